@@ -36,6 +36,7 @@ NVFLAGS += os.environ.get("COMDGB_NVCC_EXTRA", "").split()
 UNITS = [
     ("md_kernels.cu", ["-fmad=false"]),
     ("force_fp64.cu", ["-fmad=false"]),
+    ("poly64.cu", ["-fmad=false"]),
     ("force_mixed.cu", []),
     ("api.cu", []),
     ("noalloc.cu", ["-fmad=false"]),

@@ -41,13 +41,10 @@ constexpr int ADJ_THREADS = 64;  // CTA of the basis-sum kernels
 constexpr int NQ = 6;            // sums per coefficient index: see adj_basis_kernel
 
 // the FP64 series of the simulation and their second derivatives
-struct ChebSet {
-  double c[9][NC];  // 0 phi 1 rho 2 F 3 dphi 4 drho 5 dF 6 d2phi 7 d2rho 8 d2F
-  double a[9], b[9];
-};
+typedef PolySeries ChebSet;
 
 // eamCheb (cheby.c:276-310), the reference's operation order
-__device__ __forceinline__ double cheb_val(const ChebSet &S, int q, double x) {
+__device__ double cheb_val(const ChebSet &S, int q, double x) {
   const double a = S.a[q], b = S.b[q];
   if (x < a) x = a;
   const double y = (2.0 * x - a - b) / (b - a), y2 = 2.0 * y;
@@ -66,6 +63,51 @@ __device__ __forceinline__ double cheb_val(const ChebSet &S, int q, double x) {
 // position derivatives below a are 0.)
 __device__ __forceinline__ double cheb_der(const ChebSet &S, int qd, int q, double x) {
   return x < S.a[q] ? 0.0 : cheb_val(S, qd, x);
+}
+
+// Pair functions of one distance from the polynomial table, or from the
+// series outside it (rare: kept out of line).
+__device__ __noinline__ double grho_series(const ChebSet &S, double r2) {
+  const double r = sqrt(r2);
+  return cheb_val(S, 4, r) / r;
+}
+// rho'(r) / r
+__device__ __forceinline__ double pair_grho(const ChebSet &S, const PolyTables &P, double r2) {
+  int k;
+  double t;
+  return poly_at(P.pair, r2, k, t) ? poly_col(P.pair, PF_GRHO, k, t) : grho_series(S, r2);
+}
+// the terms of the Hessian: phi'/r and rho'/r, the position derivative of
+// the density over r (dr), and (phi'' - phi'/r) / r^2, (rho'' - rho'/r) / r^2
+struct HessTerms {
+  double gphi, grho, dr, hphi, hrho;
+};
+__device__ __noinline__ HessTerms hess_series(const ChebSet &S, double r2) {
+  const double r = sqrt(r2), ir = 1.0 / r, ir2 = ir * ir;
+  HessTerms h;
+  h.gphi = cheb_val(S, 3, r) * ir;
+  h.grho = cheb_val(S, 4, r) * ir;
+  h.dr = cheb_der(S, 4, 1, r) * ir;
+  h.hphi = (cheb_der(S, 6, 0, r) - h.gphi) * ir2;
+  h.hrho = (cheb_der(S, 7, 1, r) - h.grho) * ir2;
+  return h;
+}
+__device__ __forceinline__ HessTerms hess_terms(const ChebSet &S, const PolyTables &P, double r2) {
+  int k, kh;
+  double t, th;
+  if (!poly_at(P.pair, r2, k, t) || !poly_at(P.hess, r2, kh, th)) return hess_series(S, r2);
+  HessTerms h;
+  h.gphi = poly_col(P.pair, PF_GPHI, k, t);
+  h.grho = h.dr = poly_col(P.pair, PF_GRHO, k, t);
+  h.hphi = poly_col(P.hess, HF_PHI, kh, th);
+  h.hrho = poly_col(P.hess, HF_RHO, kh, th);
+  return h;
+}
+// F''(rho)
+__device__ __forceinline__ double embed_d2(const ChebSet &S, const PolyTables &P, double rho) {
+  int k;
+  double t;
+  return poly_at(P.embed, rho, k, t) ? poly_col(P.embed, EF_D2F, k, t) : cheb_der(S, 8, 2, rho);
 }
 
 struct Lam {
@@ -105,8 +147,9 @@ __global__ void adj_lambda_kernel(Slots s, const int *atom_slot, int ntot, const
 
 // W_i = sum_j v_ij rho'(r_ij) over the embedding-force pairs (r2 < rc2,
 // eam.c:612) and X_i = F''(rho_i) W_i, per slot
-__global__ void adj_w_kernel(ForceArgs A, const __grid_constant__ ChebSet S, double rc2,
-                             const d4 *lam, double *wout, double *xout) {
+__global__ void adj_w_kernel(ForceArgs A, const __grid_constant__ ChebSet S,
+                             PolyTables poly, double rc2, const d4 *lam, double *wout,
+                             double *xout) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= A.ntot) return;
   const int slot = A.atom_slot[a];
@@ -118,14 +161,13 @@ __global__ void adj_w_kernel(ForceArgs A, const __grid_constant__ ChebSet S, dou
   for_each_neighbor<double, true>(A, a, b, i, xi, yi, zi, rc2,
                                   [&](int js, double dx, double dy, double dz, double r2) {
                                     if (r2 >= rc2) return;
-                                    const double r = sqrt(r2);
                                     const d4 lj = lam[js];
-                                    const double v = ((li.x - lj.x) * dx + (li.y - lj.y) * dy +
-                                                      (li.z - lj.z) * dz) / r;
-                                    W += v * cheb_val(S, 4, r);
+                                    const double vr = (li.x - lj.x) * dx + (li.y - lj.y) * dy +
+                                                      (li.z - lj.z) * dz;
+                                    W += vr * pair_grho(S, poly, r2);
                                   });
   wout[slot] = W;
-  xout[slot] = cheb_der(S, 8, 2, A.s.rho[slot]) * W;
+  xout[slot] = embed_d2(S, poly, A.s.rho[slot]) * W;
 }
 
 // y of x on [a, b] after the clamp at a, and 2/(b - a)
@@ -288,9 +330,12 @@ __global__ void __launch_bounds__(128) adj_lj_kernel(ForceArgs A, double eps, do
 //   g  = phi'(r) + (F'_k + F'_j) rho'(r)      (embedding part for r2 < rc2)
 //   g' = phi''(r) + (F'_k + F'_j) rho''(r)
 //   += g (du - v rhat)/r + v g' rhat + (X_k + X_j) d rho/dr rhat
-// with X = F'' W (adj_w_kernel at lambda = u).  Written by atom id.
-__global__ void adj_hvp_kernel(ForceArgs A, const __grid_constant__ ChebSet S, double rc2,
-                               const d4 *u, const double *X, double *hv) {
+// with X = F'' W (adj_w_kernel at lambda = u), computed as
+//   (g/r) du + [(du . d) (g' - g/r)/r^2 + (X_k + X_j) (d rho/dr)/r] d,
+// d = r_k - r_j, whose functions of r^2 are columns of the polynomial table
+// (no square root, no division).  Written by atom id.
+__global__ void adj_hvp_kernel(ForceArgs A, const __grid_constant__ ChebSet S, PolyTables poly,
+                               double rc2, const d4 *u, const double *X, double *hv) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= A.ntot) return;
   const int slot = A.atom_slot[a];
@@ -303,19 +348,16 @@ __global__ void adj_hvp_kernel(ForceArgs A, const __grid_constant__ ChebSet S, d
   for_each_neighbor<double, true>(
       A, a, b, i, xi, yi, zi, rc2, [&](int js, double dx, double dy, double dz, double r2) {
         if (r2 > rc2) return;
-        const double r = sqrt(r2), ir = 1.0 / r;
-        const double ex = dx * ir, ey = dy * ir, ez = dz * ir;
+        const HessTerms h = hess_terms(S, poly, r2);
         const d4 uj = u[js];
         const double ux = uk.x - uj.x, uy = uk.y - uj.y, uz = uk.z - uj.z;
-        const double v = ux * ex + uy * ey + uz * ez;
-        const double fs = Fk + A.s.fi[js];
-        const bool emb = r2 < rc2;
-        const double g = cheb_val(S, 3, r) + (emb ? fs * cheb_val(S, 4, r) : 0.0);
-        const double gp = cheb_der(S, 6, 0, r) + (emb ? fs * cheb_der(S, 7, 1, r) : 0.0);
-        const double c = (Xk + X[js]) * cheb_der(S, 4, 1, r) + v * gp - g * v * ir;
-        hx += g * ux * ir + c * ex;
-        hy += g * uy * ir + c * ey;
-        hz += g * uz * ir + c * ez;
+        const double ud = ux * dx + uy * dy + uz * dz;
+        const double fs = r2 < rc2 ? Fk + A.s.fi[js] : 0.0;
+        const double g = h.gphi + fs * h.grho;
+        const double c = ud * (h.hphi + fs * h.hrho) + (Xk + X[js]) * h.dr;
+        hx += g * ux + c * dx;
+        hy += g * uy + c * dy;
+        hz += g * uz + c * dz;
       });
   const int id = A.s.id[slot];
   if ((unsigned)id >= (unsigned)A.ntot) return;
@@ -366,16 +408,6 @@ __global__ void adj_block_sum_kernel(const double *x, int n, double *partial) {
 // host side
 // ---------------------------------------------------------------------------
 namespace {
-
-// chder / genDer (cheby.c:180-270): derivative coefficients of an n-term
-// series on [a, b], the reference's recurrence and scaling
-void cheb_derive(double a, double b, const double *c, double *cd, int n) {
-  cd[n - 1] = 0.0;
-  cd[n - 2] = 2.0 * (n - 1) * c[n - 1];
-  for (int j = n - 2; j > 0; j--) cd[j - 1] = cd[j + 1] + 2 * (j)*c[j];
-  const double con = 2.0 / (b - a);
-  for (int j = 0; j < n; j++) cd[j] = cd[j] * con;
-}
 
 ChebSet cheb_set(const comdgb_sim *h) {
   ChebSet S{};
@@ -482,8 +514,8 @@ int set_lambda(comdgb_sim *h, Work &W, const ChebSet &S, const double *d_target,
   adj_lambda_kernel<<<blocks(h->ntot), 256, 0, h->stream>>>(h->s, h->atom_slot, h->ntot, d_target,
                                                            d_u, W.lam, W.loss);
   if (h->opts.potential == COMDGB_POT_EAM_CHEBY)
-    adj_w_kernel<<<blocks(h->ntot, 128), 128, 0, h->stream>>>(force_args(h), S, h->eam64c.rc2,
-                                                              W.lam, W.w, W.x);
+    adj_w_kernel<<<blocks(h->ntot, 128), 128, 0, h->stream>>>(force_args(h), S, h->eam64c.poly,
+                                                              h->eam64c.rc2, W.lam, W.w, W.x);
   CK(cudaGetLastError());
   return 0;
 }
@@ -662,7 +694,8 @@ int comdgb_sim_traj_energy_grad(comdgb_sim *h, int n, double dt, int every, doub
       adj_scale_kernel<<<blocks(nv), 256, 0, h->stream>>>(-dt_atu, pb, u, nv);
       if ((rc = set_lambda(h, W, S, nullptr, u))) return rc;
       adj_hvp_kernel<<<blocks(h->ntot, 128), 128, 0, h->stream>>>(force_args(h), S,
-                                                                 h->eam64c.rc2, W.lam, W.x, hv);
+                                                                 h->eam64c.poly, h->eam64c.rc2,
+                                                                 W.lam, W.x, hv);
       if ((rc = eam_rows(h, W, S, true, rows))) return rc;
       for (int q = 0; q < 3; q++)
         for (int k = 0; k < NC; k++) cbar[q * NC + k] += rows[(2 * q + 1) * NC + k];

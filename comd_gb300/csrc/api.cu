@@ -181,6 +181,16 @@ double cheb_host(const double *c, double a, double b, double x) {
   return y * d - dd + 0.5 * c[0];
 }
 
+// chder / genDer (cheby.c:180-270): derivative coefficients of an n-term
+// series on [a, b], the reference's recurrence and scaling
+void cheb_derive(double a, double b, const double *c, double *cd, int n) {
+  cd[n - 1] = 0.0;
+  cd[n - 2] = 2.0 * (n - 1) * c[n - 1];
+  for (int j = n - 2; j > 0; j--) cd[j - 1] = cd[j + 1] + 2 * (j)*c[j];
+  const double con = 2.0 / (b - a);
+  for (int j = 0; j < n; j++) cd[j] = cd[j] * con;
+}
+
 // The degree-31 polynomial of series c on [a, b] written in the Chebyshev
 // basis of [lo, b]: sampled at the 32 Chebyshev nodes of [lo, b] (exact for
 // a degree-31 polynomial) and transformed back.  Identical function to
@@ -422,6 +432,53 @@ int build_pair_seg(comdgb_sim *h, const double coef[6][CG_NCHEB], const double a
   return 0;
 }
 
+// The polynomial tables of an FP64 simulation (poly64.cuh) from the installed
+// series.  Returns 0, or -1 when a CUDA call failed.
+int build_poly64(comdgb_sim *h, const double coef[6][CG_NCHEB], const double a[6],
+                 const double b[6], double pair_lo, double rc, PolyTables *out) {
+  *out = PolyTables{};
+  PolySeries S;
+  for (int q = 0; q < 9; q++) {
+    const int from = q < 6 ? q : q - 3;
+    if (q < 6) memcpy(S.c[q], coef[q], sizeof S.c[q]);
+    else cheb_derive(a[from], b[from], coef[from], S.c[q], CG_NCHEB);
+    S.a[q] = a[from];
+    S.b[q] = b[from];
+  }
+  double lo = pair_lo;
+  for (int s : {0, 1, 3, 4}) lo = std::max(lo, a[s]);
+  int base[PT_COUNT], n[PT_COUNT], bad[PT_COUNT], err = 0;
+  poly_range(PT_PAIR, lo, rc, &base[PT_PAIR], &n[PT_PAIR]);
+  poly_range(PT_HESS, lo, rc, &base[PT_HESS], &n[PT_HESS]);
+  poly_range(PT_EMBED, std::max(a[2], a[5]), std::min(b[2], b[5]), &base[PT_EMBED], &n[PT_EMBED]);
+  if (!h->poly_series) {
+    h->poly_series = track(h, dalloc<PolySeries>(1, &err));
+    h->poly_bad = track(h, dalloc<int>(PT_COUNT, &err));
+    if (err) return -1;
+  }
+  cudaStream_t st = h->stream;
+  bool ok =
+      cudaMemcpyAsync(h->poly_series, &S, sizeof S, cudaMemcpyHostToDevice, st) == cudaSuccess &&
+      cudaMemcpyAsync(h->poly_bad, n, sizeof n, cudaMemcpyHostToDevice, st) == cudaSuccess;
+  for (int e = 0; e < PT_COUNT; e++) {
+    const size_t need = poly_size(e, n[e]);
+    if (need > h->poly_cap[e]) {
+      h->poly_buf[e] = track(h, dalloc<double2>(need, &err));
+      if (err) return -1;
+      h->poly_cap[e] = need;
+    }
+    launch_poly_fit(e, h->poly_series, base[e], n[e], h->poly_buf[e], h->poly_bad + e, st);
+  }
+  ok = ok &&
+       cudaMemcpyAsync(bad, h->poly_bad, sizeof bad, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
+       cudaStreamSynchronize(st) == cudaSuccess;
+  if (!ok) return -1;
+  out->pair = Poly64<PT_PAIR>{h->poly_buf[PT_PAIR], base[PT_PAIR], bad[PT_PAIR]};
+  out->hess = Poly64<PT_HESS>{h->poly_buf[PT_HESS], base[PT_HESS], bad[PT_HESS]};
+  out->embed = Poly64<PT_EMBED>{h->poly_buf[PT_EMBED], base[PT_EMBED], bad[PT_EMBED]};
+  return 0;
+}
+
 int fit_cheb_gpu(comdgb_sim *h, const eampotential_t *pot, double coef[6][CG_NCHEB],
                  double a[6], double b[6]) {
   int err = 0;
@@ -545,8 +602,11 @@ void cgapi::install_lj(comdgb_sim *h, double eps, double sigma, double cutoff) {
 int cgapi::install_cheby(comdgb_sim *h, const double coef[6][CG_NCHEB], const double a[6],
                          const double b[6]) {
   fill_cheb(h->eam64c.ch, h->eam32c.ch, h->eam32c.chlo, coef, a, b, h->pair_lo);
-  if (build_pair_seg(h, coef, a, b, h->pair_lo, h->cutoff, &h->seg_built))
-    return set_err(COMDGB_ERR_NOMEM, "cudaMalloc failed for the pair segment table");
+  // each precision has its own tables of the pair functions
+  h->seg_built = no_pair_seg();
+  if (h->mixed ? build_pair_seg(h, coef, a, b, h->pair_lo, h->cutoff, &h->seg_built)
+               : build_poly64(h, coef, a, b, h->pair_lo, h->cutoff, &h->eam64c.poly))
+    return set_err(COMDGB_ERR_NOMEM, "cudaMalloc failed for the pair function tables");
   h->eam32c.seg = h->pair_table_off ? no_pair_seg() : h->seg_built;
   for (int q = 0; q < 6; q++) {
     for (int j = 0; j < CG_NCHEB; j++) h->cheb_coef[q][j] = coef[q][j];

@@ -21,6 +21,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "poly64.cuh"
 
 namespace cg {
 
@@ -119,9 +120,10 @@ struct PrecT<float> {
 };
 
 // FP64: dr = drbox + r_i - r_j and r2 accumulated in the reference's order
-__device__ __forceinline__ double pair_r2(const BoxOff<double> &o, double xi, double yi,
-                                          double zi, double xj, double yj, double zj, double &dx,
-                                          double &dy, double &dz) {
+// (the list build: which pairs are within the cutoff)
+__device__ __forceinline__ double pair_r2_ref(const BoxOff<double> &o, double xi, double yi,
+                                              double zi, double xj, double yj, double zj,
+                                              double &dx, double &dy, double &dz) {
   dx = (o.x + xi) - xj;
   dy = (o.y + yi) - yj;
   dz = (o.z + zi) - zj;
@@ -129,6 +131,16 @@ __device__ __forceinline__ double pair_r2(const BoxOff<double> &o, double xi, do
   r2 = r2 + dy * dy;
   r2 = r2 + dz * dz;
   return r2;
+}
+// the same with fused sums (the passes: two FP64 operations and two roundings
+// fewer per pair)
+__device__ __forceinline__ double pair_r2(const BoxOff<double> &o, double xi, double yi,
+                                          double zi, double xj, double yj, double zj, double &dx,
+                                          double &dy, double &dz) {
+  dx = (o.x + xi) - xj;
+  dy = (o.y + yi) - yj;
+  dz = (o.z + zi) - zj;
+  return fma(dz, dz, fma(dy, dy, dx * dx));
 }
 
 // FP32: coordinates are relative to the box centre (|x| <= boxsize/2) and
@@ -597,7 +609,7 @@ static __global__ void __launch_bounds__(NB_THREADS) nbr_build64_kernel(ForceArg
         code = cc[c];
         int e = code >> 6, k = code & 63;
         double dx, dy, dz;
-        double r2 = pair_r2(s_dr[e], xi, yi, zi, cx[c], cy[c], cz[c], dx, dy, dz);
+        double r2 = pair_r2_ref(s_dr[e], xi, yi, zi, cx[c], cy[c], cz[c], dx, dy, dz);
         hit = (r2 <= rc2) && !(s_box[e] == b && k == i);
       }
       const unsigned m = __ballot_sync(0xffffffffu, hit);
@@ -621,6 +633,7 @@ struct EamPot {
   Cheb<T> ch;
   ChebLow32 chlo;  // FP32 only
   PairSeg seg;     // FP32 Chebyshev only
+  PolyTables poly; // FP64 Chebyshev only
   T rc2;
 };
 
@@ -694,6 +707,13 @@ __device__ __forceinline__ void eam_pair_terms(const EamPot<T, EVAL> &P, T r, T 
 template <class T, int EVAL>
 __device__ __forceinline__ void eam_embed(const EamPot<T, EVAL> &P, T rho, T &F, T &dF) {
   if (EVAL == EVAL_CHEBY) {
+    int k;
+    double t;
+    if (sizeof(T) == 8 && poly_at(P.poly.embed, (double)rho, k, t)) {
+      F = (T)poly_col(P.poly.embed, EF_F, k, t);
+      dF = (T)poly_col(P.poly.embed, EF_DF, k, t);
+      return;
+    }
     F = cheb_series(P, 2, rho);
     dF = cheb_series(P, 5, rho);
   } else {
@@ -736,7 +756,19 @@ static __device__ __forceinline__ bool eam_pair_w(const EamPot<float, EVAL_CHEBY
   rho = seg_cubic(cr, t);
   return true;
 }
-// the series for a pair below the table (FP32 Chebyshev only)
+// FP64 Chebyshev: the polynomials of poly64.cuh
+static __device__ __forceinline__ bool eam_pair_w(const EamPot<double, EVAL_CHEBY> &P,
+                                                  const float4 *, double r2, double &phi,
+                                                  double &w, double &rho) {
+  int k;
+  double t;
+  if (!poly_at(P.poly.pair, r2, k, t)) return false;
+  phi = poly_col(P.poly.pair, PF_PHI, k, t);
+  w = poly_col(P.poly.pair, PF_GPHI, k, t);
+  rho = poly_col(P.poly.pair, PF_RHO, k, t);
+  return true;
+}
+// the series for a pair below the table (Chebyshev only)
 template <class T, int EVAL>
 __device__ __forceinline__ void pair_w_series(const EamPot<T, EVAL> &, T, T &, T &, T &) {}
 static __device__ __noinline__ void pair_w_series(const EamPot<float, EVAL_CHEBY> &P, float r2,
@@ -746,9 +778,21 @@ static __device__ __noinline__ void pair_w_series(const EamPot<float, EVAL_CHEBY
   cheb_pair32(P, r, phi, dphi, rho);
   w = dphi * inv_r;
 }
+static __device__ __noinline__ void pair_w_series(const EamPot<double, EVAL_CHEBY> &P, double r2,
+                                                  double &phi, double &w, double &rho) {
+  double r, inv_r, dphi;
+  r_and_inv(r2, r, inv_r);
+  eam_pair_terms<double, EVAL_CHEBY>(P, r, phi, dphi, rho);
+  w = dphi * inv_r;
+}
 template <class T, int EVAL>
 __device__ __forceinline__ bool below_seg(const EamPot<T, EVAL> &, T) {
   return false;
+}
+static __device__ __forceinline__ bool below_seg(const EamPot<double, EVAL_CHEBY> &P, double r2) {
+  int k;
+  double t;
+  return !poly_at(P.poly.pair, r2, k, t);
 }
 static __device__ __forceinline__ bool below_seg(const EamPot<float, EVAL_CHEBY> &P, float r2) {
   return !((r2 - P.seg.s_lo) * P.seg.inv_h >= 0.f);
@@ -774,6 +818,15 @@ static __device__ __forceinline__ bool eam_embed_w(const EamPot<float, EVAL_CHEB
   wr = fsum * (P.seg.dscale * seg_dcubic(sm[k], u - (float)k));
   return true;
 }
+static __device__ __forceinline__ bool eam_embed_w(const EamPot<double, EVAL_CHEBY> &P,
+                                                   const float4 *, double r2, double fsum,
+                                                   double &wr) {
+  int k;
+  double t;
+  if (!poly_at(P.poly.pair, r2, k, t)) return false;
+  wr = fsum * poly_col(P.poly.pair, PF_GRHO, k, t);
+  return true;
+}
 template <class T, int EVAL>
 __device__ __forceinline__ T embed_w_series(const EamPot<T, EVAL> &, T, T) {
   return T(0);
@@ -781,6 +834,13 @@ __device__ __forceinline__ T embed_w_series(const EamPot<T, EVAL> &, T, T) {
 static __device__ __noinline__ float embed_w_series(const EamPot<float, EVAL_CHEBY> &P, float r2,
                                                     float fsum) {
   float r, inv_r;
+  r_and_inv(r2, r, inv_r);
+  return fsum * (cheb_series(P, 4, r) * inv_r);
+}
+
+static __device__ __noinline__ double embed_w_series(const EamPot<double, EVAL_CHEBY> &P,
+                                                     double r2, double fsum) {
+  double r, inv_r;
   r_and_inv(r2, r, inv_r);
   return fsum * (cheb_series(P, 4, r) * inv_r);
 }

@@ -1,0 +1,110 @@
+// poly64.cuh -- the FP64 Chebyshev potential as piecewise polynomials.
+//
+// A 32-term Clenshaw sum costs 93 FP64 operations (and its argument a square
+// root and a division), and the FP64 pipe issues about two lanes per SM per
+// clock, so summing the series for every pair bounds the FP64 kernels.  The
+// pair functions are instead degree-5 polynomials in s = r^2 (no square
+// root) on segments that are the 256 equal parts of each binade of s: the
+// segment index is the top bits of s, its centre the index with the next bit
+// set, so an evaluation takes one FP64 subtraction and five fused
+// multiply-adds.  The embedding function has the same form in rho.  At
+// 256,000 atoms the first FP64 pass took 8,342 us with the series and takes
+// 750 us, the second 3,267 and 577 us.
+//
+// Accuracy: the coefficients interpolate the series at six Chebyshev nodes
+// of each segment, with the series summed in double-double arithmetic, and
+// are rounded once.  The fit compares every polynomial with its series and
+// the table ends before the first segment that is further off than half an
+// FP64 ulp of the sum of the series' coefficients' magnitudes, less than a
+// Clenshaw sum in FP64 loses by rounding; arguments outside the table take
+// the series.  EAM Cu over 2.1 to 4.96 A, rms error against the series in
+// extended precision, Clenshaw in FP64 -> polynomial: phi 4.7e-17 -> 9.5e-19,
+// phi'/r 6.6e-17 -> 5.0e-18, rho 3.4e-18 -> 3.5e-19, rho'/r 2.0e-18 ->
+// 2.5e-19 (Ha, A).  The Hessian's columns vary faster near the cutoff and
+// have twice the segments; the embedding function's table reaches densities
+// of 0.46 there, four times the lattice's.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace cg {
+
+constexpr int POLY_REC = 3;  // double2 per polynomial: degree 5
+
+// The tables: pair functions (rho, phi, phi'/r, rho'/r), the Hessian's (the
+// s-derivatives of phi'/r and rho'/r, doubled: (phi'' - phi'/r) / s and
+// (rho'' - rho'/r) / s), and F, F' and F'' of rho; 2^bits segments a binade.
+enum { PT_PAIR = 0, PT_HESS, PT_EMBED, PT_COUNT };
+enum { PF_RHO = 0, PF_PHI, PF_GPHI, PF_GRHO, PF_COUNT };
+enum { HF_PHI = 0, HF_RHO, HF_COUNT };
+enum { EF_F = 0, EF_DF, EF_D2F, EF_COUNT };
+template <int TABLE>
+struct PolyShape;
+template <>
+struct PolyShape<PT_PAIR> {
+  static constexpr int bits = 8, cols = PF_COUNT;
+};
+template <>
+struct PolyShape<PT_HESS> {
+  static constexpr int bits = 9, cols = HF_COUNT;
+};
+template <>
+struct PolyShape<PT_EMBED> {
+  static constexpr int bits = 8, cols = EF_COUNT;
+};
+
+// segment k of the table: arguments whose top bits are base + k; column q of
+// it at c + (k * cols + q) * POLY_REC.  n = 0: no table.
+template <int TABLE>
+struct Poly64 {
+  const double2 *c;
+  int base, n;
+};
+struct PolyTables {
+  Poly64<PT_PAIR> pair;
+  Poly64<PT_HESS> hess;
+  Poly64<PT_EMBED> embed;
+};
+
+// segment k and offset t from its centre; false outside the table (NaN
+// included)
+template <int TABLE>
+__device__ __forceinline__ bool poly_at(const Poly64<TABLE> &p, double x, int &k, double &t) {
+  constexpr int sh = 20 - PolyShape<TABLE>::bits;
+  const int i = __double2hiint(x) >> sh;
+  t = __dsub_rn(x, __hiloint2double((i << sh) | (1 << (sh - 1)), 0));
+  k = i - p.base;
+  return (unsigned)k < (unsigned)p.n;
+}
+
+__device__ __forceinline__ double poly_eval(const double2 *c, double t) {
+  const double2 a = __ldg(c), b = __ldg(c + 1), d = __ldg(c + 2);
+  return __fma_rn(
+      __fma_rn(__fma_rn(__fma_rn(__fma_rn(d.y, t, d.x), t, b.y), t, b.x), t, a.y), t, a.x);
+}
+
+// column q at segment k
+template <int TABLE>
+__device__ __forceinline__ double poly_col(const Poly64<TABLE> &p, int q, int k, double t) {
+  return poly_eval(p.c + (size_t)(k * PolyShape<TABLE>::cols + q) * POLY_REC, t);
+}
+
+// the series a table is made from: coefficients of phi, rho, F, their first
+// and second derivatives (order 0 phi 1 rho 2 F 3 dphi 4 drho 5 dF 6 d2phi
+// 7 d2rho 8 d2F) and the intervals
+struct PolySeries {
+  double c[9][32];
+  double a[9], b[9];
+};
+
+// First segment and number of segments of a table: pair distances over (lo,
+// rc], densities over whole segments of [a, b]; double2 each takes.
+void poly_range(int table, double lo, double hi, int *base, int *n);
+size_t poly_size(int table, int n);
+
+// Fits n segments of a table into c on the device; *first_bad (device) is
+// lowered to the first segment with a polynomial that misses its series.
+void launch_poly_fit(int table, const PolySeries *series, int base, int n, double2 *c,
+                     int *first_bad, cudaStream_t st);
+
+}  // namespace cg

@@ -101,6 +101,12 @@ struct comdgb_sim {
   double cheb_a[6] = {}, cheb_b[6] = {};
   double pair_lo = 0.0;
   float4 *seg_buf = nullptr;
+  // FP64 polynomial tables (poly64.cuh): the fit's input, the tables' storage
+  // with its capacity in double2, and the first segment each misses
+  cg::PolySeries *poly_series = nullptr;
+  double2 *poly_buf[cg::PT_COUNT] = {};
+  size_t poly_cap[cg::PT_COUNT] = {};
+  int *poly_bad = nullptr;
   // the FP32 pair segment table as built (seg_built) and whether the mixed
   // Chebyshev evaluator uses it (comdgb_sim_set_pair_table)
   cg::PairSeg seg_built{};
@@ -186,6 +192,8 @@ cg::ForceArgs force_args(comdgb_sim *h);
 comdgb_sim *find_attached(const void *s);  // the handle of an attached simflat_t
 int do_force(comdgb_sim *h);       // force call (graph), energy and stress to the host
 int check_status(comdgb_sim *h);
+// genDer (cheby.c:219-270): the derivative series of an n-term series on [a, b]
+void cheb_derive(double a, double b, const double *c, double *cd, int n);
 double cheb_host(const double *c, double a, double b, double x);  // eamCheb on the host
 void drop_graphs(comdgb_sim *h);  // after a change of potential parameters
 void install_lj(comdgb_sim *h, double eps, double sigma, double cutoff);
