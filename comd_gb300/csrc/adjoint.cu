@@ -37,8 +37,8 @@ using namespace cgapi;
 namespace {
 
 constexpr int NC = CG_NCHEB;
-constexpr int ADJ_THREADS = 64;  // CTA of the basis-sum kernels
-constexpr int NQ = 6;            // sums per coefficient index: see adj_basis_kernel
+constexpr int BASIS_THREADS = 128;  // CTA of the basis-sum kernels
+constexpr int NQ = 4;               // sums per coefficient index at most: three over pairs, one over atoms
 
 // the FP64 series of the simulation and their second derivatives
 typedef PolySeries ChebSet;
@@ -170,115 +170,168 @@ __global__ void adj_w_kernel(ForceArgs A, const __grid_constant__ ChebSet S,
   xout[slot] = embed_d2(S, poly, A.s.rho[slot]) * W;
 }
 
-// y of x on [a, b] after the clamp at a, and 2/(b - a)
-__device__ __forceinline__ void cheb_y(const ChebSet &S, int q, double x, double &y, double &sc) {
+// y of x on [a, b] after the clamp at a
+__device__ __forceinline__ double cheb_y(const ChebSet &S, int q, double x) {
   const double a = S.a[q], b = S.b[q];
   if (x < a) x = a;
-  y = (2.0 * x - a - b) / (b - a);
-  sc = 2.0 / (b - a);
+  return (2.0 * x - a - b) / (b - a);
 }
 
-// Per-CTA basis sums, row q*NC + k of acc (one column per thread):
-//   0 dU/dc^phi   1 dD/dc^phi   2 dU/dc^rho   3 dD/dc^rho   4 dU/dc^F   5 dD/dc^F
-// lam / x may be null (energy only).  Writes the CTA's NQ*NC row sums.
-__global__ void __launch_bounds__(ADJ_THREADS)
-    adj_basis_kernel(ForceArgs A, const __grid_constant__ ChebSet S, double rc2, Lam L,
-                     const double *wsl, double *partial) {
-  extern __shared__ double acc[];  // [NQ*NC][ADJ_THREADS]
-  const int tid = threadIdx.x;
-  for (int r = 0; r < NQ * NC; r++) acc[r * ADJ_THREADS + tid] = 0.0;
-  const bool same = S.a[0] == S.a[1] && S.b[0] == S.b[1];
-  for (int a = blockIdx.x * blockDim.x + tid; a < A.ntot; a += gridDim.x * blockDim.x) {
-    const int slot = A.atom_slot[a];
-    const int b = slot >> 6, i = slot & 63;
-    double xi, yi, zi;
-    PrecT<double>::pos(A.s, slot, xi, yi, zi);
-    const double fpi = A.s.fi[slot];
-    const double Xi = L.x ? L.x[slot] : 0.0, Wi = wsl ? wsl[slot] : 0.0;
-    d4 li;
-    li.x = li.y = li.z = 0.0;
-    if (L.lam) li = L.lam[slot];
-    {  // F(rho_i) terms
-      double y, sc;
-      cheb_y(S, 2, A.s.rho[slot], y, sc);
-      double t0 = 1.0, t1 = y, u0 = 1.0, u1 = 2.0 * y;
-      acc[(4 * NC + 0) * ADJ_THREADS + tid] += 0.5;
-      for (int k = 1; k < NC; k++) {
-        // t1 = T_k, u0 = U_{k-1}
-        acc[(4 * NC + k) * ADJ_THREADS + tid] += t1;
-        acc[(5 * NC + k) * ADJ_THREADS + tid] += Wi * sc * (double)k * u0;
-        const double t2 = 2.0 * y * t1 - t0, u2 = 2.0 * y * u1 - u0;
-        t0 = t1;
-        t1 = t2;
-        u0 = u1;
-        u1 = u2;
-      }
+// Sums over the pairs of w T_k(y), k < 32, for the weights of the gradients:
+// without lambda w = 1 (phi) and F'_i + F'_j (rho); with it v (phi) and
+// (F'_i + F'_j) v and X_i + X_j (rho).  The sums of the derivative basis
+// B'_k = T'_k 2/(b - a) follow on the host, T'_k = k U_{k-1} being twice the
+// sum of the T_j of the other parity below k (basis_derivative).
+//
+// Bound by FP64 operations: one for the recurrence and one per weight and k,
+// 124 a pair with lambda.  A thread keeps all its sums in registers (96
+// doubles; a column of shared memory per thread, read and written for every
+// k, took 10.45 ms at 256,000 atoms, this 2.16 ms) and LANES threads share
+// an atom's list.  Each pair is taken at one of its atoms, the lower slot if
+// the slots' sum is even and the higher if it is odd, so every thread finds
+// about half of its entries; it skips the others before the sums, or half of
+// the lanes would stand idle in them.
+template <int NW>
+struct BasisAcc {
+  double s[NW][NC];
+};
+template <int NW, bool SAME>
+__device__ __forceinline__ void basis_add(BasisAcc<NW> &A, double yp, double yr, const double *w) {
+  double t0 = 1.0, t1 = yp, r0 = 1.0, r1 = yr;
+  const double yp2 = 2.0 * yp, yr2 = 2.0 * yr;
+#pragma unroll
+  for (int k = 0; k < NC; k++) {
+    A.s[0][k] = fma(w[0], t0, A.s[0][k]);
+#pragma unroll
+    for (int q = 1; q < NW; q++) A.s[q][k] = fma(w[q], SAME ? t0 : r0, A.s[q][k]);
+    const double t2 = fma(yp2, t1, -t0);
+    t0 = t1;
+    t1 = t2;
+    if (!SAME) {
+      const double r2 = fma(yr2, r1, -r0);
+      r0 = r1;
+      r1 = r2;
     }
-    for_each_neighbor<double, true>(
-        A, a, b, i, xi, yi, zi, rc2, [&](int js, double dx, double dy, double dz, double r2) {
-          if (js <= slot || r2 > rc2) return;
-          const double r = sqrt(r2);
-          double v = 0.0;
-          if (L.lam) {
-            const d4 lj = L.lam[js];
-            v = ((li.x - lj.x) * dx + (li.y - lj.y) * dy + (li.z - lj.z) * dz) / r;
-          }
-          const double fsum = fpi + A.s.fi[js];
-          const double ap = v;                                 // x B'_k / sc
-          const double ar = r2 < rc2 ? fsum * v : 0.0;         // x B'_k / sc
-          const double br = L.x ? Xi + L.x[js] : 0.0;          // x B_k
-          double yp, sp, yr, sr;
-          cheb_y(S, 0, r, yp, sp);
-          cheb_y(S, 1, r, yr, sr);
-          // phi series
-          {
-            double t0 = 1.0, t1 = yp, u0 = 1.0, u1 = 2.0 * yp;
-            acc[(0 * NC + 0) * ADJ_THREADS + tid] += 0.5;
-            for (int k = 1; k < NC; k++) {
-              acc[(0 * NC + k) * ADJ_THREADS + tid] += t1;
-              acc[(1 * NC + k) * ADJ_THREADS + tid] += ap * sp * (double)k * u0;
-              if (same) {
-                acc[(2 * NC + k) * ADJ_THREADS + tid] += fsum * t1;
-                acc[(3 * NC + k) * ADJ_THREADS + tid] += ar * sr * (double)k * u0 + br * t1;
-              }
-              const double t2 = 2.0 * yp * t1 - t0, u2 = 2.0 * yp * u1 - u0;
-              t0 = t1;
-              t1 = t2;
-              u0 = u1;
-              u1 = u2;
-            }
-          }
-          acc[(2 * NC + 0) * ADJ_THREADS + tid] += 0.5 * fsum;
-          acc[(3 * NC + 0) * ADJ_THREADS + tid] += 0.5 * br;
-          if (!same) {
-            double t0 = 1.0, t1 = yr, u0 = 1.0, u1 = 2.0 * yr;
-            for (int k = 1; k < NC; k++) {
-              acc[(2 * NC + k) * ADJ_THREADS + tid] += fsum * t1;
-              acc[(3 * NC + k) * ADJ_THREADS + tid] += ar * sr * (double)k * u0 + br * t1;
-              const double t2 = 2.0 * yr * t1 - t0, u2 = 2.0 * yr * u1 - u0;
-              t0 = t1;
-              t1 = t2;
-              u0 = u1;
-              u1 = u2;
-            }
-          }
-        });
+  }
+}
+
+// the CTA's sums of NROW per-thread values, to out[0..NROW): warp trees,
+// then the warps in order
+template <int NROW, int NT>
+__device__ __forceinline__ void block_rows(const double *v, double *sh, double *out) {
+#pragma unroll
+  for (int r = 0; r < NROW; r++) {
+    double t = v[r];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if ((threadIdx.x & 31) == 0) sh[(threadIdx.x >> 5) * NROW + r] = t;
   }
   __syncthreads();
-  for (int r = tid; r < NQ * NC; r += ADJ_THREADS) {
+  for (int r = threadIdx.x; r < NROW; r += NT) {
     double t = 0.0;
-    for (int c = 0; c < ADJ_THREADS; c++) t += acc[r * ADJ_THREADS + c];
-    partial[(size_t)blockIdx.x * NQ * NC + r] = t;
+    for (int w = 0; w < NT / 32; w++) t += sh[w * NROW + r];
+    out[r] = t;
   }
 }
 
-// out[r] = sum over n partial rows (fixed order)
-__global__ void adj_sum_kernel(const double *partial, int n, int width, double *out) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= width) return;
+template <int NW, bool SAME, int LANES>
+__global__ void __launch_bounds__(BASIS_THREADS)
+    adj_basis_kernel(ForceArgs A, const __grid_constant__ ChebSet S, double rc2, Lam L,
+                     double *partial) {
+  __shared__ double sh[BASIS_THREADS / 32 * NW * NC];
+  BasisAcc<NW> acc;
+#pragma unroll
+  for (int q = 0; q < NW; q++)
+#pragma unroll
+    for (int k = 0; k < NC; k++) acc.s[q][k] = 0.0;
+  const int sub = threadIdx.x % LANES;
+  for (int a = (blockIdx.x * BASIS_THREADS + threadIdx.x) / LANES; a < A.ntot;
+       a += gridDim.x * BASIS_THREADS / LANES) {
+    const int slot = A.atom_slot[a];
+    const int b = slot >> 6, ebase = b * CG_NNBR, n = A.nbr_n[a];
+    const d4 ri = A.s.r[slot];
+    const double fpi = A.s.fi[slot];
+    d4 li;
+    double Xi = 0.0;
+    if (NW == 3) {
+      li = L.lam[slot];
+      Xi = L.x[slot];
+    }
+    auto mine = [&](int js) { return ((js > slot) ^ ((js + slot) & 1)) != 0; };
+    auto pair = [&](int js, double dx, double dy, double dz, double r2) {
+      if (r2 > rc2) return;
+      const double r = sqrt(r2), fsum = fpi + A.s.fi[js];
+      double w[3];
+      if (NW == 3) {
+        const d4 lj = L.lam[js];
+        w[0] = ((li.x - lj.x) * dx + (li.y - lj.y) * dy + (li.z - lj.z) * dz) / r;
+        w[1] = r2 < rc2 ? fsum * w[0] : 0.0;
+        w[2] = Xi + L.x[js];
+      } else {
+        w[0] = 1.0;
+        w[1] = fsum;
+      }
+      const double yp = cheb_y(S, 0, r);
+      basis_add<NW, SAME>(acc, yp, SAME ? yp : cheb_y(S, 1, r), w);
+    };
+    const bool over = n > A.cap;
+    if (over && sub == 0)  // overflowed list: the stencil, by one lane
+      scan_stencil<double>(A, b, slot & 63, ri.x, ri.y, ri.z, rc2,
+                           [&](int js, double dx, double dy, double dz, double r2) {
+                             if (mine(js)) pair(js, dx, dy, dz, r2);
+                           });
+    const uint16_t *lst = A.nbr + (size_t)a * A.cap;
+    int t = over ? n : sub;
+    while (true) {
+      int js = 0, e = 0;
+      bool got = false;
+      for (; t < n && !got; t += LANES) {
+        const uint32_t code = lst[t];
+        e = code >> 6;
+        js = __ldg(A.et.box + ebase + e) * CG_MAXATOMS + (code & 63);
+        got = mine(js);
+      }
+      if (!got) break;
+      const d4 rj = A.s.r[js];
+      double dx, dy, dz;
+      const double r2 = pair_r2(PrecT<double>::drbox(A.et, ebase + e), ri.x, ri.y, ri.z, rj.x,
+                                rj.y, rj.z, dx, dy, dz);
+      pair(js, dx, dy, dz, r2);
+    }
+  }
+  block_rows<NW * NC, BASIS_THREADS>(&acc.s[0][0], sh, partial + (size_t)blockIdx.x * NW * NC);
+}
+
+// sums over the atoms of w T_k(y(rho_i)) for the F series: w = 1, or W_i
+__global__ void __launch_bounds__(BASIS_THREADS)
+    adj_embed_basis_kernel(ForceArgs A, const __grid_constant__ ChebSet S, const double *wsl,
+                           double *partial) {
+  __shared__ double sh[BASIS_THREADS / 32 * NC];
+  BasisAcc<1> acc;
+#pragma unroll
+  for (int k = 0; k < NC; k++) acc.s[0][k] = 0.0;
+  for (int a = blockIdx.x * BASIS_THREADS + threadIdx.x; a < A.ntot;
+       a += gridDim.x * BASIS_THREADS) {
+    const int slot = A.atom_slot[a];
+    const double y = cheb_y(S, 2, A.s.rho[slot]), w = wsl ? wsl[slot] : 1.0;
+    basis_add<1, true>(acc, y, y, &w);
+  }
+  block_rows<NC, BASIS_THREADS>(&acc.s[0][0], sh, partial + (size_t)blockIdx.x * NC);
+}
+
+// out[r] = sum over n partial rows, one CTA per r: thread t takes rows t, t +
+// 256, ..., then a tree (a fixed order; one thread over 1,000 rows took 65 us)
+__global__ void __launch_bounds__(256)
+    adj_sum_kernel(const double *partial, int n, int width, double *out) {
+  __shared__ double sh[256];
   double t = 0.0;
-  for (int q = 0; q < n; q++) t += partial[(size_t)q * width + r];
-  out[r] = t;
+  for (int q = threadIdx.x; q < n; q += 256) t += partial[(size_t)q * width + blockIdx.x];
+  sh[threadIdx.x] = t;
+  __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) out[blockIdx.x] = sh[0];
 }
 
 // LJ (ljForce.c:151-215, U = 4 eps sum_{i<j} (s^12 - s^6), s = sigma/r, no
@@ -436,7 +489,7 @@ int work(comdgb_sim *h, Work *&Wp) {
   int dev = 0, nsm = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  W.nblk = std::max(1, std::min(2 * nsm, (h->ntot + ADJ_THREADS - 1) / ADJ_THREADS));
+  W.nblk = 2 * nsm;  // resident CTAs of the basis sums
   W.lam = track(h, dalloc<d4>(ns, &err));
   W.w = track(h, dalloc<double>(ns, &err));
   W.x = track(h, dalloc<double>(ns, &err));
@@ -452,8 +505,6 @@ int work(comdgb_sim *h, Work *&Wp) {
     W.lam = nullptr;
     return set_err(COMDGB_ERR_NOMEM, "cudaMalloc failed for adjoint scratch");
   }
-  CK(cudaFuncSetAttribute(adj_basis_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          (int)(sizeof(double) * NQ * NC * ADJ_THREADS)));
   return 0;
 }
 
@@ -487,24 +538,78 @@ unsigned blocks(long n, int t = 256) { return (unsigned)((n + t - 1) / t); }
 int loss_sum(comdgb_sim *h, Work &W, double *loss) {
   const int nb = std::min(1024, (int)blocks(h->ntot));
   adj_block_sum_kernel<<<nb, 256, 0, h->stream>>>(W.loss, h->ntot, W.partial);
-  adj_sum_kernel<<<1, 32, 0, h->stream>>>(W.partial, nb, 1, W.out);
+  adj_sum_kernel<<<1, 256, 0, h->stream>>>(W.partial, nb, 1, W.out);
   CK(cudaMemcpyAsync(loss, W.out, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   return 0;
 }
 
-// EAM Chebyshev basis sums at the current forces and per-step list: rows
-// 0..5 (see adj_basis_kernel) into out[6*NC] on the host.  lam/x/w null:
-// energy rows only.
-int eam_rows(comdgb_sim *h, Work &W, const ChebSet &S, bool with_lam, double *rows) {
-  ForceArgs A = force_args(h);
+// sums of w T'_k(y) from those of w T_k: T'_k = k U_{k-1}, and U_{k-1} = 2
+// (T_{k-1} + T_{k-3} + ...), T_0 counted half
+void basis_derivative(const double *t, double *d) {
+  for (int k = 0; k < NC; k++) {
+    double u = 0.0;
+    for (int j = k - 1; j >= 0; j -= 2) u += j == 0 ? 0.5 * t[j] : t[j];
+    d[k] = 2.0 * k * u;
+  }
+}
+
+template <int NW>
+void launch_basis(comdgb_sim *h, Work &W, const ChebSet &S, Lam L) {
+  const ForceArgs A = force_args(h);
   const double rc2 = h->eam64c.rc2;
-  Lam L{with_lam ? W.lam : nullptr, with_lam ? W.x : nullptr};
-  adj_basis_kernel<<<W.nblk, ADJ_THREADS, sizeof(double) * NQ * NC * ADJ_THREADS, h->stream>>>(
-      A, S, rc2, L, with_lam ? W.w : nullptr, W.partial);
-  adj_sum_kernel<<<blocks(NQ * NC, 64), 64, 0, h->stream>>>(W.partial, W.nblk, NQ * NC, W.out);
-  CK(cudaMemcpyAsync(rows, W.out, sizeof(double) * NQ * NC, cudaMemcpyDeviceToHost, h->stream));
+  const bool same = S.a[0] == S.a[1] && S.b[0] == S.b[1];
+  // one thread per atom fills the card from about 150,000 atoms on (two CTAs
+  // an SM, four rounds of atoms); below, four threads share an atom: at 3,960
+  // atoms 220 us with one and 96 us with four (256,000: 2,157 and 2,774 us)
+  const int lanes = h->ntot >= 4 * W.nblk * BASIS_THREADS ? 1 : 4;
+  const long need = ((long)h->ntot * lanes + BASIS_THREADS - 1) / BASIS_THREADS;
+  const int grid = (int)std::max(1L, std::min((long)W.nblk, need));
+  auto run = [&](auto kernel) { kernel<<<grid, BASIS_THREADS, 0, h->stream>>>(A, S, rc2, L, W.partial); };
+  if (lanes == 1) {
+    if (same) run(adj_basis_kernel<NW, true, 1>);
+    else run(adj_basis_kernel<NW, false, 1>);
+  } else {
+    if (same) run(adj_basis_kernel<NW, true, 4>);
+    else run(adj_basis_kernel<NW, false, 4>);
+  }
+  adj_sum_kernel<<<NW * NC, 256, 0, h->stream>>>(W.partial, grid, NW * NC, W.out);
+}
+
+// The gradient in the coefficients at the current forces and per-step list,
+// to g[3*NC] on the host: dU/dc, or with lambda set dD/dc.
+int eam_grad(comdgb_sim *h, Work &W, const ChebSet &S, bool with_lam, double *g) {
+  if (with_lam) launch_basis<3>(h, W, S, Lam{W.lam, W.x});
+  else launch_basis<2>(h, W, S, Lam{nullptr, nullptr});
+  const int nw = with_lam ? 3 : 2;
+  const int nb = std::max(1, std::min(W.nblk, (h->ntot + BASIS_THREADS - 1) / BASIS_THREADS));
+  adj_embed_basis_kernel<<<nb, BASIS_THREADS, 0, h->stream>>>(force_args(h), S,
+                                                              with_lam ? W.w : nullptr, W.partial);
+  adj_sum_kernel<<<NC, 256, 0, h->stream>>>(W.partial, nb, NC, W.out + nw * NC);
+  double t[NQ * NC];
+  CK(cudaMemcpyAsync(t, W.out, sizeof(double) * (nw + 1) * NC, cudaMemcpyDeviceToHost,
+                     h->stream));
   CK(cudaStreamSynchronize(h->stream));
+  const double *phi = t, *rho = t + NC, *f = t + nw * NC;
+  if (!with_lam) {
+    for (int k = 0; k < NC; k++) {
+      const double c = k == 0 ? 0.5 : 1.0;
+      g[k] = c * phi[k];
+      g[NC + k] = c * rho[k];
+      g[2 * NC + k] = c * f[k];
+    }
+  } else {
+    const double *x = t + 2 * NC;
+    double d[3][NC];
+    basis_derivative(phi, d[0]);
+    basis_derivative(rho, d[1]);
+    basis_derivative(f, d[2]);
+    for (int k = 0; k < NC; k++)
+      for (int q = 0; q < 3; q++) {
+        g[q * NC + k] = d[q][k] * (2.0 / (S.b[q] - S.a[q]));
+        if (q == 1) g[q * NC + k] += k == 0 ? 0.5 * x[k] : x[k];
+      }
+  }
   return check_status(h);
 }
 
@@ -525,7 +630,7 @@ int lj_sums(comdgb_sim *h, Work &W, bool with_lam, double *out4) {
   const int nb = std::min(W.nblk, 1024);
   adj_lj_kernel<<<nb, 128, 0, h->stream>>>(force_args(h), h->lj_eps, h->lj_sigma, h->lj64.rc2,
                                            with_lam ? W.lam : nullptr, W.partial);
-  adj_sum_kernel<<<1, 32, 0, h->stream>>>(W.partial, nb, 4, W.out);
+  adj_sum_kernel<<<4, 256, 0, h->stream>>>(W.partial, nb, 4, W.out);
   CK(cudaMemcpyAsync(out4, W.out, sizeof(double) * 4, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   return check_status(h);
@@ -597,11 +702,7 @@ int comdgb_sim_energy_grad(comdgb_sim *h, double *energy, double *grad) {
     grad[1] = o[1];
     return 0;
   }
-  double rows[NQ * NC];
-  if ((rc = eam_rows(h, W, cheb_set(h), false, rows))) return rc;
-  for (int q = 0; q < 3; q++)
-    for (int k = 0; k < NC; k++) grad[q * NC + k] = rows[(2 * q) * NC + k];
-  return 0;
+  return eam_grad(h, W, cheb_set(h), false, grad);
 }
 
 int comdgb_sim_force_loss_grad(comdgb_sim *h, const double *target, double *loss, double *grad) {
@@ -626,11 +727,7 @@ int comdgb_sim_force_loss_grad(comdgb_sim *h, const double *target, double *loss
     grad[1] = -o[3];
     return 0;
   }
-  double rows[NQ * NC];
-  if ((rc = eam_rows(h, W, S, true, rows))) return rc;
-  for (int q = 0; q < 3; q++)
-    for (int k = 0; k < NC; k++) grad[q * NC + k] = rows[(2 * q + 1) * NC + k];
-  return 0;
+  return eam_grad(h, W, S, true, grad);
 }
 
 // Reverse velocity Verlet.  Forward: x_{n+1} = Phi(x_n) with r_a = r_n + c p_n,
@@ -673,10 +770,8 @@ int comdgb_sim_traj_energy_grad(comdgb_sim *h, int n, double dt, int every, doub
   if ((rc = force_fresh(h))) return rc;
   if (j) *j = h->e;
   if ((rc = snapshot_copy(h, *fin, true))) return rc;
-  double rows[NQ * NC], cbar[3 * NC];
-  if ((rc = eam_rows(h, W, S, false, rows))) return rc;
-  for (int q = 0; q < 3; q++)
-    for (int k = 0; k < NC; k++) cbar[q * NC + k] = rows[(2 * q) * NC + k];
+  double g[3 * NC], cbar[3 * NC];
+  if ((rc = eam_grad(h, W, S, false, cbar))) return rc;
   adj_force_by_id_kernel<<<blocks(h->ntot), 256, 0, h->stream>>>(h->s, h->atom_slot, h->ntot, rb);
   CK(cudaMemsetAsync(pb, 0, sizeof(double) * nv, h->stream));
   // backward, segment by segment: recompute the segment's mid-step states
@@ -696,9 +791,8 @@ int comdgb_sim_traj_energy_grad(comdgb_sim *h, int n, double dt, int every, doub
       adj_hvp_kernel<<<blocks(h->ntot, 128), 128, 0, h->stream>>>(force_args(h), S,
                                                                  h->eam64c.poly, h->eam64c.rc2,
                                                                  W.lam, W.x, hv);
-      if ((rc = eam_rows(h, W, S, true, rows))) return rc;
-      for (int q = 0; q < 3; q++)
-        for (int k = 0; k < NC; k++) cbar[q * NC + k] += rows[(2 * q + 1) * NC + k];
+      if ((rc = eam_grad(h, W, S, true, g))) return rc;
+      for (int q = 0; q < 3 * NC; q++) cbar[q] += g[q];
       adj_axpy_kernel<<<blocks(nv), 256, 0, h->stream>>>(1.0, hv, rb, nv);
       adj_axpy_kernel<<<blocks(nv), 256, 0, h->stream>>>(c, rb, pb, nv);
     }
