@@ -75,6 +75,7 @@ ForceArgs force_args(comdgb_sim *h) {
   A.ntot = h->ntot;
   A.nbr = h->nbr;
   A.nbr_n = h->nbr_n;
+  A.npair = h->npair;
   A.cap = h->cap;
   A.atom_stress = h->atom_stress;
   A.status = h->status;
@@ -149,6 +150,24 @@ Table<T> upload_table(comdgb_sim *h, const potentialarray_t *a, int *err) {
   t.invDx = (T)a->invDx;
   t.n = n;
   t.seg = nullptr;
+  t.rec = nullptr;
+  if (sizeof(T) == 8) {
+    const double *w = a->values;
+    std::vector<double2> rec(3 * (size_t)n);
+    for (int i = 0; i < n; i++) {
+      const double g0 = w[i + 1] - w[i - 1], g1 = w[i + 2] - w[i];
+      rec[3 * i] = make_double2(w[i], 0.5 * g0);
+      rec[3 * i + 1] = make_double2(0.5 * (w[i + 1] + w[i - 1] - 2.0 * w[i]), 0.0);
+      rec[3 * i + 2] = i <= 0 ? make_double2(0.0, 0.0)
+                              : make_double2(0.5 * g0 * a->invDx, 0.5 * (g1 - g0) * a->invDx);
+    }
+    double2 *dr = track(h, dalloc<double2>(rec.size(), err));
+    if (*err) return t;
+    cudaMemcpy(dr, rec.data(), sizeof(double2) * rec.size(), cudaMemcpyHostToDevice);
+    t.rec = dr;
+    t.off = (T)(-(a->x0 * a->invDx));
+    t.umax = (T)((a->xn - a->x0) * a->invDx);
+  }
   if (sizeof(T) == 4) {
     // per-interval coefficients of eamInterpolateDeriv (eam.c:422-431) in FP64
     const double *w = a->values;
@@ -529,6 +548,8 @@ int setup_potential(comdgb_sim *h, const simflat_t *s) {
     h->eam64t.rho = upload_table<double>(h, ep->rho, &err);
     h->eam64t.f = upload_table<double>(h, ep->f, &err);
     h->eam64t.rc2 = rc2;
+    h->eam64t.same_grid = ep->phi->n == ep->rho->n && ep->phi->x0 == ep->rho->x0 &&
+                          ep->phi->xn == ep->rho->xn && ep->phi->invDx == ep->rho->invDx;
     h->eam32t.phi = upload_table<float>(h, ep->phi, &err);
     h->eam32t.rho = upload_table<float>(h, ep->rho, &err);
     h->eam32t.f = upload_table<float>(h, ep->f, &err);
@@ -655,6 +676,21 @@ void enqueue_classify_finish(comdgb_sim *h, bool lazy = false) {
                       lazy ? h->status : nullptr);
 }
 
+// The squared cutoff of an FP32 list build for pairs within rc: wider by more
+// than the FP32 distances err.  Mixed precision tests the same FP32 positions
+// in its passes: a few ulps.  FP64 tests its own: a pair's FP32 difference is
+// off by the roundings of two box-centred positions (half a box each), of two
+// box offsets (up to 1.5 boxes) and of the difference, 6 * 2^-24 box widths
+// per axis at most, atoms up to an Angstrom outside their boxes included.
+float list_cutoff(const comdgb_sim *h, double rc) {
+  if (h->mixed) return (float)(rc * rc) * (1.0f + 4e-6f);
+  double width = 0.0;
+  for (const RepGeo &R : h->reps)
+    for (int j = 0; j < 3; j++) width = std::max(width, R.boxsize[j]);
+  const double err = 6.0 / 16777216.0 * (width + 1.0);
+  return (float)(rc * rc * (1.0 + 1e-6) + 4.0 * rc * err);
+}
+
 void enqueue_force_parts(comdgb_sim *h, cudaEvent_t *ev, int &evi, bool obs = true,
                          bool host_out = false) {
   // ev (optional) records after each group: compact, nbr, pass1, pass2.
@@ -680,7 +716,7 @@ void enqueue_force_parts(comdgb_sim *h, cudaEvent_t *ev, int &evi, bool obs = tr
   if (h->fo.list) {
     // force order (positions were placed by the half step before, or by
     // fo_track): the list build if due, then the passes
-    launch_nbr_build<float>(A, (float)(rcl * rcl), st, &h->tune);
+    launch_nbr_build(A, list_cutoff(h, rcl), st, &h->tune);
     launch_rebuild_done(h->status, st);
     if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
     if (pot == COMDGB_POT_LJ) {
@@ -698,38 +734,33 @@ void enqueue_force_parts(comdgb_sim *h, cudaEvent_t *ev, int &evi, bool obs = tr
     if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
     return;
   }
-  if (h->mixed) {
-    float rc2 = h->pl.vlist ? (float)(rcl * rcl)
-                            : (pot == COMDGB_POT_LJ ? h->lj32.rc2 : (float)(h->cutoff * h->cutoff));
-    launch_nbr_build<float>(A, rc2, st);
-  } else {
-    double rc2 = h->pl.vlist ? rcl * rcl
-                             : (pot == COMDGB_POT_LJ ? h->lj64.rc2 : h->cutoff * h->cutoff);
-    launch_nbr_build<double>(A, rc2, st);
+  // the build and the cut work on FP32 copies (mixed precision keeps them)
+  if (!h->mixed) launch_pos32_atoms(h->g, h->s, h->atom_slot, h->ntot, st);
+  launch_nbr_build(A, list_cutoff(h, h->pl.vlist ? rcl : h->cutoff), st);
+  if (h->pl.vlist) {
+    launch_rebuild_done(h->status, st);
+    launch_nbr_cut(A, list_cutoff(h, h->cutoff), st);
   }
-  if (h->pl.vlist) launch_rebuild_done(h->status, st);
   if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
   if (pot == COMDGB_POT_LJ) {
     if (h->mixed) launch_lj<float>(A, h->lj32, st);
-    else launch_lj<double>(A, h->lj64, st);
+    else launch_lj64(A, h->lj64, st, obs);
     if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
     if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
     return;
   }
-  if (pot == COMDGB_POT_EAM_TABLE) {
-    if (h->mixed) launch_eam_pass1<float, EVAL_TABLE>(A, h->eam32t, st);
-    else launch_eam_pass1<double, EVAL_TABLE>(A, h->eam64t, st);
+  for (int pass = 0; pass < 2; pass++) {
+    if (pot == COMDGB_POT_EAM_TABLE) {
+      if (!h->mixed) launch_eam64<EVAL_TABLE>(A, h->eam64t, pass, st, obs);
+      else if (pass == 0) launch_eam_pass1<float, EVAL_TABLE>(A, h->eam32t, st);
+      else launch_eam_pass2<float, EVAL_TABLE>(A, h->eam32t, st);
+    } else {
+      if (!h->mixed) launch_eam64<EVAL_CHEBY>(A, h->eam64c, pass, st, obs);
+      else if (pass == 0) launch_eam_pass1<float, EVAL_CHEBY>(A, h->eam32c, st);
+      else launch_eam_pass2<float, EVAL_CHEBY>(A, h->eam32c, st);
+    }
     if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
-    if (h->mixed) launch_eam_pass2<float, EVAL_TABLE>(A, h->eam32t, st);
-    else launch_eam_pass2<double, EVAL_TABLE>(A, h->eam64t, st);
-  } else {
-    if (h->mixed) launch_eam_pass1<float, EVAL_CHEBY>(A, h->eam32c, st);
-    else launch_eam_pass1<double, EVAL_CHEBY>(A, h->eam64c, st);
-    if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
-    if (h->mixed) launch_eam_pass2<float, EVAL_CHEBY>(A, h->eam32c, st);
-    else launch_eam_pass2<double, EVAL_CHEBY>(A, h->eam64c, st);
   }
-  if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
 }
 
 int count_kernel_nodes(cudaGraph_t graph);
@@ -830,7 +861,7 @@ void enqueue_fo_step_force(comdgb_sim *h, double dt_atu, cudaEvent_t *ev, int &e
   launch_compact(h->g, h->s.natoms, h->box_start, h->atom_slot, h->ntot, h->cpart, h->ncpart,
                  rs, h->status);
   const double rcl = h->cutoff + h->skin;
-  launch_nbr_build<float>(A, (float)(rcl * rcl), rs, &h->tune);
+  launch_nbr_build(A, list_cutoff(h, rcl), rs, &h->tune);
   if (bs) h->rebuild_kernels = cond_end(h);
   // (mixed precision keeps no position increments in f: ST_DELTA stays 0)
   cudaStream_t os = cond_begin(h, -1);
@@ -911,9 +942,9 @@ void enqueue_step(comdgb_sim *h, double dt_atu, cudaEvent_t *ev, int part) {
     if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
     enqueue_classify_finish(h);
     if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
-    // inside the sequence (OPEN, MID): the CLOSE part and the force call
-    // that ends nTimeSteps follow, so nothing reads this call's energies
-    enqueue_force_parts(h, ev, evi, part == PART_FULL);  // the atom list of the new layout
+    // inside a sequence (OPEN, MID, and every FP64 step) a force call that ends
+    // nTimeSteps follows, so nothing reads this call's energies
+    enqueue_force_parts(h, ev, evi, part == PART_FULL && h->mixed);
     if (part != PART_FULL) return;
   }
   cudaMemsetAsync(h->status + ST_REBIN_SERIAL, 0, sizeof(int), st);
@@ -1665,6 +1696,7 @@ int create(const simflat_t *const *sims, int nrep, const comdgb_opts *o, comdgb_
   // (the force-order passes keep their own lists and never read this one)
   h->nbr = track(h, dalloc<uint16_t>((h->fo.list ? 0 : (size_t)h->ntot * h->cap) + 8, &err));
   h->nbr_n = track(h, dalloc<int>((size_t)h->ntot + 1, &err));
+  h->npair = track(h, dalloc<int>((size_t)h->ntot + 1, &err));
   h->atom_stress = track(h, dalloc<double>((size_t)h->ntot + 1, &err));
   h->nrpart = reduce_partials(h->ntot);
   h->rpart = track(h, dalloc<double>(2 * (size_t)h->nrpart, &err));
@@ -1678,9 +1710,10 @@ int create(const simflat_t *const *sims, int nrep, const comdgb_opts *o, comdgb_
     delete h;
     return set_err(COMDGB_ERR_NOMEM, "cudaMalloc failed (%zu slots)", ns);
   }
-  if (prepare_force_kernels<double>() != cudaSuccess || prepare_force_kernels<float>() != cudaSuccess)
+  if (prepare_force_kernels() != cudaSuccess)
     err = 1;
   cudaMemsetAsync(h->nbr_n, 0, sizeof(int) * ((size_t)h->ntot + 1), h->stream);
+  cudaMemsetAsync(h->npair, 0, sizeof(int) * ((size_t)h->ntot + 1), h->stream);
   cudaMemsetAsync(h->atom_stress, 0, sizeof(double) * ((size_t)h->ntot + 1), h->stream);
   for (int r = 0; r < nrep; r++)
     cudaMemcpyAsync(h->dcenter + 3 * (size_t)h->reps[r].box0, sims[r]->dcenter,

@@ -296,6 +296,10 @@ struct Table {
   // computed in FP64 from v[i-1..i+2] so no FP32 differences of nearby table
   // values are formed: value = c0 + u(c1 + u c2), deriv = d0 + u d1
   const float4 *seg;
+  // FP64 path: the same coefficients, per interval (c0, c1) (c2, 0) (d0, d1),
+  // and u = r * invDx + off, at most umax
+  const double2 *rec;
+  T off, umax;
 };
 
 // Chebyshev series of the reference: 0 phi, 1 rho, 2 F, 3 dphi, 4 drho, 5 dF
@@ -450,23 +454,81 @@ struct DSum {
   __device__ __forceinline__ double value() const { return s; }
 };
 
-// eamInterpolateDeriv (eam.c:401-434), same operation order
-template <class T>
-__device__ __forceinline__ void table_eval(const Table<T> &a, T r, T &value, T &deriv) {
-  if (r < a.x0) r = a.x0;
-  else if (r > a.xn) r = a.xn;
-  r = (r - a.x0) * a.invDx;
-  T fl = floor(r);
-  int i1 = (int)fl;
-  r = r - fl;
-  // a NaN argument must not index outside the table (valid r gives 0..n-1)
-  i1 = i1 < 0 ? 0 : (i1 > a.n - 1 ? a.n - 1 : i1);
-  const T *v = a.v;
-  T vm = __ldg(v + i1 - 1), v0 = __ldg(v + i1), v1 = __ldg(v + i1 + 1), v2 = __ldg(v + i1 + 2);
-  T gi = v1 - vm;
-  T gi1 = v2 - v0;
-  value = v0 + T(0.5) * r * (r * (v1 + vm - T(2.0) * v0) + gi);
-  deriv = (i1 <= 0) ? T(0) : T(0.5) * (gi + r * (gi1 - gi)) * a.invDx;
+// FP64 1/s, and r = sqrt(s) with 1/r, for the per-pair functions: the FP32
+// approximation of the leading bits of s (moved to FP32 and back by integer
+// operations) and one step of third order, 1/s = y (1 + e + e^2), e = 1 - s y,
+// and s^(-1/2) = y (1 + e/2 + 3 e^2/8), e = 1 - s y^2 (Householder's method):
+// e is below 2^-21, so the terms left out are below 2^-63.  r is then
+// corrected by its residual.  Three and nine FP64 operations where the exact
+// division and square root take about twice as many.  Arguments far from 1
+// (none that a pair distance takes), zero and NaN go the exact way.
+__device__ __forceinline__ float leading_f32(double s, int hi) {
+  return __int_as_float((int)((unsigned)(hi - 0x38000000) << 3) |
+                        (int)((unsigned)__double2loint(s) >> 29));
+}
+__device__ __forceinline__ double widen_f32(float y) {  // a positive normal number
+  const int b = __float_as_int(y);
+  return __hiloint2double((b >> 3) + 0x38000000, b << 29);
+}
+__device__ __forceinline__ bool f32_range(int hi) {
+  return (unsigned)(hi - 0x3c000000) < 0x08000000u;  // 2^-63 to 2^65
+}
+__device__ __forceinline__ double reciprocal(double s) {
+  const int hi = __double2hiint(s);
+  if (!f32_range(hi)) return __ddiv_rn(1.0, s);
+  const double y = widen_f32(__frcp_rn(leading_f32(s, hi)));
+  const double e = fma(-s, y, 1.0);
+  return fma(fma(e, e, e), y, y);
+}
+__device__ __forceinline__ void r_and_inv(double s, double &r, double &inv) {
+  const int hi = __double2hiint(s);
+  if (!f32_range(hi)) {
+    r = sqrt(s);
+    inv = __ddiv_rn(1.0, r);
+    return;
+  }
+  const double y = widen_f32(rsqrtf(leading_f32(s, hi)));
+  const double e = fma(-__dmul_rn(s, y), y, 1.0);
+  inv = fma(__dmul_rn(y, e), fma(e, 0.375, 0.5), y);
+  const double g = __dmul_rn(s, inv);
+  r = fma(fma(-g, g, s), __dmul_rn(0.5, inv), g);
+}
+
+// eamInterpolateDeriv (eam.c:401-434) from per-interval coefficients: the
+// interval i of r (clamped to the table) and the offset u in it.  The
+// interval is the integer part of the leading bits of u, which truncation
+// keeps; the clamps compare bits.  A NaN keeps u NaN and some valid interval.
+struct TableAt {
+  int i;
+  double u;
+};
+__device__ __forceinline__ TableAt table_at(const Table<double> &a, double r) {
+  const long long inf = 0x7ff0000000000000LL, mag = 0x7fffffffffffffffLL;
+  double u = fma(r, a.invDx, a.off);
+  const long long b = __double_as_longlong(u);
+  if (b < 0 && (b & mag) <= inf) u = 0.0;
+  else if (b > __double_as_longlong(a.umax) && b <= inf) u = a.umax;
+  const int hi = __double2hiint(u);
+  TableAt t;
+  t.i = hi < 0x3ff00000 ? 0 : min((int)leading_f32(u, hi), a.n - 1);
+  t.i = max(t.i, 0);
+  t.u = __dsub_rn(u, __dsub_rn(__hiloint2double(0x43300000, t.i), 4503599627370496.0));
+  return t;
+}
+__device__ __forceinline__ double table_value(const Table<double> &a, TableAt t) {
+  const double2 c = __ldg(a.rec + 3 * t.i);
+  const double c2 = __ldg(reinterpret_cast<const double *>(a.rec + 3 * t.i + 1));
+  return fma(t.u, fma(t.u, c2, c.y), c.x);
+}
+__device__ __forceinline__ double table_deriv(const Table<double> &a, TableAt t) {
+  const double2 d = __ldg(a.rec + 3 * t.i + 2);
+  return fma(t.u, d.y, d.x);
+}
+__device__ __forceinline__ void table_eval(const Table<double> &a, double r, double &value,
+                                           double &deriv) {
+  const TableAt t = table_at(a, r);
+  value = table_value(a, t);
+  deriv = table_deriv(a, t);
 }
 
 // FP32 table lookup from the per-interval coefficients (same function)

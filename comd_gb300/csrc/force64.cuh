@@ -1,0 +1,314 @@
+// force64.cuh -- the FP64 force passes over the per-step list.
+//
+// What bounds them is the FP64 pipe: about two lanes per SM per clock, so a
+// warp's FP64 instruction holds it for 16 clocks while every other pipe (and
+// the loads) wait for nothing.  So the passes count FP64 operations:
+//   * density first, then forces, as in force order: rho alone in the first
+//     pass (17 operations a pair with the Chebyshev polynomials), phi'/r and
+//     rho'/r in the second, and phi and the stress only where the caller can
+//     read them (OBS);
+//   * the cutoff test compares bit patterns, and 1/r and r come from the FP32
+//     reciprocal square root (MUFU) and one cubic step, not from FP64 division;
+//   * LANES threads share an atom's list (lane l takes entries l, l + LANES,
+//     ...; the sums are combined in a fixed order).  A thread per atom leaves
+//     most of the 152 SMs idle on small systems, and on larger ones the last
+//     wave of long threads runs nearly empty.
+// F'(rho_j) reaches the second pass in the unused fourth component of r: one
+// 32-byte gather a pair.
+// Measured at 256,000 atoms (no energies), both passes: table potential 3,156
+// us before (phi, phi' and rho, then rho', a thread per atom, FP64 division and
+// square root, the skin list walked in FP64) and 1,221 now, Chebyshev 1,327 and
+// 950.
+#pragma once
+
+#include "force_kernels.cuh"
+
+namespace cg {
+
+constexpr int F64_THREADS = 128;
+
+// r2 beyond the cutoff, by the bits of non-negative doubles; a NaN is not (it
+// reaches the sums, as in a floating-point comparison)
+__device__ __forceinline__ bool beyond(double r2, double rc2) {
+  const long long x = __double_as_longlong(r2);
+  return x > __double_as_longlong(rc2) && x <= 0x7ff0000000000000LL;
+}
+__device__ __forceinline__ bool below(double r2, double rc2) {
+  return __double_as_longlong(r2) < __double_as_longlong(rc2);
+}
+
+// The atom and sub-lane of this thread; false when its whole warp has none.
+// Groups past the last atom repeat it (no divergence in the shuffles) and
+// store nothing (live).
+template <int LANES>
+__device__ __forceinline__ bool lane_atom(int ntot, int &a, int &sub, bool &live) {
+  const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if ((q & ~31L) / LANES >= ntot) return false;
+  const long at = q / LANES;
+  live = at < ntot;
+  a = live ? (int)at : ntot - 1;
+  sub = (int)(q % LANES);
+  return true;
+}
+
+template <int LANES>
+__device__ __forceinline__ double lane_sum(double v) {
+#pragma unroll
+  for (int o = LANES / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// This lane's entries of atom a's list: fn(r_j, dx, dy, dz, r2), entries past
+// the cutoff included; an overflowed list's stencil is scanned by lane 0.
+template <int LANES, class F>
+__device__ __forceinline__ void walk64(const ForceArgs &A, int a, int sub, int slot,
+                                       const d4 &ri, double rc2, F &&fn) {
+  const int n = A.nbr_n[a], b = slot >> 6;
+  if (n > A.cap) {
+    if (sub == 0)
+      scan_stencil<double>(A, b, slot & 63, ri.x, ri.y, ri.z, rc2,
+                           [&](int js, double dx, double dy, double dz, double r2) {
+                             fn(A.s.r[js], dx, dy, dz, r2);
+                           });
+    return;
+  }
+  const int ebase = b * CG_NNBR;
+  const uint16_t *lst = A.nbr + (size_t)a * A.cap;
+#pragma unroll 2
+  for (int t = sub; t < n; t += LANES) {
+    const uint32_t code = __ldg(lst + t);
+    const int e = code >> 6;
+    const d4 rj = A.s.r[__ldg(A.et.box + ebase + e) * CG_MAXATOMS + (code & 63)];
+    double dx, dy, dz;
+    const double r2 = pair_r2(PrecT<double>::drbox(A.et, ebase + e), ri.x, ri.y, ri.z, rj.x, rj.y,
+                              rj.z, dx, dy, dz);
+    fn(rj, dx, dy, dz, r2);
+  }
+}
+
+// rho(r); phi, phi'/r and rho'/r.  false: outside the polynomial tables
+static __device__ __forceinline__ bool rho64(const EamPot<double, EVAL_CHEBY> &P, double r2,
+                                             double &rho) {
+  int k;
+  double t;
+  if (!poly_at(P.poly.pair, r2, k, t)) return false;
+  rho = poly_col(P.poly.pair, PF_RHO, k, t);
+  return true;
+}
+template <bool OBS>
+static __device__ __forceinline__ bool force64(const EamPot<double, EVAL_CHEBY> &P, double r2,
+                                               double &phi, double &wphi, double &wrho) {
+  int k;
+  double t;
+  if (!poly_at(P.poly.pair, r2, k, t)) return false;
+  if (OBS) phi = poly_col(P.poly.pair, PF_PHI, k, t);
+  wphi = poly_col(P.poly.pair, PF_GPHI, k, t);
+  wrho = poly_col(P.poly.pair, PF_GRHO, k, t);
+  return true;
+}
+static __device__ __forceinline__ bool outside64(const EamPot<double, EVAL_CHEBY> &P, double r2) {
+  return below_seg(P, r2);
+}
+static __device__ __noinline__ double rho64_series(const EamPot<double, EVAL_CHEBY> &P, double r2) {
+  double r, inv;
+  r_and_inv(r2, r, inv);
+  return cheb_series(P, 1, r);
+}
+static __device__ __noinline__ void force64_series(const EamPot<double, EVAL_CHEBY> &P, double r2,
+                                                   double &phi, double &wphi, double &wrho) {
+  double r, inv;
+  r_and_inv(r2, r, inv);
+  phi = cheb_series(P, 0, r);
+  wphi = cheb_series(P, 3, r) * inv;
+  wrho = cheb_series(P, 4, r) * inv;
+}
+// the table potential has no outside
+static __device__ __forceinline__ bool rho64(const EamPot<double, EVAL_TABLE> &P, double r2,
+                                             double &rho) {
+  double r, inv;
+  r_and_inv(r2, r, inv);
+  rho = table_value(P.rho, table_at(P.rho, r));
+  return true;
+}
+template <bool OBS>
+static __device__ __forceinline__ bool force64(const EamPot<double, EVAL_TABLE> &P, double r2,
+                                               double &phi, double &wphi, double &wrho) {
+  double r, inv;
+  r_and_inv(r2, r, inv);
+  const TableAt p = table_at(P.phi, r);
+  const TableAt q = P.same_grid ? p : table_at(P.rho, r);
+  if (OBS) phi = table_value(P.phi, p);
+  wphi = table_deriv(P.phi, p) * inv;
+  wrho = table_deriv(P.rho, q) * inv;
+  return true;
+}
+static __device__ __forceinline__ bool outside64(const EamPot<double, EVAL_TABLE> &, double) {
+  return false;
+}
+static __device__ __forceinline__ double rho64_series(const EamPot<double, EVAL_TABLE> &, double) {
+  return 0.0;
+}
+static __device__ __forceinline__ void force64_series(const EamPot<double, EVAL_TABLE> &, double,
+                                                      double &, double &, double &) {}
+
+// rho_i = sum of rho(r_ij), F'(rho_i) for the force pass; OBS: also rho, F'
+// and F(rho_i) (left in f's fourth component) and the pairs counted
+template <int EVAL, int LANES, bool OBS>
+__global__ void __launch_bounds__(F64_THREADS)
+    eam64_density_kernel(ForceArgs A, const __grid_constant__ EamPot<double, EVAL> P) {
+  int a, sub;
+  bool live;
+  if (!lane_atom<LANES>(A.ntot, a, sub, live)) return;
+  const int slot = A.atom_slot[a];
+  const d4 ri = A.s.r[slot];
+  const double rc2 = P.rc2;
+  double rho = 0.0;
+  int cnt = 0;
+  bool low = false;
+  walk64<LANES>(A, a, sub, slot, ri, rc2, [&](const d4 &, double, double, double, double r2) {
+    if (beyond(r2, rc2)) return;
+    cnt++;
+    double v;
+    if (rho64(P, r2, v)) rho = __dadd_rn(rho, v);
+    else low = true;
+  });
+  if (low)  // pairs below the table: the series, in a second sweep
+    walk64<LANES>(A, a, sub, slot, ri, rc2, [&](const d4 &, double, double, double, double r2) {
+      if (!beyond(r2, rc2) && outside64(P, r2)) rho = __dadd_rn(rho, rho64_series(P, r2));
+    });
+  rho = lane_sum<LANES>(rho);
+  if (OBS)
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+  double F, dF;
+  eam_embed<double, EVAL>(P, rho, F, dF);
+  if (sub != 0 || !live) return;
+  A.s.r[slot].w = dF;
+  if (OBS) {
+    A.s.rho[slot] = rho;
+    A.s.fi[slot] = dF;
+    A.s.f[slot].w = F;
+    A.npair[a] = cnt;
+  }
+}
+
+// f_i = sum of (phi'(r) + (F'_i + F'_j) rho'(r)) dr/r (eam.c:534-545,
+// 595-653); OBS: the per-atom energy and the x-x embedding stress
+template <int EVAL, int LANES, bool OBS>
+__global__ void __launch_bounds__(F64_THREADS)
+    eam64_force_kernel(ForceArgs A, const __grid_constant__ EamPot<double, EVAL> P) {
+  int a, sub;
+  bool live;
+  if (!lane_atom<LANES>(A.ntot, a, sub, live)) return;
+  const int slot = A.atom_slot[a];
+  const d4 ri = A.s.r[slot];
+  const double rc2 = P.rc2, fii = ri.w;
+  double fx = 0.0, fy = 0.0, fz = 0.0, ep = 0.0, sx = 0.0;
+  bool low = false;
+  auto add = [&](const d4 &rj, double dx, double dy, double dz, double r2, double phi, double wphi,
+                 double wrho) {
+    const double we = below(r2, rc2) ? __dmul_rn(__dadd_rn(fii, rj.w), wrho) : 0.0;
+    const double w = __dadd_rn(wphi, we);
+    fx = fma(w, dx, fx);
+    fy = fma(w, dy, fy);
+    fz = fma(w, dz, fz);
+    if (OBS) {
+      ep = __dadd_rn(ep, phi);
+      sx = fma(__dmul_rn(we, dx), dx, sx);
+    }
+  };
+  walk64<LANES>(A, a, sub, slot, ri, rc2, [&](const d4 &rj, double dx, double dy, double dz,
+                                              double r2) {
+    if (beyond(r2, rc2)) return;
+    double phi = 0.0, wphi, wrho;
+    if (force64<OBS>(P, r2, phi, wphi, wrho)) add(rj, dx, dy, dz, r2, phi, wphi, wrho);
+    else low = true;
+  });
+  if (low)
+    walk64<LANES>(A, a, sub, slot, ri, rc2, [&](const d4 &rj, double dx, double dy, double dz,
+                                                double r2) {
+      if (beyond(r2, rc2) || !outside64(P, r2)) return;
+      double phi, wphi, wrho;
+      force64_series(P, r2, phi, wphi, wrho);
+      add(rj, dx, dy, dz, r2, phi, wphi, wrho);
+    });
+  fx = lane_sum<LANES>(fx);
+  fy = lane_sum<LANES>(fy);
+  fz = lane_sum<LANES>(fz);
+  if (OBS) {
+    ep = lane_sum<LANES>(ep);
+    sx = lane_sum<LANES>(sx);
+  }
+  if (sub != 0 || !live) return;
+  d4 f;
+  f.x = fx;
+  f.y = fy;
+  f.z = fz;
+  f.w = 0.0;
+  if (OBS) {
+    f.w = fma(0.5, ep, A.s.f[slot].w);
+    A.atom_stress[a] = sx;
+  }
+  A.s.f[slot] = f;
+}
+
+// LJ: ljForce.c:151-215 as full pairs; the kinetic stress term is added once
+// per (atom, non-empty neighbour box) as at ljForce.c:175
+template <int LANES, bool OBS>
+__global__ void __launch_bounds__(F64_THREADS) lj64_kernel(ForceArgs A, LjPot<double> P) {
+  int a, sub;
+  bool live;
+  if (!lane_atom<LANES>(A.ntot, a, sub, live)) return;
+  const int slot = A.atom_slot[a], b = slot >> 6;
+  const d4 ri = A.s.r[slot];
+  const double s6 = P.s6, s12 = P.s6x12, c4 = P.eps4s6, rc2 = P.rc2;
+  double fx = 0.0, fy = 0.0, fz = 0.0, ep = 0.0, sx = 0.0;
+  int cnt = 0;
+  walk64<LANES>(A, a, sub, slot, ri, rc2, [&](const d4 &, double dx, double dy, double dz,
+                                              double r2) {
+    if (beyond(r2, rc2)) return;
+    const double ir2 = reciprocal(r2);
+    const double r6 = __dmul_rn(__dmul_rn(ir2, ir2), ir2);
+    const double fr = __dmul_rn(__dmul_rn(__dmul_rn(c4, r6), ir2), fma(s12, r6, -6.0));
+    fx = fma(fr, dx, fx);
+    fy = fma(fr, dy, fy);
+    fz = fma(fr, dz, fz);
+    if (OBS) {
+      cnt++;
+      ep = fma(r6, fma(s6, r6, -1.0), ep);
+      sx = fma(__dmul_rn(fr, dx), dx, sx);
+    }
+  });
+  fx = lane_sum<LANES>(fx);
+  fy = lane_sum<LANES>(fy);
+  fz = lane_sum<LANES>(fz);
+  int nonempty = 0;
+  if (OBS) {
+    ep = lane_sum<LANES>(ep);
+    sx = lane_sum<LANES>(sx);
+    const int ne = A.et.n[b];
+    for (int e = sub; e < ne; e += LANES)
+      nonempty += A.s.natoms[A.et.box[b * CG_NNBR + e]] > 0;
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) {
+      cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+      nonempty += __shfl_xor_sync(0xffffffffu, nonempty, o);
+    }
+  }
+  if (sub != 0 || !live) return;
+  d4 f;
+  f.x = fx;
+  f.y = fy;
+  f.z = fz;
+  f.w = 0.0;
+  if (OBS) {
+    f.w = 0.5 * ep;
+    const d4 p = A.s.p[slot];
+    const double kin = __ddiv_rn(__dmul_rn(p.x, p.x), A.s.mass[slot]);
+    A.atom_stress[a] = sx - (double)nonempty * kin;
+    A.npair[a] = cnt;
+  }
+  A.s.f[slot] = f;
+}
+
+}  // namespace cg

@@ -1,15 +1,15 @@
-// force_kernels.cuh -- link-cell force kernels, templated on the pair
-// arithmetic type T (double: the plain FP64 kernels; float: mixed precision).
+// force_kernels.cuh -- list builds (both precisions) and the mixed-precision
+// link-cell force kernels; the FP64 passes are in force64.cuh.
 //
 // Work decomposition (full pairs: every atom sums over all its neighbours,
 // so per-atom sums need no atomics and are deterministic):
 //   nbr_build   one CTA per box.  The box's stencil entries (27 neighbour
 //               boxes with the reference's multiplicity) are staged from HBM
-//               into shared memory; each warp takes one atom of the box and
-//               tests 32 candidates per iteration, compacting hits with a
-//               ballot into the atom's neighbour list (uint16 codes: entry
-//               index << 6 | slot).  Cutoff test as pass 1 of eamForce:
-//               r2 <= rc2 (eam.c:521, ljForce.c:193).
+//               into shared memory; each warp tests atoms of the box against
+//               32 candidates per iteration, compacting hits with a ballot
+//               into the atom's neighbour list (uint16 codes: entry index
+//               << 6 | slot).  The passes test r2 <= rc2 (eam.c:521,
+//               ljForce.c:193) again.
 //   eam_pass1   one thread per atom over its list: pair phi, phi', rho
 //               (eam.c:484-549), then F(rho) and F'(rho) fused in
 //               (eam.c:576-594).
@@ -36,7 +36,8 @@ struct ForceArgs {
   const int *box_start;  // [nboxes+1] first atom index of each box
   int ntot;
   uint16_t *nbr;         // [ntot*cap]
-  int *nbr_n;            // [ntot] true neighbour count
+  int *nbr_n;            // [ntot] list length (> cap: overflowed)
+  int *npair;            // [ntot] neighbours within the cutoff (written by the passes)
   int cap;
   double *atom_stress;   // [ntot] per-atom share of the scalar stress
   int *status;
@@ -119,21 +120,8 @@ struct PrecT<float> {
   }
 };
 
-// FP64: dr = drbox + r_i - r_j and r2 accumulated in the reference's order
-// (the list build: which pairs are within the cutoff)
-__device__ __forceinline__ double pair_r2_ref(const BoxOff<double> &o, double xi, double yi,
-                                              double zi, double xj, double yj, double zj,
-                                              double &dx, double &dy, double &dz) {
-  dx = (o.x + xi) - xj;
-  dy = (o.y + yi) - yj;
-  dz = (o.z + zi) - zj;
-  double r2 = dx * dx;
-  r2 = r2 + dy * dy;
-  r2 = r2 + dz * dz;
-  return r2;
-}
-// the same with fused sums (the passes: two FP64 operations and two roundings
-// fewer per pair)
+// FP64: dr = drbox + r_i - r_j as the reference forms it, r2 with fused sums
+// (two FP64 operations and two roundings fewer per pair)
 __device__ __forceinline__ double pair_r2(const BoxOff<double> &o, double xi, double yi,
                                           double zi, double xj, double yj, double zj, double &dx,
                                           double &dy, double &dz) {
@@ -175,58 +163,14 @@ __device__ void scan_stencil(const ForceArgs &A, int b, int i, T xi, T yi, T zi,
   }
 }
 
-// Persistent list of atom (b, i): neighbour ids, looked up in their current
-// slots; the pair's box offset is the stencil entry of the two current boxes,
-// so dr is formed exactly as with the per-step list.
-// With `a` >= 0 the pairs within rc2 are also written, as slot codes, to the
-// per-step list of compact atom a (for the passes that follow).
-template <class T, class F>
-__device__ __forceinline__ void for_each_persistent(const ForceArgs &A, int a, int b, int i, T xi,
-                                                    T yi, T zi, T rc2, F &&fn) {
-  const int idi = A.s.id[b * CG_MAXATOMS + i];
-  const int n = A.pl.vcount[idi];
-  if (n > A.pl.vcap) {
-    scan_stencil<T>(A, b, i, xi, yi, zi, rc2, fn);
-    if (a >= 0) A.nbr_n[a] = A.cap + 1;  // later passes scan the stencil too
-    return;
-  }
-  uint16_t *emit = a >= 0 ? A.nbr + (size_t)a * A.cap : nullptr;
-  int cnt = 0;
-  const int *lst = A.pl.vlist + (size_t)idi * A.pl.vcap;
-#pragma unroll 1
-  for (int t = 0; t < n; t++) {
-    const int js = __ldg(A.pl.slot_of + __ldg(lst + t));
-    const int e = stencil_entry(A.g, b, js >> 6);
-    if (e < 0) continue;
-    T xj, yj, zj, dx, dy, dz;
-    BoxOff<T> bo = PrecT<T>::drbox(A.et, b * CG_NNBR + e);
-    PrecT<T>::pos(A.s, js, xj, yj, zj);
-    T r2 = pair_r2(bo, xi, yi, zi, xj, yj, zj, dx, dy, dz);
-    if (emit && r2 <= rc2) {
-      if (cnt < A.cap) emit[cnt] = (uint16_t)((e << 6) | (js & 63));
-      cnt++;
-    }
-    fn(js, dx, dy, dz, r2);
-  }
-  if (a >= 0) {
-    A.nbr_n[a] = cnt;
-    if (cnt > A.cap) atomicAdd(A.status + ST_NBR_OVERFLOW, 1);
-  }
-}
-
 // Visit the atom's neighbour list (or its stencil when the list overflowed).
-// The first pass of a force call with persistent lists (PERSIST_FIRST)
-// walks the skin list instead and leaves the exact per-step list behind.
+// Entries a hair past the cutoff are among them: the passes test r2 again.
 // VEC: read eight codes per 16-byte load and unroll over them (light
 // passes: independent gathers in flight); otherwise one copy of the pair
 // code in the loop (heavy passes: instruction cache).
-template <class T, bool VEC = false, bool PERSIST_FIRST = false, class F>
+template <class T, bool VEC = false, class F>
 __device__ __forceinline__ void for_each_neighbor(const ForceArgs &A, int a, int b, int i, T xi,
                                                   T yi, T zi, T rc2, F &&fn) {
-  if (PERSIST_FIRST && A.pl.vlist) {
-    for_each_persistent<T>(A, a, b, i, xi, yi, zi, rc2, fn);
-    return;
-  }
   const int n = A.nbr_n[a];
   if (n > A.cap) {
     scan_stencil<T>(A, b, i, xi, yi, zi, rc2, fn);
@@ -356,9 +300,13 @@ __device__ __forceinline__ int entry_of(const int *s_off, int ne, int c) {
 // sentinels.  Each warp takes two atoms per candidate load and parks every
 // chunk's ballot in warp-private shared memory; the warp then writes each
 // atom's list cooperatively (one mask word per lane, prefix sum of the
-// popcounts, each lane emits its own bits).  The cutoff of the build is
-// widened by a hair so the list is a superset of the pairs the passes accept
-// with their exact dr.
+// popcounts, each lane emits its own bits).  The cutoff of the build (rc2b)
+// is widened by more than the FP32 distances err (list_cutoff in api.cu), so
+// the list holds every pair that the passes accept with their exact dr.  The
+// FP64 simulations use the same build on FP32 copies of their positions: an
+// FP64 test of every candidate, 12 operations for each of seven candidates
+// per neighbour, took 1,785 us for the lists of 256,000 atoms, this
+// 270 us.
 #define NB_CHUNKS (NB_MAXC / 32)  // 54
 #define NB_ATOMS 4                 // atoms tested per candidate load
 // Modes: LIST_STEP writes the per-step list (uint16 codes); LIST_ID (runs
@@ -421,7 +369,7 @@ __device__ __forceinline__ void build_count(const ForceArgs &A, int row, int tot
 // the lists of the atoms of box b (not empty): NT threads (the CTA), NA
 // atoms tested per candidate load, the shared arrays of the kernel
 template <int MODE, int NT, int NA>
-__device__ __forceinline__ void build_box32(const ForceArgs &A, float rc2, int b, float4 *cand,
+__device__ __forceinline__ void build_box32(const ForceArgs &A, float rc2b, int b, float4 *cand,
                                             uint32_t (*s_mask)[NA][NB_CHUNKS], int *s_box,
                                             int *s_off, int *s_code, BoxOff<float> *s_dr) {
   const int ni = A.s.natoms[b];
@@ -449,7 +397,6 @@ __device__ __forceinline__ void build_box32(const ForceArgs &A, float rc2, int b
     }
   }
   __syncthreads();
-  const float rc2b = rc2 * (1.0f + 4e-6f);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   static_assert(NA % 2 == 0, "atoms are tested in pairs");
   for (int i0 = NA * warp; i0 < ni; i0 += NA * (NT / 32)) {
@@ -552,7 +499,7 @@ __device__ __forceinline__ void build_box32(const ForceArgs &A, float rc2, int b
 // rebuild due (most steps, with skin lists) costs one check per resident
 // CTA instead of one CTA per box.
 template <int MODE, int NT = NB_THREADS, int NA = NB_ATOMS>
-static __global__ void __launch_bounds__(NT) nbr_build32_kernel(ForceArgs A, float rc2) {
+static __global__ void __launch_bounds__(NT) nbr_build32_kernel(ForceArgs A, float rc2b) {
   __shared__ __align__(16) float4 cand[NB_MAXC];
   __shared__ uint32_t s_mask[NT / 32][NA][NB_CHUNKS];
   __shared__ int s_box[CG_NNBR], s_off[CG_NNBR + 1], s_code[CG_NNBR];
@@ -560,67 +507,51 @@ static __global__ void __launch_bounds__(NT) nbr_build32_kernel(ForceArgs A, flo
   if (build_skipped<MODE>(A)) return;
   for (int b = blockIdx.x; b < A.g.nboxes; b += gridDim.x) {
     if (A.s.natoms[b] == 0) continue;
-    build_box32<MODE, NT, NA>(A, rc2, b, cand, s_mask, s_box, s_off, s_code, s_dr);
+    build_box32<MODE, NT, NA>(A, rc2b, b, cand, s_mask, s_box, s_off, s_code, s_dr);
     __syncthreads();  // the next box restages the shared arrays
   }
 }
 
-// FP64: the reference's dr = (drbox + r_i) - r_j, operation by operation
-template <int MODE>
-static __global__ void __launch_bounds__(NB_THREADS) nbr_build64_kernel(ForceArgs A, double rc2) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double *cx = reinterpret_cast<double *>(smem_raw);
-  double *cy = cx + NB_MAXC;
-  double *cz = cy + NB_MAXC;
-  uint16_t *cc = reinterpret_cast<uint16_t *>(cz + NB_MAXC);
-  __shared__ int s_box[CG_NNBR], s_off[CG_NNBR + 1];
-  __shared__ BoxOff<double> s_dr[CG_NNBR];
-  if (build_skipped<MODE>(A)) return;
-  const int b = blockIdx.x;
-  const int ni = A.s.natoms[b];
-  if (ni == 0) return;
-  const int ne = stage_entries<double>(A, b, s_box, s_off, s_dr);
-  const int ncand = s_off[ne];
-  for (int c = threadIdx.x; c < ncand; c += NB_THREADS) {
-    int e = entry_of(s_off, ne, c);
-    int k = c - s_off[e];
-    d4 q = A.s.r[s_box[e] * CG_MAXATOMS + k];
-    cx[c] = q.x;
-    cy[c] = q.y;
-    cz[c] = q.z;
-    cc[c] = (uint16_t)((e << 6) | k);
+// The per-step list of every atom from its id-keyed skin list (LIST_ID),
+// one warp per atom, 32 entries a round: the neighbour's current slot, its
+// stencil entry as seen from the atom's box, an FP32 distance test (rc2b is
+// widened as the build's, so no pair within the cutoff is lost) and a ballot
+// to pack the codes.  The passes then walk the entries near the cutoff alone.
+static __global__ void __launch_bounds__(NB_THREADS) nbr_cut_kernel(ForceArgs A, float rc2b) {
+  const int a = (blockIdx.x * NB_THREADS + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (a >= A.ntot) return;
+  const int slot = A.atom_slot[a], b = slot >> 6, idi = A.s.id[slot];
+  const int n = A.pl.vcount[idi];
+  if (n > A.pl.vcap) {  // overflowed skin list: the passes scan the stencil
+    if (lane == 0) A.nbr_n[a] = A.cap + 1;
+    return;
   }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned lt = (1u << lane) - 1u;
-  for (int i = warp; i < ni; i += NB_THREADS / 32) {
-    double xi, yi, zi;
-    PrecT<double>::pos(A.s, b * CG_MAXATOMS + i, xi, yi, zi);
-    if (MODE != LIST_ID && A.box_start[b] + i >= A.ntot) break;  // only after an overflow
-    const int row = (lane == 0) ? build_row<MODE>(A, b, i) : 0;
-    const int a = __shfl_sync(0xffffffffu, row, 0);
-    const int cap = build_cap<MODE>(A);
-    int cnt = 0;
-    for (int c0 = 0; c0 < ncand; c0 += 32) {
-      const int c = c0 + lane;
-      bool hit = false;
-      uint16_t code = 0;
-      if (c < ncand) {
-        code = cc[c];
-        int e = code >> 6, k = code & 63;
-        double dx, dy, dz;
-        double r2 = pair_r2_ref(s_dr[e], xi, yi, zi, cx[c], cy[c], cz[c], dx, dy, dz);
-        hit = (r2 <= rc2) && !(s_box[e] == b && k == i);
+  const float4 pi = __ldg(A.s.pos32 + slot);
+  const int *lst = A.pl.vlist + (size_t)idi * A.pl.vcap;
+  uint16_t *out = A.nbr + (size_t)a * A.cap;
+  int cnt = 0;
+  for (int t0 = 0; t0 < n; t0 += 32) {
+    bool hit = false;
+    uint32_t code = 0;
+    if (t0 + lane < n) {
+      const int js = __ldg(A.pl.slot_of + __ldg(lst + t0 + lane));
+      const int e = stencil_entry(A.g, b, js >> 6);
+      if (e >= 0) {
+        const float4 q = __ldg(A.s.pos32 + js);
+        float dx, dy, dz;
+        hit = pair_r2(PrecT<float>::drbox(A.et, b * CG_NNBR + e), pi.x, pi.y, pi.z, q.x, q.y, q.z,
+                      dx, dy, dz) <= rc2b;
+        code = (e << 6) | (js & 63);
       }
-      const unsigned m = __ballot_sync(0xffffffffu, hit);
-      const int pos = cnt + __popc(m & lt);
-      if (hit && pos < cap)
-        build_store<MODE>(A, a, pos,
-                             MODE == LIST_ID ? A.s.id[s_box[code >> 6] * CG_MAXATOMS + (code & 63)]
-                                     : (int)code);
-      cnt += __popc(m);
     }
-    if (lane == 0) build_count<MODE>(A, a, cnt);
+    const uint32_t m = __ballot_sync(0xffffffffu, hit);
+    const int pos = cnt + __popc(m & ((1u << lane) - 1u));
+    if (hit && pos < A.cap) out[pos] = (uint16_t)code;
+    cnt += __popc(m);
+  }
+  if (lane == 0) {
+    A.nbr_n[a] = cnt;
+    if (cnt > A.cap) atomicAdd(A.status + ST_NBR_OVERFLOW, 1);
   }
 }
 
@@ -635,6 +566,7 @@ struct EamPot {
   PairSeg seg;     // FP32 Chebyshev only
   PolyTables poly; // FP64 Chebyshev only
   T rc2;
+  bool same_grid;  // the tables of phi and rho have the same intervals
 };
 
 template <int EVAL>
@@ -653,12 +585,7 @@ __device__ __forceinline__ float cheb_series(const EamPot<float, EVAL> &P, int s
   return cheb_low32(P.chlo, s, x);
 }
 
-// r and 1/r from r^2: FP64 as the reference (sqrt, then divide); FP32 from
-// rsqrt refined by one Newton step (about 1 ulp)
-__device__ __forceinline__ void r_and_inv(double r2, double &r, double &inv) {
-  r = sqrt(r2);
-  inv = 1.0 / r;
-}
+// r and 1/r from r^2: rsqrt refined by one Newton step (about 1 ulp)
 __device__ __forceinline__ void r_and_inv(float r2, float &r, float &inv) {
   float y = rsqrtf(r2);
   y = y * fmaf(-0.5f * r2, y * y, 1.5f);
@@ -943,10 +870,11 @@ __global__ void __launch_bounds__(PASS_THREADS)
     Pass1Acc<T> acc;
     acc.zero();
     eam_pass1_sum(P, seg_sm, acc, [&](auto &&fn) {
-      for_each_neighbor<T, false, true>(A, a, b, i, xi, yi, zi, P.rc2,
+      for_each_neighbor<T>(A, a, b, i, xi, yi, zi, P.rc2,
                                         [&](int, T dx, T dy, T dz, T r2) { fn(T(0), dx, dy, dz, r2); });
     });
     eam_pass1_store(A, P, acc, slot);
+    A.npair[a] = acc.cnt;
   }
 }
 
@@ -1271,7 +1199,7 @@ __device__ __forceinline__ void fo_density_store(const ForceArgs &A,
   A.s.fi32[slot] = dF;
   A.fo.pf[a] = make_float4(pi.x, pi.y, pi.z, dF);
   A.fo.ncut[a] = ncut;
-  A.nbr_n[a] = cnt;
+  A.npair[a] = cnt;
 }
 
 #ifdef COMDGB_FO1_MAXNREG  // sweep variant: a register cap instead of the launch bound
@@ -1491,8 +1419,10 @@ __global__ void __launch_bounds__(128) lj_pass_kernel(ForceArgs A, LjPot<T> P) {
   fx.zero(); fy.zero(); fz.zero(); ep.zero(); sx.zero();
   const T s6 = P.s6, s12 = P.s6x12, c4 = P.eps4s6;
   const T rc2 = P.rc2;
+  int cnt = 0;
   auto fn = [&](int js, T dx, T dy, T dz, T r2) {
     if (r2 > rc2) return;
+    cnt++;
     T ir2 = T(1.0) / r2;
     T r6 = ir2 * ir2 * ir2;
     ep.add(T(0.5) * r6 * (s6 * r6 - T(1.0)));
@@ -1502,7 +1432,7 @@ __global__ void __launch_bounds__(128) lj_pass_kernel(ForceArgs A, LjPot<T> P) {
     fz.add(dz * fr);
     sx.add(fr * dx * dx);
   };
-  for_each_neighbor<T, false, true>(A, a, b, i, xi, yi, zi, rc2, fn);
+  for_each_neighbor<T>(A, a, b, i, xi, yi, zi, rc2, fn);
   // kinetic term: -p_x^2/m per non-empty stencil entry
   int ne = A.et.n[b], nonempty = 0;
   for (int e = 0; e < ne; e++) nonempty += A.s.natoms[A.et.box[b * CG_NNBR + e]] > 0;
@@ -1515,6 +1445,7 @@ __global__ void __launch_bounds__(128) lj_pass_kernel(ForceArgs A, LjPot<T> P) {
   fo.w = ep.value();
   A.s.f[slot] = fo;
   A.atom_stress[a] = sx.value() - (double)nonempty * kin;
+  A.npair[a] = cnt;
 }
 
 // LJ in force order (mixed precision, persistent lists)
@@ -1557,7 +1488,7 @@ __global__ void __launch_bounds__(PASS_THREADS) fo_lj_kernel(ForceArgs A, LjPot<
       double kin = __ddiv_rn(__dmul_rn(p.x, p.x), A.s.mass[slot]);
       A.atom_stress[a] = sx.value() - (double)nonempty * kin;
     }
-    A.nbr_n[a] = cnt;
+    A.npair[a] = cnt;
   }
 }
 

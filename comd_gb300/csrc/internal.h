@@ -97,6 +97,8 @@ void launch_zc_upload(const HostSlots &hs, Slots s, int nboxes, bool forces, cud
 void launch_zc_download(const HostSlots &hs, Slots s, int nboxes, bool state, bool forces,
                         cudaStream_t st, int max_blocks = 0);
 void launch_pos32(const Geom &g, Slots s, cudaStream_t st, const int *only_if_overflow = nullptr);
+// the same over the atom list alone
+void launch_pos32_atoms(const Geom &g, Slots s, const int *atom_slot, int ntot, cudaStream_t st);
 void launch_bin_atoms(const Geom &g, const double *dcenter, Slots s, int n, const double *xyz,
                       const double *pxyz, const int *ids, const int *types, const double *masses,
                       int *tmp_index, int *status, cudaStream_t st);
@@ -130,17 +132,24 @@ struct Tune {
   int pass2_blocks_fast = 0;  // the same for the force pass without energies (OBS = false)
 };
 
-// ---- force_fp64.cu (T = double) / force_mixed.cu (T = float) ----
-template <class T>
+// ---- force_mixed.cu ----
 cudaError_t prepare_force_kernels();
-template <class T>
-void launch_nbr_build(const ForceArgs &A, T rc2, cudaStream_t st, const Tune *tune = nullptr);
+// the list build of the list mode (force order, id-keyed or per step), from
+// the FP32 positions pos32: every pair within rc2b (widened, list_cutoff)
+void launch_nbr_build(const ForceArgs &A, float rc2b, cudaStream_t st, const Tune *tune = nullptr);
+// id-keyed lists: the per-step list out of them
+void launch_nbr_cut(const ForceArgs &A, float rc2b, cudaStream_t st);
 template <class T, int EVAL>
 void launch_eam_pass1(const ForceArgs &A, const EamPot<T, EVAL> &P, cudaStream_t st);
 template <class T, int EVAL>
 void launch_eam_pass2(const ForceArgs &A, const EamPot<T, EVAL> &P, cudaStream_t st);
 template <class T>
 void launch_lj(const ForceArgs &A, const LjPot<T> &P, cudaStream_t st);
+// ---- force_fp64.cu: pass 0 (density) or 1 (forces); obs as below ----
+template <int EVAL>
+void launch_eam64(const ForceArgs &A, const EamPot<double, EVAL> &P, int pass, cudaStream_t st,
+                  bool obs);
+void launch_lj64(const ForceArgs &A, const LjPot<double> &P, cudaStream_t st, bool obs);
 // force order (mixed precision only, force_mixed.cu); pass 0 or 1.  obs:
 // the caller can read this force call's energies, stress, rho and F' (else
 // forces only: the force calls inside a step sequence)

@@ -860,7 +860,7 @@ __global__ void __launch_bounds__(RD_THREADS) reduce_force_kernel(ForceArgs A, d
     if (a < A.ntot) {
       e += A.s.f[A.atom_slot[a]].w;
       sx += A.atom_stress[a];
-      np += A.nbr_n[a];
+      np += A.npair[a];
     }
   }
   e = block_sum_d(e, shd);
@@ -1099,6 +1099,19 @@ __global__ void pos32_kernel(Geom g, Slots s, const int *only_if_overflow) {
 
 void launch_pos32(const Geom &g, Slots s, cudaStream_t st, const int *only_if_overflow) {
   pos32_kernel<<<slot_blocks(g), 256, 0, st>>>(g, s, only_if_overflow);
+}
+
+__global__ void __launch_bounds__(256) pos32_atoms_kernel(Geom g, Slots s, const int *atom_slot,
+                                                          int ntot) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a >= ntot) return;
+  const int slot = atom_slot[a];
+  const d4 r = s.r[slot];
+  s.pos32[slot] = centred32(rep_of(g, slot >> 6), r.x, r.y, r.z);
+}
+
+void launch_pos32_atoms(const Geom &g, Slots s, const int *atom_slot, int ntot, cudaStream_t st) {
+  if (ntot > 0) pos32_atoms_kernel<<<atom_blocks(ntot), 256, 0, st>>>(g, s, atom_slot, ntot);
 }
 
 // ---------------------------------------------------------------------------

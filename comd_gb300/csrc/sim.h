@@ -73,7 +73,7 @@ struct comdgb_sim {
   int *box_start = nullptr, *atom_slot = nullptr, *cpart = nullptr;
   int ncpart = 0;
   uint16_t *nbr = nullptr;
-  int *nbr_n = nullptr;
+  int *nbr_n = nullptr, *npair = nullptr;
   int cap = 0;
   // list capacities as allocated (comdgb_sim_set_list_capacity may lower the
   // capacity in use): per-step, id-keyed and force-order lists
