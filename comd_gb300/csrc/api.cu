@@ -52,12 +52,12 @@ enum { KGM_ADV_VPP, KGM_REBIN, KGM_COMPACT, KGM_NBR, KGM_PASS1, KGM_PASS2, KGM_C
 const char *kGroupNameMerged[KGM_COUNT] = {"advance_velocity_positions+classify",
                                            "rebin_plan_apply", "compact_atoms", "nbr_build",
                                            "force_pass1", "force_pass2"};
-// the middle part of a force-order sequence: the rebuild section (classify,
-// rebin, compact, list build) is one conditional graph node, and the force
-// pass ends with the velocity-Verlet update of the step boundary
-enum { KGF_REBUILD, KGF_PASS1, KGF_PASS2, KGF_COUNT };
-const char *kGroupNameFo[KGF_COUNT] = {"rebuild_if_due", "force_pass1",
-                                       "force_pass2+advance_velocity_positions"};
+// the middle part of a force-order sequence: the force pass ends with the
+// velocity-Verlet update of the step boundary, and the rebuild section that
+// may follow (classify, rebin, compact, list build) is one conditional node
+enum { KGF_PASS1, KGF_PASS2, KGF_REBUILD, KGF_COUNT };
+const char *kGroupNameFo[KGF_COUNT] = {"force_pass1", "force_pass2+advance_velocity_positions",
+                                       "rebuild_if_due"};
 
 }  // namespace
 
@@ -82,6 +82,7 @@ ForceArgs force_args(comdgb_sim *h) {
   A.pl = h->pl;
   A.fo = h->fo;
   A.vv_dt = A.vv_c = 0.0;
+  A.cond = 0;
   A.host_f = A.host_rho = A.host_fi = nullptr;
   return A;
 }
@@ -765,15 +766,10 @@ void enqueue_force_parts(comdgb_sim *h, cudaEvent_t *ev, int &evi, bool obs = tr
 
 int count_kernel_nodes(cudaGraph_t graph);
 
-// Under stream capture of h->stream: a kernel that sets a new conditional
-// handle to "status word `word` is set" (word < 0: the end of a possible
-// rebuild and "a current list overflowed", rebuild_done_cond_kernel), then
-// an IF node after it whose body is captured on h->cond_stream until
-// cond_end.  Returns that stream, or nullptr when h->stream is not capturing
-// or the node cannot be made (the caller then enqueues the body on
-// h->stream, where its kernels stand down by themselves; with word < 0 it
-// also launches rebuild_done itself).
-cudaStream_t cond_begin(comdgb_sim *h, int word) {
+// Under stream capture of h->stream: a new conditional handle of the graph
+// being captured, 0 at every launch until a kernel sets it; 0 when h->stream
+// is not capturing or there is none.
+cudaGraphConditionalHandle cond_handle(comdgb_sim *h) {
   // COMDGB_GRAPH_CONDITIONALS=0: no conditional nodes (the sections stand
   // down by themselves instead).  ncu profiles no kernel of a graph that
   // holds a conditional node, so the launch lists are taken with this set.
@@ -781,26 +777,33 @@ cudaStream_t cond_begin(comdgb_sim *h, int word) {
     const char *e = getenv("COMDGB_GRAPH_CONDITIONALS");
     return e && e[0] == '0';
   }();
-  if (off) return nullptr;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  if (off || !h->cond_stream ||
+      cudaStreamGetCaptureInfo(h->stream, &cs, nullptr, &graph, nullptr, nullptr, nullptr) !=
+          cudaSuccess ||
+      cs != cudaStreamCaptureStatusActive)
+    return 0;
+  cudaGraphConditionalHandle cond = 0;
+  if (cudaGraphConditionalHandleCreate(&cond, graph, 0, cudaGraphCondAssignDefault) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return cond;
+}
+
+// An IF node on `cond` after what h->stream has captured so far, its body
+// captured on h->cond_stream until cond_end.  Returns that stream, or nullptr
+// when there is no handle or no node (the caller then enqueues the body on
+// h->stream, where its kernels stand down by themselves).
+cudaStream_t cond_begin(comdgb_sim *h, cudaGraphConditionalHandle cond) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   cudaGraph_t graph = nullptr;
   const cudaGraphNode_t *deps = nullptr;
   size_t nd = 0;
-  if (!h->cond_stream ||
-      cudaStreamGetCaptureInfo(h->stream, &cs, nullptr, &graph, &deps, nullptr, &nd) !=
-          cudaSuccess ||
-      cs != cudaStreamCaptureStatusActive)
-    return nullptr;
-  cudaGraphConditionalHandle cond;
-  if (cudaGraphConditionalHandleCreate(&cond, graph, 0, cudaGraphCondAssignDefault) !=
-      cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  if (word < 0) launch_rebuild_done_cond(h->status, cond, h->stream);
-  else launch_status_cond(cond, h->status, word, h->stream);
-  if (cudaStreamGetCaptureInfo(h->stream, &cs, nullptr, &graph, &deps, nullptr, &nd) !=
-      cudaSuccess)
+  if (!cond || cudaStreamGetCaptureInfo(h->stream, &cs, nullptr, &graph, &deps, nullptr, &nd) !=
+                   cudaSuccess)
     return nullptr;
   std::vector<cudaGraphNode_t> dv(deps, deps + nd);
   cudaGraphNodeParams p{};
@@ -838,37 +841,41 @@ void set_fuse(comdgb_sim *h, bool on, cudaStream_t st = nullptr) {
     cudaMemsetAsync(h->status + ST_FUSE, on ? 1 : 0, sizeof(int), st ? st : h->stream);
 }
 
-// The force call of a force-order step part (OPEN or MID, mixed precision):
-// the rebuild section -- classify, rebin, compact and the list build, all
-// needed only when an atom moved more than skin/2 since the build -- as the
-// body of a conditional node; the slot-order FP32 copy refreshed (another
-// conditional node) when a list overflowed, since only the stencil scan of
-// an overflowed list reads it and the fused update does not keep it; then
-// the passes without energies, the force pass with the update of the step
-// boundary when ST_FUSE is set (dt_atu: the step).  ev: events after the
-// rebuild section and after each pass.
-void enqueue_fo_step_force(comdgb_sim *h, double dt_atu, cudaEvent_t *ev, int &evi) {
+// What follows an update of the positions inside a force-order sequence, as
+// the body of a conditional node that the update's kernel sets: classify,
+// rebin, compact and the list build, all needed only when an atom moved more
+// than skin/2 since the build, and the slot-order FP32 copy refreshed when a
+// list overflowed (only the stencil scan of an overflowed list reads it, and
+// the fused update does not keep it).  Set by the update itself, the node
+// costs a middle step of 4,000 atoms 6 us; with a kernel before it to read
+// the status word, and a second pair for the overflow, it was 18.3 us.
+void enqueue_rebuild(comdgb_sim *h, cudaGraphConditionalHandle cond) {
   ForceArgs A = force_args(h);
-  A.vv_dt = dt_atu;
-  const double dt_r = dt_atu / 2.0;
-  A.vv_c = 2.0 * dt_r / h->rmass;  // both half steps, as one multiply-add
-  cudaStream_t st = h->stream;
-  cudaStream_t bs = cond_begin(h, ST_REBUILD);
-  cudaStream_t rs = bs ? bs : st;
+  cudaStream_t bs = cond_begin(h, cond);
+  cudaStream_t rs = bs ? bs : h->stream;
   cudaMemsetAsync(h->status + ST_REBIN_SERIAL, 0, sizeof(int), rs);
   launch_classify(h->g, h->s, h->atom_slot, h->ntot, h->mixed, h->w, h->status, rs, h->status);
   launch_rebin_finish(h->g, h->s, h->mixed, h->w, h->status, rs, h->status);
   launch_compact(h->g, h->s.natoms, h->box_start, h->atom_slot, h->ntot, h->cpart, h->ncpart,
                  rs, h->status);
-  const double rcl = h->cutoff + h->skin;
-  launch_nbr_build(A, list_cutoff(h, rcl), rs, &h->tune);
-  if (bs) h->rebuild_kernels = cond_end(h);
+  launch_nbr_build(A, list_cutoff(h, h->cutoff + h->skin), rs, &h->tune);
   // (mixed precision keeps no position increments in f: ST_DELTA stays 0)
-  cudaStream_t os = cond_begin(h, -1);
-  if (!os) launch_rebuild_done(h->status, st);
-  launch_pos32(h->g, h->s, os ? os : st, h->status);
-  if (os) h->overflow_kernels = cond_end(h);
-  if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
+  launch_rebuild_done(h->status, rs);
+  launch_pos32(h->g, h->s, rs, h->status);
+  if (bs) h->rebuild_kernels = cond_end(h);
+}
+
+// The force call of a force-order step part (OPEN or MID, mixed precision):
+// the passes without energies, the force pass with the update of the step
+// boundary when ST_FUSE is set (dt_atu: the step), and the rebuild section
+// for the next part.  ev: events after each pass and after that section.
+void enqueue_fo_step_force(comdgb_sim *h, double dt_atu, cudaEvent_t *ev, int &evi) {
+  ForceArgs A = force_args(h);
+  A.vv_dt = dt_atu;
+  const double dt_r = dt_atu / 2.0;
+  A.vv_c = 2.0 * dt_r / h->rmass;  // both half steps, as one multiply-add
+  A.cond = cond_handle(h);
+  cudaStream_t st = h->stream;
   const int pot = h->opts.potential;
   if (pot == COMDGB_POT_LJ) {
     launch_fo_lj(A, h->lj32, st, false);
@@ -882,6 +889,8 @@ void enqueue_fo_step_force(comdgb_sim *h, double dt_atu, cudaEvent_t *ev, int &e
     if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
     launch_fo_eam<EVAL_CHEBY>(A, h->eam32c, 1, st, &h->tune, false);
   }
+  if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
+  enqueue_rebuild(h, A.cond);
   if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
 }
 
@@ -922,11 +931,15 @@ void enqueue_step(comdgb_sim *h, double dt_atu, cudaEvent_t *ev, int part) {
   if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
   if (lazy) {
     // force order: the opening position half step; a middle part's update
-    // was made by the force pass before it (ST_FUSE); the classification,
-    // rebox and list build only when a rebuild is due
-    if (part == PART_OPEN)
+    // was made by the force pass before it (ST_FUSE); after either the
+    // classification, rebox and list build only when a rebuild is due
+    if (part == PART_OPEN) {
+      RebinWork w = h->w;
+      w.cond = cond_handle(h);
       launch_advance_positions(h->g, h->s, h->atom_slot, h->ntot, dt_atu / 2.0, h->rmass,
-                               h->mixed, false, h->w, h->status, st, true);
+                               h->mixed, false, w, h->status, st, true);
+      enqueue_rebuild(h, w.cond);
+    }
     enqueue_fo_step_force(h, dt_atu, ev, evi);
     return;
   }

@@ -203,8 +203,12 @@ struct ForceOrder {
 // build box centre -- p32 itself while the atom is in its build box, else
 // RN(r - boxsize/2 + (b - build box) * boxsize), one rounding either way --
 // and the rebuild test on its displacement since the build.
+// A step part's rebuild section is the body of a conditional graph node whose
+// handle `cond` (0: none) starts each launch at 0: the first atom to set
+// ST_REBUILD sets it (see also cond_pending).
 __device__ __forceinline__ void fo_track_at(const Geom &g, const ForceOrder &fo, int b, int af,
-                                            const d4 &r, float4 p32, int *status) {
+                                            const d4 &r, float4 p32, int *status,
+                                            cudaGraphConditionalHandle cond) {
   const float4 q = fo.ref[af];
   const RepGeo &R = rep_of(g, b);
   int ixn[3], ixb[3];
@@ -228,8 +232,17 @@ __device__ __forceinline__ void fo_track_at(const Geom &g, const ForceOrder &fo,
     const float d = pv[k] - qv[k];
     d2 = fmaf(d, d, d2);
   }
-  if (far || !(d2 <= fo.half_skin2)) atomicExch(status + ST_REBUILD, 1);
+  if ((far || !(d2 <= fo.half_skin2)) && atomicExch(status + ST_REBUILD, 1) == 0 && cond)
+    cudaGraphSetConditional(cond, 1);
   fo.pos[af] = make_float4(pv[0], pv[1], pv[2], 0.f);
+}
+// What the atoms' own tests do not announce: a rebuild that was due already,
+// or lists that overflowed, whose stencil scans need the slot-order FP32 copy
+// refreshed after every update.  One thread of the kernel that moves the atoms.
+__device__ __forceinline__ void cond_pending(cudaGraphConditionalHandle cond, const int *status) {
+  if (cond && (*(volatile const int *)(status + ST_REBUILD) ||
+               *(volatile const int *)(status + ST_NBR_OVERFLOW)))
+    cudaGraphSetConditional(cond, 1);
 }
 // the slot of an atom moved by the rebin, in the maps the list mode keeps
 struct SlotMap {

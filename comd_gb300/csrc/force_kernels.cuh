@@ -46,6 +46,7 @@ struct ForceArgs {
   // force order, a step sequence: the velocity-Verlet coefficients of the
   // update the force pass makes when ST_FUSE is set (p -= vv_dt f, r += vv_c p)
   double vv_dt, vv_c;
+  cudaGraphConditionalHandle cond;  // the rebuild section that follows that update (0: none)
   // force order, a force call whose results go straight to an attached host
   // simflat_t (device pointers of its registered f, rho, fi; slot-indexed),
   // or null
@@ -1328,8 +1329,10 @@ __device__ __forceinline__ void fo_force_end(const ForceArgs &A, int a, int slot
   r.y = fma(p.y, A.vv_c, r.y);
   r.z = fma(p.z, A.vv_c, r.z);
   A.s.r[slot] = r;
+  if (a == 0) cond_pending(A.cond, A.status);
   const int b = slot >> 6;
-  fo_track_at(A.g, A.fo, b, a, r, centred32(rep_of(A.g, b), r.x, r.y, r.z), A.status);
+  fo_track_at(A.g, A.fo, b, a, r, centred32(rep_of(A.g, b), r.x, r.y, r.z), A.status,
+              A.cond);
 }
 
 // Force pass: f_i = sum over the cut list of (phi'(r) + (F'_i + F'_j)

@@ -181,9 +181,10 @@ __device__ __forceinline__ double div_mass(double a, double rmass, double rinv) 
 // fo_track_at for atom id (before the first build, no force-order number:
 // a rebuild is due anyway)
 __device__ __forceinline__ void fo_track(const Geom &g, const ForceOrder &fo, int b, int id,
-                                         const d4 &r, float4 p32, int *status) {
+                                         const d4 &r, float4 p32, int *status,
+                                         cudaGraphConditionalHandle cond) {
   const int af = fo.of_id[id];
-  if (af >= 0) fo_track_at(g, fo, b, af, r, p32, status);
+  if (af >= 0) fo_track_at(g, fo, b, af, r, p32, status, cond);
 }
 
 // delta: the two position half steps around a step boundary add the same
@@ -205,6 +206,7 @@ __global__ void __launch_bounds__(256) advance_kernel(Geom g, Slots s, const int
                                                       int *status) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= ntot) return;
+  if (POS && a == 0) cond_pending(w.cond, status);
   const int slot = atom_slot[a];
   const int b = slot >> 6;
   d4 r = s.r[slot];
@@ -281,7 +283,7 @@ __global__ void __launch_bounds__(256) advance_kernel(Geom g, Slots s, const int
       // list reads the slot-order copy (the classification before a rebuild
       // rewrites it for every atom)
       if (!lazy32 || *(volatile const int *)(status + ST_NBR_OVERFLOW)) s.pos32[slot] = p32;
-      if (w.fo.of_id) fo_track(g, w.fo, b, s.id[slot], r, p32, status);
+      if (w.fo.of_id) fo_track(g, w.fo, b, s.id[slot], r, p32, status, w.cond);
     }
     if ((!VEL || twice) && w.pl.rref) {
       // persistent lists: the half step before a force call decides
@@ -636,7 +638,7 @@ __global__ void __launch_bounds__(256) fo_track_kernel(Geom g, Slots s, ForceOrd
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= ntot) return;
   const int slot = atom_slot[a];
-  fo_track(g, fo, slot >> 6, s.id[slot], s.r[slot], s.pos32[slot], status);
+  fo_track(g, fo, slot >> 6, s.id[slot], s.r[slot], s.pos32[slot], status, 0);
 }
 
 void launch_fo_track(const Geom &g, Slots s, const ForceOrder &fo, const int *atom_slot,
@@ -663,30 +665,6 @@ void launch_skin_check(const Geom &g, Slots s, Persist pl, bool mixed, int *stat
 
 void launch_rebuild_done(int *status, cudaStream_t st) {
   rebuild_done_kernel<<<1, 1, 0, st>>>(status);
-}
-
-// rebuild_done_kernel, then the condition of a conditional graph node: some
-// list of the current lists overflowed
-__global__ void rebuild_done_cond_kernel(int *status, cudaGraphConditionalHandle cond) {
-  if (status[ST_REBUILD]) {
-    status[ST_REBUILDS] += 1;
-    status[ST_REBUILD] = 0;
-    status[ST_NBR_OVERFLOW] = status[ST_OVF_BUILD];
-    status[ST_OVF_BUILD] = 0;
-  }
-  cudaGraphSetConditional(cond, status[ST_NBR_OVERFLOW] != 0 ? 1u : 0u);
-}
-void launch_rebuild_done_cond(int *status, cudaGraphConditionalHandle cond, cudaStream_t st) {
-  rebuild_done_cond_kernel<<<1, 1, 0, st>>>(status, cond);
-}
-
-// the condition of a conditional graph node: status word `word` is set
-__global__ void status_cond_kernel(cudaGraphConditionalHandle cond, const int *status, int word) {
-  cudaGraphSetConditional(cond, *(volatile const int *)(status + word) != 0 ? 1u : 0u);
-}
-void launch_status_cond(cudaGraphConditionalHandle cond, const int *status, int word,
-                        cudaStream_t st) {
-  status_cond_kernel<<<1, 1, 0, st>>>(cond, status, word);
 }
 
 // ---------------------------------------------------------------------------

@@ -159,7 +159,6 @@ struct comdgb_sim {
   // cond_stream; its kernel nodes run only in steps that rebuild
   cudaStream_t cond_stream = nullptr;
   int rebuild_kernels = 0;
-  int overflow_kernels = 0;  // the slot-order copy's refresh after a list overflow
   std::string trace_note;    // phases of the last drop-in call (COMDGB_TRACE_CALLS)
   // host last results
   double e = 0.0, stress = 0.0;
