@@ -529,6 +529,36 @@ int fit_cheb_gpu(comdgb_sim *h, const eampotential_t *pot, double coef[6][CG_NCH
   return 0;
 }
 
+// the tables of phi and rho (the same intervals) as FoTab
+FoTab build_fotab(comdgb_sim *h, const potentialarray_t *phi, const potentialarray_t *rho,
+                  int *err) {
+  const int n = phi->n;
+  std::vector<float4> v(3 * (size_t)n);
+  auto value = [&](const potentialarray_t *a, int i) {
+    const double *w = a->values;
+    return make_float4((float)w[i], (float)(0.5 * (w[i + 1] - w[i - 1])),
+                       (float)(0.5 * (w[i + 1] + w[i - 1] - 2.0 * w[i])), 0.f);
+  };
+  auto deriv = [&](const potentialarray_t *a, int i, float *d) {
+    const double *w = a->values;
+    const double gi = w[i + 1] - w[i - 1], gi1 = w[i + 2] - w[i];
+    d[0] = i <= 0 ? 0.f : (float)(0.5 * gi * a->invDx);
+    d[1] = i <= 0 ? 0.f : (float)(0.5 * (gi1 - gi) * a->invDx);
+  };
+  for (int i = 0; i < n; i++) {
+    float d[4];
+    deriv(phi, i, d);
+    deriv(rho, i, d + 2);
+    v[i] = value(rho, i);
+    v[(size_t)n + i] = value(phi, i);
+    v[2 * (size_t)n + i] = make_float4(d[0], d[1], d[2], d[3]);
+  }
+  float4 *p = track(h, dalloc<float4>(v.size(), err));
+  if (*err) return FoTab{};
+  cudaMemcpy(p, v.data(), sizeof(float4) * v.size(), cudaMemcpyHostToDevice);
+  return FoTab{p, p + n, p + 2 * (size_t)n, (float)phi->x0, (float)phi->xn, (float)phi->invDx, n};
+}
+
 int setup_potential(comdgb_sim *h, const simflat_t *s) {
   int err = 0;
   const comdgb_opts &o = h->opts;
@@ -555,6 +585,8 @@ int setup_potential(comdgb_sim *h, const simflat_t *s) {
     h->eam32t.rho = upload_table<float>(h, ep->rho, &err);
     h->eam32t.f = upload_table<float>(h, ep->f, &err);
     h->eam32t.rc2 = (float)rc2;
+    if (h->mixed && h->eam64t.same_grid && ep->phi->n <= FOTAB_MAX)
+      h->eam32t.tab = build_fotab(h, ep->phi, ep->rho, &err);
     if (err) return set_err(COMDGB_ERR_NOMEM, "cudaMalloc failed for EAM tables");
     return 0;
   }

@@ -315,6 +315,18 @@ struct Table {
   T off, umax;
 };
 
+// The FP32 tables of phi and rho as the force-order passes read them, one
+// 16-byte record per interval: rho and phi (c0, c1, c2, -), and the
+// derivatives of both (phi d0, phi d1, rho d0, rho d1), the coefficients of
+// Table::seg.  Only when the two tables have the same intervals and at most
+// FOTAB_MAX of them (64 KB staged); n = 0 otherwise.
+constexpr int FOTAB_MAX = 4096;
+struct FoTab {
+  const float4 *rho, *phi, *der;
+  float x0, xn, invDx;
+  int n;
+};
+
 // Chebyshev series of the reference: 0 phi, 1 rho, 2 F, 3 dphi, 4 drho, 5 dF
 template <class T>
 struct Cheb {

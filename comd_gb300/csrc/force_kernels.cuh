@@ -566,6 +566,7 @@ struct EamPot {
   ChebLow32 chlo;  // FP32 only
   PairSeg seg;     // FP32 Chebyshev only
   PolyTables poly; // FP64 Chebyshev only
+  FoTab tab;       // FP32 tables only
   T rc2;
   bool same_grid;  // the tables of phi and rho have the same intervals
 };
@@ -784,14 +785,6 @@ __device__ __forceinline__ void stage_seg(float4 *sm, const float4 *src, int nre
   __syncthreads();
 }
 
-// the density pass's rho table (nrec cubics from src) as RHO_COPIES
-// interleaved copies: record q of the shared array is segment q / RHO_COPIES
-__device__ __forceinline__ void stage_rho_copies(float4 *sm, const float4 *src, int nrec) {
-  for (int q = threadIdx.x; q < nrec * RHO_COPIES; q += blockDim.x)
-    sm[q] = __ldg(src + q / RHO_COPIES);
-  __syncthreads();
-}
-
 // ---------------------------------------------------------------------------
 // EAM pass 1: density, pair energy and pair force of one atom.  `visit`
 // runs the atom's neighbour traversal with a pair functor.
@@ -980,6 +973,7 @@ constexpr int FO1_THREADS = 512;  // pass 1 (density): 2 CTAs of 64 registers pe
 #endif
 constexpr int FO_PREFETCH = COMDGB_FO_PREFETCH;
 constexpr int FO1_UNROLL = COMDGB_FO1_UNROLL, FO2_UNROLL = COMDGB_FO2_UNROLL;
+constexpr int FO1_BATCH = 4, FO2_BATCH = 4;  // entries loaded before the first is used
 
 __device__ __forceinline__ void prefetch_l1(const void *p) {
   asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
@@ -1043,16 +1037,40 @@ __device__ __forceinline__ void fo_walk(const ForceArgs &A, const uint32_t *list
   const FoFrame fr = fo_frame<MULTI>(A, slot);
   const uint32_t *lst = list + fo_row(a, A.fo.vcap);
   const float4 *pj = NEED_FI ? A.fo.pf : A.fo.pos;
-  // the warp's list lines stream from HBM: pull line t + FO_PREFETCH into L1
-  // while line t is used (within this atom's list only)
+  if constexpr (NEED_FI) {
+    // the force pass: a batch's entries and gathers before its first pair (at
+    // 4M atoms, 4 a batch: 575 us against 604 unrolled by two with the
+    // Chebyshev tables, 650 against 895 with the table potential; 2 a batch
+    // 660 and 742, 6 a batch 627 and 672)
+    for (int t0 = 0; t0 < n; t0 += FO2_BATCH) {
+      uint32_t p[FO2_BATCH];
+      float4 q[FO2_BATCH];
+#pragma unroll
+      for (int u = 0; u < FO2_BATCH; u++) {
+        if (t0 + u + FO_PREFETCH < n) prefetch_l1(lst + (size_t)(t0 + u + FO_PREFETCH) * 32);
+        p[u] = __ldg(lst + (size_t)min(t0 + u, n - 1) * 32);
+      }
+#pragma unroll
+      for (int u = 0; u < FO2_BATCH; u++) q[u] = __ldg(pj + (p[u] >> 6));
+#pragma unroll
+      for (int u = 0; u < FO2_BATCH; u++) {
+        float dx, dy, dz;
+        const float r2 = fo_dr(fr, p[u], pi, q[u], dx, dy, dz);
+        if (t0 + u < n) fn(q[u].w, dx, dy, dz, r2);
+      }
+    }
+  } else {
+    // the warp's list lines stream from HBM: pull line t + FO_PREFETCH into L1
+    // while line t is used (within this atom's list only)
 #pragma unroll UNROLL
-  for (int t = 0; t < n; t++) {
-    if (t + FO_PREFETCH < n) prefetch_l1(lst + (size_t)(t + FO_PREFETCH) * 32);
-    const uint32_t p = __ldg(lst + (size_t)t * 32);
-    const float4 q = __ldg(pj + (p >> 6));
-    float dx, dy, dz;
-    const float r2 = fo_dr(fr, p, pi, q, dx, dy, dz);
-    fn(q.w, dx, dy, dz, r2);
+    for (int t = 0; t < n; t++) {
+      if (t + FO_PREFETCH < n) prefetch_l1(lst + (size_t)(t + FO_PREFETCH) * 32);
+      const uint32_t p = __ldg(lst + (size_t)t * 32);
+      const float4 q = __ldg(pj + (p >> 6));
+      float dx, dy, dz;
+      const float r2 = fo_dr(fr, p, pi, q, dx, dy, dz);
+      fn(q.w, dx, dy, dz, r2);
+    }
   }
 }
 
@@ -1074,31 +1092,90 @@ __device__ __forceinline__ void fo_for_each(const ForceArgs &A, int a, int slot,
 // and stress for r^2 < rc^2.
 // ---------------------------------------------------------------------------
 
-// rho(r) of one pair distance: the rho cubics of the FP32 pair table (sm),
-// or the table evaluator.  false: below the pair table (the series, in a
-// second sweep)
-template <int EVAL>
-__device__ __forceinline__ bool fo_rho(const EamPot<float, EVAL> &P, const float4 *, float r2,
-                                       float &rho) {
+// The passes' pair functions in shared memory, COPIES interleaved copies of
+// every record (record q of copy c at q * COPIES + c; lane l reads copy l mod
+// COPIES through `sm`, its own first record): the Chebyshev potential's
+// cubics (PairSeg), or the table potential's interval coefficients (FoTab:
+// one 16-byte record a pair, 48 KB for the 3,000 intervals of the Cu tables;
+// COPIES = 0 reads them from global memory, for CTAs too small to be worth
+// the staging).  At 282,000 atoms the table potential's passes took 88 + 97
+// us reading two 32-byte records a pair from global memory, 66 + 63 us so (with
+// the batched gathers).
+
+// density pass: rho
+template <int COPIES>
+__device__ __forceinline__ void stage_rho(float4 *sm, const EamPot<float, EVAL_CHEBY> &P) {
+  if (P.seg.n <= 0) return;
+  for (int q = threadIdx.x; q < P.seg.n1 * COPIES; q += blockDim.x)
+    sm[q] = __ldg(P.seg.rho1 + q / COPIES);
+  __syncthreads();
+}
+template <int COPIES>
+__device__ __forceinline__ void stage_rho(float4 *sm, const EamPot<float, EVAL_TABLE> &P) {
+  if (COPIES == 0 || P.tab.n <= 0) return;
+  for (int q = threadIdx.x; q < P.tab.n; q += blockDim.x) sm[q] = __ldg(P.tab.rho + q);
+  __syncthreads();
+}
+// force pass: phi'/r and rho'/r (Chebyshev: 2 n2 records, then with OBS the n
+// phi cubics, one copy), or phi' and rho' (table)
+template <int COPIES, bool OBS>
+__device__ __forceinline__ void stage_force(float4 *sm, const EamPot<float, EVAL_CHEBY> &P) {
+  const PairSeg &S = P.seg;
+  if (S.n <= 0) return;
+  const int m = 2 * S.n2 * COPIES;
+  for (int q = threadIdx.x; q < m; q += blockDim.x) sm[q] = __ldg(S.dcub + q / COPIES);
+  if (OBS)
+    for (int q = threadIdx.x; q < S.n; q += blockDim.x) sm[m + q] = __ldg(S.p1 + q);
+  __syncthreads();
+}
+template <int COPIES, bool OBS>
+__device__ __forceinline__ void stage_force(float4 *sm, const EamPot<float, EVAL_TABLE> &P) {
+  if (COPIES == 0 || P.tab.n <= 0) return;
+  for (int q = threadIdx.x; q < P.tab.n; q += blockDim.x) sm[q] = __ldg(P.tab.der + q);
+  __syncthreads();
+}
+// this lane's copy
+template <int EVAL, int COPIES>
+__device__ __forceinline__ const float4 *fo_copy(const float4 *sm) {
+  return EVAL == EVAL_CHEBY && COPIES > 1 ? sm + (threadIdx.x & (COPIES - 1)) : sm;
+}
+
+// interval and offset of r in the table, as table_eval
+__device__ __forceinline__ int fo_interval(const FoTab &t, float r, float &u) {
+  if (r < t.x0) r = t.x0;
+  else if (r > t.xn) r = t.xn;
+  const float v = (r - t.x0) * t.invDx, fl = floorf(v);
+  int i = (int)fl;
+  i = i < 0 ? 0 : (i > t.n - 1 ? t.n - 1 : i);
+  u = v - fl;
+  return i;
+}
+
+// rho(r) of one pair distance.  false: below the pair table (the series, in
+// a second sweep)
+template <int COPIES>
+static __device__ __forceinline__ bool fo_rho(const EamPot<float, EVAL_TABLE> &P,
+                                              const float4 *sm, float r2, float &rho) {
   float r, inv_r, v, d;
   r_and_inv(r2, r, inv_r);
-  if (EVAL == EVAL_CHEBY) {
-    rho = cheb_series(P, 1, r);
+  if (P.tab.n > 0) {
+    const int i = fo_interval(P.tab, r, v);
+    const float4 c = COPIES == 0 ? __ldg(P.tab.rho + i) : sm[i];
+    rho = fmaf(v, fmaf(v, c.z, c.y), c.x);
   } else {
-    table_eval(P.rho, r, v, d);
-    rho = v;
+    table_eval(P.rho, r, rho, d);
   }
   return true;
 }
-// (sm: this lane's copy of the density pass's rho table, n1 segments
-// RHO_COPIES records apart; the same lower end s_lo, so "below the table"
-// is below_seg's test)
+// (n1 segments of the same range as the force pass's table, so "below the
+// table" is below_seg's test)
+template <int COPIES>
 static __device__ __forceinline__ bool fo_rho(const EamPot<float, EVAL_CHEBY> &P,
                                               const float4 *sm, float r2, float &rho) {
   const float u = (r2 - P.seg.s_lo) * P.seg.inv_h1;
   if (!(u >= 0.f)) return false;
   const int k = min((int)u, P.seg.n1 - 1);
-  rho = seg_cubic(sm[k * RHO_COPIES], u - (float)k);
+  rho = seg_cubic(sm[k * COPIES], u - (float)k);
   return true;
 }
 template <int EVAL>
@@ -1111,20 +1188,23 @@ static __device__ __noinline__ float fo_rho_series(const EamPot<float, EVAL_CHEB
   return cheb_series(P, 1, r);
 }
 
-// phi (OBS only), phi'(r)/r and rho'(r)/r of one pair distance: the force
-// pass's tables (staged by stage_force_table: sm this lane's copy of the
-// derivative cubics, phi_sm the phi cubics), or the table evaluator.
-// false: below the pair table
-template <bool OBS, int EVAL>
-__device__ __forceinline__ bool fo_pair(const EamPot<float, EVAL> &P, const float4 *,
-                                        const float4 *, float r2, float &phi, float &wphi,
-                                        float &wrho) {
+// phi (OBS only), phi'(r)/r and rho'(r)/r of one pair distance.  false: below
+// the pair table
+template <bool OBS, int COPIES>
+static __device__ __forceinline__ bool fo_pair(const EamPot<float, EVAL_TABLE> &P,
+                                               const float4 *sm, const float4 *, float r2,
+                                               float &phi, float &wphi, float &wrho) {
   float r, inv_r, dphi, v, drho;
   r_and_inv(r2, r, inv_r);
-  if (EVAL == EVAL_CHEBY) {
-    phi = cheb_series(P, 0, r);
-    dphi = cheb_series(P, 3, r);
-    drho = cheb_series(P, 4, r);
+  if (P.tab.n > 0) {
+    const int i = fo_interval(P.tab, r, v);
+    const float4 d = COPIES == 0 ? __ldg(P.tab.der + i) : sm[i];
+    dphi = fmaf(v, d.y, d.x);
+    drho = fmaf(v, d.w, d.z);
+    if (OBS) {
+      const float4 c = __ldg(P.tab.phi + i);
+      phi = fmaf(v, fmaf(v, c.z, c.y), c.x);
+    }
   } else {
     table_eval(P.phi, r, phi, dphi);
     table_eval(P.rho, r, v, drho);
@@ -1135,7 +1215,7 @@ __device__ __forceinline__ bool fo_pair(const EamPot<float, EVAL> &P, const floa
 }
 // (two conflict-free 16-byte shared loads per pair, the phi cubic a third
 // only when the energy is summed)
-template <bool OBS>
+template <bool OBS, int COPIES>
 static __device__ __forceinline__ bool fo_pair(const EamPot<float, EVAL_CHEBY> &P,
                                                const float4 *sm, const float4 *phi_sm, float r2,
                                                float &phi, float &wphi, float &wrho) {
@@ -1146,8 +1226,8 @@ static __device__ __forceinline__ bool fo_pair(const EamPot<float, EVAL_CHEBY> &
     u = fmaf(r2 - P.seg.s2b, P.seg.inv_h2b, (float)P.seg.n2a);
   const int k = min((int)u, P.seg.n2 - 1);
   const float t = u - (float)k;
-  wphi = seg_cubic(sm[(2 * k) * FORCE_COPIES], t);
-  wrho = seg_cubic(sm[(2 * k + 1) * FORCE_COPIES], t);
+  wphi = seg_cubic(sm[(2 * k) * COPIES], t);
+  wrho = seg_cubic(sm[(2 * k + 1) * COPIES], t);
   if (OBS) {
     const float u1 = d * P.seg.inv_h;
     const int k1 = min((int)u1, P.seg.n - 1);
@@ -1156,17 +1236,6 @@ static __device__ __forceinline__ bool fo_pair(const EamPot<float, EVAL_CHEBY> &
   return true;
 }
 
-// the force pass's tables into shared memory, once per CTA: FORCE_COPIES
-// interleaved copies of the derivative cubics (2 n2 records each), then
-// with OBS the phi cubics (n records)
-template <bool OBS>
-__device__ __forceinline__ void stage_force_table(float4 *sm, const PairSeg &S) {
-  const int m = 2 * S.n2 * FORCE_COPIES;
-  for (int q = threadIdx.x; q < m; q += blockDim.x) sm[q] = __ldg(S.dcub + q / FORCE_COPIES);
-  if (OBS)
-    for (int q = threadIdx.x; q < S.n; q += blockDim.x) sm[m + q] = __ldg(S.p1 + q);
-  __syncthreads();
-}
 // the series for a pair below the table (FP32 Chebyshev only)
 template <int EVAL>
 __device__ __forceinline__ void fo_pair_series(const EamPot<float, EVAL> &, float, float &,
@@ -1218,8 +1287,8 @@ template <int EVAL, bool MULTI, bool OBS>
 __global__ void FO1_BOUNDS
     fo_eam_pass1_kernel(ForceArgs A, const __grid_constant__ EamPot<float, EVAL> P) {
   extern __shared__ float4 seg_sm[];
-  if (uses_seg(P)) stage_rho_copies(seg_sm, P.seg.rho1, P.seg.n1);  // the rho cubics
-  const float4 *rho_sm = seg_sm + (threadIdx.x & (RHO_COPIES - 1));  // this lane's copy
+  stage_rho<RHO_COPIES>(seg_sm, P);
+  const float4 *rho_sm = fo_copy<EVAL, RHO_COPIES>(seg_sm);
   const float rc2 = P.rc2;
   for (int a = blockIdx.x * blockDim.x + threadIdx.x; a < A.ntot; a += gridDim.x * blockDim.x) {
     const int slot = A.fo.slot[a];
@@ -1234,7 +1303,7 @@ __global__ void FO1_BOUNDS
                                  if (r2 > rc2) return;
                                  cnt++;
                                  float rho;
-                                 if (!fo_rho(P, rho_sm, r2, rho)) rho = fo_rho_series(P, r2);
+                                 if (!fo_rho<RHO_COPIES>(P, rho_sm, r2, rho)) rho = fo_rho_series(P, r2);
                                  rh.add(rho);
                                });
       fo_density_store<EVAL, OBS>(A, P, rh, a, slot, pi, cnt, A.fo.vcap + 1);
@@ -1245,19 +1314,48 @@ __global__ void FO1_BOUNDS
     const uint32_t *lst = A.fo.list + row;
     uint32_t *cut = A.fo.cut + row;
     bool low = false;
+    if (EVAL == EVAL_TABLE) {
+      // batches: the entries and the neighbours' positions of a whole batch are
+      // loaded before the first is used.  (The table's evaluation keeps the
+      // compiler from doing so in an unrolled loop: 1,047 us a pass at 4M
+      // atoms against 720; the Chebyshev pass takes 579 us unrolled, 589 so.)
+      for (int t0 = 0; t0 < n; t0 += FO1_BATCH) {
+        uint32_t p[FO1_BATCH];
+        float4 q[FO1_BATCH];
+#pragma unroll
+        for (int u = 0; u < FO1_BATCH; u++) {
+          if (t0 + u + FO_PREFETCH < n) prefetch_l1(lst + (size_t)(t0 + u + FO_PREFETCH) * 32);
+          p[u] = __ldg(lst + (size_t)min(t0 + u, n - 1) * 32);
+        }
+#pragma unroll
+        for (int u = 0; u < FO1_BATCH; u++) q[u] = __ldg(A.fo.pos + (p[u] >> 6));
+#pragma unroll
+        for (int u = 0; u < FO1_BATCH; u++) {
+          float dx, dy, dz;
+          const float r2 = fo_dr(fr, p[u], pi, q[u], dx, dy, dz);
+          if (r2 > rc2 || t0 + u >= n) continue;
+          if (COMDGB_FO_CUT) cut[(size_t)cnt * 32] = p[u];
+          cnt++;
+          float rho;
+          if (fo_rho<RHO_COPIES>(P, rho_sm, r2, rho)) rh.add(rho);
+          else low = true;
+        }
+      }
+    } else {
 #pragma unroll FO1_UNROLL
-    for (int t = 0; t < n; t++) {
-      if (t + FO_PREFETCH < n) prefetch_l1(lst + (size_t)(t + FO_PREFETCH) * 32);
-      const uint32_t p = __ldg(lst + (size_t)t * 32);
-      const float4 q = __ldg(A.fo.pos + (p >> 6));
-      float dx, dy, dz;
-      const float r2 = fo_dr(fr, p, pi, q, dx, dy, dz);
-      if (r2 > rc2) continue;
-      if (COMDGB_FO_CUT) cut[(size_t)cnt * 32] = p;
-      cnt++;
-      float rho;
-      if (fo_rho(P, rho_sm, r2, rho)) rh.add(rho);
-      else low = true;
+      for (int t = 0; t < n; t++) {
+        if (t + FO_PREFETCH < n) prefetch_l1(lst + (size_t)(t + FO_PREFETCH) * 32);
+        const uint32_t p = __ldg(lst + (size_t)t * 32);
+        const float4 q = __ldg(A.fo.pos + (p >> 6));
+        float dx, dy, dz;
+        const float r2 = fo_dr(fr, p, pi, q, dx, dy, dz);
+        if (r2 > rc2) continue;
+        if (COMDGB_FO_CUT) cut[(size_t)cnt * 32] = p;
+        cnt++;
+        float rho;
+        if (fo_rho<RHO_COPIES>(P, rho_sm, r2, rho)) rh.add(rho);
+        else low = true;
+      }
     }
     if (low)  // pairs below the table: the series, in a second sweep
       fo_walk<false, MULTI, 1>(A, A.fo.list, n, a, slot, pi, rc2,
@@ -1351,8 +1449,8 @@ template <int EVAL, bool MULTI, bool OBS>
 __global__ void __maxnreg__(OBS ? COMDGB_FO2_MAXNREG : COMDGB_FO2F_MAXNREG)
     fo_eam_pass2_kernel(ForceArgs A, const __grid_constant__ EamPot<float, EVAL> P) {
   extern __shared__ float4 seg_sm[];
-  if (uses_seg(P)) stage_force_table<OBS>(seg_sm, P.seg);
-  const float4 *dcub_sm = seg_sm + (threadIdx.x & (FORCE_COPIES - 1));  // this lane's copy
+  stage_force<FORCE_COPIES, OBS>(seg_sm, P);
+  const float4 *dcub_sm = fo_copy<EVAL, FORCE_COPIES>(seg_sm);
   const float4 *phi_sm = seg_sm + 2 * SEG2_N * FORCE_COPIES;
   const float rc2 = P.rc2;
   const bool fuse = !OBS && *(volatile const int *)(A.status + ST_FUSE);
@@ -1371,7 +1469,7 @@ __global__ void __maxnreg__(OBS ? COMDGB_FO2_MAXNREG : COMDGB_FO2F_MAXNREG)
     walk([&](float fj, float dx, float dy, float dz, float r2) {
       if (r2 > rc2) return;
       float phi, wphi, wrho;
-      if (!fo_pair<OBS>(P, dcub_sm, phi_sm, r2, phi, wphi, wrho)) {
+      if (!fo_pair<OBS, FORCE_COPIES>(P, dcub_sm, phi_sm, r2, phi, wphi, wrho)) {
         low = true;
         return;
       }

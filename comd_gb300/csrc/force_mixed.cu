@@ -1,6 +1,7 @@
 // force_mixed.cu -- the mixed-precision force kernels (FP32 pair terms on
 // box-relative coordinates, Kahan-compensated FP32 per-atom sums) and the list
 // builds, which both precisions use.
+#include "fo_lanes.cuh"
 #include "internal.h"
 
 namespace cg {
@@ -30,13 +31,11 @@ static size_t pass_smem(int pass, int eval) {
   return sizeof(float4) * (pass == 0 ? 2 : 1) * SEG_N;
 }
 
-// force order: the density pass stages its rho table (SEG1_N cubics, in
-// RHO_COPIES copies), the force pass its derivative cubics (2 SEG2_N, in
-// FORCE_COPIES copies) and, summing energies (obs), the phi cubics (SEG_N)
-static size_t fo_pass_smem(int pass, int eval, bool obs = true) {
-  if (eval != EVAL_CHEBY) return 0;
-  if (pass == 0) return sizeof(float4) * SEG1_N * RHO_COPIES;
-  return sizeof(float4) * (2 * SEG2_N * FORCE_COPIES + (obs ? SEG_N : 0));
+// force order: what a pass stages (stage_rho, stage_force)
+static size_t fo_pass_smem(int pass, int eval, bool obs, int copies, int ntab) {
+  if (eval == EVAL_TABLE) return copies > 0 ? sizeof(float4) * (size_t)ntab : 0;
+  if (pass == 0) return sizeof(float4) * SEG1_N * copies;
+  return sizeof(float4) * (2 * SEG2_N * copies + (obs ? SEG_N : 0));
 }
 
 // resident CTAs per SM of the force-order builds with NT threads, for 2, 4
@@ -61,25 +60,27 @@ template <bool OBS>
 static cudaError_t fo_occupancy() {
   int dummy = 0;
   int(&o)[3][2] = g_fo_per_sm[OBS];
-  const size_t s0 = fo_pass_smem(0, EVAL_CHEBY), s1 = fo_pass_smem(1, EVAL_CHEBY, OBS);
-  cudaError_t e = pass_occupancy(fo_eam_pass1_kernel<EVAL_TABLE, false, OBS>, 0,
+  const size_t s0 = fo_pass_smem(0, EVAL_CHEBY, OBS, RHO_COPIES, 0),
+               s1 = fo_pass_smem(1, EVAL_CHEBY, OBS, FORCE_COPIES, 0),
+               st = fo_pass_smem(0, EVAL_TABLE, OBS, 1, FOTAB_MAX);
+  cudaError_t e = pass_occupancy(fo_eam_pass1_kernel<EVAL_TABLE, false, OBS>, st,
                                  &o[0][EVAL_TABLE], FO1_THREADS);
   if (e == cudaSuccess)
     e = pass_occupancy(fo_eam_pass1_kernel<EVAL_CHEBY, false, OBS>, s0, &o[0][EVAL_CHEBY],
                        FO1_THREADS);
   if (e == cudaSuccess)
-    e = pass_occupancy(fo_eam_pass2_kernel<EVAL_TABLE, false, OBS>, 0, &o[1][EVAL_TABLE],
+    e = pass_occupancy(fo_eam_pass2_kernel<EVAL_TABLE, false, OBS>, st, &o[1][EVAL_TABLE],
                        FO2_MAX_THREADS);
   if (e == cudaSuccess)
     e = pass_occupancy(fo_eam_pass2_kernel<EVAL_CHEBY, false, OBS>, s1, &o[1][EVAL_CHEBY],
                        FO2_MAX_THREADS);
   if (e == cudaSuccess) e = pass_occupancy(fo_lj_kernel<false, OBS>, 0, &o[2][0]);
   if (e == cudaSuccess)
-    e = pass_occupancy(fo_eam_pass1_kernel<EVAL_TABLE, true, OBS>, 0, &dummy, FO1_THREADS);
+    e = pass_occupancy(fo_eam_pass1_kernel<EVAL_TABLE, true, OBS>, st, &dummy, FO1_THREADS);
   if (e == cudaSuccess)
     e = pass_occupancy(fo_eam_pass1_kernel<EVAL_CHEBY, true, OBS>, s0, &dummy, FO1_THREADS);
   if (e == cudaSuccess)
-    e = pass_occupancy(fo_eam_pass2_kernel<EVAL_TABLE, true, OBS>, 0, &dummy, FO2_MAX_THREADS);
+    e = pass_occupancy(fo_eam_pass2_kernel<EVAL_TABLE, true, OBS>, st, &dummy, FO2_MAX_THREADS);
   if (e == cudaSuccess)
     e = pass_occupancy(fo_eam_pass2_kernel<EVAL_CHEBY, true, OBS>, s1, &dummy, FO2_MAX_THREADS);
   if (e == cudaSuccess) e = pass_occupancy(fo_lj_kernel<true, OBS>, 0, &dummy);
@@ -174,10 +175,61 @@ void launch_nbr_cut(const ForceArgs &A, float rc2b, cudaStream_t st) {
         A, rc2b);
 }
 
+// Threads per atom of a force-order pass (1: the thread-per-atom kernels).  The
+// lines lie where the sums of both passes cross (us, Cu at 300 K, lattices
+// without energies; 8, 4, 2, 1 threads):
+//   Chebyshev   4,000 atoms  20.9  23.4  35.0  43.5
+//              16,384        27.1  26.3  35.0  43.8
+//              32,000          -   31.3  35.0  44.8
+//              55,296          -   45.6  43.6  46.0
+//             108,000          -   63.4  66.2  62.0
+//   table      16,384        25.7  28.7    -   50.5
+//              32,000        36.0  32.5    -   51.5
+//             108,000          -   63.4  65.4  70.1
+//             186,624          -   96.9  94.0 105.3
+//             275,684          -  139.9 132.0 130.0
+static int fo_lanes(int eval, int ntot) {
+  if (eval == EVAL_TABLE)
+    return ntot < 24000 ? 8 : ntot < 140000 ? 4 : ntot < 230000 ? 2 : 1;
+  return ntot < 12000 ? 8 : ntot < 60000 ? 4 : 1;
+}
+// and the LJ pass's, whose lists are twice as long
+static int fo_lj_lanes(int ntot) { return ntot < 24000 ? 8 : ntot < 100000 ? 4 : 1; }
+static unsigned fol_blocks(int ntot, int lanes) {
+  return (unsigned)(((long)ntot * lanes + FOL_THREADS - 1) / FOL_THREADS);
+}
+template <int EVAL, bool OBS, int LANES, int COPIES>
+static void launch_fol_eam(const ForceArgs &A, const EamPot<float, EVAL> &P, int pass,
+                           cudaStream_t st) {
+  const size_t smem = fo_pass_smem(pass, EVAL, OBS, COPIES, P.tab.n);
+  const unsigned g = fol_blocks(A.ntot, LANES);
+  const bool multi = A.g.nrep > 1;
+  if (pass == 0) {
+    if (multi) fol_eam_pass1_kernel<EVAL, true, OBS, LANES, COPIES><<<g, FOL_THREADS, smem, st>>>(A, P);
+    else fol_eam_pass1_kernel<EVAL, false, OBS, LANES, COPIES><<<g, FOL_THREADS, smem, st>>>(A, P);
+  } else {
+    if (multi) fol_eam_pass2_kernel<EVAL, true, OBS, LANES, COPIES><<<g, FOL_THREADS, smem, st>>>(A, P);
+    else fol_eam_pass2_kernel<EVAL, false, OBS, LANES, COPIES><<<g, FOL_THREADS, smem, st>>>(A, P);
+  }
+}
+template <bool OBS, int LANES>
+static void launch_fol_lj(const ForceArgs &A, const LjPot<float> &P, cudaStream_t st) {
+  const unsigned g = fol_blocks(A.ntot, LANES);
+  if (A.g.nrep > 1) fol_lj_kernel<true, OBS, LANES><<<g, FOL_THREADS, 0, st>>>(A, P);
+  else fol_lj_kernel<false, OBS, LANES><<<g, FOL_THREADS, 0, st>>>(A, P);
+}
+
 template <int EVAL, bool OBS>
 static void launch_fo_eam_obs(const ForceArgs &A, const EamPot<float, EVAL> &P, int pass,
                               cudaStream_t st, const Tune *tune) {
-  const size_t smem = P.seg.n > 0 ? fo_pass_smem(pass, EVAL, OBS) : 0;
+  // the tables once a CTA, or (table potential) from global memory
+  constexpr int copies = EVAL == EVAL_TABLE ? 0 : 1;
+  switch (fo_lanes(EVAL, A.ntot)) {
+    case 8: return launch_fol_eam<EVAL, OBS, 8, copies>(A, P, pass, st);
+    case 4: return launch_fol_eam<EVAL, OBS, 4, copies>(A, P, pass, st);
+    case 2: return launch_fol_eam<EVAL, OBS, 2, copies>(A, P, pass, st);
+  }
+  const size_t smem = fo_pass_smem(pass, EVAL, OBS, pass == 0 ? RHO_COPIES : FORCE_COPIES, P.tab.n);
   const bool multi = A.g.nrep > 1;
   if (pass == 0) {
     const int g0 = pass_grid(0, EVAL, A.ntot, true, FO1_THREADS, OBS);
@@ -213,7 +265,7 @@ template void launch_fo_eam<EVAL_CHEBY>(const ForceArgs &, const EamPot<float, E
 template <int EVAL, bool OBS>
 static int fo_pass2_per_sm(bool multi, int threads) {
   int per_sm = 0;
-  const size_t smem = fo_pass_smem(1, EVAL, OBS);
+  const size_t smem = fo_pass_smem(1, EVAL, OBS, FORCE_COPIES, FOTAB_MAX);
   const cudaError_t e =
       multi ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                   &per_sm, fo_eam_pass2_kernel<EVAL, true, OBS>, threads, smem)
@@ -235,6 +287,12 @@ int fo_pass2_blocks(int eval, bool multi, int threads, bool obs) {
 
 void launch_fo_lj(const ForceArgs &A, const LjPot<float> &P, cudaStream_t st, bool obs) {
   if (A.ntot <= 0) return;
+  const int lanes = fo_lj_lanes(A.ntot);
+  if (lanes > 1) {
+    if (lanes == 8) obs ? launch_fol_lj<true, 8>(A, P, st) : launch_fol_lj<false, 8>(A, P, st);
+    else obs ? launch_fol_lj<true, 4>(A, P, st) : launch_fol_lj<false, 4>(A, P, st);
+    return;
+  }
   const int grid = pass_grid(2, 0, A.ntot, true, PASS_THREADS, obs);
   const bool multi = A.g.nrep > 1;
   if (obs) {
