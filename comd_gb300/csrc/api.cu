@@ -724,8 +724,10 @@ float list_cutoff(const comdgb_sim *h, double rc) {
   return (float)(rc * rc * (1.0 + 1e-6) + 4.0 * rc * err);
 }
 
+// compact: first the atom list of the layout a rebin has just made (every
+// other call that changes the layout leaves the list current).
 void enqueue_force_parts(comdgb_sim *h, cudaEvent_t *ev, int &evi, bool obs = true,
-                         bool host_out = false) {
+                         bool host_out = false, bool compact = true) {
   // ev (optional) records after each group: compact, nbr, pass1, pass2.
   // obs = false: a force call inside a step sequence, whose energies, stress,
   // rho and F' the next force call overwrites before the caller can read
@@ -740,8 +742,9 @@ void enqueue_force_parts(comdgb_sim *h, cudaEvent_t *ev, int &evi, bool obs = tr
   }
   cudaStream_t st = h->stream;
   cudaMemsetAsync(h->status + ST_DELTA, 0, sizeof(int), st);  // f is about to hold forces
-  launch_compact(h->g, h->s.natoms, h->box_start, h->atom_slot, h->ntot, h->cpart, h->ncpart,
-                 st);
+  if (compact)
+    launch_compact(h->g, h->s.natoms, h->box_start, h->atom_slot, h->ntot, h->cpart, h->ncpart,
+                   st);
   if (ev) cudaEventRecordWithFlags(ev[evi++], st, cudaEventRecordExternal);
   const int pot = h->opts.potential;
   // persistent lists are built with rc + skin, and only when a rebuild is due
@@ -928,7 +931,7 @@ void enqueue_fo_step_force(comdgb_sim *h, double dt_atu, cudaEvent_t *ev, int &e
 
 void enqueue_reduce(comdgb_sim *h) {
   ForceArgs A = force_args(h);
-  launch_reduce(A, h->rpart, h->ripart, h->nrpart, h->d_out, h->d_iout, h->stream);
+  launch_reduce(A, h->rpart, h->ripart, h->nrpart, h->rdone, h->d_out, h->d_iout, h->stream);
   if (h->nrep > 1) launch_rep_reduce(A, h->rep_out, h->stream);
 }
 
@@ -1033,7 +1036,7 @@ int capture(comdgb_sim *h, cudaGraphExec_t *exec, double dt_atu, int part, bool 
     if (h->pl.vlist) launch_skin_check(h->g, h->s, h->pl, h->mixed, h->status, h->stream);
     if (h->fo.list && !tracked)
       launch_fo_track(h->g, h->s, h->fo, h->atom_slot, h->ntot, h->status, h->stream);
-    enqueue_force_parts(h, nullptr, evi, true, host_out);
+    enqueue_force_parts(h, nullptr, evi, true, host_out, false);
     enqueue_reduce(h);
   }
   CK(cudaStreamEndCapture(h->stream, &graph));
@@ -1741,11 +1744,13 @@ int create(const simflat_t *const *sims, int nrep, const comdgb_opts *o, comdgb_
   // (the force-order passes keep their own lists and never read this one)
   h->nbr = track(h, dalloc<uint16_t>((h->fo.list ? 0 : (size_t)h->ntot * h->cap) + 8, &err));
   h->nbr_n = track(h, dalloc<int>((size_t)h->ntot + 1, &err));
-  h->npair = track(h, dalloc<int>((size_t)h->ntot + 1, &err));
+  // (the force-order passes have their own list lengths)
+  h->npair = h->fo.list ? h->nbr_n : track(h, dalloc<int>((size_t)h->ntot + 1, &err));
   h->atom_stress = track(h, dalloc<double>((size_t)h->ntot + 1, &err));
   h->nrpart = reduce_partials(h->ntot);
   h->rpart = track(h, dalloc<double>(2 * (size_t)h->nrpart, &err));
   h->ripart = track(h, dalloc<long long>(h->nrpart, &err));
+  h->rdone = track(h, dalloc<unsigned>(1, &err));
   h->d_out = track(h, dalloc<double>(4, &err));
   h->d_iout = track(h, dalloc<long long>(2, &err));
   h->status = track(h, dalloc<int>(ST_COUNT, &err));
@@ -1755,9 +1760,9 @@ int create(const simflat_t *const *sims, int nrep, const comdgb_opts *o, comdgb_
     delete h;
     return set_err(COMDGB_ERR_NOMEM, "cudaMalloc failed (%zu slots)", ns);
   }
-  if (prepare_force_kernels() != cudaSuccess)
-    err = 1;
+  if (prepare_force_kernels() != cudaSuccess || prepare_md_kernels() != cudaSuccess) err = 1;
   cudaMemsetAsync(h->nbr_n, 0, sizeof(int) * ((size_t)h->ntot + 1), h->stream);
+  cudaMemsetAsync(h->rdone, 0, sizeof(unsigned), h->stream);
   cudaMemsetAsync(h->npair, 0, sizeof(int) * ((size_t)h->ntot + 1), h->stream);
   cudaMemsetAsync(h->atom_stress, 0, sizeof(double) * ((size_t)h->ntot + 1), h->stream);
   for (int r = 0; r < nrep; r++)
@@ -2038,8 +2043,6 @@ int comdgb_sim_energy(comdgb_sim *h, double *e, double *stress) {
 int comdgb_sim_kinetic(comdgb_sim *h, double *ek) {
   if (!h || !ek) return set_err(COMDGB_ERR_ARG, "null argument");
   CK(cudaSetDevice(h->device));
-  launch_compact(h->g, h->s.natoms, h->box_start, h->atom_slot, h->ntot, h->cpart, h->ncpart,
-                 h->stream);
   launch_kinetic(h->g, h->s, h->atom_slot, h->ntot, h->rmass, h->rpart, h->nrpart, h->d_out + 2,
                  h->stream);
   CK(cudaMemcpyAsync(ek, h->d_out + 2, sizeof(double), cudaMemcpyDeviceToHost, h->stream));

@@ -268,8 +268,6 @@ int comdgb_sim_centrosymmetry(comdgb_sim *h, int r, int approx, double *out, dou
   }
   cudaStream_t st = h->stream;
   CK(cudaMemsetAsync(h->centro, 0, sizeof(double) * (size_t)h->nslots, st));  // empty slots 0
-  // the atom list of the current layout
-  launch_compact(h->g, h->s.natoms, h->box_start, h->atom_slot, h->ntot, h->cpart, h->ncpart, st);
   if (h->ntot > 0)
     centro_kernel<<<(h->ntot + CT - 1) / CT, CT, 0, st>>>(h->g, h->s, h->dcenter, h->atom_slot,
                                                            h->ntot, approx, h->centro);

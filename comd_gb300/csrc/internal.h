@@ -71,8 +71,9 @@ void launch_rebin_finish(const Geom &g, Slots s, bool mixed, const RebinWork &w,
 void launch_compact(const Geom &g, const int *natoms, int *box_start, int *atom_slot, int ntot,
                     int *partials, int npart, cudaStream_t st, const int *only_if = nullptr);
 int compact_partials(int nboxes);
+cudaError_t prepare_md_kernels();
 void launch_reduce(const ForceArgs &A, double *partials, long long *ipartials, int npart,
-                   double *out, long long *iout, cudaStream_t st);
+                   unsigned *done, double *out, long long *iout, cudaStream_t st);
 int reduce_partials(int ntot);
 void launch_kinetic(const Geom &g, Slots s, const int *atom_slot, int ntot, double rmass,
                     double *partials, int npart, double *out, cudaStream_t st);

@@ -671,13 +671,9 @@ void launch_rebuild_done(int *status, cudaStream_t st) {
 // compaction: box_start = exclusive scan of natoms; atom_slot[a] = slot
 // ---------------------------------------------------------------------------
 #define CP_THREADS 256
-#ifndef COMDGB_CP_PER
-#define COMDGB_CP_PER 1  // boxes per thread in the compaction scans (1: 20 us at 110,592 boxes, 2: 27, 4: 37)
-#endif
-#define CP_PER COMDGB_CP_PER
-#define CP_CHUNK (CP_THREADS * CP_PER)
-
-int compact_partials(int nboxes) { return (nboxes + CP_CHUNK - 1) / CP_CHUNK; }
+#define CP_SMALL 8192    // boxes one CTA scans (24,389 boxes: 16 us so, 9 in three kernels)
+#define CP_SCAN 1024     // its threads
+int compact_partials(int nboxes) { return (nboxes + CP_THREADS - 1) / CP_THREADS; }
 
 __device__ __forceinline__ int block_excl_scan(int v, int *sh, int &total) {
   // sh has CP_THREADS/32 ints
@@ -704,17 +700,58 @@ __device__ __forceinline__ int block_excl_scan(int v, int *sh, int &total) {
   return pre + x - v;
 }
 
+// Up to CP_SMALL boxes one CTA scans the occupancies (thread t the boxes t *
+// per + q, staged in shared memory by coalesced loads).
+__global__ void __launch_bounds__(CP_SCAN) compact_scan_kernel(const int *natoms, int nboxes,
+                                                               int *box_start,
+                                                               const int *only_if) {
+  __shared__ int sh[CP_SCAN / 32];
+  extern __shared__ int cnt[];
+  if (stood_down(only_if)) return;
+  const int per = (nboxes + CP_SCAN - 1) / CP_SCAN;
+  for (int b = threadIdx.x; b < nboxes; b += CP_SCAN) cnt[b] = natoms[b];
+  __syncthreads();
+  const int b0 = threadIdx.x * per, b1 = min(b0 + per, nboxes);
+  int v = 0;
+  for (int b = b0; b < b1; b++) v += cnt[b];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int x = v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) sh[wid] = x;
+  __syncthreads();
+  if (wid == 0) {
+    int t = sh[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) t += y;
+    }
+    sh[lane] = t;
+  }
+  __syncthreads();
+  int off = x - v + (wid > 0 ? sh[wid - 1] : 0);
+  for (int b = b0; b < b1; b++) {
+    const int n = cnt[b];
+    cnt[b] = off;
+    off += n;
+  }
+  if (threadIdx.x == CP_SCAN - 1) box_start[nboxes] = sh[CP_SCAN / 32 - 1];
+  __syncthreads();
+  for (int b = threadIdx.x; b < nboxes; b += CP_SCAN) box_start[b] = cnt[b];
+}
+
+// Above, every CTA sums its 256 boxes, one CTA scans the sums, and
+// compact_offsets_kernel scans its boxes from there.
 __global__ void __launch_bounds__(CP_THREADS) compact_sum_kernel(const int *natoms, int nboxes,
                                                                  int *partials,
                                                                  const int *only_if) {
   __shared__ int sh[CP_THREADS / 32];
   if (stood_down(only_if)) return;
-  int base = blockIdx.x * CP_CHUNK + threadIdx.x * CP_PER;
-  int v = 0;
-  for (int q = 0; q < CP_PER; q++)
-    if (base + q < nboxes) v += natoms[base + q];
+  const int b = blockIdx.x * CP_THREADS + threadIdx.x;
   int total;
-  block_excl_scan(v, sh, total);
+  block_excl_scan(b < nboxes ? natoms[b] : 0, sh, total);
   if (threadIdx.x == 0) partials[blockIdx.x] = total;
 }
 
@@ -734,52 +771,56 @@ __global__ void __launch_bounds__(CP_THREADS) compact_scan_partials_kernel(int *
   }
 }
 
-// box offsets from the block's scan, then each warp writes whole boxes'
-// atom entries (coalesced)
-__global__ void __launch_bounds__(CP_THREADS) compact_write_kernel(const int *natoms, int nboxes,
-                                                                   const int *partials,
-                                                                   int *box_start,
-                                                                   int *atom_slot, int ntot,
-                                                                   const int *only_if) {
+__global__ void __launch_bounds__(CP_THREADS) compact_offsets_kernel(const int *natoms, int nboxes,
+                                                                     const int *partials,
+                                                                     int *box_start,
+                                                                     const int *only_if) {
   __shared__ int sh[CP_THREADS / 32];
-  __shared__ int s_off[CP_CHUNK], s_n[CP_CHUNK];
   if (stood_down(only_if)) return;
-  const int b0 = blockIdx.x * CP_CHUNK;
-  int loc[CP_PER];
-  int v = 0;
-  for (int q = 0; q < CP_PER; q++) {
-    const int b = b0 + threadIdx.x * CP_PER + q;
-    loc[q] = b < nboxes ? natoms[b] : 0;
-    v += loc[q];
-  }
+  const int b = blockIdx.x * CP_THREADS + threadIdx.x;
+  const int n = b < nboxes ? natoms[b] : 0;
   int total;
-  int off = block_excl_scan(v, sh, total) + partials[blockIdx.x];
-  for (int q = 0; q < CP_PER; q++) {
-    const int i = threadIdx.x * CP_PER + q, b = b0 + i;
-    s_off[i] = off;
-    s_n[i] = loc[q];
-    if (b < nboxes) {
-      box_start[b] = off;
-      if (b == nboxes - 1) box_start[nboxes] = off + loc[q];
-    }
-    off += loc[q];
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, nbk = min(CP_CHUNK, nboxes - b0);
-  for (int i = threadIdx.x >> 5; i < nbk; i += CP_THREADS / 32) {
-    const int o = s_off[i], n = s_n[i], base = (b0 + i) * CG_MAXATOMS;
-    // the counts sum to ntot unless a reported overflow left them inconsistent
-    for (int k = lane; k < n; k += 32)
-      if (o + k < ntot) atom_slot[o + k] = base + k;
+  const int off = block_excl_scan(n, sh, total) + partials[blockIdx.x];
+  if (b < nboxes) {
+    box_start[b] = off;
+    if (b == nboxes - 1) box_start[nboxes] = off + n;
   }
 }
 
+// each warp writes the atom entries of four boxes, eight lanes a box
+__global__ void __launch_bounds__(256) compact_write_kernel(const int *natoms, int nboxes,
+                                                            const int *box_start, int *atom_slot,
+                                                            int ntot, const int *only_if) {
+  if (stood_down(only_if)) return;
+  const int b = (blockIdx.x * 256 + threadIdx.x) >> 3, lane = threadIdx.x & 7;
+  if (b >= nboxes) return;
+  const int o = box_start[b], n = natoms[b], base = b * CG_MAXATOMS;
+  // the counts sum to ntot unless a reported overflow left them inconsistent
+  for (int k = lane; k < n; k += 8)
+    if (o + k < ntot) atom_slot[o + k] = base + k;
+}
+
+// (216 boxes: 6 us for the scan and the write, 13 for three kernels of which
+// the last wrote a warp's 32 boxes one after the other)
 void launch_compact(const Geom &g, const int *natoms, int *box_start, int *atom_slot, int ntot,
                     int *partials, int npart, cudaStream_t st, const int *only_if) {
-  compact_sum_kernel<<<npart, CP_THREADS, 0, st>>>(natoms, g.nboxes, partials, only_if);
-  compact_scan_partials_kernel<<<1, CP_THREADS, 0, st>>>(partials, npart, only_if);
-  compact_write_kernel<<<npart, CP_THREADS, 0, st>>>(natoms, g.nboxes, partials, box_start,
-                                                     atom_slot, ntot, only_if);
+  if (g.nboxes <= CP_SMALL) {
+    compact_scan_kernel<<<1, CP_SCAN, sizeof(int) * (size_t)g.nboxes, st>>>(natoms, g.nboxes,
+                                                                           box_start, only_if);
+  } else {
+    compact_sum_kernel<<<npart, CP_THREADS, 0, st>>>(natoms, g.nboxes, partials, only_if);
+    compact_scan_partials_kernel<<<1, CP_THREADS, 0, st>>>(partials, npart, only_if);
+    compact_offsets_kernel<<<npart, CP_THREADS, 0, st>>>(natoms, g.nboxes, partials, box_start,
+                                                         only_if);
+  }
+  compact_write_kernel<<<(unsigned)((8L * g.nboxes + 255) / 256), 256, 0, st>>>(
+      natoms, g.nboxes, box_start, atom_slot, ntot, only_if);
+}
+
+// before any launch or capture: the scan's shared memory
+cudaError_t prepare_md_kernels() {
+  return cudaFuncSetAttribute(compact_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)(sizeof(int) * CP_SMALL));
 }
 
 // ids of a replica's slots, offset by its first atom
@@ -795,7 +836,7 @@ void launch_add_offset(int *v, long n, int off, cudaStream_t st) {
 // deterministic reductions: energy (sum of f[3]), stress share, pair count
 // ---------------------------------------------------------------------------
 #define RD_THREADS 256
-#define RD_PER 16
+#define RD_PER 4
 
 int reduce_partials(int ntot) {
   int n = (ntot + RD_THREADS * RD_PER - 1) / (RD_THREADS * RD_PER);
@@ -826,13 +867,21 @@ __device__ __forceinline__ long long block_sum_l(long long v, long long *sh) {
   return t;
 }
 
+// Every CTA sums its atoms; the one that finishes last sums the CTAs' partials
+// in a fixed order (thread t takes partials t, t + RD_THREADS, ..., then the
+// block tree), so every run gives the same bits.  `done` counts the CTAs and
+// wraps to 0.
 __global__ void __launch_bounds__(RD_THREADS) reduce_force_kernel(ForceArgs A, double *partials,
-                                                                  long long *ipartials) {
+                                                                  long long *ipartials,
+                                                                  unsigned *done, double *out,
+                                                                  long long *iout) {
   __shared__ double shd[RD_THREADS / 32];
   __shared__ long long shl[RD_THREADS / 32];
+  __shared__ bool last;
   int base = blockIdx.x * RD_THREADS * RD_PER;
   double e = 0.0, sx = 0.0;
   long long np = 0;
+#pragma unroll
   for (int q = 0; q < RD_PER; q++) {
     int a = base + q * RD_THREADS + threadIdx.x;
     if (a < A.ntot) {
@@ -848,25 +897,18 @@ __global__ void __launch_bounds__(RD_THREADS) reduce_force_kernel(ForceArgs A, d
     partials[2 * blockIdx.x] = e;
     partials[2 * blockIdx.x + 1] = sx;
     ipartials[blockIdx.x] = np;
+    __threadfence();
+    last = atomicInc(done, gridDim.x - 1) == gridDim.x - 1;
   }
-}
-
-// The block partials summed by one CTA in a fixed order (thread t sums
-// partials t, t + RD_THREADS, ... in turn, then the block tree), so every
-// run gives the same bits.  (One thread summing them serially took 150 us
-// for the ~1000 partials of 4 M atoms.)
-__global__ void __launch_bounds__(RD_THREADS) reduce_final_kernel(const double *partials,
-                                                                  const long long *ipartials,
-                                                                  int npart, double *out,
-                                                                  long long *iout) {
-  __shared__ double shd[RD_THREADS / 32];
-  __shared__ long long shl[RD_THREADS / 32];
-  double e = 0.0, sx = 0.0;
-  long long np = 0;
-  for (int q = threadIdx.x; q < npart; q += RD_THREADS) {
-    e += partials[2 * q];
-    sx += partials[2 * q + 1];
-    np += ipartials[q];
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  e = sx = 0.0;
+  np = 0;
+  for (int q = threadIdx.x; q < (int)gridDim.x; q += RD_THREADS) {
+    e += __ldcg(partials + 2 * q);
+    sx += __ldcg(partials + 2 * q + 1);
+    np += __ldcg(ipartials + q);
   }
   e = block_sum_d(e, shd);
   sx = block_sum_d(sx, shd);
@@ -879,9 +921,8 @@ __global__ void __launch_bounds__(RD_THREADS) reduce_final_kernel(const double *
 }
 
 void launch_reduce(const ForceArgs &A, double *partials, long long *ipartials, int npart,
-                   double *out, long long *iout, cudaStream_t st) {
-  reduce_force_kernel<<<npart, RD_THREADS, 0, st>>>(A, partials, ipartials);
-  reduce_final_kernel<<<1, RD_THREADS, 0, st>>>(partials, ipartials, npart, out, iout);
+                   unsigned *done, double *out, long long *iout, cudaStream_t st) {
+  reduce_force_kernel<<<npart, RD_THREADS, 0, st>>>(A, partials, ipartials, done, out, iout);
 }
 
 // per replica (one block each, fixed order): energy sum f.w and stress share
@@ -921,7 +962,7 @@ __global__ void __launch_bounds__(RD_THREADS) kinetic_kernel(Slots s, const int 
   if (threadIdx.x == 0) partials[blockIdx.x] = ek;
 }
 
-// (the partials summed as in reduce_final_kernel)
+// (the partials summed as in reduce_force_kernel)
 __global__ void __launch_bounds__(RD_THREADS) kinetic_final_kernel(const double *partials,
                                                                    int npart, double rmass,
                                                                    double *out) {

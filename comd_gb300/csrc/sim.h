@@ -81,6 +81,7 @@ struct comdgb_sim {
   double *atom_stress = nullptr;
   double *rpart = nullptr;
   long long *ripart = nullptr;
+  unsigned *rdone = nullptr;   // CTAs of the force reduction that have finished
   int nrpart = 0;
   double *d_out = nullptr;     // [0] energy sum [1] stress sum [2] kinetic
   long long *d_iout = nullptr; // [0] directed pair count
@@ -126,6 +127,9 @@ struct comdgb_sim {
   // centrosymmetry (centro.cu): one value per slot, then the range of the
   // last replica asked for
   double *centro = nullptr;
+  // by-id gather (clsman_io.cu): six doubles per atom, ids seen; on first use
+  double *gather_out = nullptr;
+  int *gather_seen = nullptr;
   cg::Tune tune;  // launch shapes of the force-order kernels (comdgb_sim_set_launch)
   // graphs
   // merge_rebox (mixed precision): a sequence of steps reboxes once per step

@@ -462,14 +462,14 @@ class DeviceSim:
     def atom_stress(self, r=0):
         """per-atom stress x volume of the last virial() call, replica r's slot
         layout: array [nboxes * 64, 6] (empty slots 0)"""
-        a = np.zeros((self._nboxes[r] * 64, 6))
+        a = np.empty((self._nboxes[r] * 64, 6))
         check(self.L.comdgb_sim_atom_stress(self.h, r, a.ctypes.data_as(C.POINTER(C.c_double))))
         return a
 
     def centrosymmetry(self, r=0, approx=False):
         """(per-slot centrosymmetry of replica r [nboxes * 64], min, max)"""
         P = C.POINTER(C.c_double)
-        out = np.zeros(self._nboxes[r] * 64)
+        out = np.empty(self._nboxes[r] * 64)
         lo, hi = C.c_double(), C.c_double()
         check(self.L.comdgb_sim_centrosymmetry(self.h, r, int(approx), out.ctypes.data_as(P),
                                                C.byref(lo), C.byref(hi)))
@@ -479,7 +479,7 @@ class DeviceSim:
     def gather(self, r=0):
         """replica r's atoms in id order: [ntot, 6] = position (box corner + r),
         momentum"""
-        a = np.zeros((self._ntot[r], 6))
+        a = np.empty((self._ntot[r], 6))
         check(self.L.comdgb_sim_gather(self.h, r, a.ctypes.data_as(C.POINTER(C.c_double))))
         return a
 
