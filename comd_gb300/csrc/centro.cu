@@ -27,6 +27,8 @@
 // the exact sum: a pairing outside the window cannot be the reference's
 // minimum, and the result is the reference's value bit for bit.
 // APPROX_CENTROSYM's greedy pairing (:528-557) is the `approx` variant.
+#include <algorithm>
+
 #include "sim.h"
 
 using namespace cg;
@@ -90,8 +92,37 @@ __device__ __forceinline__ void pairing_dfs(const float (*p)[CT], int t, const f
   }
 }
 
+// the FP32 extent of every box's atoms (relative to its centre): lo, then hi;
+// without bounds when a position is not a number, and nothing in an empty box
+__global__ void __launch_bounds__(256) box_extent_kernel(Slots s, int nboxes, float4 *ext) {
+  const int b = blockIdx.x * 256 + threadIdx.x;
+  if (b >= nboxes) return;
+  const float inf = __int_as_float(0x7f800000);
+  float4 lo = make_float4(inf, inf, inf, 0.f), hi = make_float4(-inf, -inf, -inf, 0.f);
+  const int n = s.natoms[b];
+  for (int k = 0; k < n; k++) {
+    const float4 q = __ldg(s.pos32 + b * CG_MAXATOMS + k);
+    if (!(q.x + q.y + q.z == q.x + q.y + q.z)) {
+      lo = make_float4(-inf, -inf, -inf, 0.f);
+      hi = make_float4(inf, inf, inf, 0.f);
+      break;
+    }
+    lo = make_float4(fminf(lo.x, q.x), fminf(lo.y, q.y), fminf(lo.z, q.z), 0.f);
+    hi = make_float4(fmaxf(hi.x, q.x), fmaxf(hi.y, q.y), fmaxf(hi.z, q.z), 0.f);
+  }
+  ext[2 * b] = lo;
+  ext[2 * b + 1] = hi;
+}
+
+// how far p (a coordinate) lies outside [lo + f, hi + f], by the operations of
+// the candidates' test: no atom of the box gives a smaller |(q - p) + f|
+__device__ __forceinline__ float outside(float lo, float hi, float p, float f) {
+  return fmaxf(fmaxf((lo - p) + f, -((hi - p) + f)), 0.f);
+}
+
 __global__ void __launch_bounds__(CT) centro_kernel(Geom g, Slots s, const double *dcenter,
                                                     const int *atom_slot, int ntot, int approx,
+                                                    float slack, const float4 *ext,
                                                     double *out) {
   // per thread (column t): held vectors, their r^2 (integer images) and the
   // pair terms rounded to FP32.  Warps run the scan and the pairing phases
@@ -138,38 +169,75 @@ __global__ void __launch_bounds__(CT) centro_kernel(Geom g, Slots s, const doubl
         }
     }
   };
-  // own box: box-relative differences
-  for (int j = 0; j < ni; j++) {
-    if (j == i) continue;
-    const d4 rj = s.r[b * CG_MAXATOMS + j];
-    offer(__dsub_rn(rj.x, ri.x), __dsub_rn(rj.y, ri.y), __dsub_rn(rj.z, ri.z));
-  }
+  // Candidates past the largest of twelve held are refused by the FP64 test in
+  // `offer`; an FP32 test in front of it (box-centred positions; est < cut
+  // holds for every candidate that `offer` would take, the FP32 distance
+  // erring by less than `own` and 1e-6 of it) refuses nearly all of them first,
+  // and whole boxes by their extent.  Within a box every thread runs on to its
+  // next candidate that passes, so that the insertions of a warp's threads,
+  // the expensive part, happen together.  At 256,000 atoms 1.95 ms where an
+  // FP64 test of every candidate took 3.64; one loop over all candidates,
+  // whose box changes diverge, took 3.31.
   const double cxi = __dadd_rn(dcenter[3 * b + 0], ri.x);
   const double cyi = __dadd_rn(dcenter[3 * b + 1], ri.y);
   const double czi = __dadd_rn(dcenter[3 * b + 2], ri.z);
-  for (int cx = bx - 1; cx <= bx + 1; cx++)
-    for (int cy = by - 1; cy <= by + 1; cy++)
-      for (int cz = bz - 1; cz <= bz + 1; cz++) {
-        if (cx == bx && cy == by && cz == bz) continue;
-        float ox = 0.0f, oy = 0.0f, oz = 0.0f;
-        int qx = cx, qy = cy, qz = cz;
-        if (qx < 0) { qx = nx - 1; ox = __double2float_rn(-R.bounds[0]); }
-        if (qx >= nx) { qx = 0; ox = __double2float_rn(R.bounds[0]); }
-        if (qy < 0) { qy = ny - 1; oy = __double2float_rn(-R.bounds[1]); }
-        if (qy >= ny) { qy = 0; oy = __double2float_rn(R.bounds[1]); }
-        if (qz < 0) { qz = nz - 1; oz = __double2float_rn(-R.bounds[2]); }
-        if (qz >= nz) { qz = 0; oz = __double2float_rn(R.bounds[2]); }
-        const int b2 = R.box0 + qz * nx * ny + qy * nx + qx;
-        const double ex = __dadd_rn((double)ox, dcenter[3 * b2 + 0]);
-        const double ey = __dadd_rn((double)oy, dcenter[3 * b2 + 1]);
-        const double ez = __dadd_rn((double)oz, dcenter[3 * b2 + 2]);
-        const int nj = s.natoms[b2];
-        for (int j = 0; j < nj; j++) {
-          const d4 rj = s.r[b2 * CG_MAXATOMS + j];
-          offer(__dsub_rn(__dadd_rn(ex, rj.x), cxi), __dsub_rn(__dadd_rn(ey, rj.y), cyi),
-                __dsub_rn(__dadd_rn(ez, rj.z), czi));
-        }
+  const float4 pi = __ldg(s.pos32 + io);
+  const float own = slack + 1e-6f * (fabsf(pi.x) + fabsf(pi.y) + fabsf(pi.z));
+  float cut = 3.0e38f;  // est must be below it
+  // the candidates of box b2 with corner offset e (own box: relative)
+  auto scan = [&](int b2, int nj, bool same, double ex, double ey, double ez, float fx, float fy,
+                  float fz) {
+    int j = 0;
+    while (true) {
+      bool got = false;
+      for (; j < nj; j++) {
+        const float4 q = __ldg(s.pos32 + b2 * CG_MAXATOMS + j);
+        const float tx = (q.x - pi.x) + fx, ty = (q.y - pi.y) + fy, tz = (q.z - pi.z) + fz;
+        // (not >=: a NaN goes on to the exact test)
+        got = !(tx * tx + ty * ty + tz * tz >= cut) && !(same && j == i);
+        if (got) break;
       }
+      if (!got) break;
+      const d4 rj = s.r[b2 * CG_MAXATOMS + j];
+      j++;
+      if (same)
+        offer(__dsub_rn(rj.x, ri.x), __dsub_rn(rj.y, ri.y), __dsub_rn(rj.z, ri.z));
+      else
+        offer(__dsub_rn(__dadd_rn(ex, rj.x), cxi), __dsub_rn(__dadd_rn(ey, rj.y), cyi),
+              __dsub_rn(__dadd_rn(ez, rj.z), czi));
+      if (nb == 12) {
+        // est < (r + e)^2, e the FP32 vector's error: slack for the box offset,
+        // and roundings of the atom's own position and of the distance
+        const float r2 = __double2float_ru(__longlong_as_double(rmax));
+        const float r = sqrtf(r2), e = own + 1e-6f * r;
+        cut = (r2 + e * (2.0f * r + e) + 1e-30f) * 1.000001f;
+      }
+    }
+  };
+  scan(b, ni, true, 0.0, 0.0, 0.0, 0.f, 0.f, 0.f);
+  for (int cell = 0; cell < 27; cell++) {  // x-outer, z-inner
+    if (cell == 13) continue;
+    float ox = 0.0f, oy = 0.0f, oz = 0.0f;
+    int qx = bx + cell / 9 - 1, qy = by + cell / 3 % 3 - 1, qz = bz + cell % 3 - 1;
+    if (qx < 0) { qx = nx - 1; ox = __double2float_rn(-R.bounds[0]); }
+    if (qx >= nx) { qx = 0; ox = __double2float_rn(R.bounds[0]); }
+    if (qy < 0) { qy = ny - 1; oy = __double2float_rn(-R.bounds[1]); }
+    if (qy >= ny) { qy = 0; oy = __double2float_rn(R.bounds[1]); }
+    if (qz < 0) { qz = nz - 1; oz = __double2float_rn(-R.bounds[2]); }
+    if (qz >= nz) { qz = 0; oz = __double2float_rn(R.bounds[2]); }
+    const int b2 = R.box0 + qz * nx * ny + qy * nx + qx;
+    const double ex = __dadd_rn((double)ox, dcenter[3 * b2 + 0]);
+    const double ey = __dadd_rn((double)oy, dcenter[3 * b2 + 1]);
+    const double ez = __dadd_rn((double)oz, dcenter[3 * b2 + 2]);
+    const float fx = (float)(ex - dcenter[3 * b + 0]), fy = (float)(ey - dcenter[3 * b + 1]),
+                fz = (float)(ez - dcenter[3 * b + 2]);
+    // a box whose atoms all fail the test is passed over whole
+    const float4 lo = __ldg(ext + 2 * b2), hi = __ldg(ext + 2 * b2 + 1);
+    const float gx = outside(lo.x, hi.x, pi.x, fx), gy = outside(lo.y, hi.y, pi.y, fy),
+                gz = outside(lo.z, hi.z, pi.z, fz);
+    if (gx * gx + gy * gy + gz * gz >= cut) continue;
+    scan(b2, s.natoms[b2], false, ex, ey, ez, fx, fy, fz);
+  }
   double c = 1000.0;
   if (nb >= 12) {
     if (approx) {
@@ -224,31 +292,26 @@ __global__ void __launch_bounds__(CT) centro_kernel(Geom g, Slots s, const doubl
   out[io] = c;
 }
 
-// min / max over the replica's atoms (minCentro from 1000, maxCentro from 0)
-__global__ void centro_range_kernel(Geom g, const int *natoms, const double *c, int r,
-                                    double *range) {
-  __shared__ double lo_s[256], hi_s[256];
-  const RepGeo &R = g.rep[r];
+// min / max over the replica's atoms (minCentro from 1000, maxCentro from 0),
+// into range[0] and range[1], which hold those two: the values are not
+// negative, so their bits are ordered as they are.  (One CTA over all boxes
+// took 342 us at 256,000 atoms.)
+__global__ void __launch_bounds__(256)
+    centro_range_kernel(Slots s, const int *atom_slot, const double *c, int a0, int na,
+                        unsigned long long *range) {
   double lo = 1000.0, hi = 0.0;
-  for (int b = R.box0 + threadIdx.x; b < R.box0 + R.nb; b += blockDim.x)
-    for (int i = 0; i < natoms[b]; i++) {
-      const double x = c[b * CG_MAXATOMS + i];
-      lo = x < lo ? x : lo;
-      hi = x > hi ? x : hi;
-    }
-  lo_s[threadIdx.x] = lo;
-  hi_s[threadIdx.x] = hi;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) {
-      lo_s[threadIdx.x] = fmin(lo_s[threadIdx.x], lo_s[threadIdx.x + o]);
-      hi_s[threadIdx.x] = fmax(hi_s[threadIdx.x], hi_s[threadIdx.x + o]);
-    }
-    __syncthreads();
+  for (int a = a0 + blockIdx.x * 256 + threadIdx.x; a < a0 + na; a += gridDim.x * 256) {
+    const double x = c[atom_slot[a]];
+    lo = x < lo ? x : lo;
+    hi = x > hi ? x : hi;
   }
-  if (threadIdx.x == 0) {
-    range[0] = lo_s[0];
-    range[1] = hi_s[0];
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicMin(range, (unsigned long long)__double_as_longlong(lo));
+    atomicMax(range + 1, (unsigned long long)__double_as_longlong(hi));
   }
 }
 
@@ -263,22 +326,43 @@ int comdgb_sim_centrosymmetry(comdgb_sim *h, int r, int approx, double *out, dou
   CK(cudaSetDevice(h->device));
   int err = 0;
   if (!h->centro) {
-    h->centro = track(h, dalloc<double>((size_t)h->nslots + 2, &err));
+    double *c = dalloc<double>((size_t)h->nslots + 2, &err);
+    float4 *x = dalloc<float4>(2 * (size_t)h->g.nboxes, &err);
+    if (!err) {
+      h->centro = track(h, c);
+      h->centro_ext = track(h, x);
+    } else {
+      cudaGetLastError();
+      cudaFree(c);
+      cudaFree(x);
+    }
     if (err) return set_err(COMDGB_ERR_NOMEM, "centrosymmetry buffer");
   }
   cudaStream_t st = h->stream;
   CK(cudaMemsetAsync(h->centro, 0, sizeof(double) * (size_t)h->nslots, st));  // empty slots 0
-  if (h->ntot > 0)
-    centro_kernel<<<(h->ntot + CT - 1) / CT, CT, 0, st>>>(h->g, h->s, h->dcenter, h->atom_slot,
-                                                           h->ntot, approx, h->centro);
-  centro_range_kernel<<<1, 256, 0, st>>>(h->g, h->s.natoms, h->centro, r,
-                                         h->centro + h->nslots);
-  CK(cudaGetLastError());
   const RepGeo &R = h->reps[r];
+  double range[2] = {1000.0, 0.0};
+  CK(cudaMemcpyAsync(h->centro + h->nslots, range, sizeof range, cudaMemcpyHostToDevice, st));
+  if (h->ntot > 0) {
+    // the error that the box offsets (up to two widths) bring to an FP32 vector
+    double width = 0.0;
+    for (const RepGeo &q : h->reps)
+      for (int j = 0; j < 3; j++) width = std::max(width, q.boxsize[j]);
+    const float slack = (float)(1.7320508 * 16.0 / 16777216.0 * 2.0 * width);
+    launch_pos32_atoms(h->g, h->s, h->atom_slot, h->ntot, st);
+    box_extent_kernel<<<(h->g.nboxes + 255) / 256, 256, 0, st>>>(h->s, h->g.nboxes,
+                                                                 h->centro_ext);
+    centro_kernel<<<(h->ntot + CT - 1) / CT, CT, 0, st>>>(h->g, h->s, h->dcenter, h->atom_slot,
+                                                           h->ntot, approx, slack,
+                                                           h->centro_ext, h->centro);
+    centro_range_kernel<<<2 * h->sms, 256, 0, st>>>(
+        h->s, h->atom_slot, h->centro, R.a0, R.na,
+        reinterpret_cast<unsigned long long *>(h->centro + h->nslots));
+  }
+  CK(cudaGetLastError());
   if (out)
     CK(cudaMemcpyAsync(out, h->centro + (size_t)R.box0 * CG_MAXATOMS,
                        sizeof(double) * (size_t)R.nb * CG_MAXATOMS, cudaMemcpyDeviceToHost, st));
-  double range[2];
   CK(cudaMemcpyAsync(range, h->centro + h->nslots, sizeof range, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   if (cmin) *cmin = range[0];

@@ -127,6 +127,7 @@ struct comdgb_sim {
   // centrosymmetry (centro.cu): one value per slot, then the range of the
   // last replica asked for
   double *centro = nullptr;
+  float4 *centro_ext = nullptr;  // and the extent of every box's atoms
   // by-id gather (clsman_io.cu): six doubles per atom, ids seen; on first use
   double *gather_out = nullptr;
   int *gather_seen = nullptr;
