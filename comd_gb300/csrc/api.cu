@@ -77,6 +77,9 @@ ForceArgs force_args(comdgb_sim *h) {
   A.nbr_n = h->nbr_n;
   A.npair = h->npair;
   A.cap = h->cap;
+  A.fx = h->fx;
+  A.fxu = h->fxu;
+  A.fx_rc2 = h->fx ? (u64)ldexp(h->cutoff * h->cutoff, 64 - 2 * h->fxu.m) : 0;
   A.atom_stress = h->atom_stress;
   A.status = h->status;
   A.pl = h->pl;
@@ -771,7 +774,7 @@ void enqueue_force_parts(comdgb_sim *h, cudaEvent_t *ev, int &evi, bool obs = tr
     return;
   }
   // the build and the cut work on FP32 copies (mixed precision keeps them)
-  if (!h->mixed) launch_pos32_atoms(h->g, h->s, h->atom_slot, h->ntot, st);
+  if (!h->mixed) launch_pos32_atoms(h->g, h->s, h->atom_slot, h->ntot, st, h->fx, h->fxu);
   launch_nbr_build(A, list_cutoff(h, h->pl.vlist ? rcl : h->cutoff), st);
   if (h->pl.vlist) {
     launch_rebuild_done(h->status, st);
@@ -1697,6 +1700,14 @@ int create(const simflat_t *const *sims, int nrep, const comdgb_opts *o, comdgb_
   h->cap = 0;
   for (int r = 0; r < nrep; r++) h->cap = std::max(h->cap, neighbor_capacity(sims[r], rc));
   h->cutoff = rc;
+  if (!h->mixed && o->potential >= 0) {
+    // 2^(m-1) above every distance in the per-step list
+    const double far = 1.001 * sqrt((double)list_cutoff(h, rc));
+    h->fxu.m = (std::isfinite(far) && far > 0.0 ? std::ilogb(far) : 0) + 2;
+    h->fxu.down = std::ldexp(1.0, -h->fxu.m);
+    h->et.fx = track(h, dalloc<d4>(nb * CG_NNBR, &err));
+    h->fx = track(h, dalloc<d4>(ns, &err));
+  }
   if (use_persistent_lists(h, sims, nrep, o)) {
     int vcap = 0;
     for (int r = 0; r < nrep; r++)
@@ -1768,7 +1779,7 @@ int create(const simflat_t *const *sims, int nrep, const comdgb_opts *o, comdgb_
   for (int r = 0; r < nrep; r++)
     cudaMemcpyAsync(h->dcenter + 3 * (size_t)h->reps[r].box0, sims[r]->dcenter,
                     (size_t)h->reps[r].nb * 3 * sizeof(double), cudaMemcpyHostToDevice, h->stream);
-  launch_entry_table(h->g, h->dcenter, h->et, h->boxc, h->stream);
+  launch_entry_table(h->g, h->dcenter, h->et, h->fxu, h->boxc, h->stream);
   int rc2 = setup_potential(h, s);
   for (int r = 0; r < nrep && !rc2; r++) rc2 = upload_rep(h, r, sims[r]);
   if (!rc2) rc2 = upload_done(h);

@@ -18,6 +18,8 @@
 #include <cstring>
 #include <cuda_runtime.h>
 
+#include "fixed64.cuh"
+
 #define CG_MAXATOMS 64
 #define CG_NNBR 27
 #define CG_NCHEB 32
@@ -134,6 +136,8 @@ struct EntryTab {
   int *box;        // [nboxes*27] neighbour box id
   d4 *dr64;     // [nboxes*27] drbox (x, y, z, 0)
   float4 *dr32;    // [nboxes*27] drbox rounded to FP32
+  d4 *fx;          // [nboxes*27] FP64 simulations: drbox in fixed point (the bits of
+                   // three 64-bit integers) and the neighbour box id (low word of w)
 };
 
 // device status words

@@ -4,38 +4,34 @@
 // warp's FP64 instruction holds it for 16 clocks while every other pipe (and
 // the loads) wait for nothing.  So the passes count FP64 operations:
 //   * density first, then forces, as in force order: rho alone in the first
-//     pass (17 operations a pair with the Chebyshev polynomials), phi'/r and
+//     pass (7 operations a pair with the Chebyshev polynomials), phi'/r and
 //     rho'/r in the second, and phi and the stress only where the caller can
 //     read them (OBS);
-//   * the cutoff test compares bit patterns, and 1/r and r come from the FP32
-//     reciprocal square root (MUFU) and one cubic step, not from FP64 division;
+//   * distances are formed in fixed point (fixed64.cuh), and 1/r and r come
+//     from the FP32 reciprocal square root (MUFU) and one cubic step, not from
+//     FP64 division;
 //   * LANES threads share an atom's list (lane l takes entries l, l + LANES,
 //     ...; the sums are combined in a fixed order).  A thread per atom leaves
 //     most of the 152 SMs idle on small systems, and on larger ones the last
 //     wave of long threads runs nearly empty.
-// F'(rho_j) reaches the second pass in the unused fourth component of r: one
-// 32-byte gather a pair.
-// Measured at 256,000 atoms (no energies), both passes: table potential 3,156
-// us before (phi, phi' and rho, then rho', a thread per atom, FP64 division and
-// square root, the skin list walked in FP64) and 1,221 now, Chebyshev 1,327 and
-// 950.
+// F'(rho_j) reaches the second pass in the fourth component of the position
+// record: one 32-byte gather a pair.
+// Measured at 256,000 atoms (no energies), density + forces: table potential
+// 3,156 us before (phi, phi' and rho, then rho', a thread per atom, FP64
+// division and square root, the skin list walked in FP64), 541 + 682 with the
+// list above in FP64 geometry, 354 + 469 in fixed point; Chebyshev 1,327, 350
+// + 560, 159 + 321, where the pipe's two lanes a clock would take 135 + 310.
+// Relative rms error of the forces against extended precision (504 atoms, Cu
+// at 300 K): Chebyshev 4.6e-14 before, 2.4e-15 now, table 2.2e-15 and 1.8e-15,
+// LJ 1.4e-15 and 0.9e-15; energies and densities are closer as well.
 #pragma once
 
+#include "fixed64.cuh"
 #include "force_kernels.cuh"
 
 namespace cg {
 
 constexpr int F64_THREADS = 128;
-
-// r2 beyond the cutoff, by the bits of non-negative doubles; a NaN is not (it
-// reaches the sums, as in a floating-point comparison)
-__device__ __forceinline__ bool beyond(double r2, double rc2) {
-  const long long x = __double_as_longlong(r2);
-  return x > __double_as_longlong(rc2) && x <= 0x7ff0000000000000LL;
-}
-__device__ __forceinline__ bool below(double r2, double rc2) {
-  return __double_as_longlong(r2) < __double_as_longlong(rc2);
-}
 
 // The atom and sub-lane of this thread; false when its whole warp has none.
 // Groups past the last atom repeat it (no divergence in the shuffles) and
@@ -58,56 +54,75 @@ __device__ __forceinline__ double lane_sum(double v) {
   return v;
 }
 
-// This lane's entries of atom a's list: fn(r_j, dx, dy, dz, r2), entries past
-// the cutoff included; an overflowed list's stencil is scanned by lane 0.
+// A pair: the differences and r^2 in fixed point, F'(rho_j)
+struct Pair64 {
+  long long x, y, z;
+  u64 s;
+  double fj;
+};
+__device__ __forceinline__ Pair64 pair64(long long x, long long y, long long z, double fj) {
+  return Pair64{x, y, z, fx_square(fx_abs(x)) + fx_square(fx_abs(y)) + fx_square(fx_abs(z)), fj};
+}
+
+// This lane's entries of atom a's list: fn(pair), entries past the cutoff
+// included; an overflowed list's stencil is scanned by lane 0.  fi: the
+// atom's record.
 template <int LANES, class F>
-__device__ __forceinline__ void walk64(const ForceArgs &A, int a, int sub, int slot,
-                                       const d4 &ri, double rc2, F &&fn) {
+__device__ __forceinline__ void walk64(const ForceArgs &A, int a, int sub, int slot, const d4 &fi,
+                                       double rc2, F &&fn) {
   const int n = A.nbr_n[a], b = slot >> 6;
   if (n > A.cap) {
-    if (sub == 0)
+    if (sub == 0) {
+      const d4 ri = A.s.r[slot];
       scan_stencil<double>(A, b, slot & 63, ri.x, ri.y, ri.z, rc2,
-                           [&](int js, double dx, double dy, double dz, double r2) {
-                             fn(A.s.r[js], dx, dy, dz, r2);
+                           [&](int js, double dx, double dy, double dz, double) {
+                             fn(pair64(fx_from(dx, A.fxu), fx_from(dy, A.fxu),
+                                       fx_from(dz, A.fxu), A.fx[js].w));
                            });
+    }
     return;
   }
-  const int ebase = b * CG_NNBR;
+  const long long xi = __double_as_longlong(fi.x), yi = __double_as_longlong(fi.y),
+                  zi = __double_as_longlong(fi.z);
+  const d4 *off = A.et.fx + b * CG_NNBR;
   const uint16_t *lst = A.nbr + (size_t)a * A.cap;
-#pragma unroll 2
+#pragma unroll 1
   for (int t = sub; t < n; t += LANES) {
     const uint32_t code = __ldg(lst + t);
-    const int e = code >> 6;
-    const d4 rj = A.s.r[__ldg(A.et.box + ebase + e) * CG_MAXATOMS + (code & 63)];
-    double dx, dy, dz;
-    const double r2 = pair_r2(PrecT<double>::drbox(A.et, ebase + e), ri.x, ri.y, ri.z, rj.x, rj.y,
-                              rj.z, dx, dy, dz);
-    fn(rj, dx, dy, dz, r2);
+    const d4 o = off[code >> 6];  // the offset, and the neighbour box
+    const d4 q = A.fx[__double2loint(o.w) * CG_MAXATOMS + (code & 63)];
+    fn(pair64(xi + __double_as_longlong(o.x) - __double_as_longlong(q.x),
+              yi + __double_as_longlong(o.y) - __double_as_longlong(q.y),
+              zi + __double_as_longlong(o.z) - __double_as_longlong(q.z), q.w));
   }
 }
 
 // rho(r); phi, phi'/r and rho'/r.  false: outside the polynomial tables
-static __device__ __forceinline__ bool rho64(const EamPot<double, EVAL_CHEBY> &P, double r2,
-                                             double &rho) {
+static __device__ __forceinline__ bool rho64(const EamPot<double, EVAL_CHEBY> &P, u64 s,
+                                             const FxUnit &u, double &rho) {
   int k;
-  double t;
-  if (!poly_at(P.poly.pair, r2, k, t)) return false;
-  rho = poly_col(P.poly.pair, PF_RHO, k, t);
+  double x;
+  if (!poly_at(P.poly.pair, s, 2 * u.m - 64, k, x)) return false;
+  rho = poly_col(P.poly.pair, PF_RHO, k, x);
   return true;
 }
 template <bool OBS>
-static __device__ __forceinline__ bool force64(const EamPot<double, EVAL_CHEBY> &P, double r2,
-                                               double &phi, double &wphi, double &wrho) {
+static __device__ __forceinline__ bool force64(const EamPot<double, EVAL_CHEBY> &P, u64 s,
+                                               const FxUnit &u, double &phi, double &wphi,
+                                               double &wrho) {
   int k;
-  double t;
-  if (!poly_at(P.poly.pair, r2, k, t)) return false;
-  if (OBS) phi = poly_col(P.poly.pair, PF_PHI, k, t);
-  wphi = poly_col(P.poly.pair, PF_GPHI, k, t);
-  wrho = poly_col(P.poly.pair, PF_GRHO, k, t);
+  double x;
+  if (!poly_at(P.poly.pair, s, 2 * u.m - 64, k, x)) return false;
+  if (OBS) phi = poly_col(P.poly.pair, PF_PHI, k, x);
+  wphi = poly_col(P.poly.pair, PF_GPHI, k, x);
+  wrho = poly_col(P.poly.pair, PF_GRHO, k, x);
   return true;
 }
-static __device__ __forceinline__ bool outside64(const EamPot<double, EVAL_CHEBY> &P, double r2) {
-  return below_seg(P, r2);
+static __device__ __forceinline__ bool outside64(const EamPot<double, EVAL_CHEBY> &P, u64 s,
+                                                 const FxUnit &u) {
+  int k;
+  double x;
+  return !poly_at(P.poly.pair, s, 2 * u.m - 64, k, x);
 }
 static __device__ __noinline__ double rho64_series(const EamPot<double, EVAL_CHEBY> &P, double r2) {
   double r, inv;
@@ -123,26 +138,28 @@ static __device__ __noinline__ void force64_series(const EamPot<double, EVAL_CHE
   wrho = cheb_series(P, 4, r) * inv;
 }
 // the table potential has no outside
-static __device__ __forceinline__ bool rho64(const EamPot<double, EVAL_TABLE> &P, double r2,
-                                             double &rho) {
+static __device__ __forceinline__ bool rho64(const EamPot<double, EVAL_TABLE> &P, u64 s,
+                                             const FxUnit &u, double &rho) {
   double r, inv;
-  r_and_inv(r2, r, inv);
+  r_and_inv(fx_area(s, u), r, inv);
   rho = table_value(P.rho, table_at(P.rho, r));
   return true;
 }
 template <bool OBS>
-static __device__ __forceinline__ bool force64(const EamPot<double, EVAL_TABLE> &P, double r2,
-                                               double &phi, double &wphi, double &wrho) {
+static __device__ __forceinline__ bool force64(const EamPot<double, EVAL_TABLE> &P, u64 s,
+                                               const FxUnit &u, double &phi, double &wphi,
+                                               double &wrho) {
   double r, inv;
-  r_and_inv(r2, r, inv);
+  r_and_inv(fx_area(s, u), r, inv);
   const TableAt p = table_at(P.phi, r);
   const TableAt q = P.same_grid ? p : table_at(P.rho, r);
   if (OBS) phi = table_value(P.phi, p);
-  wphi = table_deriv(P.phi, p) * inv;
-  wrho = table_deriv(P.rho, q) * inv;
+  wphi = __dmul_rn(table_deriv(P.phi, p), inv);
+  wrho = __dmul_rn(table_deriv(P.rho, q), inv);
   return true;
 }
-static __device__ __forceinline__ bool outside64(const EamPot<double, EVAL_TABLE> &, double) {
+static __device__ __forceinline__ bool outside64(const EamPot<double, EVAL_TABLE> &, u64,
+                                                 const FxUnit &) {
   return false;
 }
 static __device__ __forceinline__ double rho64_series(const EamPot<double, EVAL_TABLE> &, double) {
@@ -160,21 +177,22 @@ __global__ void __launch_bounds__(F64_THREADS)
   bool live;
   if (!lane_atom<LANES>(A.ntot, a, sub, live)) return;
   const int slot = A.atom_slot[a];
-  const d4 ri = A.s.r[slot];
-  const double rc2 = P.rc2;
+  const d4 fi = A.fx[slot];
+  const u64 rc2 = A.fx_rc2;
   double rho = 0.0;
   int cnt = 0;
   bool low = false;
-  walk64<LANES>(A, a, sub, slot, ri, rc2, [&](const d4 &, double, double, double, double r2) {
-    if (beyond(r2, rc2)) return;
+  walk64<LANES>(A, a, sub, slot, fi, P.rc2, [&](const Pair64 &q) {
+    if (q.s > rc2) return;
     cnt++;
     double v;
-    if (rho64(P, r2, v)) rho = __dadd_rn(rho, v);
+    if (rho64(P, q.s, A.fxu, v)) rho = __dadd_rn(rho, v);
     else low = true;
   });
   if (low)  // pairs below the table: the series, in a second sweep
-    walk64<LANES>(A, a, sub, slot, ri, rc2, [&](const d4 &, double, double, double, double r2) {
-      if (!beyond(r2, rc2) && outside64(P, r2)) rho = __dadd_rn(rho, rho64_series(P, r2));
+    walk64<LANES>(A, a, sub, slot, fi, P.rc2, [&](const Pair64 &q) {
+      if (q.s <= rc2 && outside64(P, q.s, A.fxu))
+        rho = __dadd_rn(rho, rho64_series(P, fx_area(q.s, A.fxu)));
     });
   rho = lane_sum<LANES>(rho);
   if (OBS)
@@ -183,7 +201,7 @@ __global__ void __launch_bounds__(F64_THREADS)
   double F, dF;
   eam_embed<double, EVAL>(P, rho, F, dF);
   if (sub != 0 || !live) return;
-  A.s.r[slot].w = dF;
+  A.fx[slot].w = dF;
   if (OBS) {
     A.s.rho[slot] = rho;
     A.s.fi[slot] = dF;
@@ -201,36 +219,39 @@ __global__ void __launch_bounds__(F64_THREADS)
   bool live;
   if (!lane_atom<LANES>(A.ntot, a, sub, live)) return;
   const int slot = A.atom_slot[a];
-  const d4 ri = A.s.r[slot];
-  const double rc2 = P.rc2, fii = ri.w;
+  const d4 fi = A.fx[slot];
+  const u64 rc2 = A.fx_rc2;
+  const double fii = fi.w;
   double fx = 0.0, fy = 0.0, fz = 0.0, ep = 0.0, sx = 0.0;
   bool low = false;
-  auto add = [&](const d4 &rj, double dx, double dy, double dz, double r2, double phi, double wphi,
-                 double wrho) {
-    const double we = below(r2, rc2) ? __dmul_rn(__dadd_rn(fii, rj.w), wrho) : 0.0;
-    const double w = __dadd_rn(wphi, we);
-    fx = fma(w, dx, fx);
-    fy = fma(w, dy, fy);
-    fz = fma(w, dz, fz);
+  auto add = [&](const Pair64 &q, double phi, double wphi, double wrho) {
+    const double fs = q.s < rc2 ? __dadd_rn(fii, q.fj) : 0.0;
+    const double dx = fx_length(q.x, A.fxu);
+    double w;
     if (OBS) {
+      const double we = __dmul_rn(fs, wrho);
+      w = __dadd_rn(wphi, we);
       ep = __dadd_rn(ep, phi);
       sx = fma(__dmul_rn(we, dx), dx, sx);
+    } else {
+      w = fma(fs, wrho, wphi);
     }
+    fx = fma(w, dx, fx);
+    fy = fma(w, fx_length(q.y, A.fxu), fy);
+    fz = fma(w, fx_length(q.z, A.fxu), fz);
   };
-  walk64<LANES>(A, a, sub, slot, ri, rc2, [&](const d4 &rj, double dx, double dy, double dz,
-                                              double r2) {
-    if (beyond(r2, rc2)) return;
+  walk64<LANES>(A, a, sub, slot, fi, P.rc2, [&](const Pair64 &q) {
+    if (q.s > rc2) return;
     double phi = 0.0, wphi, wrho;
-    if (force64<OBS>(P, r2, phi, wphi, wrho)) add(rj, dx, dy, dz, r2, phi, wphi, wrho);
+    if (force64<OBS>(P, q.s, A.fxu, phi, wphi, wrho)) add(q, phi, wphi, wrho);
     else low = true;
   });
   if (low)
-    walk64<LANES>(A, a, sub, slot, ri, rc2, [&](const d4 &rj, double dx, double dy, double dz,
-                                                double r2) {
-      if (beyond(r2, rc2) || !outside64(P, r2)) return;
+    walk64<LANES>(A, a, sub, slot, fi, P.rc2, [&](const Pair64 &q) {
+      if (q.s > rc2 || !outside64(P, q.s, A.fxu)) return;
       double phi, wphi, wrho;
-      force64_series(P, r2, phi, wphi, wrho);
-      add(rj, dx, dy, dz, r2, phi, wphi, wrho);
+      force64_series(P, fx_area(q.s, A.fxu), phi, wphi, wrho);
+      add(q, phi, wphi, wrho);
     });
   fx = lane_sum<LANES>(fx);
   fy = lane_sum<LANES>(fy);
@@ -260,19 +281,19 @@ __global__ void __launch_bounds__(F64_THREADS) lj64_kernel(ForceArgs A, LjPot<do
   bool live;
   if (!lane_atom<LANES>(A.ntot, a, sub, live)) return;
   const int slot = A.atom_slot[a], b = slot >> 6;
-  const d4 ri = A.s.r[slot];
-  const double s6 = P.s6, s12 = P.s6x12, c4 = P.eps4s6, rc2 = P.rc2;
+  const d4 fi = A.fx[slot];
+  const double s6 = P.s6, s12 = P.s6x12, c4 = P.eps4s6;
   double fx = 0.0, fy = 0.0, fz = 0.0, ep = 0.0, sx = 0.0;
   int cnt = 0;
-  walk64<LANES>(A, a, sub, slot, ri, rc2, [&](const d4 &, double dx, double dy, double dz,
-                                              double r2) {
-    if (beyond(r2, rc2)) return;
-    const double ir2 = reciprocal(r2);
+  walk64<LANES>(A, a, sub, slot, fi, P.rc2, [&](const Pair64 &q) {
+    if (q.s > A.fx_rc2) return;
+    const double ir2 = reciprocal(fx_area(q.s, A.fxu));
     const double r6 = __dmul_rn(__dmul_rn(ir2, ir2), ir2);
     const double fr = __dmul_rn(__dmul_rn(__dmul_rn(c4, r6), ir2), fma(s12, r6, -6.0));
+    const double dx = fx_length(q.x, A.fxu);
     fx = fma(fr, dx, fx);
-    fy = fma(fr, dy, fy);
-    fz = fma(fr, dz, fz);
+    fy = fma(fr, fx_length(q.y, A.fxu), fy);
+    fz = fma(fr, fx_length(q.z, A.fxu), fz);
     if (OBS) {
       cnt++;
       ep = fma(r6, fma(s6, r6, -1.0), ep);

@@ -5,26 +5,27 @@
 
 namespace cg {
 
-// Four threads per atom up to 2^20 atoms, then one.  4,000 atoms (LJ): 34 us
-// with four, 55 with two, 96 with one.  256,000 (table, density pass): 540 us
-// with four, 565 with two, 562 with one, 694 with eight (lists of 42 entries
-// leave the eighth lanes short).  1,048,576: 2,137 us with one, 2,235 with two.
-static bool four_lanes(int ntot) { return ntot < (1 << 20); }
-static unsigned blocks64(int ntot, int lanes) {
-  return (unsigned)(((long)ntot * lanes + F64_THREADS - 1) / F64_THREADS);
-}
+// Threads per atom.  Density + force pass without energies in us, Chebyshev
+// (16, 4, 1 threads): 4,000 atoms 22, 36, 99; 27,436 atoms 85, 66, 108; 256,000
+// atoms 658, 480, 523; 1,048,576 atoms 2,648, 1,903, 1,838 (lists of 42 entries
+// leave lanes of 16 short).  Eight threads lie between at every size, two at
+// 27,436 atoms 71.
+static int lanes64(int ntot) { return ntot < 12000 ? 16 : ntot < (1 << 19) ? 4 : 1; }
 
+template <int EVAL, bool OBS, int LANES>
+static void launch_eam64_lanes(const ForceArgs &A, const EamPot<double, EVAL> &P, int pass,
+                               cudaStream_t st) {
+  const unsigned n = (unsigned)(((long)A.ntot * LANES + F64_THREADS - 1) / F64_THREADS);
+  if (pass == 0) eam64_density_kernel<EVAL, LANES, OBS><<<n, F64_THREADS, 0, st>>>(A, P);
+  else eam64_force_kernel<EVAL, LANES, OBS><<<n, F64_THREADS, 0, st>>>(A, P);
+}
 template <int EVAL, bool OBS>
 static void launch_eam64_obs(const ForceArgs &A, const EamPot<double, EVAL> &P, int pass,
                              cudaStream_t st) {
-  const unsigned n4 = blocks64(A.ntot, 4), n1 = blocks64(A.ntot, 1);
-  if (pass == 0) {
-    if (four_lanes(A.ntot)) eam64_density_kernel<EVAL, 4, OBS><<<n4, F64_THREADS, 0, st>>>(A, P);
-    else eam64_density_kernel<EVAL, 1, OBS><<<n1, F64_THREADS, 0, st>>>(A, P);
-  } else {
-    if (four_lanes(A.ntot)) eam64_force_kernel<EVAL, 4, OBS><<<n4, F64_THREADS, 0, st>>>(A, P);
-    else eam64_force_kernel<EVAL, 1, OBS><<<n1, F64_THREADS, 0, st>>>(A, P);
-  }
+  const int lanes = lanes64(A.ntot);
+  if (lanes == 16) launch_eam64_lanes<EVAL, OBS, 16>(A, P, pass, st);
+  else if (lanes == 4) launch_eam64_lanes<EVAL, OBS, 4>(A, P, pass, st);
+  else launch_eam64_lanes<EVAL, OBS, 1>(A, P, pass, st);
 }
 
 template <int EVAL>
@@ -39,10 +40,17 @@ template void launch_eam64<EVAL_TABLE>(const ForceArgs &, const EamPot<double, E
 template void launch_eam64<EVAL_CHEBY>(const ForceArgs &, const EamPot<double, EVAL_CHEBY> &, int,
                                        cudaStream_t, bool);
 
+template <bool OBS, int LANES>
+static void launch_lj64_lanes(const ForceArgs &A, const LjPot<double> &P, cudaStream_t st) {
+  const unsigned n = (unsigned)(((long)A.ntot * LANES + F64_THREADS - 1) / F64_THREADS);
+  lj64_kernel<LANES, OBS><<<n, F64_THREADS, 0, st>>>(A, P);
+}
 template <bool OBS>
 static void launch_lj64_obs(const ForceArgs &A, const LjPot<double> &P, cudaStream_t st) {
-  if (four_lanes(A.ntot)) lj64_kernel<4, OBS><<<blocks64(A.ntot, 4), F64_THREADS, 0, st>>>(A, P);
-  else lj64_kernel<1, OBS><<<blocks64(A.ntot, 1), F64_THREADS, 0, st>>>(A, P);
+  const int lanes = lanes64(A.ntot);
+  if (lanes == 16) launch_lj64_lanes<OBS, 16>(A, P, st);
+  else if (lanes == 4) launch_lj64_lanes<OBS, 4>(A, P, st);
+  else launch_lj64_lanes<OBS, 1>(A, P, st);
 }
 void launch_lj64(const ForceArgs &A, const LjPot<double> &P, cudaStream_t st, bool obs) {
   if (A.ntot <= 0) return;

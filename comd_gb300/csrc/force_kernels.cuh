@@ -39,6 +39,11 @@ struct ForceArgs {
   int *nbr_n;            // [ntot] list length (> cap: overflowed)
   int *npair;            // [ntot] neighbours within the cutoff (written by the passes)
   int cap;
+  // FP64: positions in fixed point and F'(rho) by slot (the bits of three
+  // 64-bit integers; w), their unit, and rc^2 in that of their squares
+  d4 *fx;
+  FxUnit fxu;
+  u64 fx_rc2;
   double *atom_stress;   // [ntot] per-atom share of the scalar stress
   int *status;
   Persist pl;            // persistent lists keyed by id (FP64)

@@ -27,8 +27,8 @@ struct RebinWork {
 
 // ---- md_kernels.cu ----
 // packed box coordinates (g.boxc must point at boxc) and the stencil table
-void launch_entry_table(const Geom &g, const double *dcenter, EntryTab et, int *boxc,
-                        cudaStream_t st);
+void launch_entry_table(const Geom &g, const double *dcenter, EntryTab et, const FxUnit &fxu,
+                        int *boxc, cudaStream_t st);
 double mass_reciprocal(double rmass);
 // The Verlet and classify kernels run one thread per atom of the compacted
 // atom list atom_slot (which must match the current layout).
@@ -99,8 +99,9 @@ void launch_zc_upload(const HostSlots &hs, Slots s, int nboxes, bool forces, cud
 void launch_zc_download(const HostSlots &hs, Slots s, int nboxes, bool state, bool forces,
                         cudaStream_t st, int max_blocks = 0);
 void launch_pos32(const Geom &g, Slots s, cudaStream_t st, const int *only_if_overflow = nullptr);
-// the same over the atom list alone
-void launch_pos32_atoms(const Geom &g, Slots s, const int *atom_slot, int ntot, cudaStream_t st);
+// the same over the atom list alone; fx: also the FP64 passes' records
+void launch_pos32_atoms(const Geom &g, Slots s, const int *atom_slot, int ntot, cudaStream_t st,
+                        d4 *fx = nullptr, const FxUnit &fxu = FxUnit{});
 void launch_bin_atoms(const Geom &g, const double *dcenter, Slots s, int n, const double *xyz,
                       const double *pxyz, const int *ids, const int *types, const double *masses,
                       int *tmp_index, int *status, cudaStream_t st);

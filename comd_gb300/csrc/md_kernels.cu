@@ -19,7 +19,16 @@ namespace cg {
 // stencil table: getNeighborBoxes (domains.c:391-430) + min-image drbox
 // (eam.c:494-502), one thread per box
 // ---------------------------------------------------------------------------
-__global__ void entry_table_kernel(Geom g, const double *dcenter, EntryTab et) {
+__device__ __forceinline__ d4 fx_entry(const FxUnit &u, const double *dr, int box) {
+  d4 v;
+  v.x = __longlong_as_double(fx_from(dr[0], u));
+  v.y = __longlong_as_double(fx_from(dr[1], u));
+  v.z = __longlong_as_double(fx_from(dr[2], u));
+  v.w = __hiloint2double(0, box);
+  return v;
+}
+
+__global__ void entry_table_kernel(Geom g, const double *dcenter, EntryTab et, FxUnit fxu) {
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= g.nboxes) return;
   int base = b * CG_NNBR;
@@ -30,6 +39,8 @@ __global__ void entry_table_kernel(Geom g, const double *dcenter, EntryTab et) {
     et.dr64[base] = d4{0.0, 0.0, 0.0, 0.0};
     et.dr32[2 * base] = make_float4(0.f, 0.f, 0.f, 0.f);
     et.dr32[2 * base + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const double none[3] = {0.0, 0.0, 0.0};
+    if (et.fx) et.fx[base] = fx_entry(fxu, none, b);
     et.n[b] = 1;
     return;
   }
@@ -51,6 +62,7 @@ __global__ void entry_table_kernel(Geom g, const double *dcenter, EntryTab et) {
         }
         et.box[base + cnt] = nb;
         et.dr64[base + cnt] = d4{dr[0], dr[1], dr[2], 0.0};
+        if (et.fx) et.fx[base + cnt] = fx_entry(fxu, dr, nb);
         float hi[3];
         for (int d = 0; d < 3; d++) hi[d] = (float)dr[d];
         et.dr32[2 * (base + cnt)] = make_float4(hi[0], hi[1], hi[2], 0.f);
@@ -71,10 +83,10 @@ __global__ void box_coord_kernel(Geom g, int *boxc) {
   boxc[b] = ix[0] | (ix[1] << 10) | (ix[2] << 20);
 }
 
-void launch_entry_table(const Geom &g, const double *dcenter, EntryTab et, int *boxc,
-                        cudaStream_t st) {
+void launch_entry_table(const Geom &g, const double *dcenter, EntryTab et, const FxUnit &fxu,
+                        int *boxc, cudaStream_t st) {
   box_coord_kernel<<<(g.nboxes + 127) / 128, 128, 0, st>>>(g, boxc);
-  entry_table_kernel<<<(g.nboxes + 127) / 128, 128, 0, st>>>(g, dcenter, et);
+  entry_table_kernel<<<(g.nboxes + 127) / 128, 128, 0, st>>>(g, dcenter, et, fxu);
 }
 
 // ---------------------------------------------------------------------------
@@ -1120,17 +1132,27 @@ void launch_pos32(const Geom &g, Slots s, cudaStream_t st, const int *only_if_ov
   pos32_kernel<<<slot_blocks(g), 256, 0, st>>>(g, s, only_if_overflow);
 }
 
+// fx (optional): also the fixed-point records of an FP64 force call
 __global__ void __launch_bounds__(256) pos32_atoms_kernel(Geom g, Slots s, const int *atom_slot,
-                                                          int ntot) {
+                                                          int ntot, d4 *fx, FxUnit fxu) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= ntot) return;
   const int slot = atom_slot[a];
   const d4 r = s.r[slot];
   s.pos32[slot] = centred32(rep_of(g, slot >> 6), r.x, r.y, r.z);
+  if (!fx) return;
+  d4 v;
+  v.x = __longlong_as_double(fx_from(r.x, fxu));
+  v.y = __longlong_as_double(fx_from(r.y, fxu));
+  v.z = __longlong_as_double(fx_from(r.z, fxu));
+  v.w = 0.0;
+  fx[slot] = v;
 }
 
-void launch_pos32_atoms(const Geom &g, Slots s, const int *atom_slot, int ntot, cudaStream_t st) {
-  if (ntot > 0) pos32_atoms_kernel<<<atom_blocks(ntot), 256, 0, st>>>(g, s, atom_slot, ntot);
+void launch_pos32_atoms(const Geom &g, Slots s, const int *atom_slot, int ntot, cudaStream_t st,
+                        d4 *fx, const FxUnit &fxu) {
+  if (ntot > 0)
+    pos32_atoms_kernel<<<atom_blocks(ntot), 256, 0, st>>>(g, s, atom_slot, ntot, fx, fxu);
 }
 
 // ---------------------------------------------------------------------------

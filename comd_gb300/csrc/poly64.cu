@@ -5,7 +5,7 @@
 // lo with about 106 bits; sums by Knuth's two-sum, products by one fused
 // multiply-add, Dekker's scheme).  Six lanes then form one monomial
 // coefficient each from the samples, by the inverse of the nodes'
-// Vandermonde matrix (the same for all segments but for powers of two), and
+// Vandermonde matrix (the same for all segments), and
 // round it once; the two others check the ends, where the error of
 // interpolation at these nodes peaks.  FP64 operations bound it: 0.37 ms
 // for the Cu tables, once per potential (2.75 ms with one thread per
@@ -141,7 +141,6 @@ __global__ void __launch_bounds__(FIT_THREADS)
     end = add(mul(end, from(x)), pj);
   }
   if (lane < NP) {
-    for (int j = 0; j < lane; j++) p = {p.h / half, p.l / half};
     reinterpret_cast<double *>(c + (size_t)id * POLY_REC)[lane] = p.h + p.l;
   } else if (!(fabs(sub(end, sample).h) <= column_bound<TABLE>(S, q, mid))) {
     atomicMin(first_bad, k);

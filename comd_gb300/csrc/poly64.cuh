@@ -5,9 +5,9 @@
 // clock, so summing the series for every pair bounds the FP64 kernels.  The
 // pair functions are instead degree-5 polynomials in s = r^2 (no square
 // root) on segments that are the 256 equal parts of each binade of s: the
-// segment index is the top bits of s, its centre the index with the next bit
-// set, so an evaluation takes one FP64 subtraction and five fused
-// multiply-adds.  The embedding function has the same form in rho.  At
+// segment index is the top bits of s and the offset x in it, from -1 to 1, the
+// bits below, so an evaluation takes six FP64 operations: one for x, five
+// fused multiply-adds.  The embedding function has the same form in rho.  At
 // 256,000 atoms the first FP64 pass took 8,342 us with the series and takes
 // 750 us, the second 3,267 and 577 us.
 //
@@ -54,7 +54,7 @@ struct PolyShape<PT_EMBED> {
 };
 
 // segment k of the table: arguments whose top bits are base + k; column q of
-// it at c + (k * cols + q) * POLY_REC.  n = 0: no table.
+// it, coefficients in x, at c + (k * cols + q) * POLY_REC.  n = 0: no table.
 template <int TABLE>
 struct Poly64 {
   const double2 *c;
@@ -66,14 +66,29 @@ struct PolyTables {
   Poly64<PT_EMBED> embed;
 };
 
-// segment k and offset t from its centre; false outside the table (NaN
-// included)
+// segment k and offset x in it; false outside the table (NaN included)
 template <int TABLE>
-__device__ __forceinline__ bool poly_at(const Poly64<TABLE> &p, double x, int &k, double &t) {
-  constexpr int sh = 20 - PolyShape<TABLE>::bits;
-  const int i = __double2hiint(x) >> sh;
-  t = __dsub_rn(x, __hiloint2double((i << sh) | (1 << (sh - 1)), 0));
-  k = i - p.base;
+__device__ __forceinline__ bool poly_at(const Poly64<TABLE> &p, double v, int &k, double &x) {
+  constexpr int bits = PolyShape<TABLE>::bits, sh = 20 - bits;
+  const int hi = __double2hiint(v), lo = __double2loint(v);
+  // 1 + the fraction of the segment
+  const double y = __hiloint2double(0x3ff00000 | ((hi << bits) & 0xfffff) |
+                                        (int)((unsigned)lo >> (32 - bits)), lo << bits);
+  x = __fma_rn(2.0, y, -3.0);
+  k = (hi >> sh) - p.base;
+  return (unsigned)k < (unsigned)p.n;
+}
+// the same from a fixed-point argument s * 2^e, s > 0 (fixed64.cuh)
+template <int TABLE>
+__device__ __forceinline__ bool poly_at(const Poly64<TABLE> &p, unsigned long long s, int e,
+                                        int &k, double &x) {
+  constexpr int bits = PolyShape<TABLE>::bits;
+  const int lz = __clzll((long long)s);
+  const unsigned long long m = (s << (lz & 63)) << 1;  // the bits below the leading one
+  const unsigned long long f = m << bits;
+  const double y = __hiloint2double(0x3ff00000 | (int)(f >> 44), (int)(unsigned)(f >> 12));
+  x = __fma_rn(2.0, y, -3.0);
+  k = ((1023 + 63 + e - lz) << bits) + (int)(m >> (64 - bits)) - p.base;
   return (unsigned)k < (unsigned)p.n;
 }
 

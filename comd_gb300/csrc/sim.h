@@ -78,6 +78,9 @@ struct comdgb_sim {
   // list capacities as allocated (comdgb_sim_set_list_capacity may lower the
   // capacity in use): per-step, id-keyed and force-order lists
   int cap_alloc = 0, pl_vcap_alloc = 0, fo_vcap_alloc = 0;
+  // FP64: fixed-point positions by slot and their unit (fixed64.cuh)
+  d4 *fx = nullptr;
+  cg::FxUnit fxu{};
   double *atom_stress = nullptr;
   double *rpart = nullptr;
   long long *ripart = nullptr;

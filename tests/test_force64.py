@@ -1,0 +1,61 @@
+"""The FP64 passes against the oracle where their shape changes: either side of
+12,000 atoms (16 and 4 threads an atom) and past 2^19 (one), with an atom taken
+out so that the atoms do not fill the last warp, and box widths that put the
+fixed-point unit on both sides of a power of two (LJ cutoffs of 3.9 and 4.1 A).
+Tolerances as in the FP64 parity tests: the sums differ in order alone."""
+import pytest
+
+import comd_gb300 as cg
+from helpers import Case, compare_forces
+from test_fo_lanes import without_last_atom
+
+pytestmark = pytest.mark.gpu
+
+
+def check(c):
+    c.oracle_force()
+    d = c.device(cg.PREC_FP64)
+    e, _ = d.force()
+    d.download(c.s)
+    d.close()
+    cmp = compare_forces(c.s, c.o)
+    assert cmp["f_max_rel"] < 1e-11 and cmp["e_max_rel"] < 1e-11, cmp
+    if c.potential != cg.POT_LJ:
+        assert cmp["rho_max_rel"] < 1e-12 and cmp["fi_max_rel"] < 1e-12, cmp
+    assert abs(e - c.o.contents.e) <= 1e-12 * abs(c.o.contents.e)
+
+
+@pytest.mark.parametrize("potential", [cg.POT_EAM_TABLE, cg.POT_EAM_CHEBY, cg.POT_LJ])
+@pytest.mark.parametrize("edges", [(7, 6, 8), (15, 14, 15)])
+def test_threads_per_atom(oracle, potential, edges):
+    c = Case(oracle, potential, n=edges, temp=300.0)
+    try:
+        without_last_atom(c)
+        check(c)
+    finally:
+        c.close()
+
+
+def test_one_thread_per_atom(oracle):
+    c = Case(oracle, cg.POT_EAM_TABLE, n=(51, 51, 51), temp=300.0)
+    try:
+        without_last_atom(c)
+        check(c)
+    finally:
+        c.close()
+
+
+@pytest.mark.parametrize("cutoff", [3.9, 4.1])
+def test_fixed_point_unit(oracle, cutoff):
+    c = Case(oracle, cg.POT_LJ, n=(7, 7, 8), temp=300.0, amp=0.03)
+    pot = cg.lj_potential(2.315, 0.167 / 27.211386245988, cutoff, 63.55)
+    try:
+        oracle.free(c.o)
+        cg.free_host(c.s)
+        c.pot, c.s = pot, cg.fcc(7, 7, 8, 3.615, 1.0, 1.0, pot)
+        cg.seed(c.s, 3, cg.DISP_GAUSSIAN, 0.03, 300.0, 63.55)
+        assert oracle.rebox(c.s) == 0
+        c.o = oracle.clone(c.s)
+        check(c)
+    finally:
+        c.close()
