@@ -532,6 +532,35 @@ int fit_cheb_gpu(comdgb_sim *h, const eampotential_t *pot, double coef[6][CG_NCH
   return 0;
 }
 
+// The polynomials of the table potential's intervals up to the cutoff (the same
+// intervals for phi and rho).  A table that starts below 0, ends before the
+// cutoff or has more intervals than the FP32 estimate of the index tells apart
+// keeps the formula, and so does one where the polynomials miss it past the
+// first quarter of the intervals.
+int build_tabpoly(comdgb_sim *h, const potentialarray_t *phi) {
+  const double last = (h->cutoff - phi->x0) * phi->invDx;
+  if (!(phi->x0 >= 0.0 && h->cutoff <= phi->xn && last >= 0.0 && last <= phi->n &&
+        h->cutoff * phi->invDx <= TABPOLY_MAX))
+    return 0;
+  const int n = std::min(phi->n, (int)last + 1);
+  int err = 0, bad = 0;
+  double4_32a *out = track(h, dalloc<double4_32a>(tabpoly_size(n), &err));
+  int *flag = track(h, dalloc<int>(1, &err));
+  if (err) return set_err(COMDGB_ERR_NOMEM, "cudaMalloc failed for EAM tables");
+  CK(cudaMemsetAsync(flag, 0, sizeof(int), h->stream));
+  launch_tab_fit(TabFit{h->eam64t.phi.v, h->eam64t.rho.v, phi->x0, phi->invDx, n}, h->fxu, out,
+                 flag, h->stream);
+  CK(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  const double r_lo = phi->x0 + (bad + 0.5) / phi->invDx;  // inside the first good interval
+  const u64 s_lo = bad ? (u64)std::ldexp(r_lo * r_lo, 64 - 2 * h->fxu.m) : 0;
+  if (bad < n / 4)
+    h->eam64t.tpoly = TabPoly{out, out + 2 * (size_t)n, out + 5 * (size_t)n,
+                              (float)std::ldexp(phi->invDx, h->fxu.m - 16),
+                              (float)(-phi->x0 * phi->invDx), n, s_lo};
+  return 0;
+}
+
 // the tables of phi and rho (the same intervals) as FoTab
 FoTab build_fotab(comdgb_sim *h, const potentialarray_t *phi, const potentialarray_t *rho,
                   int *err) {
@@ -588,6 +617,10 @@ int setup_potential(comdgb_sim *h, const simflat_t *s) {
     h->eam32t.rho = upload_table<float>(h, ep->rho, &err);
     h->eam32t.f = upload_table<float>(h, ep->f, &err);
     h->eam32t.rc2 = (float)rc2;
+    if (!err && !h->mixed && h->eam64t.same_grid) {
+      const int rc = build_tabpoly(h, ep->phi);
+      if (rc) return rc;
+    }
     if (h->mixed && h->eam64t.same_grid && ep->phi->n <= FOTAB_MAX)
       h->eam32t.tab = build_fotab(h, ep->phi, ep->rho, &err);
     if (err) return set_err(COMDGB_ERR_NOMEM, "cudaMalloc failed for EAM tables");

@@ -137,9 +137,43 @@ static __device__ __noinline__ void force64_series(const EamPot<double, EVAL_CHE
   wphi = cheb_series(P, 3, r) * inv;
   wrho = cheb_series(P, 4, r) * inv;
 }
-// the table potential has no outside
+// The record of s (rec doubles of 32 bytes each) and the argument t = s - S0
+// of its polynomials: the interval by an FP32 estimate, good to within one,
+// and the ends in the record.
+template <int REC>
+__device__ __forceinline__ const d4 *tab_record(const TabPoly &T, const d4 *tab, u64 s,
+                                                const FxUnit &u, d4 &first, double &t) {
+  const float sf = (float)(unsigned)(s >> 32);
+  int i = (int)fmaf(sf * rsqrtf(sf), T.ku, T.off);  // (sf = 0: NaN, interval 0)
+  i = max(0, min(i, T.n - 1));
+  const d4 *rec = tab + REC * i;
+  first = rec[0];
+  const u64 lo = (u64)__double_as_longlong(first.x), hi = (u64)__double_as_longlong(first.y);
+  const int step = s < lo ? (i > 0 ? -1 : 0) : s >= hi ? 1 : 0;
+  if (step != 0) {
+    rec += REC * step;
+    first = rec[0];
+  }
+  const u64 s0 = (u64)__double_as_longlong(first.x);
+  t = fx_area(s > s0 ? s - s0 : 0, u);  // (below the table: its lower end)
+  return rec;
+}
+__device__ __forceinline__ double quartic(double c0, double c1, double c2, double c3, double c4,
+                                          double t) {
+  return fma(fma(fma(fma(c4, t, c3), t, c2), t, c1), t, c0);
+}
+
 static __device__ __forceinline__ bool rho64(const EamPot<double, EVAL_TABLE> &P, u64 s,
                                              const FxUnit &u, double &rho) {
+  if (P.tpoly.n > 0) {
+    if (s < P.tpoly.s_lo) return false;
+    d4 a;
+    double t;
+    const d4 *rec = tab_record<2>(P.tpoly, P.tpoly.rho, s, u, a, t);
+    const d4 b = rec[1];
+    rho = quartic(a.z, a.w, b.x, b.y, b.z, t);
+    return true;
+  }
   double r, inv;
   r_and_inv(fx_area(s, u), r, inv);
   rho = table_value(P.rho, table_at(P.rho, r));
@@ -149,6 +183,21 @@ template <bool OBS>
 static __device__ __forceinline__ bool force64(const EamPot<double, EVAL_TABLE> &P, u64 s,
                                                const FxUnit &u, double &phi, double &wphi,
                                                double &wrho) {
+  if (P.tpoly.n > 0) {
+    if (s < P.tpoly.s_lo) return false;
+    d4 a;
+    double t;
+    const d4 *rec = tab_record<3>(P.tpoly, P.tpoly.force, s, u, a, t);
+    const d4 b = rec[1], c = rec[2];
+    wphi = quartic(a.z, a.w, b.x, b.y, b.z, t);
+    wrho = quartic(b.w, c.x, c.y, c.z, c.w, t);
+    if (OBS) {
+      const d4 *f = P.tpoly.phi + 2 * ((rec - P.tpoly.force) / 3);
+      const d4 e = f[0];
+      phi = quartic(e.x, e.y, e.z, e.w, f[1].x, t);
+    }
+    return true;
+  }
   double r, inv;
   r_and_inv(fx_area(s, u), r, inv);
   const TableAt p = table_at(P.phi, r);
@@ -158,15 +207,24 @@ static __device__ __forceinline__ bool force64(const EamPot<double, EVAL_TABLE> 
   wrho = __dmul_rn(table_deriv(P.rho, q), inv);
   return true;
 }
-static __device__ __forceinline__ bool outside64(const EamPot<double, EVAL_TABLE> &, u64,
+static __device__ __forceinline__ bool outside64(const EamPot<double, EVAL_TABLE> &P, u64 s,
                                                  const FxUnit &) {
-  return false;
+  return P.tpoly.n > 0 && s < P.tpoly.s_lo;
 }
-static __device__ __forceinline__ double rho64_series(const EamPot<double, EVAL_TABLE> &, double) {
-  return 0.0;
+static __device__ __noinline__ double rho64_series(const EamPot<double, EVAL_TABLE> &P, double r2) {
+  double r, inv;
+  r_and_inv(r2, r, inv);
+  return table_value(P.rho, table_at(P.rho, r));
 }
-static __device__ __forceinline__ void force64_series(const EamPot<double, EVAL_TABLE> &, double,
-                                                      double &, double &, double &) {}
+static __device__ __noinline__ void force64_series(const EamPot<double, EVAL_TABLE> &P, double r2,
+                                                   double &phi, double &wphi, double &wrho) {
+  double r, inv, dphi, v, drho;
+  r_and_inv(r2, r, inv);
+  table_eval(P.phi, r, phi, dphi);
+  table_eval(P.rho, r, v, drho);
+  wphi = dphi * inv;
+  wrho = drho * inv;
+}
 
 // rho_i = sum of rho(r_ij), F'(rho_i) for the force pass; OBS: also rho, F'
 // and F(rho_i) (left in f's fourth component) and the pairs counted
@@ -189,7 +247,7 @@ __global__ void __launch_bounds__(F64_THREADS)
     if (rho64(P, q.s, A.fxu, v)) rho = __dadd_rn(rho, v);
     else low = true;
   });
-  if (low)  // pairs below the table: the series, in a second sweep
+  if (low)  // pairs below the polynomials: the series or the interpolation, in a second sweep
     walk64<LANES>(A, a, sub, slot, fi, P.rc2, [&](const Pair64 &q) {
       if (q.s <= rc2 && outside64(P, q.s, A.fxu))
         rho = __dadd_rn(rho, rho64_series(P, fx_area(q.s, A.fxu)));

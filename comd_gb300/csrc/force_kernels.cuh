@@ -571,6 +571,7 @@ struct EamPot {
   ChebLow32 chlo;  // FP32 only
   PairSeg seg;     // FP32 Chebyshev only
   PolyTables poly; // FP64 Chebyshev only
+  TabPoly tpoly;   // FP64 tables only
   FoTab tab;       // FP32 tables only
   T rc2;
   bool same_grid;  // the tables of phi and rho have the same intervals

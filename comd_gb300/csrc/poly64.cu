@@ -178,6 +178,85 @@ void fit(const PolySeries *series, int base, int n, double2 *c, int *first_bad, 
         series, node_matrix(), base, n, c, first_bad);
 }
 
+// a double-double number times 2^e as an integer (below 2^63)
+__device__ __forceinline__ u64 to_fixed(dd a, int e) {
+  return (u64)((long long)ldexp(a.h, e) + __double2ll_rd(ldexp(a.l, e) + (ldexp(a.h, e) - floor(ldexp(a.h, e)))));
+}
+
+// One thread per (interval, function): five Chebyshev nodes in s, Newton's
+// differences, monomials in s - S0.
+__global__ void __launch_bounds__(FIT_THREADS)
+    tab_fit_kernel(TabFit T, FxUnit u, double4_32a *out, int *bad) {
+  constexpr int M = 5;
+  const int id = blockIdx.x * FIT_THREADS + threadIdx.x;
+  const int i = id >> 2, q = id & 3;  // rho, phi, phi'/r, rho'/r
+  if (i >= T.n) return;
+  const int up = 64 - 2 * u.m;
+  const double *w = (q == 0 || q == 3) ? T.rho : T.phi;
+  const dd inv = from(T.invDx);
+  const dd r0 = add(from(T.x0), div(from((double)i), inv));
+  const dd r1 = add(from(T.x0), div(from((double)(i + 1)), inv));
+  const u64 S0 = to_fixed(mul(r0, r0), up), S1 = to_fixed(mul(r1, r1), up);
+  const dd s0 = {ldexp((double)(S0 >> 32), 32 - up), ldexp((double)(unsigned)S0, -up)};
+  const double width = ldexp((double)(S1 - S0), -up);
+  // the coefficients the formula takes (its table_value and table_deriv)
+  const double g0 = w[i + 1] - w[i - 1], g1 = w[i + 2] - w[i];
+  const double c0 = w[i], c1 = 0.5 * g0, c2 = 0.5 * (w[i + 1] + w[i - 1] - 2.0 * w[i]);
+  const double d0 = i <= 0 ? 0.0 : 0.5 * g0 * T.invDx, d1 = i <= 0 ? 0.0 : 0.5 * (g1 - g0) * T.invDx;
+  auto eval = [&](double t) {
+    const dd r = root(add(quick(s0.h, s0.l), from(t)));
+    const dd v = mul(sub(r, r0), inv);
+    if (q < 2) return add(from(c0), mul(v, add(from(c1), mul(v, from(c2)))));
+    return div(add(from(d0), mul(v, from(d1))), r);
+  };
+  double t[M];
+  dd v[M], p[M];
+#pragma unroll
+  for (int j = 0; j < M; j++) {
+    t[j] = width * (0.5 + 0.5 * cospi((j + 0.5) / M));
+    v[j] = eval(t[j]);
+    p[j] = from(0.0);
+  }
+#pragma unroll
+  for (int m = 1; m < M; m++)
+#pragma unroll
+    for (int j = M - 1; j >= m; j--)
+      v[j] = div(sub(v[j], v[j - 1]), sub(from(t[j]), from(t[j - m])));
+#pragma unroll
+  for (int m = M - 1; m >= 0; m--) {
+#pragma unroll
+    for (int j = M - 1; j > 0; j--) p[j] = sub(p[j - 1], mul(p[j], from(t[m])));
+    p[0] = add(neg(mul(p[0], from(t[m]))), v[m]);
+  }
+  double c[M];
+#pragma unroll
+  for (int j = 0; j < M; j++) c[j] = p[j].h + p[j].l;
+  for (int e = 0; e < 2; e++) {  // both ends
+    const double at = e ? width : 0.0;
+    dd s = from(0.0);
+#pragma unroll
+    for (int j = M - 1; j >= 0; j--) s = add(mul(s, from(at)), p[j]);
+    // half an ulp of the value at the lower end, and of r in the rest
+    const double steps = r0.h * T.invDx;
+    const double size = q < 2 ? fabs(c0) + steps * (fabs(c1) + fabs(c2))
+                              : (fabs(d0) + steps * fabs(d1)) / r0.h;
+    if (!(fabs(sub(s, eval(at)).h) <= 0x1p-53 * size)) atomicMax(bad, i + 1);
+  }
+  // the ends of the first and the last interval are open
+  const double lo = __longlong_as_double((long long)S0);
+  const double hi = __longlong_as_double(i == T.n - 1 ? 0x7fffffffffffffffLL : (long long)S1);
+  double *rho = reinterpret_cast<double *>(out) + 8 * (size_t)i;
+  double *frc = reinterpret_cast<double *>(out + 2 * (size_t)T.n) + 12 * (size_t)i;
+  double *phi = reinterpret_cast<double *>(out + 5 * (size_t)T.n) + 8 * (size_t)i;
+  double *to = q == 0 ? rho + 2 : q == 1 ? phi : q == 2 ? frc + 2 : frc + 7;
+#pragma unroll
+  for (int j = 0; j < M; j++) to[j] = c[j];
+  if (q == 0 || q == 2) {
+    (q == 0 ? rho : frc)[0] = lo;
+    (q == 0 ? rho : frc)[1] = hi;
+  }
+}
+
 int index_of(double x, int bits) {
   unsigned long long b;
   memcpy(&b, &x, sizeof b);
@@ -217,6 +296,11 @@ void launch_poly_fit(int table, const PolySeries *series, int base, int n, doubl
   if (table == PT_PAIR) fit<PT_PAIR>(series, base, n, c, first_bad, st);
   else if (table == PT_HESS) fit<PT_HESS>(series, base, n, c, first_bad, st);
   else fit<PT_EMBED>(series, base, n, c, first_bad, st);
+}
+
+void launch_tab_fit(const TabFit &t, const FxUnit &u, double4_32a *out, int *bad,
+                    cudaStream_t st) {
+  tab_fit_kernel<<<(4 * t.n + FIT_THREADS - 1) / FIT_THREADS, FIT_THREADS, 0, st>>>(t, u, out, bad);
 }
 
 }  // namespace cg

@@ -27,6 +27,8 @@
 
 #include <cuda_runtime.h>
 
+#include "fixed64.cuh"
+
 namespace cg {
 
 constexpr int POLY_REC = 3;  // double2 per polynomial: degree 5
@@ -121,5 +123,41 @@ size_t poly_size(int table, int n);
 // lowered to the first segment with a polynomial that misses its series.
 void launch_poly_fit(int table, const PolySeries *series, int base, int n, double2 *c,
                      int *first_bad, cudaStream_t st);
+
+// The table potential in the same spirit.  eamInterpolateDeriv (eam.c:401-434)
+// is a quadratic in r on each of the table's intervals and its derivative
+// linear, so phi, rho, phi'/r and rho'/r are smooth functions of s = r^2
+// there: degree-4 polynomials in s from the interval's lower end, in place of
+// a square root, a division and the index arithmetic (14 FP64 operations a
+// pair of the density pass, now five).  The interval has to be the exact one,
+// the derivative having a kink at each end: an FP32 estimate of r gives it to
+// within one, the record's own ends (integers, fixed64.cuh) decide.
+// Fitted and checked as the series' polynomials are: within what half an ulp
+// of the value or of r changes.  Pairs below s_lo, inside the first interval
+// after the last that misses it (the Cu tables' first, next to their guard
+// value, at 1 A), take the formula.
+// 256,000 atoms, density + forces: 354 + 469 -> 132 + 271 us.
+struct TabPoly {
+  const double4_32a *rho;    // [2 n] (S0, S1, c0, c1) (c2, c3, c4, -), S the bits of the ends
+  const double4_32a *force;  // [3 n] (S0, S1, a0, a1) (a2, a3, a4, b0) (b1, b2, b3, b4):
+                             // a phi'/r, b rho'/r
+  const double4_32a *phi;    // [2 n] (c0, c1, c2, c3) (c4, -, -, -)
+  float ku, off;             // the interval from sqrt(s >> 32): ku * that + off
+  int n;                     // 0: none
+  u64 s_lo;
+};
+constexpr int TABPOLY_MAX = 1 << 16;
+constexpr size_t tabpoly_size(int n) { return 7 * (size_t)n; }  // in 32-byte records
+
+// a table as the fit reads it: values v[-1 .. n + 1]
+struct TabFit {
+  const double *phi, *rho;
+  double x0, invDx;
+  int n;
+};
+// into out (the three arrays one after the other); *bad (0 at first) becomes
+// one more than the last interval with a polynomial that misses its formula
+void launch_tab_fit(const TabFit &t, const FxUnit &u, double4_32a *out, int *bad,
+                    cudaStream_t st);
 
 }  // namespace cg

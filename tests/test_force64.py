@@ -2,10 +2,13 @@
 12,000 atoms (16 and 4 threads an atom) and past 2^19 (one), with an atom taken
 out so that the atoms do not fill the last warp, and box widths that put the
 fixed-point unit on both sides of a power of two (LJ cutoffs of 3.9 and 4.1 A).
-Tolerances as in the FP64 parity tests: the sums differ in order alone."""
+A table's intervals are polynomials in r^2 up to the cutoff, the ones near its
+lower end the formula: pairs are put on both sides of every end there, and below
+the table.  Tolerances as in the FP64 parity tests: the sums differ in order alone."""
 import pytest
 
 import comd_gb300 as cg
+from comd_gb300.abi import slot_views
 from helpers import Case, compare_forces
 from test_fo_lanes import without_last_atom
 
@@ -56,6 +59,25 @@ def test_fixed_point_unit(oracle, cutoff):
         cg.seed(c.s, 3, cg.DISP_GAUSSIAN, 0.03, 300.0, 63.55)
         assert oracle.rebox(c.s) == 0
         c.o = oracle.clone(c.s)
+        check(c)
+    finally:
+        c.close()
+
+
+# distances in table intervals from the table's lower end; the derivative jumps
+# at 1 and 0 (its first interval counts as flat), so none lies on an end
+@pytest.mark.parametrize("at", [-200.3, -0.5, 0.5, 0.9999, 1.0001, 1.5, 1.9999, 2.0001, 7.3, 150.2])
+def test_close_pair_of_a_table(oracle, at):
+    c = Case(oracle, cg.POT_EAM_TABLE, n=(6, 6, 7), temp=300.0, amp=0.03)
+    try:
+        phi = c.pot.ptr.contents.phi.contents
+        v = slot_views(c.s)
+        assert v["natoms"][0] > 1
+        v["r"][1] = v["r"][0]
+        v["r"][1, 0] += phi.x0 + at / phi.invDx
+        assert oracle.rebox(c.s) == 0
+        c.oracle.free(c.o)
+        c.o = c.oracle.clone(c.s)
         check(c)
     finally:
         c.close()
