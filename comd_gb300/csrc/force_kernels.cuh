@@ -212,76 +212,53 @@ __device__ __forceinline__ void for_each_neighbor(const ForceArgs &A, int a, int
 // neighbour-list build: one CTA per box, one warp per atom of the box
 // ---------------------------------------------------------------------------
 #define NB_THREADS 128
-#define NB_MAXC (CG_NNBR * CG_MAXATOMS)
+#define NB_TILE 768  // candidates staged at a time (27 boxes of 64 are 1,728)
 
-// stencil entries of box b: boxes, box offsets and candidate offsets (warp 0)
-template <class T>
+// The stencil entries of box b (warp 0): boxes, box offsets, candidate offsets
+// and, in s_code, each entry's stencil index (the passes take the box offset
+// from it).  SORT: by neighbour box (ties by entry), so that every list comes
+// out in ascending neighbour slot -- atoms in force order are in box order,
+// and lanes of a warp then walk the position array together.  The lanes take
+// the entries in the order that an interior box's come out in; only where the
+// boxes wrap are they ranked.
+template <bool SORT>
 __device__ __forceinline__ int stage_entries(const ForceArgs &A, int b, int *s_box, int *s_off,
-                                             BoxOff<T> *s_dr) {
+                                             BoxOff<float> *s_dr, int *s_code) {
   const int ne = A.et.n[b];
   if (threadIdx.x < 32) {
-    const int e = threadIdx.x;
-    int n = 0;
-    if (e < ne) {
-      int jb = A.et.box[b * CG_NNBR + e];
-      s_box[e] = jb;
-      s_dr[e] = PrecT<T>::drbox(A.et, b * CG_NNBR + e);
-      n = min(A.s.natoms[jb], CG_MAXATOMS);  // (more only in a reported overflow)
+    const int l = threadIdx.x;
+    const bool in = l < ne;
+    const int e = SORT && ne == CG_NNBR ? (l % 3) * 9 + ((l / 3) % 3) * 3 + l / 9 : l;
+    const int jb = in ? A.et.box[b * CG_NNBR + e] : 0x7fffffff;
+    int rank = l;
+    if (SORT) {
+      const int before = __shfl_up_sync(0xffffffffu, jb, 1);
+      if (!__all_sync(0xffffffffu, l == 0 || !in || before < jb)) {
+        rank = 0;
+        for (int q = 0; q < ne; q++) {
+          const int jq = __shfl_sync(0xffffffffu, jb, q), eq = __shfl_sync(0xffffffffu, e, q);
+          rank += jq < jb || (jq == jb && eq < e);
+        }
+      }
     }
-    int x = n;  // inclusive warp scan
-    for (int o = 1; o < 32; o <<= 1) {
-      int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (e >= o) x += y;
+    if (in) {
+      s_box[rank] = jb;
+      s_dr[rank] = PrecT<float>::drbox(A.et, b * CG_NNBR + e);
+      s_code[rank] = e;
+      // (more than 64 only in a reported overflow)
+      s_off[rank + 1] = min(A.s.natoms[jb], CG_MAXATOMS);
     }
-    if (e < ne) s_off[e + 1] = x;
-    if (e == 0) s_off[0] = 0;
+    __syncwarp();
+    int x = in ? s_off[l + 1] : 0;
+    for (int o = 1; o < 32; o <<= 1) {  // inclusive scan
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (l >= o) x += y;
+    }
+    if (in) s_off[l + 1] = x;
+    if (l == 0) s_off[0] = 0;
   }
   __syncthreads();
   return ne;
-}
-
-// FP32 lists: the staged entries sorted by neighbour box (ties by entry),
-// so that every list comes out in ascending neighbour slot -- atoms in force
-// order are in box order, and lanes of a warp then walk the position array
-// together.  s_code keeps each entry's stencil index (the passes take the
-// box offset from it); s_off is rebuilt in the new order.
-__device__ __forceinline__ void order_entries_by_box(int ne, int *s_box, int *s_off,
-                                                     BoxOff<float> *s_dr, int *s_code) {
-  if (threadIdx.x < 32) {
-    const int e = threadIdx.x;
-    const int jb = e < ne ? s_box[e] : 0x7fffffff;
-    BoxOff<float> dr{};
-    int n = 0;
-    if (e < ne) {
-      dr = s_dr[e];
-      n = s_off[e + 1] - s_off[e];
-    }
-    int rank = 0;
-    for (int q = 0; q < ne; q++) {
-      const int jq = __shfl_sync(0xffffffffu, jb, q);
-      rank += (jq < jb) || (jq == jb && q < e);
-    }
-    // n of the entry at each rank, for the new prefix
-    int x = 0;
-    for (int q = 0; q < ne; q++) {
-      const int rq = __shfl_sync(0xffffffffu, rank, q);
-      const int nq = __shfl_sync(0xffffffffu, n, q);
-      if (rq == e) x = nq;
-    }
-    __syncwarp();
-    if (e < ne) {
-      s_box[rank] = jb;
-      s_dr[rank] = dr;
-      s_code[rank] = e;
-    }
-    for (int o = 1; o < 32; o <<= 1) {  // inclusive scan over ranks
-      const int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (e >= o) x += y;
-    }
-    if (e < ne) s_off[e + 1] = x;
-    if (e == 0) s_off[0] = 0;
-  }
-  __syncthreads();
 }
 
 // force-order entry code of stencil entry e = (dx+1)*9 + (dy+1)*3 + (dz+1)
@@ -291,29 +268,19 @@ __device__ __forceinline__ int fo_code(int e) {
   return (e / 9) | (((e / 3) % 3) << 2) | ((e % 3) << 4);
 }
 
-__device__ __forceinline__ int entry_of(const int *s_off, int ne, int c) {
-  int lo = 0, hi = ne - 1;  // last e with s_off[e] <= c
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (s_off[mid] <= c) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
-
-// FP32: candidates staged as (x - drbox, y - drbox, z - drbox, code) in the
+// FP32: candidates staged as (x - drbox, y - drbox, z - drbox, key) in the
 // centre box's frame, padded to whole 32-candidate chunks with far-away
-// sentinels.  Each warp takes two atoms per candidate load and parks every
-// chunk's ballot in warp-private shared memory; the warp then writes each
-// atom's list cooperatively (one mask word per lane, prefix sum of the
-// popcounts, each lane emits its own bits).  The cutoff of the build (rc2b)
+// sentinels.  A warp tests NA atoms against every chunk it loads and appends
+// the hits of each to its list at once: the ballot's bits below the lane give
+// the place.  The cutoff of the build (rc2b)
 // is widened by more than the FP32 distances err (list_cutoff in api.cu), so
 // the list holds every pair that the passes accept with their exact dr.  The
 // FP64 simulations use the same build on FP32 copies of their positions: an
 // FP64 test of every candidate, 12 operations for each of seven candidates
-// per neighbour, took 1,785 us for the lists of 256,000 atoms, this
-// 270 us.
-#define NB_CHUNKS (NB_MAXC / 32)  // 54
+// per neighbour, took 1,785 us for the lists of 256,000 atoms.
+// Bound by the instructions issued.  Parking the ballots in shared memory and
+// finding the h-th set bit (__fns) for full-warp stores took more of them
+// than the tests: 270 us for those lists, 129 now (65% of the issue slots).
 #define NB_ATOMS 4                 // atoms tested per candidate load
 // Modes: LIST_STEP writes the per-step list (uint16 codes); LIST_ID (runs
 // only when a rebuild is due) writes neighbour ids into the atom's id-keyed
@@ -349,14 +316,6 @@ __device__ __forceinline__ int build_row(const ForceArgs &A, int b, int i) {
 }
 
 template <int MODE>
-__device__ __forceinline__ void build_store(const ForceArgs &A, int row, int h, int value) {
-  if (MODE == LIST_ID) A.pl.vlist[(size_t)row * A.pl.vcap + h] = value;
-  else if (MODE == LIST_FO)
-    A.fo.list[((size_t)(row >> 5) * A.fo.vcap + h) * 32 + (row & 31)] = (uint32_t)value;
-  else A.nbr[(size_t)row * A.cap + h] = (uint16_t)value;
-}
-
-template <int MODE>
 __device__ __forceinline__ int build_cap(const ForceArgs &A) {
   return MODE == LIST_ID ? A.pl.vcap : MODE == LIST_FO ? A.fo.vcap : A.cap;
 }
@@ -372,131 +331,120 @@ __device__ __forceinline__ void build_count(const ForceArgs &A, int row, int tot
     atomicAdd(A.status + (MODE == LIST_STEP ? ST_NBR_OVERFLOW : ST_OVF_BUILD), 1);
 }
 
-// the lists of the atoms of box b (not empty): NT threads (the CTA), NA
-// atoms tested per candidate load, the shared arrays of the kernel
+// a candidate's key: what its list entry holds (LIST_STEP: bit 16 set in the
+// atom's own box)
+template <int MODE>
+__device__ __forceinline__ int build_key(const ForceArgs &A, int jb, int e, int k, bool own) {
+  if (MODE == LIST_ID) return A.s.id[jb * CG_MAXATOMS + k];
+  // force order: with periodic nbx >= 3 the entry index is the code
+  if (MODE == LIST_FO) return (int)(((unsigned)(A.box_start[jb] + k) << 6) | fo_code(e));
+  return (own ? 1 << 16 : 0) | (e << 6) | k;
+}
+
+// The lists of the atoms of box b (not empty): NT threads (the CTA), NA atoms
+// tested per candidate load, the shared arrays of the kernel.
 template <int MODE, int NT, int NA>
 __device__ __forceinline__ void build_box32(const ForceArgs &A, float rc2b, int b, float4 *cand,
-                                            uint32_t (*s_mask)[NA][NB_CHUNKS], int *s_box,
-                                            int *s_off, int *s_code, BoxOff<float> *s_dr) {
-  const int ni = A.s.natoms[b];
-  const int ne = stage_entries<float>(A, b, s_box, s_off, s_dr);
-  if (MODE != LIST_ID) order_entries_by_box(ne, s_box, s_off, s_dr, s_code);
-  const int ncand = s_off[ne];
-  const int nchunk = (ncand + 31) >> 5;
-  for (int c = threadIdx.x; c < (nchunk << 5); c += NT) {
-    if (c < ncand) {
-      int e = entry_of(s_off, ne, c);
-      int k = c - s_off[e];
-      float4 q = __ldg(A.s.pos32 + s_box[e] * CG_MAXATOMS + k);
-      BoxOff<float> o = s_dr[e];
-      // force order: with periodic nbx >= 3 the entry index is the code
-      const int tag = MODE == LIST_ID   ? A.s.id[s_box[e] * CG_MAXATOMS + k]
-                      : MODE == LIST_FO ? (int)(((unsigned)(A.box_start[s_box[e]] + k) << 6) |
-                                                fo_code(s_code[e]))
-                                        : ((s_code[e] << 6) | k);
-      // negated, so the test below is one packed add per axis: pa + (-c)
-      // rounds exactly as pa - c
-      cand[c] = make_float4(-((q.x - o.x) - o.lx), -((q.y - o.y) - o.ly), -((q.z - o.z) - o.lz),
-                            __int_as_float(tag));
-    } else {
-      cand[c] = make_float4(-1e18f, -1e18f, -1e18f, 0.f);
-    }
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+                                            int *s_cnt, int *s_box, int *s_off, int *s_code,
+                                            BoxOff<float> *s_dr) {
   static_assert(NA % 2 == 0, "atoms are tested in pairs");
-  for (int i0 = NA * warp; i0 < ni; i0 += NA * (NT / 32)) {
-    const int na = min(NA, ni - i0);
-    // the atoms in pairs, one per half of the packed FP32x2 operations (two
-    // pair tests per instruction; r^2 = dx*dx, + dy*dy, + dz*dz rounded as
-    // fmaf(dz, dz, fmaf(dy, dy, dx * dx)))
-    float2 px[NA / 2], py[NA / 2], pz[NA / 2];
+  const int ni = min(A.s.natoms[b], CG_MAXATOMS);
+  const int ne = stage_entries<MODE != LIST_ID>(A, b, s_box, s_off, s_dr, s_code);
+  const int ncand = s_off[ne];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t below = (1u << lane) - 1u;
+  const int cap = build_cap<MODE>(A);
+  const int a0 = MODE == LIST_ID ? 0 : A.box_start[b];
+  // the lists of the box's rows: offsets below are of 32 bits
+  uint16_t *step = MODE == LIST_STEP ? A.nbr + (size_t)a0 * cap : nullptr;
+  uint32_t *fo = MODE == LIST_FO ? A.fo.list + (size_t)(a0 >> 5) * 32 * cap : nullptr;
+  for (int base = 0; base < ncand; base += NB_TILE) {
+    const int nc = min(NB_TILE, ncand - base), nchunk = (nc + 31) >> 5;
+    if (base > 0) __syncthreads();  // the tile before is done with
+    // 16 threads an entry
+    for (int e = threadIdx.x >> 4; e < ne; e += NT / 16) {
+      const int jb = s_box[e], off = s_off[e], end = min(s_off[e + 1], base + nc);
+      const BoxOff<float> o = s_dr[e];
+      for (int c = max(off, base) + (threadIdx.x & 15); c < end; c += 16) {
+        const float4 q = __ldg(A.s.pos32 + jb * CG_MAXATOMS + (c - off));
+        // negated, so the test below is one packed add per axis: pa + (-c)
+        // rounds exactly as pa - c
+        cand[c - base] =
+            make_float4(-((q.x - o.x) - o.lx), -((q.y - o.y) - o.ly), -((q.z - o.z) - o.lz),
+                        __int_as_float(build_key<MODE>(A, jb, s_code[e], c - off, jb == b)));
+      }
+    }
+    for (int c = nc + threadIdx.x; c < (nchunk << 5); c += NT)
+      cand[c] = make_float4(-1e18f, -1e18f, -1e18f, 0.f);
+    __syncthreads();
+    for (int i0 = NA * warp; i0 < ni; i0 += NA * (NT / 32)) {
+      // (rows past the last only after an overflow)
+      const int na = min(NA, MODE == LIST_ID ? ni - i0 : min(ni - i0, A.ntot - a0 - i0));
+      if (na <= 0) break;
+      // the atoms in pairs, one per half of the packed FP32x2 operations (two
+      // pair tests per instruction; r^2 = dx*dx, + dy*dy, + dz*dz rounded as
+      // fmaf(dz, dz, fmaf(dy, dy, dx * dx))); a missing atom is far away from
+      // all candidates
+      float2 px[NA / 2], py[NA / 2], pz[NA / 2];
+      int cnt[NA], id[NA];
 #pragma unroll
-    for (int u = 0; u < NA / 2; u++) {
-      const float4 a0 = __ldg(A.s.pos32 + b * CG_MAXATOMS + i0 + (2 * u < na ? 2 * u : 0));
-      const float4 a1 = __ldg(A.s.pos32 + b * CG_MAXATOMS + i0 + (2 * u + 1 < na ? 2 * u + 1 : 0));
-      px[u] = make_float2(a0.x, a1.x);
-      py[u] = make_float2(a0.y, a1.y);
-      pz[u] = make_float2(a0.z, a1.z);
-    }
-    for (int q = 0; q < nchunk; q++) {
-      const float4 cq = cand[(q << 5) + lane];
-      const float2 cx = make_float2(cq.x, cq.x), cy = make_float2(cq.y, cq.y),
-                   cz = make_float2(cq.z, cq.z);
+      for (int u = 0; u < NA; u++) {
+        float4 p = make_float4(-1e18f, -1e18f, -1e18f, 0.f);
+        cnt[u] = id[u] = 0;
+        if (u < na) {
+          const int slot = b * CG_MAXATOMS + i0 + u;
+          p = __ldg(A.s.pos32 + slot);
+          if (MODE == LIST_ID) id[u] = A.s.id[slot];
+          if (base > 0) cnt[u] = s_cnt[i0 + u];
+        }
+        (u & 1 ? px[u / 2].y : px[u / 2].x) = p.x;
+        (u & 1 ? py[u / 2].y : py[u / 2].x) = p.y;
+        (u & 1 ? pz[u / 2].y : pz[u / 2].x) = p.z;
+      }
+      // the candidate's place counted from atom i0, an atom u being none of
+      // its own neighbours (it sits in every stencil entry of its own box)
+      auto append = [&](int u, float r2, int key, int from) {
+        const bool self = MODE == LIST_ID ? key == id[u] : from == u;
+        const bool hit = r2 <= rc2b && !self;
+        const uint32_t m = __ballot_sync(0xffffffffu, hit);
+        const int h = cnt[u] + __popc(m & below);
+        if (hit && h < cap) {
+          if (MODE == LIST_ID) A.pl.vlist[(size_t)id[u] * cap + h] = key;
+          else if (MODE == LIST_STEP) step[(i0 + u) * cap + h] = (uint16_t)key;
+          else {
+            const int row = (a0 & 31) + i0 + u;
+            fo[((row >> 5) * cap + h) * 32 + (row & 31)] = (uint32_t)key;
+          }
+        }
+        cnt[u] += __popc(m);
+      };
+      for (int q = 0; q < nchunk; q++) {
+        const float4 cq = cand[(q << 5) + lane];
+        const float2 cx = make_float2(cq.x, cq.x), cy = make_float2(cq.y, cq.y),
+                     cz = make_float2(cq.z, cq.z);
+        const int key = __float_as_int(cq.w);
+        const int from = MODE == LIST_FO ? (int)((unsigned)key >> 6) - a0 - i0
+                                         : (key & (1 << 16 | 63)) - (1 << 16) - i0;
 #pragma unroll
-      for (int u = 0; u < NA / 2; u++) {
-        const float2 dx = __fadd2_rn(px[u], cx), dy = __fadd2_rn(py[u], cy),
-                     dz = __fadd2_rn(pz[u], cz);
-        float2 r2 = __fmul2_rn(dx, dx);
-        r2 = __ffma2_rn(dy, dy, r2);
-        r2 = __ffma2_rn(dz, dz, r2);
-        const uint32_t m0 = __ballot_sync(0xffffffffu, r2.x <= rc2b);
-        const uint32_t m1 = __ballot_sync(0xffffffffu, r2.y <= rc2b);
-        if (lane == 0) {
-          s_mask[warp][2 * u][q] = m0;
-          s_mask[warp][2 * u + 1][q] = m1;
+        for (int u = 0; u < NA; u += 2) {
+          const float2 dx = __fadd2_rn(px[u / 2], cx), dy = __fadd2_rn(py[u / 2], cy),
+                       dz = __fadd2_rn(pz[u / 2], cz);
+          float2 r2 = __fmul2_rn(dx, dx);
+          r2 = __ffma2_rn(dy, dy, r2);
+          r2 = __ffma2_rn(dz, dz, r2);
+          append(u, r2.x, key, from);
+          append(u + 1, r2.y, key, from);
         }
       }
+      if (lane < na) {
+        int mine = cnt[0];
+#pragma unroll
+        for (int u = 1; u < NA; u++) mine = lane == u ? cnt[u] : mine;
+        s_cnt[i0 + lane] = mine;
+        if (base + NB_TILE >= ncand) build_count<MODE>(A, build_row<MODE>(A, b, i0 + lane), mine);
+      }
+      __syncwarp();
     }
-    __syncwarp();
-    // the atom itself sits in every stencil entry of its own box (one entry
-    // unless nbx < 3): clear those bits
-    if (lane < na)
-      for (int e = 0; e < ne; e++)
-        if (s_box[e] == b) {
-          const int c = s_off[e] + i0 + lane;
-          s_mask[warp][lane][c >> 5] &= ~(1u << (c & 31));
-        }
-    __syncwarp();
-    for (int t = 0; t < na; t++) {
-      const uint32_t *ms = s_mask[warp][t];
-      if (MODE != LIST_ID && A.box_start[b] + i0 + t >= A.ntot) break;  // only after an overflow
-      const int row = (lane == 0) ? build_row<MODE>(A, b, i0 + t) : 0;
-      const int a = __shfl_sync(0xffffffffu, row, 0);
-      const int cap = build_cap<MODE>(A);
-      // chunk words in candidate order: word w is held by lane w & 31 (w < 32
-      // in `lo`, w >= 32 in `hi`); inclusive prefix of the hit counts
-      const uint32_t lo = lane < nchunk ? ms[lane] : 0u;
-      const uint32_t hi = lane + 32 < nchunk ? ms[lane + 32] : 0u;
-      int xl = __popc(lo), xh = __popc(hi);
-      for (int o = 1; o < 32; o <<= 1) {
-        const int yl = __shfl_up_sync(0xffffffffu, xl, o);
-        const int yh = __shfl_up_sync(0xffffffffu, xh, o);
-        if (lane >= o) {
-          xl += yl;
-          xh += yh;
-        }
-      }
-      const int tot_lo = __shfl_sync(0xffffffffu, xl, 31);
-      const int total = tot_lo + __shfl_sync(0xffffffffu, xh, 31);
-      // one hit per lane per round: find its word by binary search over the
-      // prefix, then its bit with fns
-      for (int h0 = 0; h0 < total; h0 += 32) {
-        const int h = h0 + lane;
-        const bool second = h >= tot_lo;
-        const int hh = second ? h - tot_lo : h;
-        int l = 0;
-        for (int step = 16; step > 0; step >>= 1) {
-          const int vl = __shfl_sync(0xffffffffu, xl, l + step - 1);
-          const int vh = __shfl_sync(0xffffffffu, xh, l + step - 1);
-          if ((second ? vh : vl) <= hh) l += step;
-        }
-        const int prev_l = __shfl_sync(0xffffffffu, xl, (l + 31) & 31);
-        const int prev_h = __shfl_sync(0xffffffffu, xh, (l + 31) & 31);
-        const uint32_t wl = __shfl_sync(0xffffffffu, lo, l);
-        const uint32_t wh = __shfl_sync(0xffffffffu, hi, l);
-        if (h < total && h < cap) {
-          const int before = l ? (second ? prev_h : prev_l) : 0;
-          const uint32_t word = second ? wh : wl;
-          const unsigned bit = __fns(word, 0, hh - before + 1);
-          const int c = ((second ? l + 32 : l) << 5) + (int)(bit & 31u);
-          if (bit < 32u && c < (nchunk << 5))
-            build_store<MODE>(A, a, h, __float_as_int(cand[c].w));
-        }
-      }
-      if (lane == 0) build_count<MODE>(A, a, total);
-    }
-    __syncwarp();
   }
 }
 
@@ -506,14 +454,14 @@ __device__ __forceinline__ void build_box32(const ForceArgs &A, float rc2b, int 
 // CTA instead of one CTA per box.
 template <int MODE, int NT = NB_THREADS, int NA = NB_ATOMS>
 static __global__ void __launch_bounds__(NT) nbr_build32_kernel(ForceArgs A, float rc2b) {
-  __shared__ __align__(16) float4 cand[NB_MAXC];
-  __shared__ uint32_t s_mask[NT / 32][NA][NB_CHUNKS];
+  __shared__ __align__(16) float4 cand[NB_TILE];
+  __shared__ int s_cnt[CG_MAXATOMS];
   __shared__ int s_box[CG_NNBR], s_off[CG_NNBR + 1], s_code[CG_NNBR];
   __shared__ BoxOff<float> s_dr[CG_NNBR];
   if (build_skipped<MODE>(A)) return;
   for (int b = blockIdx.x; b < A.g.nboxes; b += gridDim.x) {
     if (A.s.natoms[b] == 0) continue;
-    build_box32<MODE, NT, NA>(A, rc2b, b, cand, s_mask, s_box, s_off, s_code, s_dr);
+    build_box32<MODE, NT, NA>(A, rc2b, b, cand, s_cnt, s_box, s_off, s_code, s_dr);
     __syncthreads();  // the next box restages the shared arrays
   }
 }

@@ -121,7 +121,7 @@ cudaError_t prepare_force_kernels() {
     if (e == cudaSuccess) e = build_occupancy_nt<256>(g_build_per_sm[2]);
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &g_build_step_per_sm, nbr_build32_kernel<LIST_STEP>, NB_THREADS, 0);
+          &g_build_step_per_sm, nbr_build32_kernel<LIST_STEP, NB_THREADS, 2>, NB_THREADS, 0);
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
           &g_build_id_per_sm, nbr_build32_kernel<LIST_ID>, NB_THREADS, 0);
@@ -164,8 +164,10 @@ void launch_nbr_build(const ForceArgs &A, float rc2b, cudaStream_t st, const Tun
     nbr_build32_kernel<LIST_ID><<<build_grid(A.g.nboxes, g_build_id_per_sm), NB_THREADS, 0, st>>>(
         A, rc2b);
   else
-    nbr_build32_kernel<LIST_STEP><<<build_grid(A.g.nboxes, g_build_step_per_sm), NB_THREADS, 0,
-                                    st>>>(A, rc2b);
+    // two atoms per load: boxes of a per-step list hold 10 to 20 atoms.  32 to
+    // 128 threads and 2 to 8 atoms: 129 (this) to 158 us at 256,000 atoms
+    nbr_build32_kernel<LIST_STEP, NB_THREADS, 2>
+        <<<build_grid(A.g.nboxes, g_build_step_per_sm), NB_THREADS, 0, st>>>(A, rc2b);
 }
 
 void launch_nbr_cut(const ForceArgs &A, float rc2b, cudaStream_t st) {

@@ -81,3 +81,29 @@ def test_close_pair_of_a_table(oracle, at):
         check(c)
     finally:
         c.close()
+
+
+# more candidates around a box than the list build stages at once: per-step
+# lists of a lattice compressed to 2.5 A, id-keyed skin lists and force-order
+# lists of wide boxes (mixed precision: its force-call tolerances)
+@pytest.mark.parametrize("precision,edges,bf,lat", [
+    (cg.PREC_FP64, (11, 10, 10), 1.0, 2.5), (cg.PREC_FP64, (14, 14, 15), 1.45, None),
+    (cg.PREC_MIXED, (14, 14, 15), 1.45, None)])
+def test_two_tiles_of_candidates(oracle, precision, edges, bf, lat):
+    c = Case(oracle, cg.POT_EAM_TABLE, n=edges, bf=bf, lat=lat, temp=300.0, amp=0.02)
+    try:
+        assert 27 * c.s.contents.ntot > 900 * c.s.contents.nboxes
+        if precision == cg.PREC_FP64:
+            check(c)
+            return
+        c.oracle_force()
+        d = c.device(precision)
+        assert d.list_info()[0]
+        d.force()
+        d.download(c.s)
+        d.close()
+        cmp = compare_forces(c.s, c.o)
+        assert cmp["f_rel_rms"] < 1e-5 and cmp["f_max_rel"] < 1e-4, cmp
+        assert cmp["rho_max_rel"] < 1e-6 and cmp["fi_max_rel"] < 1e-5, cmp
+    finally:
+        c.close()
