@@ -28,7 +28,9 @@
 // fixed order: results are deterministic.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
+#include "force64.cuh"
 #include "sim.h"
 
 using namespace cg;
@@ -65,17 +67,19 @@ __device__ __forceinline__ double cheb_der(const ChebSet &S, int qd, int q, doub
   return x < S.a[q] ? 0.0 : cheb_val(S, qd, x);
 }
 
-// Pair functions of one distance from the polynomial table, or from the
-// series outside it (rare: kept out of line).
+// Pair functions of one distance (r^2 in fixed point) from the polynomial
+// table, or from the series outside it (rare: kept out of line).
 __device__ __noinline__ double grho_series(const ChebSet &S, double r2) {
   const double r = sqrt(r2);
   return cheb_val(S, 4, r) / r;
 }
 // rho'(r) / r
-__device__ __forceinline__ double pair_grho(const ChebSet &S, const PolyTables &P, double r2) {
+__device__ __forceinline__ double pair_grho(const ChebSet &S, const PolyTables &P, u64 s,
+                                            const FxUnit &u) {
   int k;
   double t;
-  return poly_at(P.pair, r2, k, t) ? poly_col(P.pair, PF_GRHO, k, t) : grho_series(S, r2);
+  return poly_at(P.pair, s, 2 * u.m - 64, k, t) ? poly_col(P.pair, PF_GRHO, k, t)
+                                                : grho_series(S, fx_area(s, u));
 }
 // the terms of the Hessian: phi'/r and rho'/r, the position derivative of
 // the density over r (dr), and (phi'' - phi'/r) / r^2, (rho'' - rho'/r) / r^2
@@ -92,10 +96,12 @@ __device__ __noinline__ HessTerms hess_series(const ChebSet &S, double r2) {
   h.hrho = (cheb_der(S, 7, 1, r) - h.grho) * ir2;
   return h;
 }
-__device__ __forceinline__ HessTerms hess_terms(const ChebSet &S, const PolyTables &P, double r2) {
+__device__ __forceinline__ HessTerms hess_terms(const ChebSet &S, const PolyTables &P, u64 s,
+                                                const FxUnit &u) {
   int k, kh;
   double t, th;
-  if (!poly_at(P.pair, r2, k, t) || !poly_at(P.hess, r2, kh, th)) return hess_series(S, r2);
+  if (!poly_at(P.pair, s, 2 * u.m - 64, k, t) || !poly_at(P.hess, s, 2 * u.m - 64, kh, th))
+    return hess_series(S, fx_area(s, u));
   HessTerms h;
   h.gphi = poly_col(P.pair, PF_GPHI, k, t);
   h.grho = h.dr = poly_col(P.pair, PF_GRHO, k, t);
@@ -146,26 +152,29 @@ __global__ void adj_lambda_kernel(Slots s, const int *atom_slot, int ntot, const
 }
 
 // W_i = sum_j v_ij rho'(r_ij) over the embedding-force pairs (r2 < rc2,
-// eam.c:612) and X_i = F''(rho_i) W_i, per slot
-__global__ void adj_w_kernel(ForceArgs A, const __grid_constant__ ChebSet S,
-                             PolyTables poly, double rc2, const d4 *lam, double *wout,
-                             double *xout) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= A.ntot) return;
+// eam.c:612) and X_i = F''(rho_i) W_i, per slot.  The walk of the FP64 passes
+// (fixed-point distances, LANES threads an atom): a thread per atom in FP64
+// geometry took 63 us at 3,960 atoms and 500 us at 256,000, this 12 and 279.
+template <int LANES>
+__global__ void __launch_bounds__(F64_THREADS)
+    adj_w_kernel(ForceArgs A, const __grid_constant__ ChebSet S, PolyTables poly, double rc2,
+                 const d4 *lam, double *wout, double *xout) {
+  int a, sub;
+  bool live;
+  if (!lane_atom<LANES>(A.ntot, a, sub, live)) return;
   const int slot = A.atom_slot[a];
-  const int b = slot >> 6, i = slot & 63;
-  double xi, yi, zi;
-  PrecT<double>::pos(A.s, slot, xi, yi, zi);
   const d4 li = lam[slot];
   double W = 0.0;
-  for_each_neighbor<double, true>(A, a, b, i, xi, yi, zi, rc2,
-                                  [&](int js, double dx, double dy, double dz, double r2) {
-                                    if (r2 >= rc2) return;
-                                    const d4 lj = lam[js];
-                                    const double vr = (li.x - lj.x) * dx + (li.y - lj.y) * dy +
-                                                      (li.z - lj.z) * dz;
-                                    W += vr * pair_grho(S, poly, r2);
-                                  });
+  walk64<LANES>(A, a, sub, slot, A.fx[slot], rc2, [&](const Pair64 &q) {
+    if (q.s >= A.fx_rc2) return;
+    const d4 lj = lam[q.j];
+    const double vr = (li.x - lj.x) * fx_length(q.x, A.fxu) +
+                      (li.y - lj.y) * fx_length(q.y, A.fxu) +
+                      (li.z - lj.z) * fx_length(q.z, A.fxu);
+    W += vr * pair_grho(S, poly, q.s, A.fxu);
+  });
+  W = lane_sum<LANES>(W);
+  if (sub != 0 || !live) return;
   wout[slot] = W;
   xout[slot] = embed_d2(S, poly, A.s.rho[slot]) * W;
 }
@@ -185,12 +194,13 @@ __device__ __forceinline__ double cheb_y(const ChebSet &S, int q, double x) {
 //
 // Bound by FP64 operations: one for the recurrence and one per weight and k,
 // 124 a pair with lambda.  A thread keeps all its sums in registers (96
-// doubles; a column of shared memory per thread, read and written for every
-// k, took 10.45 ms at 256,000 atoms, this 2.16 ms) and LANES threads share
-// an atom's list.  Each pair is taken at one of its atoms, the lower slot if
-// the slots' sum is even and the higher if it is odd, so every thread finds
-// about half of its entries; it skips the others before the sums, or half of
-// the lanes would stand idle in them.
+// doubles).  Each pair is taken at one of its atoms, the lower slot if the
+// slots' sum is even and the higher if it is odd.  So that no lane idles in
+// those operations, a warp collects the pairs it takes, over all its atoms, in
+// a queue in shared memory and works on 32 at a time; the distances are formed
+// in fixed point, r without division.  At 256,000 and 3,960 atoms: 10,450 and
+// 750 us with sums in shared memory, 2,158 and 94 us with several threads an
+// atom each at its own pairs, 1,403 and 45 us now.
 template <int NW>
 struct BasisAcc {
   double s[NW][NC];
@@ -215,16 +225,32 @@ __device__ __forceinline__ void basis_add(BasisAcc<NW> &A, double yp, double yr,
   }
 }
 
-// the CTA's sums of NROW per-thread values, to out[0..NROW): warp trees,
-// then the warps in order
-template <int NROW, int NT>
-__device__ __forceinline__ void block_rows(const double *v, double *sh, double *out) {
+// A lane hands half of its 2 N rows to its partner O lanes on and adds the
+// other half, down to O = 1: a fifth of the additions of a tree per row.
+// Returns the lane's first row.
+template <int N, int O>
+__device__ __forceinline__ int split_rows(double *v, int lane) {
+  if constexpr (O == 0) {
+    return 0;
+  } else {
+    const bool upper = lane & O;
 #pragma unroll
-  for (int r = 0; r < NROW; r++) {
-    double t = v[r];
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-    if ((threadIdx.x & 31) == 0) sh[(threadIdx.x >> 5) * NROW + r] = t;
+    for (int r = 0; r < N; r++) {
+      const double keep = upper ? v[N + r] : v[r], give = upper ? v[r] : v[N + r];
+      v[r] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+    }
+    return (upper ? N : 0) + split_rows<N / 2, O / 2>(v, lane);
   }
+}
+
+// the CTA's sums of NROW per-thread values (a multiple of 32), to
+// out[0..NROW): over the lanes of each warp, then the warps in order
+template <int NROW, int NT>
+__device__ __forceinline__ void block_rows(double *v, double *sh, double *out) {
+  static_assert(NROW % 32 == 0, "rows are split over the lanes");
+  const int first = split_rows<NROW / 2, 16>(v, threadIdx.x & 31);
+#pragma unroll
+  for (int r = 0; r < NROW / 32; r++) sh[(threadIdx.x >> 5) * NROW + first + r] = v[r];
   __syncthreads();
   for (int r = threadIdx.x; r < NROW; r += NT) {
     double t = 0.0;
@@ -233,71 +259,91 @@ __device__ __forceinline__ void block_rows(const double *v, double *sh, double *
   }
 }
 
-template <int NW, bool SAME, int LANES>
+template <int NW, bool SAME>
 __global__ void __launch_bounds__(BASIS_THREADS)
     adj_basis_kernel(ForceArgs A, const __grid_constant__ ChebSet S, double rc2, Lam L,
                      double *partial) {
-  __shared__ double sh[BASIS_THREADS / 32 * NW * NC];
+  constexpr int WARPS = BASIS_THREADS / 32;
+  __shared__ double sh[WARPS * NW * NC];
+  __shared__ uint2 s_queue[WARPS][64];  // (slot i, entry)
+  uint2 *queue = s_queue[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const double scale[2] = {1.0 / (S.b[0] - S.a[0]), 1.0 / (S.b[1] - S.a[1])};
   BasisAcc<NW> acc;
 #pragma unroll
   for (int q = 0; q < NW; q++)
 #pragma unroll
     for (int k = 0; k < NC; k++) acc.s[q][k] = 0.0;
-  const int sub = threadIdx.x % LANES;
-  for (int a = (blockIdx.x * BASIS_THREADS + threadIdx.x) / LANES; a < A.ntot;
-       a += gridDim.x * BASIS_THREADS / LANES) {
-    const int slot = A.atom_slot[a];
-    const int b = slot >> 6, ebase = b * CG_NNBR, n = A.nbr_n[a];
-    const d4 ri = A.s.r[slot];
-    const double fpi = A.s.fi[slot];
-    d4 li;
-    double Xi = 0.0;
+  auto mine = [](int js, int slot) { return ((js > slot) ^ ((js + slot) & 1)) != 0; };
+  // cheb_y: 2 (r - a) / (b - a) - 1, the quotient corrected once
+  auto y_of = [&](int q, double r) {
+    const double d = fmax(r, S.a[q]) - S.a[q], t = d * scale[q];
+    return fma(2.0, fma(fma(-t, S.b[q] - S.a[q], d), scale[q], t), -1.0);
+  };
+  auto pair = [&](int slot, const d4 &fi, const Pair64 &q) {
+    if (q.s > A.fx_rc2) return;
+    double r, inv;
+    r_and_inv(fx_area(q.s, A.fxu), r, inv);
+    const double fsum = fi.w + q.fj;
+    double w[3];
     if (NW == 3) {
-      li = L.lam[slot];
-      Xi = L.x[slot];
+      const d4 li = L.lam[slot], lj = L.lam[q.j];
+      w[0] = ((li.x - lj.x) * fx_length(q.x, A.fxu) + (li.y - lj.y) * fx_length(q.y, A.fxu) +
+              (li.z - lj.z) * fx_length(q.z, A.fxu)) * inv;
+      w[1] = q.s < A.fx_rc2 ? fsum * w[0] : 0.0;
+      w[2] = L.x[slot] + L.x[q.j];
+    } else {
+      w[0] = 1.0;
+      w[1] = fsum;
     }
-    auto mine = [&](int js) { return ((js > slot) ^ ((js + slot) & 1)) != 0; };
-    auto pair = [&](int js, double dx, double dy, double dz, double r2) {
-      if (r2 > rc2) return;
-      const double r = sqrt(r2), fsum = fpi + A.s.fi[js];
-      double w[3];
-      if (NW == 3) {
-        const d4 lj = L.lam[js];
-        w[0] = ((li.x - lj.x) * dx + (li.y - lj.y) * dy + (li.z - lj.z) * dz) / r;
-        w[1] = r2 < rc2 ? fsum * w[0] : 0.0;
-        w[2] = Xi + L.x[js];
-      } else {
-        w[0] = 1.0;
-        w[1] = fsum;
+    const double yp = y_of(0, r);
+    basis_add<NW, SAME>(acc, yp, SAME ? yp : y_of(1, r), w);
+  };
+  int queued = 0;
+  auto work = [&](int n) {  // the queue's first n <= 32 pairs
+    if (lane < n) {
+      const uint2 e = queue[lane];
+      const int slot = (int)e.x;
+      const d4 fi = A.fx[slot];
+      pair(slot, fi, pair64(A, fi, A.et.fx + (slot >> 6) * CG_NNBR, e.y));
+    }
+    __syncwarp();
+  };
+  for (int a = blockIdx.x * WARPS + (threadIdx.x >> 5); a < A.ntot; a += gridDim.x * WARPS) {
+    const int slot = A.atom_slot[a], n = A.nbr_n[a], ebase = (slot >> 6) * CG_NNBR;
+    if (n > A.cap) {  // overflowed list: the stencil, by one lane
+      if (lane == 0) {
+        const d4 fi = A.fx[slot];
+        walk64<1>(A, a, 0, slot, fi, rc2, [&](const Pair64 &q) {
+          if (mine(q.j, slot)) pair(slot, fi, q);
+        });
       }
-      const double yp = cheb_y(S, 0, r);
-      basis_add<NW, SAME>(acc, yp, SAME ? yp : cheb_y(S, 1, r), w);
-    };
-    const bool over = n > A.cap;
-    if (over && sub == 0)  // overflowed list: the stencil, by one lane
-      scan_stencil<double>(A, b, slot & 63, ri.x, ri.y, ri.z, rc2,
-                           [&](int js, double dx, double dy, double dz, double r2) {
-                             if (mine(js)) pair(js, dx, dy, dz, r2);
-                           });
+      __syncwarp();
+      continue;
+    }
     const uint16_t *lst = A.nbr + (size_t)a * A.cap;
-    int t = over ? n : sub;
-    while (true) {
-      int js = 0, e = 0;
-      bool got = false;
-      for (; t < n && !got; t += LANES) {
-        const uint32_t code = lst[t];
-        e = code >> 6;
-        js = __ldg(A.et.box + ebase + e) * CG_MAXATOMS + (code & 63);
-        got = mine(js);
+    for (int t0 = 0; t0 < n; t0 += 32) {
+      uint32_t code = 0;
+      bool take = false;
+      if (t0 + lane < n) {
+        code = __ldg(lst + t0 + lane);
+        take = mine(__ldg(A.et.box + ebase + (code >> 6)) * CG_MAXATOMS + (int)(code & 63), slot);
       }
-      if (!got) break;
-      const d4 rj = A.s.r[js];
-      double dx, dy, dz;
-      const double r2 = pair_r2(PrecT<double>::drbox(A.et, ebase + e), ri.x, ri.y, ri.z, rj.x,
-                                rj.y, rj.z, dx, dy, dz);
-      pair(js, dx, dy, dz, r2);
+      const uint32_t m = __ballot_sync(0xffffffffu, take);
+      if (take) queue[queued + __popc(m & ((1u << lane) - 1u))] = make_uint2(slot, code);
+      queued += __popc(m);
+      __syncwarp();
+      if (queued < 32) continue;
+      work(32);
+      queued -= 32;
+      uint2 e;
+      if (lane < queued) e = queue[32 + lane];
+      __syncwarp();
+      if (lane < queued) queue[lane] = e;
+      __syncwarp();
     }
   }
+  work(queued);
   block_rows<NW * NC, BASIS_THREADS>(&acc.s[0][0], sh, partial + (size_t)blockIdx.x * NW * NC);
 }
 
@@ -386,32 +432,37 @@ __global__ void __launch_bounds__(128) adj_lj_kernel(ForceArgs A, double eps, do
 // with X = F'' W (adj_w_kernel at lambda = u), computed as
 //   (g/r) du + [(du . d) (g' - g/r)/r^2 + (X_k + X_j) (d rho/dr)/r] d,
 // d = r_k - r_j, whose functions of r^2 are columns of the polynomial table
-// (no square root, no division).  Written by atom id.
-__global__ void adj_hvp_kernel(ForceArgs A, const __grid_constant__ ChebSet S, PolyTables poly,
-                               double rc2, const d4 *u, const double *X, double *hv) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= A.ntot) return;
+// (no square root, no division).  Written by atom id.  The walk of adj_w_kernel;
+// a thread per atom took 108 us at 3,960 atoms, this 25.
+template <int LANES>
+__global__ void __launch_bounds__(F64_THREADS)
+    adj_hvp_kernel(ForceArgs A, const __grid_constant__ ChebSet S, PolyTables poly, double rc2,
+                   const d4 *u, const double *X, double *hv) {
+  int a, sub;
+  bool live;
+  if (!lane_atom<LANES>(A.ntot, a, sub, live)) return;
   const int slot = A.atom_slot[a];
-  const int b = slot >> 6, i = slot & 63;
-  double xi, yi, zi;
-  PrecT<double>::pos(A.s, slot, xi, yi, zi);
-  const d4 uk = u[slot];
-  const double Fk = A.s.fi[slot], Xk = X[slot];
+  const d4 fi = A.fx[slot], uk = u[slot];
+  const double Xk = X[slot];
   double hx = 0.0, hy = 0.0, hz = 0.0;
-  for_each_neighbor<double, true>(
-      A, a, b, i, xi, yi, zi, rc2, [&](int js, double dx, double dy, double dz, double r2) {
-        if (r2 > rc2) return;
-        const HessTerms h = hess_terms(S, poly, r2);
-        const d4 uj = u[js];
-        const double ux = uk.x - uj.x, uy = uk.y - uj.y, uz = uk.z - uj.z;
-        const double ud = ux * dx + uy * dy + uz * dz;
-        const double fs = r2 < rc2 ? Fk + A.s.fi[js] : 0.0;
-        const double g = h.gphi + fs * h.grho;
-        const double c = ud * (h.hphi + fs * h.hrho) + (Xk + X[js]) * h.dr;
-        hx += g * ux + c * dx;
-        hy += g * uy + c * dy;
-        hz += g * uz + c * dz;
-      });
+  walk64<LANES>(A, a, sub, slot, fi, rc2, [&](const Pair64 &q) {
+    if (q.s > A.fx_rc2) return;
+    const HessTerms h = hess_terms(S, poly, q.s, A.fxu);
+    const d4 uj = u[q.j];
+    const double dx = fx_length(q.x, A.fxu), dy = fx_length(q.y, A.fxu), dz = fx_length(q.z, A.fxu);
+    const double ux = uk.x - uj.x, uy = uk.y - uj.y, uz = uk.z - uj.z;
+    const double ud = ux * dx + uy * dy + uz * dz;
+    const double fs = q.s < A.fx_rc2 ? fi.w + q.fj : 0.0;
+    const double g = h.gphi + fs * h.grho;
+    const double c = ud * (h.hphi + fs * h.hrho) + (Xk + X[q.j]) * h.dr;
+    hx += g * ux + c * dx;
+    hy += g * uy + c * dy;
+    hz += g * uz + c * dz;
+  });
+  hx = lane_sum<LANES>(hx);
+  hy = lane_sum<LANES>(hy);
+  hz = lane_sum<LANES>(hz);
+  if (sub != 0 || !live) return;
   const int id = A.s.id[slot];
   if ((unsigned)id >= (unsigned)A.ntot) return;
   hv[3 * (size_t)id] = hx;
@@ -534,6 +585,15 @@ int need_fp64(comdgb_sim *h) {
 
 unsigned blocks(long n, int t = 256) { return (unsigned)((n + t - 1) / t); }
 
+// fn(threads per atom), as the force passes take them
+template <class F>
+void by_lanes(const comdgb_sim *h, F &&fn) {
+  const int lanes = lanes64(h->ntot);
+  if (lanes == 16) fn(std::integral_constant<int, 16>());
+  else if (lanes == 4) fn(std::integral_constant<int, 4>());
+  else fn(std::integral_constant<int, 1>());
+}
+
 // sum of W.loss[0..ntot) to the host
 int loss_sum(comdgb_sim *h, Work &W, double *loss) {
   const int nb = std::min(1024, (int)blocks(h->ntot));
@@ -559,20 +619,11 @@ void launch_basis(comdgb_sim *h, Work &W, const ChebSet &S, Lam L) {
   const ForceArgs A = force_args(h);
   const double rc2 = h->eam64c.rc2;
   const bool same = S.a[0] == S.a[1] && S.b[0] == S.b[1];
-  // one thread per atom fills the card from about 150,000 atoms on (two CTAs
-  // an SM, four rounds of atoms); below, four threads share an atom: at 3,960
-  // atoms 220 us with one and 96 us with four (256,000: 2,157 and 2,774 us)
-  const int lanes = h->ntot >= 4 * W.nblk * BASIS_THREADS ? 1 : 4;
-  const long need = ((long)h->ntot * lanes + BASIS_THREADS - 1) / BASIS_THREADS;
-  const int grid = (int)std::max(1L, std::min((long)W.nblk, need));
+  const long warps = BASIS_THREADS / 32;
+  const int grid = (int)std::max(1L, std::min((long)W.nblk, (h->ntot + warps - 1) / warps));
   auto run = [&](auto kernel) { kernel<<<grid, BASIS_THREADS, 0, h->stream>>>(A, S, rc2, L, W.partial); };
-  if (lanes == 1) {
-    if (same) run(adj_basis_kernel<NW, true, 1>);
-    else run(adj_basis_kernel<NW, false, 1>);
-  } else {
-    if (same) run(adj_basis_kernel<NW, true, 4>);
-    else run(adj_basis_kernel<NW, false, 4>);
-  }
+  if (same) run(adj_basis_kernel<NW, true>);
+  else run(adj_basis_kernel<NW, false>);
   adj_sum_kernel<<<NW * NC, 256, 0, h->stream>>>(W.partial, grid, NW * NC, W.out);
 }
 
@@ -619,8 +670,11 @@ int set_lambda(comdgb_sim *h, Work &W, const ChebSet &S, const double *d_target,
   adj_lambda_kernel<<<blocks(h->ntot), 256, 0, h->stream>>>(h->s, h->atom_slot, h->ntot, d_target,
                                                            d_u, W.lam, W.loss);
   if (h->opts.potential == COMDGB_POT_EAM_CHEBY)
-    adj_w_kernel<<<blocks(h->ntot, 128), 128, 0, h->stream>>>(force_args(h), S, h->eam64c.poly,
-                                                              h->eam64c.rc2, W.lam, W.w, W.x);
+    by_lanes(h, [&](auto lanes) {
+      constexpr int L = decltype(lanes)::value;
+      adj_w_kernel<L><<<blocks((long)h->ntot * L, F64_THREADS), F64_THREADS, 0, h->stream>>>(
+          force_args(h), S, h->eam64c.poly, h->eam64c.rc2, W.lam, W.w, W.x);
+    });
   CK(cudaGetLastError());
   return 0;
 }
@@ -788,9 +842,11 @@ int comdgb_sim_traj_energy_grad(comdgb_sim *h, int n, double dt, int every, doub
       adj_axpy_kernel<<<blocks(nv), 256, 0, h->stream>>>(c, rb, pb, nv);
       adj_scale_kernel<<<blocks(nv), 256, 0, h->stream>>>(-dt_atu, pb, u, nv);
       if ((rc = set_lambda(h, W, S, nullptr, u))) return rc;
-      adj_hvp_kernel<<<blocks(h->ntot, 128), 128, 0, h->stream>>>(force_args(h), S,
-                                                                 h->eam64c.poly, h->eam64c.rc2,
-                                                                 W.lam, W.x, hv);
+      by_lanes(h, [&](auto lanes) {
+        constexpr int L = decltype(lanes)::value;
+        adj_hvp_kernel<L><<<blocks((long)h->ntot * L, F64_THREADS), F64_THREADS, 0, h->stream>>>(
+            force_args(h), S, h->eam64c.poly, h->eam64c.rc2, W.lam, W.x, hv);
+      });
       if ((rc = eam_grad(h, W, S, true, g))) return rc;
       for (int q = 0; q < 3 * NC; q++) cbar[q] += g[q];
       adj_axpy_kernel<<<blocks(nv), 256, 0, h->stream>>>(1.0, hv, rb, nv);

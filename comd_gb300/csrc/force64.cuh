@@ -33,6 +33,13 @@ namespace cg {
 
 constexpr int F64_THREADS = 128;
 
+// Threads per atom.  Density + force pass without energies in us, Chebyshev
+// (16, 4, 1 threads): 4,000 atoms 22, 36, 99; 27,436 atoms 85, 66, 108; 256,000
+// atoms 658, 480, 523; 1,048,576 atoms 2,648, 1,903, 1,838 (lists of 42 entries
+// leave lanes of 16 short).  Eight threads lie between at every size, two at
+// 27,436 atoms 71.
+inline int lanes64(int ntot) { return ntot < 12000 ? 16 : ntot < (1 << 19) ? 4 : 1; }
+
 // The atom and sub-lane of this thread; false when its whole warp has none.
 // Groups past the last atom repeat it (no divergence in the shuffles) and
 // store nothing (live).
@@ -54,14 +61,26 @@ __device__ __forceinline__ double lane_sum(double v) {
   return v;
 }
 
-// A pair: the differences and r^2 in fixed point, F'(rho_j)
+// A pair: the differences and r^2 in fixed point, F'(rho_j), j's slot
 struct Pair64 {
   long long x, y, z;
   u64 s;
   double fj;
+  int j;
 };
-__device__ __forceinline__ Pair64 pair64(long long x, long long y, long long z, double fj) {
-  return Pair64{x, y, z, fx_square(fx_abs(x)) + fx_square(fx_abs(y)) + fx_square(fx_abs(z)), fj};
+__device__ __forceinline__ Pair64 pair64(long long x, long long y, long long z, double fj, int j) {
+  return Pair64{x, y, z, fx_square(fx_abs(x)) + fx_square(fx_abs(y)) + fx_square(fx_abs(z)), fj, j};
+}
+// the pair of atom i (its record) and entry code of its box's stencil (off)
+__device__ __forceinline__ Pair64 pair64(const ForceArgs &A, const d4 &fi, const d4 *off,
+                                         uint32_t code) {
+  const d4 o = off[code >> 6];  // the offset, and the neighbour box
+  const int j = __double2loint(o.w) * CG_MAXATOMS + (code & 63);
+  const d4 q = A.fx[j];
+  return pair64(
+      __double_as_longlong(fi.x) + __double_as_longlong(o.x) - __double_as_longlong(q.x),
+      __double_as_longlong(fi.y) + __double_as_longlong(o.y) - __double_as_longlong(q.y),
+      __double_as_longlong(fi.z) + __double_as_longlong(o.z) - __double_as_longlong(q.z), q.w, j);
 }
 
 // This lane's entries of atom a's list: fn(pair), entries past the cutoff
@@ -77,24 +96,15 @@ __device__ __forceinline__ void walk64(const ForceArgs &A, int a, int sub, int s
       scan_stencil<double>(A, b, slot & 63, ri.x, ri.y, ri.z, rc2,
                            [&](int js, double dx, double dy, double dz, double) {
                              fn(pair64(fx_from(dx, A.fxu), fx_from(dy, A.fxu),
-                                       fx_from(dz, A.fxu), A.fx[js].w));
+                                       fx_from(dz, A.fxu), A.fx[js].w, js));
                            });
     }
     return;
   }
-  const long long xi = __double_as_longlong(fi.x), yi = __double_as_longlong(fi.y),
-                  zi = __double_as_longlong(fi.z);
   const d4 *off = A.et.fx + b * CG_NNBR;
   const uint16_t *lst = A.nbr + (size_t)a * A.cap;
 #pragma unroll 1
-  for (int t = sub; t < n; t += LANES) {
-    const uint32_t code = __ldg(lst + t);
-    const d4 o = off[code >> 6];  // the offset, and the neighbour box
-    const d4 q = A.fx[__double2loint(o.w) * CG_MAXATOMS + (code & 63)];
-    fn(pair64(xi + __double_as_longlong(o.x) - __double_as_longlong(q.x),
-              yi + __double_as_longlong(o.y) - __double_as_longlong(q.y),
-              zi + __double_as_longlong(o.z) - __double_as_longlong(q.z), q.w));
-  }
+  for (int t = sub; t < n; t += LANES) fn(pair64(A, fi, off, __ldg(lst + t)));
 }
 
 // rho(r); phi, phi'/r and rho'/r.  false: outside the polynomial tables

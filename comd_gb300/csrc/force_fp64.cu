@@ -5,13 +5,6 @@
 
 namespace cg {
 
-// Threads per atom.  Density + force pass without energies in us, Chebyshev
-// (16, 4, 1 threads): 4,000 atoms 22, 36, 99; 27,436 atoms 85, 66, 108; 256,000
-// atoms 658, 480, 523; 1,048,576 atoms 2,648, 1,903, 1,838 (lists of 42 entries
-// leave lanes of 16 short).  Eight threads lie between at every size, two at
-// 27,436 atoms 71.
-static int lanes64(int ntot) { return ntot < 12000 ? 16 : ntot < (1 << 19) ? 4 : 1; }
-
 template <int EVAL, bool OBS, int LANES>
 static void launch_eam64_lanes(const ForceArgs &A, const EamPot<double, EVAL> &P, int pass,
                                cudaStream_t st) {
