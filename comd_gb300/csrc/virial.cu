@@ -21,6 +21,12 @@
 // list (mixed precision), with F' from that call.  Per-atom sums are
 // compensated in FP32 and plain in FP64; the sums over atoms are FP64 in a
 // fixed order (deterministic).
+//
+// FP64: bound by that pipe, as the force passes are, so the walk is theirs
+// (fixed-point distances, the pair functions as polynomials, several threads
+// an atom).  256,000 atoms, Chebyshev: 891 us with a thread per atom in FP64
+// geometry, 464 now.
+#include "force64.cuh"
 #include "sim.h"
 
 using namespace cg;
@@ -29,7 +35,7 @@ using namespace cgapi;
 namespace {
 
 constexpr int VIR_THREADS = 256;
-constexpr int VIR_PARTS = 64;  // partial sums per replica
+constexpr int VIR_PARTS = 304;  // partial sums per replica, at most
 
 template <class T>
 struct VirAcc {
@@ -114,6 +120,73 @@ __global__ void __launch_bounds__(VIR_THREADS)
   }
 }
 
+// FP64: the pair weight g of the terms above, times dr (x) dr
+struct Vir64 {
+  double c[6];
+  __device__ __forceinline__ void add(double g, const Pair64 &q, const FxUnit &u) {
+    const double dx = fx_length(q.x, u), dy = fx_length(q.y, u), dz = fx_length(q.z, u);
+    const double gx = g * dx, gy = g * dy, gz = g * dz;
+    c[0] = fma(gx, dx, c[0]);
+    c[1] = fma(gy, dy, c[1]);
+    c[2] = fma(gz, dz, c[2]);
+    c[3] = fma(gy, dz, c[3]);
+    c[4] = fma(gx, dz, c[4]);
+    c[5] = fma(gx, dy, c[5]);
+  }
+  // half of the sums over LANES lanes
+  template <int LANES>
+  __device__ __forceinline__ void store(bool mine, double *out) {
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+      const double v = 0.5 * lane_sum<LANES>(c[q]);
+      if (mine) out[q] = v;
+    }
+  }
+};
+template <int EVAL, int LANES>
+__global__ void __launch_bounds__(F64_THREADS)
+    eam64_virial_kernel(ForceArgs A, const __grid_constant__ EamPot<double, EVAL> P, double *out) {
+  int a, sub;
+  bool live;
+  if (!lane_atom<LANES>(A.ntot, a, sub, live)) return;
+  const int slot = A.atom_slot[a];
+  const d4 fi = A.fx[slot];
+  const u64 rc2 = A.fx_rc2;
+  Vir64 acc{};
+  bool low = false;
+  walk64<LANES>(A, a, sub, slot, fi, P.rc2, [&](const Pair64 &q) {
+    if (q.s > rc2) return;
+    double phi, w, wr;
+    if (force64<false>(P, q.s, A.fxu, phi, w, wr))
+      acc.add(-fma(q.s < rc2 ? fi.w + q.fj : 0.0, wr, w), q, A.fxu);
+    else
+      low = true;
+  });
+  if (low)
+    walk64<LANES>(A, a, sub, slot, fi, P.rc2, [&](const Pair64 &q) {
+      if (q.s > rc2 || !outside64(P, q.s, A.fxu)) return;
+      double phi, w, wr;
+      force64_series(P, fx_area(q.s, A.fxu), phi, w, wr);
+      acc.add(-fma(q.s < rc2 ? fi.w + q.fj : 0.0, wr, w), q, A.fxu);
+    });
+  acc.template store<LANES>(sub == 0 && live, out + 6 * (size_t)slot);
+}
+template <int LANES>
+__global__ void __launch_bounds__(F64_THREADS)
+    lj64_virial_kernel(ForceArgs A, LjPot<double> P, double *out) {
+  int a, sub;
+  bool live;
+  if (!lane_atom<LANES>(A.ntot, a, sub, live)) return;
+  const int slot = A.atom_slot[a];
+  Vir64 acc{};
+  walk64<LANES>(A, a, sub, slot, A.fx[slot], P.rc2, [&](const Pair64 &q) {
+    if (q.s > A.fx_rc2) return;
+    const double ir2 = reciprocal(fx_area(q.s, A.fxu)), r6 = ir2 * ir2 * ir2;
+    acc.add(P.eps4s6 * r6 * ir2 * fma(P.s6x12, r6, -6.0), q, A.fxu);
+  });
+  acc.template store<LANES>(sub == 0 && live, out + 6 * (size_t)slot);
+}
+
 template <class T, bool FO>
 __global__ void __launch_bounds__(VIR_THREADS) lj_virial_kernel(ForceArgs A, LjPot<T> P,
                                                                 double *out) {
@@ -150,7 +223,7 @@ __global__ void __launch_bounds__(VIR_THREADS) lj_virial_kernel(ForceArgs A, LjP
 __global__ void __launch_bounds__(VIR_THREADS)
     virial_reduce_kernel(Geom g, Slots s, const int *atom_slot, double rmass, double *w,
                          double *part) {
-  __shared__ double red[VIR_THREADS];
+  __shared__ double red[VIR_THREADS / 32][12];
   const RepGeo &R = g.rep[blockIdx.y];
   double acc[12];
 #pragma unroll
@@ -159,8 +232,8 @@ __global__ void __launch_bounds__(VIR_THREADS)
        a += gridDim.x * blockDim.x) {
     const int slot = atom_slot[a];
     const d4 p = s.p[slot];
-    const double k[6] = {p.x * p.x / rmass, p.y * p.y / rmass, p.z * p.z / rmass,
-                         p.y * p.z / rmass, p.x * p.z / rmass, p.x * p.y / rmass};
+    const double vx = p.x / rmass, vy = p.y / rmass, vz = p.z / rmass;
+    const double k[6] = {p.x * vx, p.y * vy, p.z * vz, p.y * vz, p.x * vz, p.x * vy};
     double *ws = w + 6 * (size_t)slot;
 #pragma unroll
     for (int c = 0; c < 6; c++) {
@@ -170,25 +243,29 @@ __global__ void __launch_bounds__(VIR_THREADS)
       ws[c] = -(v + k[c]);
     }
   }
+  const int lane = threadIdx.x & 31;
+#pragma unroll
   for (int c = 0; c < 12; c++) {
-    red[threadIdx.x] = acc[c];
-    __syncthreads();
-    for (int o = VIR_THREADS / 2; o > 0; o >>= 1) {
-      if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) part[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 12 + c] = red[0];
-    __syncthreads();
+    double v = acc[c];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) red[threadIdx.x >> 5][c] = v;
   }
+  __syncthreads();
+  if (threadIdx.x >= 12) return;
+  double v = 0.0;
+  for (int w = 0; w < VIR_THREADS / 32; w++) v += red[w][threadIdx.x];
+  part[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 12 + threadIdx.x] = v;
 }
 
-// out[12 r + c] = sum over the parts of replica r, in part order
-__global__ void virial_final_kernel(const double *part, int nparts, double *out) {
-  const int r = blockIdx.x, c = threadIdx.x;
-  if (c >= 12) return;
+// out[12 r + c] = sum over the parts of replica r, a warp each: lane l takes
+// parts l, l + 32, ..., then a tree (one thread over 64 parts took 8 us)
+__global__ void __launch_bounds__(12 * 32)
+    virial_final_kernel(const double *part, int nparts, double *out) {
+  const int r = blockIdx.x, c = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double v = 0.0;
-  for (int x = 0; x < nparts; x++) v += part[((size_t)r * nparts + x) * 12 + c];
-  out[12 * r + c] = v;
+  for (int x = lane; x < nparts; x += 32) v += part[((size_t)r * nparts + x) * 12 + c];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (lane == 0) out[12 * r + c] = v;
 }
 
 size_t eam_virial_smem(const comdgb_sim *h) {
@@ -204,11 +281,32 @@ int allow_smem(K kernel, size_t smem) {
   return 0;
 }
 
+template <int LANES>
+void launch_virial64(comdgb_sim *h, double *out) {
+  const ForceArgs A = force_args(h);
+  const unsigned n = (unsigned)(((long)h->ntot * LANES + F64_THREADS - 1) / F64_THREADS);
+  if (h->opts.potential == COMDGB_POT_LJ)
+    lj64_virial_kernel<LANES><<<n, F64_THREADS, 0, h->stream>>>(A, h->lj64, out);
+  else if (h->opts.potential == COMDGB_POT_EAM_TABLE)
+    eam64_virial_kernel<EVAL_TABLE, LANES><<<n, F64_THREADS, 0, h->stream>>>(A, h->eam64t, out);
+  else
+    eam64_virial_kernel<EVAL_CHEBY, LANES><<<n, F64_THREADS, 0, h->stream>>>(A, h->eam64c, out);
+}
+
 // the per-slot virial of the state the last force call saw
 int launch_virial(comdgb_sim *h, double *out) {
   const ForceArgs A = force_args(h);
   cudaStream_t st = h->stream;
   const int pot = h->opts.potential;
+  if (!h->mixed) {
+    const int lanes = lanes64(h->ntot);
+    if (h->ntot <= 0) return 0;
+    if (lanes == 16) launch_virial64<16>(h, out);
+    else if (lanes == 4) launch_virial64<4>(h, out);
+    else launch_virial64<1>(h, out);
+    CK(cudaGetLastError());
+    return 0;
+  }
   int dev_sms = 1;
   CK(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, h->device));
   long need = ((long)h->ntot + VIR_THREADS - 1) / VIR_THREADS;
@@ -217,28 +315,22 @@ int launch_virial(comdgb_sim *h, double *out) {
   const bool fo = h->fo.list != nullptr;
   if (pot == COMDGB_POT_LJ) {
     if (fo) lj_virial_kernel<float, true><<<grid, VIR_THREADS, 0, st>>>(A, h->lj32, out);
-    else if (h->mixed) lj_virial_kernel<float, false><<<grid, VIR_THREADS, 0, st>>>(A, h->lj32, out);
-    else lj_virial_kernel<double, false><<<grid, VIR_THREADS, 0, st>>>(A, h->lj64, out);
+    else lj_virial_kernel<float, false><<<grid, VIR_THREADS, 0, st>>>(A, h->lj32, out);
   } else if (pot == COMDGB_POT_EAM_TABLE) {
     if (fo)
       eam_virial_kernel<float, EVAL_TABLE, true><<<grid, VIR_THREADS, 0, st>>>(A, h->eam32t, out);
-    else if (h->mixed)
-      eam_virial_kernel<float, EVAL_TABLE, false><<<grid, VIR_THREADS, 0, st>>>(A, h->eam32t, out);
     else
-      eam_virial_kernel<double, EVAL_TABLE, false><<<grid, VIR_THREADS, 0, st>>>(A, h->eam64t, out);
+      eam_virial_kernel<float, EVAL_TABLE, false><<<grid, VIR_THREADS, 0, st>>>(A, h->eam32t, out);
   } else {
     int rc;
     if (fo) {
       if ((rc = allow_smem(eam_virial_kernel<float, EVAL_CHEBY, true>, smem))) return rc;
       eam_virial_kernel<float, EVAL_CHEBY, true><<<grid, VIR_THREADS, smem, st>>>(A, h->eam32c,
                                                                                   out);
-    } else if (h->mixed) {
+    } else {
       if ((rc = allow_smem(eam_virial_kernel<float, EVAL_CHEBY, false>, smem))) return rc;
       eam_virial_kernel<float, EVAL_CHEBY, false><<<grid, VIR_THREADS, smem, st>>>(A, h->eam32c,
                                                                                    out);
-    } else {
-      eam_virial_kernel<double, EVAL_CHEBY, false><<<grid, VIR_THREADS, 0, st>>>(A, h->eam64c,
-                                                                                 out);
     }
   }
   CK(cudaGetLastError());
@@ -272,9 +364,13 @@ int compute_virial(comdgb_sim *h) {
   cudaStream_t st = h->stream;
   CK(cudaMemsetAsync(h->vir_slot, 0, sizeof(double) * 6 * (size_t)h->nslots, st));
   if ((rc = launch_virial(h, h->vir_slot))) return rc;
-  virial_reduce_kernel<<<dim3(VIR_PARTS, h->nrep), VIR_THREADS, 0, st>>>(
+  // as many parts as an average replica fills (64 of them took 106 us at
+  // 256,000 atoms, 304 take 40)
+  const int parts =
+      std::max(1, std::min(VIR_PARTS, (h->ntot / h->nrep + VIR_THREADS - 1) / VIR_THREADS));
+  virial_reduce_kernel<<<dim3(parts, h->nrep), VIR_THREADS, 0, st>>>(
       h->g, h->s, h->atom_slot, h->rmass, h->vir_slot, h->vir_part);
-  virial_final_kernel<<<h->nrep, 32, 0, st>>>(h->vir_part, VIR_PARTS, h->vir_out);
+  virial_final_kernel<<<h->nrep, 12 * 32, 0, st>>>(h->vir_part, parts, h->vir_out);
   CK(cudaGetLastError());
   h->vir_sums.resize(12 * (size_t)h->nrep);
   CK(cudaMemcpyAsync(h->vir_sums.data(), h->vir_out, sizeof(double) * h->vir_sums.size(),
