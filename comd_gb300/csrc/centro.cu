@@ -15,17 +15,19 @@
 // The parameter is the minimum over the 10395 pairings of the 12 vectors of
 // the sum of |r_a + r_b|^2, accumulated in a float over the pairs in the
 // order of their lower index (testCentro, :560-664).  The 66 pair terms are
-// rounded to FP32 once; a depth-first search over the pairings (the lowest
-// unpaired vector paired first, as the visualiser's loops pair them) finds
-// the least plain-FP32 sum, cutting every branch whose partial sum already
-// reaches the best complete one (partial sums of non-negative terms never
-// decrease, so the cut loses nothing; the greedy pairing gives the first
-// bound).  A second search visits the pairings whose FP32 sum lies within
-// 4e-6 of that least and sums them exactly as testCentro does (double terms,
-// each partial sum rounded to float).  Both sums round at most six float
-// additions of non-negative terms, so each is within 12 units of 2^-24 of
-// the exact sum: a pairing outside the window cannot be the reference's
-// minimum, and the result is the reference's value bit for bit.
+// formed in FP32 once; a depth-first search over the pairings (the lowest
+// unpaired vector paired first, as the visualiser's loops pair them) cuts every
+// branch whose partial FP32 sum is past a window above the least complete one
+// so far (partial sums of non-negative terms never decrease, so the cut loses
+// nothing; the greedy pairing gives the first window), and the pairings it
+// keeps are summed exactly as testCentro does (double terms, each partial sum
+// rounded to float).  The window holds the reference's minimum: with m the
+// largest component, an FP32 component of r_a + r_b is off by at most d =
+// 2^-22 m, so the FP32 sum F of a pairing and its exact sum T differ by at
+// most 2 d sqrt(18 T) + 18 d^2 + 6e-7 T; the reference's sum is within 12 units
+// of 2^-24 of T.  A pairing with the least reference sum thus has an F of at
+// most F' + 18.5 d sqrt(F') + 340 d^2 + 3e-6 F', F' any pairing's; the window
+// is wider than that.  The result is the reference's value bit for bit.
 // APPROX_CENTROSYM's greedy pairing (:528-557) is the `approx` variant.
 #include <algorithm>
 
@@ -44,51 +46,30 @@ __device__ __forceinline__ int pidx(int a, int b) { return 11 * a - (a * (a - 1)
 
 __device__ __forceinline__ long long key(double rsq) { return __double_as_longlong(rsq); }
 
+struct V3 {
+  double x, y, z;
+};
 // |a + b|^2 of two held vectors, the reference's order
-__device__ __forceinline__ double pair_term(const double (*v)[3][CT], int a, int b, int t) {
-  const double x = __dadd_rn(v[a][0][t], v[b][0][t]);
-  const double y = __dadd_rn(v[a][1][t], v[b][1][t]);
-  const double z = __dadd_rn(v[a][2][t], v[b][2][t]);
+__device__ __forceinline__ double pair_term(const V3 &a, const V3 &b) {
+  const double x = __dadd_rn(a.x, b.x), y = __dadd_rn(a.y, b.y), z = __dadd_rn(a.z, b.z);
   return __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
 }
 
-// Depth-first over the pairings: the lowest unpaired entry is paired next,
-// with its partners in index order.  A branch whose partial FP32 sum reaches
-// `bound` (STRICT) or exceeds it is cut.  leaf(sum, nn, pp) gets every
-// pairing kept; its pairs are (nn[l], pp[l]), l = 0..5, lower index first.
-template <bool STRICT, class Leaf>
-__device__ __forceinline__ void pairing_dfs(const float (*p)[CT], int t, const float &bound,
-                                            Leaf &&leaf) {
-  int nn[6], pp[6];
-  float acc[6];
-  int used = 1, lvl = 0;
-  nn[0] = 0;
-  pp[0] = 0;
-  acc[0] = 0.0f;
-  while (true) {
-    int q = pp[lvl] + 1;
-    while (q < 12 && (used >> q & 1)) q++;
-    if (q >= 12) {  // this level's partners are done
-      used &= ~(1 << nn[lvl]);
-      if (lvl == 0) break;
-      lvl--;
-      used &= ~(1 << pp[lvl]);
-      continue;
-    }
-    pp[lvl] = q;
-    const float a = __fadd_rn(acc[lvl], p[pidx(nn[lvl], q)][t]);
-    if (STRICT ? a >= bound : a > bound) continue;
-    if (lvl == 5) {
-      leaf(a, nn, pp);
-      continue;
-    }
-    used |= 1 << q;
-    lvl++;
-    acc[lvl] = a;
-    const int n = __ffs(~used) - 1;
-    nn[lvl] = n;
-    pp[lvl] = n;
-    used |= 1 << n;
+// Depth-first over the pairings from level L (pairs formed) on: the lowest
+// unpaired entry is paired next, with its partners in index order.  A branch
+// whose partial sum exceeds `bound` is cut.  leaf(sum, pairs) gets every pairing
+// kept, pair l in bits 8 l: its lower index, then its higher.
+template <int L, class P, class Leaf>
+__device__ __forceinline__ void pairing_dfs(P &&p, int used, float acc, unsigned long long pairs,
+                                            const float &bound, Leaf &&leaf) {
+  const int n = __ffs(~used) - 1;
+  for (int m = ~used & 0xfff & ~(1 << n); m != 0; m &= m - 1) {
+    const int q = __ffs(m) - 1;
+    const float a = __fadd_rn(acc, p(pidx(n, q)));
+    if (a > bound) continue;
+    const unsigned long long with = pairs | (unsigned long long)(n | q << 4) << (8 * L);
+    if constexpr (L == 5) leaf(a, with);
+    else pairing_dfs<L + 1>(p, used | 1 << n | 1 << q, a, with, bound, leaf);
   }
 }
 
@@ -120,17 +101,24 @@ __device__ __forceinline__ float outside(float lo, float hi, float p, float f) {
   return fmaxf(fmaxf((lo - p) + f, -((hi - p) + f)), 0.f);
 }
 
+// What bounds the exact variant is latency in divergent code: 12 of 32 lanes
+// active, and as many warps as shared memory holds.  So a thread keeps there
+// only the r^2 and the candidate's number of its held vectors, and later the
+// 66 terms in the place of the r^2 (288 bytes a thread; with the vectors it was
+// 648, and nine warps an SM), and the exact sums wait until its search is over,
+// when the warp forms them together.  256,000 atoms: 1,947 us -> 1,230 us
+// (1,383 with 80 registers and 24 warps an SM).
+template <bool APPROX>
 __global__ void __launch_bounds__(CT) centro_kernel(Geom g, Slots s, const double *dcenter,
-                                                    const int *atom_slot, int ntot, int approx,
-                                                    float slack, const float4 *ext,
-                                                    double *out) {
-  // per thread (column t): held vectors, their r^2 (integer images) and the
-  // pair terms rounded to FP32.  Warps run the scan and the pairing phases
-  // at different times with no barrier between them, so no array is shared
-  // between the phases.
-  __shared__ double v[12][3][CT];
-  __shared__ long long vk[12][CT];
-  __shared__ float p32[NPAIR][CT];
+                                                    const int *atom_slot, int ntot, float slack,
+                                                    const float4 *ext, double *out) {
+  // A thread's column t: 33 of 8 bytes (the twelve r^2 as integer images, later
+  // the terms in pairs) and the held candidates' numbers.  Warps run the scan
+  // and the pairing phases at different times with no barrier between them:
+  // the columns of two threads share no byte.
+  __shared__ uint2 col[APPROX ? 12 : (NPAIR + 1) / 2][CT];
+  __shared__ unsigned short held[12][CT];  // cell * 64 + atom
+  __shared__ double vs[APPROX ? 36 : 1][APPROX ? CT : 1];
   const int t = threadIdx.x;
   const int a = blockIdx.x * CT + t;
   if (a >= ntot) return;
@@ -144,9 +132,13 @@ __global__ void __launch_bounds__(CT) centro_kernel(Geom g, Slots s, const doubl
   const d4 ri = s.r[io];
   int nb = 0, kmax = 0;
   long long rmax = 0;
-  auto offer = [&](double dx, double dy, double dz) {
+  auto held_rsq = [&](int k) {
+    const uint2 r = col[k][t];
+    return (long long)((unsigned long long)r.y << 32 | r.x);
+  };
+  auto offer = [&](const V3 &d, int number) {
     const double rsq =
-        __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+        __dadd_rn(__dadd_rn(__dmul_rn(d.x, d.x), __dmul_rn(d.y, d.y)), __dmul_rn(d.z, d.z));
     const long long kk = key(rsq);
     int i1;
     if (nb < 12) {
@@ -155,18 +147,19 @@ __global__ void __launch_bounds__(CT) centro_kernel(Geom g, Slots s, const doubl
       if (kk > rmax) return;
       i1 = kmax;
     }
-    v[i1][0][t] = dx;
-    v[i1][1][t] = dy;
-    v[i1][2][t] = dz;
-    vk[i1][t] = kk;
+    col[i1][t] = make_uint2((unsigned)kk, (unsigned)(kk >> 32));
+    held[i1][t] = (unsigned short)number;
     if (nb == 12) {  // first entry of largest r^2
       kmax = 0;
-      rmax = vk[0][t];
-      for (int k = 1; k < 12; k++)
-        if (vk[k][t] > rmax) {
+      rmax = held_rsq(0);
+#pragma unroll
+      for (int k = 1; k < 12; k++) {
+        const long long r = held_rsq(k);
+        if (r > rmax) {
           kmax = k;
-          rmax = vk[k][t];
+          rmax = r;
         }
+      }
     }
   };
   // Candidates past the largest of twelve held are refused by the FP64 test in
@@ -181,12 +174,41 @@ __global__ void __launch_bounds__(CT) centro_kernel(Geom g, Slots s, const doubl
   const double cxi = __dadd_rn(dcenter[3 * b + 0], ri.x);
   const double cyi = __dadd_rn(dcenter[3 * b + 1], ri.y);
   const double czi = __dadd_rn(dcenter[3 * b + 2], ri.z);
+  // box and corner of cell (x-outer, z-inner; 13 is the own box), wrapped once
+  // per axis with the periodic offset rounded to float
+  auto corner = [&](int cell, V3 &e) {
+    float ox = 0.0f, oy = 0.0f, oz = 0.0f;
+    int qx = bx + cell / 9 - 1, qy = by + cell / 3 % 3 - 1, qz = bz + cell % 3 - 1;
+    if (qx < 0) { qx = nx - 1; ox = __double2float_rn(-R.bounds[0]); }
+    if (qx >= nx) { qx = 0; ox = __double2float_rn(R.bounds[0]); }
+    if (qy < 0) { qy = ny - 1; oy = __double2float_rn(-R.bounds[1]); }
+    if (qy >= ny) { qy = 0; oy = __double2float_rn(R.bounds[1]); }
+    if (qz < 0) { qz = nz - 1; oz = __double2float_rn(-R.bounds[2]); }
+    if (qz >= nz) { qz = 0; oz = __double2float_rn(R.bounds[2]); }
+    const int b2 = R.box0 + qz * nx * ny + qy * nx + qx;
+    e = V3{__dadd_rn((double)ox, dcenter[3 * b2 + 0]), __dadd_rn((double)oy, dcenter[3 * b2 + 1]),
+           __dadd_rn((double)oz, dcenter[3 * b2 + 2])};
+    return b2;
+  };
+  // the vector to atom j of box b2
+  auto vector = [&](int b2, int j, bool same, const V3 &e) {
+    const d4 rj = s.r[b2 * CG_MAXATOMS + j];
+    if (same) return V3{__dsub_rn(rj.x, ri.x), __dsub_rn(rj.y, ri.y), __dsub_rn(rj.z, ri.z)};
+    return V3{__dsub_rn(__dadd_rn(e.x, rj.x), cxi), __dsub_rn(__dadd_rn(e.y, rj.y), cyi),
+              __dsub_rn(__dadd_rn(e.z, rj.z), czi)};
+  };
+  auto held_vector = [&](int k) {
+    const int number = held[k][t], cell = number >> 6;
+    V3 e;
+    const int b2 = cell == 13 ? b : corner(cell, e);
+    return vector(b2, number & 63, cell == 13, e);
+  };
   const float4 pi = __ldg(s.pos32 + io);
   const float own = slack + 1e-6f * (fabsf(pi.x) + fabsf(pi.y) + fabsf(pi.z));
   float cut = 3.0e38f;  // est must be below it
-  // the candidates of box b2 with corner offset e (own box: relative)
-  auto scan = [&](int b2, int nj, bool same, double ex, double ey, double ez, float fx, float fy,
-                  float fz) {
+  // the candidates of a cell: box b2, corner e (own box: relative)
+  auto scan = [&](int cell, int b2, int nj, const V3 &e, float fx, float fy, float fz) {
+    const bool same = cell == 13;
     int j = 0;
     while (true) {
       bool got = false;
@@ -198,52 +220,44 @@ __global__ void __launch_bounds__(CT) centro_kernel(Geom g, Slots s, const doubl
         if (got) break;
       }
       if (!got) break;
-      const d4 rj = s.r[b2 * CG_MAXATOMS + j];
+      offer(vector(b2, j, same, e), cell * 64 + j);
       j++;
-      if (same)
-        offer(__dsub_rn(rj.x, ri.x), __dsub_rn(rj.y, ri.y), __dsub_rn(rj.z, ri.z));
-      else
-        offer(__dsub_rn(__dadd_rn(ex, rj.x), cxi), __dsub_rn(__dadd_rn(ey, rj.y), cyi),
-              __dsub_rn(__dadd_rn(ez, rj.z), czi));
       if (nb == 12) {
         // est < (r + e)^2, e the FP32 vector's error: slack for the box offset,
         // and roundings of the atom's own position and of the distance
         const float r2 = __double2float_ru(__longlong_as_double(rmax));
-        const float r = sqrtf(r2), e = own + 1e-6f * r;
-        cut = (r2 + e * (2.0f * r + e) + 1e-30f) * 1.000001f;
+        const float r = sqrtf(r2), err = own + 1e-6f * r;
+        cut = (r2 + err * (2.0f * r + err) + 1e-30f) * 1.000001f;
       }
     }
   };
-  scan(b, ni, true, 0.0, 0.0, 0.0, 0.f, 0.f, 0.f);
+  scan(13, b, ni, V3{0.0, 0.0, 0.0}, 0.f, 0.f, 0.f);
   for (int cell = 0; cell < 27; cell++) {  // x-outer, z-inner
     if (cell == 13) continue;
-    float ox = 0.0f, oy = 0.0f, oz = 0.0f;
-    int qx = bx + cell / 9 - 1, qy = by + cell / 3 % 3 - 1, qz = bz + cell % 3 - 1;
-    if (qx < 0) { qx = nx - 1; ox = __double2float_rn(-R.bounds[0]); }
-    if (qx >= nx) { qx = 0; ox = __double2float_rn(R.bounds[0]); }
-    if (qy < 0) { qy = ny - 1; oy = __double2float_rn(-R.bounds[1]); }
-    if (qy >= ny) { qy = 0; oy = __double2float_rn(R.bounds[1]); }
-    if (qz < 0) { qz = nz - 1; oz = __double2float_rn(-R.bounds[2]); }
-    if (qz >= nz) { qz = 0; oz = __double2float_rn(R.bounds[2]); }
-    const int b2 = R.box0 + qz * nx * ny + qy * nx + qx;
-    const double ex = __dadd_rn((double)ox, dcenter[3 * b2 + 0]);
-    const double ey = __dadd_rn((double)oy, dcenter[3 * b2 + 1]);
-    const double ez = __dadd_rn((double)oz, dcenter[3 * b2 + 2]);
-    const float fx = (float)(ex - dcenter[3 * b + 0]), fy = (float)(ey - dcenter[3 * b + 1]),
-                fz = (float)(ez - dcenter[3 * b + 2]);
+    V3 e;
+    const int b2 = corner(cell, e);
+    const float fx = (float)(e.x - dcenter[3 * b + 0]), fy = (float)(e.y - dcenter[3 * b + 1]),
+                fz = (float)(e.z - dcenter[3 * b + 2]);
     // a box whose atoms all fail the test is passed over whole
     const float4 lo = __ldg(ext + 2 * b2), hi = __ldg(ext + 2 * b2 + 1);
     const float gx = outside(lo.x, hi.x, pi.x, fx), gy = outside(lo.y, hi.y, pi.y, fy),
                 gz = outside(lo.z, hi.z, pi.z, fz);
     if (gx * gx + gy * gy + gz * gz >= cut) continue;
-    scan(b2, s.natoms[b2], false, ex, ey, ez, fx, fy, fz);
+    scan(cell, b2, s.natoms[b2], e, fx, fy, fz);
   }
   double c = 1000.0;
   if (nb >= 12) {
-    if (approx) {
+    if constexpr (APPROX) {
+      for (int k = 0; k < 12; k++) {
+        const V3 d = held_vector(k);
+        vs[3 * k][t] = d.x;
+        vs[3 * k + 1][t] = d.y;
+        vs[3 * k + 2][t] = d.z;
+      }
+      auto v = [&](int k) { return V3{vs[3 * k][t], vs[3 * k + 1][t], vs[3 * k + 2][t]}; };
       // greedy pairing; a vector with r^2 = 0 counts as paired
       int paired = 0;
-      for (int q = 0; q < 12; q++) paired |= (vk[q][t] > 0 ? 0 : 1) << q;
+      for (int q = 0; q < 12; q++) paired |= (held_rsq(q) > 0 ? 0 : 1) << q;
       c = 0.0;
       for (int j = 0; j < 11; j++) {
         if (paired >> j & 1) continue;
@@ -251,7 +265,7 @@ __global__ void __launch_bounds__(CT) centro_kernel(Geom g, Slots s, const doubl
         int kmin = -1;
         for (int k = j + 1; k < 12; k++) {
           if (paired >> k & 1) continue;
-          const double sum = pair_term(v, j, k, t);
+          const double sum = pair_term(v(j), v(k));
           if (sum < summin) {
             kmin = k;
             summin = sum;
@@ -262,8 +276,27 @@ __global__ void __launch_bounds__(CT) centro_kernel(Geom g, Slots s, const doubl
         if (kmin >= 0) paired |= 1 << kmin;
       }
     } else {
-      for (int x = 0, k = 0; x < 12; x++)
-        for (int y = x + 1; y < 12; y++, k++) p32[k][t] = __double2float_rn(pair_term(v, x, y, t));
+      float x[12], y[12], z[12], most = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 12; k++) {
+        const V3 d = held_vector(k);
+        x[k] = (float)d.x;
+        y[k] = (float)d.y;
+        z[k] = (float)d.z;
+        most = fmaxf(most, fmaxf(fabsf(x[k]), fmaxf(fabsf(y[k]), fabsf(z[k]))));
+      }
+      float low = 0.0f;
+#pragma unroll
+      for (int i = 0, k = 0; i < 12; i++)
+#pragma unroll
+        for (int j = i + 1; j < 12; j++, k++) {
+          const float sx = x[i] + x[j], sy = y[i] + y[j], sz = z[i] + z[j];
+          const float term = fmaf(sz, sz, fmaf(sy, sy, sx * sx));
+          if (k & 1) col[k >> 1][t] = make_uint2(__float_as_uint(low), __float_as_uint(term));
+          low = term;
+        }
+      const unsigned *terms = &col[0][t].x;
+      auto p = [&](int k) { return __uint_as_float(terms[(k >> 1) * (2 * CT) + (k & 1)]); };
       // first bound: the greedy pairing's FP32 sum (a complete pairing)
       float best = 0.0f;
       for (int used = 0, step = 0; step < 6; step++) {
@@ -272,21 +305,40 @@ __global__ void __launch_bounds__(CT) centro_kernel(Geom g, Slots s, const doubl
         int qb = -1;
         float pb = 0.0f;
         for (int q = n + 1; q < 12; q++)
-          if (!(used >> q & 1) && (qb < 0 || p32[pidx(n, q)][t] < pb)) {
+          if (!(used >> q & 1) && (qb < 0 || p(pidx(n, q)) < pb)) {
             qb = q;
-            pb = p32[pidx(n, q)][t];
+            pb = p(pidx(n, q));
           }
         used |= 1 << qb;
         best = __fadd_rn(best, pb);
       }
-      pairing_dfs<true>(p32, t, best, [&](float sum, const int *, const int *) { best = sum; });
-      const float window = __fadd_rn(best, __fmul_rn(best, 4e-6f)) + 1e-37f;
-      pairing_dfs<false>(p32, t, window, [&](float, const int *nn, const int *pp) {
-        float e = 0.0f;  // testCentro
-        for (int l = 0; l < 6; l++)
-          e = __double2float_rn(__dadd_rn((double)e, pair_term(v, nn[l], pp[l], t)));
+      const float d = most * 0x1p-22f;
+      auto window = [&](float f) { return f * 1.000005f + d * (24.0f * sqrtf(f) + 600.0f * d) + 1e-37f; };
+      float bound = window(best), kept = 0.0f;
+      unsigned long long pending = 0;
+      auto exact = [&](unsigned long long pairs) {  // testCentro
+        float e = 0.0f;
+        for (int l = 0; l < 6; l++) {
+          const int pair = (int)(pairs >> (8 * l)) & 255;
+          e = __double2float_rn(
+              __dadd_rn((double)e, pair_term(held_vector(pair & 15), held_vector(pair >> 4))));
+        }
         if ((double)e < c) c = (double)e;
+      };
+      // one pairing is kept for later, those that may be as good (the one kept
+      // or the new one) are summed at once
+      pairing_dfs<0>(p, 0, 0.0f, 0ull, bound, [&](float sum, unsigned long long pairs) {
+        if (sum < best) {
+          best = sum;
+          bound = window(best);
+        }
+        if (pending != 0 && !(kept > bound)) exact(pairs);
+        else {
+          pending = pairs;
+          kept = sum;
+        }
       });
+      if (pending != 0) exact(pending);
     }
   }
   out[io] = c;
@@ -352,9 +404,13 @@ int comdgb_sim_centrosymmetry(comdgb_sim *h, int r, int approx, double *out, dou
     launch_pos32_atoms(h->g, h->s, h->atom_slot, h->ntot, st);
     box_extent_kernel<<<(h->g.nboxes + 255) / 256, 256, 0, st>>>(h->s, h->g.nboxes,
                                                                  h->centro_ext);
-    centro_kernel<<<(h->ntot + CT - 1) / CT, CT, 0, st>>>(h->g, h->s, h->dcenter, h->atom_slot,
-                                                           h->ntot, approx, slack,
-                                                           h->centro_ext, h->centro);
+    const unsigned n = (h->ntot + CT - 1) / CT;
+    if (approx)
+      centro_kernel<true><<<n, CT, 0, st>>>(h->g, h->s, h->dcenter, h->atom_slot, h->ntot, slack,
+                                            h->centro_ext, h->centro);
+    else
+      centro_kernel<false><<<n, CT, 0, st>>>(h->g, h->s, h->dcenter, h->atom_slot, h->ntot, slack,
+                                             h->centro_ext, h->centro);
     centro_range_kernel<<<2 * h->sms, 256, 0, st>>>(
         h->s, h->atom_slot, h->centro, R.a0, R.na,
         reinterpret_cast<unsigned long long *>(h->centro + h->nslots));

@@ -247,3 +247,24 @@ def test_gpu_batch_centro_equals_single(oracle):
     finally:
         for s in bs:
             cg.free_host(s)
+
+
+# many pairings of nearly equal sums (a disordered box), and atoms with ties in
+# both the distances and the pairings (a lattice half of whose atoms are moved
+# by a micro-Angstrom): the FP32 window has to keep the least of them
+@pytest.mark.gpu
+@pytest.mark.parametrize("amp", [1e-6, 0.3, 0.9])
+def test_gpu_centro_with_close_pairings(oracle, amp):
+    s, _pot = perfect()
+    try:
+        v = slot_views(s)
+        m = occupied_mask(s)
+        m[::2] = False
+        v["r"][m] += np.random.default_rng(7).uniform(-amp, amp, (int(m.sum()), 3))
+        assert oracle.rebox(s) == 0
+        co, lo, hi = oracle.centro(s, False)
+        cgpu, glo, ghi = gpu_centro(s)
+        assert np.array_equal(cgpu, np.where(occupied_mask(s), co, 0.0))
+        assert (glo, ghi) == (lo, hi)
+    finally:
+        cg.free_host(s)
