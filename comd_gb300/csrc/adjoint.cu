@@ -40,6 +40,7 @@ namespace {
 
 constexpr int NC = CG_NCHEB;
 constexpr int BASIS_THREADS = 128;  // CTA of the basis-sum kernels
+constexpr int LOG_STEPS = 64;       // backward steps whose sums wait on the device
 constexpr int NQ = 4;               // sums per coefficient index at most: three over pairs, one over atoms
 
 // the FP64 series of the simulation and their second derivatives
@@ -547,6 +548,7 @@ int work(comdgb_sim *h, Work *&Wp) {
   W.loss = track(h, dalloc<double>((size_t)h->ntot + 1, &err));
   W.partial = track(h, dalloc<double>((size_t)W.nblk * NQ * NC + 4096, &err));
   W.out = track(h, dalloc<double>(NQ * NC + 8, &err));
+  W.log = track(h, dalloc<double>((size_t)LOG_STEPS * NQ * NC, &err));
   W.target = track(h, dalloc<double>(nv, &err));
   W.rb = track(h, dalloc<double>(nv, &err));
   W.pb = track(h, dalloc<double>(nv, &err));
@@ -615,7 +617,7 @@ void basis_derivative(const double *t, double *d) {
 }
 
 template <int NW>
-void launch_basis(comdgb_sim *h, Work &W, const ChebSet &S, Lam L) {
+void launch_basis(comdgb_sim *h, Work &W, const ChebSet &S, Lam L, double *out) {
   const ForceArgs A = force_args(h);
   const double rc2 = h->eam64c.rc2;
   const bool same = S.a[0] == S.a[1] && S.b[0] == S.b[1];
@@ -624,23 +626,24 @@ void launch_basis(comdgb_sim *h, Work &W, const ChebSet &S, Lam L) {
   auto run = [&](auto kernel) { kernel<<<grid, BASIS_THREADS, 0, h->stream>>>(A, S, rc2, L, W.partial); };
   if (same) run(adj_basis_kernel<NW, true>);
   else run(adj_basis_kernel<NW, false>);
-  adj_sum_kernel<<<NW * NC, 256, 0, h->stream>>>(W.partial, grid, NW * NC, W.out);
+  adj_sum_kernel<<<NW * NC, 256, 0, h->stream>>>(W.partial, grid, NW * NC, out);
 }
 
-// The gradient in the coefficients at the current forces and per-step list,
-// to g[3*NC] on the host: dU/dc, or with lambda set dD/dc.
-int eam_grad(comdgb_sim *h, Work &W, const ChebSet &S, bool with_lam, double *g) {
-  if (with_lam) launch_basis<3>(h, W, S, Lam{W.lam, W.x});
-  else launch_basis<2>(h, W, S, Lam{nullptr, nullptr});
+// The sums of the gradient in the coefficients at the current forces and
+// per-step list, to out[0 .. (2 or 3 + 1) NC) on the device.
+void enqueue_eam_sums(comdgb_sim *h, Work &W, const ChebSet &S, bool with_lam, double *out) {
+  if (with_lam) launch_basis<3>(h, W, S, Lam{W.lam, W.x}, out);
+  else launch_basis<2>(h, W, S, Lam{nullptr, nullptr}, out);
   const int nw = with_lam ? 3 : 2;
   const int nb = std::max(1, std::min(W.nblk, (h->ntot + BASIS_THREADS - 1) / BASIS_THREADS));
   adj_embed_basis_kernel<<<nb, BASIS_THREADS, 0, h->stream>>>(force_args(h), S,
                                                               with_lam ? W.w : nullptr, W.partial);
-  adj_sum_kernel<<<NC, 256, 0, h->stream>>>(W.partial, nb, NC, W.out + nw * NC);
-  double t[NQ * NC];
-  CK(cudaMemcpyAsync(t, W.out, sizeof(double) * (nw + 1) * NC, cudaMemcpyDeviceToHost,
-                     h->stream));
-  CK(cudaStreamSynchronize(h->stream));
+  adj_sum_kernel<<<NC, 256, 0, h->stream>>>(W.partial, nb, NC, out + nw * NC);
+}
+
+// the gradient g[3*NC] from those sums: dU/dc, or with lambda set dD/dc
+void eam_grad_of(const ChebSet &S, bool with_lam, const double *t, double *g) {
+  const int nw = with_lam ? 3 : 2;
   const double *phi = t, *rho = t + NC, *f = t + nw * NC;
   if (!with_lam) {
     for (int k = 0; k < NC; k++) {
@@ -661,6 +664,16 @@ int eam_grad(comdgb_sim *h, Work &W, const ChebSet &S, bool with_lam, double *g)
         if (q == 1) g[q * NC + k] += k == 0 ? 0.5 * x[k] : x[k];
       }
   }
+}
+
+// both, with the gradient on the host
+int eam_grad(comdgb_sim *h, Work &W, const ChebSet &S, bool with_lam, double *g) {
+  enqueue_eam_sums(h, W, S, with_lam, W.out);
+  double t[NQ * NC];
+  CK(cudaMemcpyAsync(t, W.out, sizeof(double) * (with_lam ? 4 : 3) * NC, cudaMemcpyDeviceToHost,
+                     h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  eam_grad_of(S, with_lam, t, g);
   return check_status(h);
 }
 
@@ -692,9 +705,9 @@ int lj_sums(comdgb_sim *h, Work &W, bool with_lam, double *out4) {
 
 // a force call whose lists are built from the current state (so forces are
 // a function of the state alone, whatever the history of list builds)
-int force_fresh(comdgb_sim *h) {
+int force_fresh(comdgb_sim *h, bool wait = true) {
   if (h->pl.slot_of) CK(cudaMemsetAsync(h->status + ST_REBUILD, 0x01, 1, h->stream));
-  return do_force(h);
+  return wait ? do_force(h) : enqueue_force(h);
 }
 
 }  // namespace
@@ -789,7 +802,10 @@ int comdgb_sim_force_loss_grad(comdgb_sim *h, const double *target, double *loss
 // the adjoints (rb, pb) of step n+1:  pb += c rb;  u = -dt pb;  rb += H(r_a) u;
 // cbar += d(u . f(r_a))/dc;  pb += c rb.  Start: rb = grad U(r_N) (= f for
 // EAM), pb = 0, cbar = dU/dc at r_N.  Adjoint vectors are kept by atom id (the
-// rebox permutes slots, not atoms).
+// rebox permutes slots, not atoms).  The host waits once a segment, and for
+// the sums of every LOG_STEPS backward steps (a wait after every half step,
+// force call and sum took 13.1 ms in 20 steps of 3,960 atoms, this 9.5): errors are
+// kept on the device, the first one of a segment is the one reported.
 int comdgb_sim_traj_energy_grad(comdgb_sim *h, int n, double dt, int every, double *j,
                                 double *grad) {
   int rc = need_fp64(h);
@@ -814,13 +830,17 @@ int comdgb_sim_traj_energy_grad(comdgb_sim *h, int n, double dt, int every, doub
     if ((rc = snap(h, si++, q))) return rc;
   if ((rc = snap(h, si++, fin))) return rc;
   const ChebSet S = cheb_set(h);
+  CK(cudaMemsetAsync(h->status + ST_NONFINITE, 0, sizeof(int), h->stream));
   // forward, keeping the state at the start of every segment
   for (int t = 0; t < n; t++) {
-    if (t % every == 0 && (rc = snapshot_copy(h, *ck[t / every], true))) return rc;
-    if ((rc = step_first_half(h, dt_atu)) || (rc = force_fresh(h)) ||
+    if (t % every == 0 &&
+        ((t && (rc = check_forces(h))) || (rc = snapshot_copy(h, *ck[t / every], true))))
+      return rc;
+    if ((rc = step_first_half(h, dt_atu)) || (rc = force_fresh(h, false)) ||
         (rc = step_second_half(h, dt_atu)))
       return rc;
   }
+  if ((rc = check_forces(h))) return rc;
   if ((rc = force_fresh(h))) return rc;
   if (j) *j = h->e;
   if ((rc = snapshot_copy(h, *fin, true))) return rc;
@@ -828,17 +848,33 @@ int comdgb_sim_traj_energy_grad(comdgb_sim *h, int n, double dt, int every, doub
   if ((rc = eam_grad(h, W, S, false, cbar))) return rc;
   adj_force_by_id_kernel<<<blocks(h->ntot), 256, 0, h->stream>>>(h->s, h->atom_slot, h->ntot, rb);
   CK(cudaMemsetAsync(pb, 0, sizeof(double) * nv, h->stream));
+  // the logged sums into cbar, in the order of the steps
+  int logged = 0;
+  std::vector<double> sums((size_t)LOG_STEPS * NQ * NC);
+  auto flush = [&]() -> int {
+    if (logged)
+      CK(cudaMemcpyAsync(sums.data(), W.log, sizeof(double) * logged * NQ * NC,
+                         cudaMemcpyDeviceToHost, h->stream));
+    if (int e = check_forces(h)) return e;
+    for (int q = 0; q < logged; q++) {
+      eam_grad_of(S, true, &sums[(size_t)q * NQ * NC], g);
+      for (int k = 0; k < 3 * NC; k++) cbar[k] += g[k];
+    }
+    logged = 0;
+    return 0;
+  };
   // backward, segment by segment: recompute the segment's mid-step states
   for (int sgm = nseg - 1; sgm >= 0; sgm--) {
     const int t0 = sgm * every, m = std::min(every, n - t0);
     if ((rc = snapshot_copy(h, *ck[sgm], false))) return rc;
     for (int t = 0; t < m; t++) {
       if ((rc = step_first_half(h, dt_atu)) || (rc = snapshot_copy(h, *mid[t], true)) ||
-          (rc = force_fresh(h)) || (rc = step_second_half(h, dt_atu)))
+          (rc = force_fresh(h, false)) || (rc = step_second_half(h, dt_atu)))
         return rc;
     }
+    if ((rc = flush())) return rc;
     for (int t = m - 1; t >= 0; t--) {
-      if ((rc = snapshot_copy(h, *mid[t], false)) || (rc = force_fresh(h))) return rc;
+      if ((rc = snapshot_copy(h, *mid[t], false)) || (rc = force_fresh(h, false))) return rc;
       adj_axpy_kernel<<<blocks(nv), 256, 0, h->stream>>>(c, rb, pb, nv);
       adj_scale_kernel<<<blocks(nv), 256, 0, h->stream>>>(-dt_atu, pb, u, nv);
       if ((rc = set_lambda(h, W, S, nullptr, u))) return rc;
@@ -847,12 +883,13 @@ int comdgb_sim_traj_energy_grad(comdgb_sim *h, int n, double dt, int every, doub
         adj_hvp_kernel<L><<<blocks((long)h->ntot * L, F64_THREADS), F64_THREADS, 0, h->stream>>>(
             force_args(h), S, h->eam64c.poly, h->eam64c.rc2, W.lam, W.x, hv);
       });
-      if ((rc = eam_grad(h, W, S, true, g))) return rc;
-      for (int q = 0; q < 3 * NC; q++) cbar[q] += g[q];
+      enqueue_eam_sums(h, W, S, true, W.log + (size_t)logged * NQ * NC);
       adj_axpy_kernel<<<blocks(nv), 256, 0, h->stream>>>(1.0, hv, rb, nv);
       adj_axpy_kernel<<<blocks(nv), 256, 0, h->stream>>>(c, rb, pb, nv);
+      if (++logged == LOG_STEPS && (rc = flush())) return rc;
     }
   }
+  if ((rc = flush())) return rc;
   CK(cudaGetLastError());
   for (int q = 0; q < 3 * NC; q++) grad[q] = cbar[q];
   if ((rc = snapshot_copy(h, *fin, false))) return rc;

@@ -715,10 +715,7 @@ int read_status(comdgb_sim *h, int *st) {
   return 0;
 }
 
-int check_status(comdgb_sim *h) {
-  int st[ST_COUNT];
-  int rc = read_status(h, st);
-  if (rc) return rc;
+static int status_error(const int *st) {
   if (st[ST_ERROR] == COMDGB_ERR_MAXATOMS)
     return set_err(COMDGB_ERR_MAXATOMS, "Increase maxatoms: a box reached %d atoms",
                    CG_MAXATOMS);
@@ -728,6 +725,21 @@ int check_status(comdgb_sim *h) {
     return set_err(COMDGB_ERR_ARG, "atom ids must be 0..ntot-1, each once (persistent lists)");
   if (st[ST_ERROR]) return set_err(st[ST_ERROR], "device error %d", st[ST_ERROR]);
   return 0;
+}
+int check_status(comdgb_sim *h) {
+  int st[ST_COUNT];
+  int rc = read_status(h, st);
+  return rc ? rc : status_error(st);
+}
+// the force calls since ST_NONFINITE was cleared, as finish_force checks one
+int check_forces(comdgb_sim *h) {
+  int st[ST_COUNT];
+  int rc = read_status(h, st);
+  if (rc) return rc;
+  if (st[ST_NONFINITE])
+    return set_err(COMDGB_ERR_NONFINITE, "total energy is %s",
+                   st[ST_NONFINITE] == 1 ? "nan" : st[ST_NONFINITE] == 2 ? "inf" : "-inf");
+  return status_error(st);
 }
 
 // ---- kernel groups of one step --------------------------------------------
@@ -1134,13 +1146,24 @@ int force_graph(comdgb_sim *h, bool after_steps, cudaGraphExec_t *out, bool host
   return 0;
 }
 
-int do_force_ex(comdgb_sim *h, bool after_steps) {
+static int launch_force(comdgb_sim *h, bool after_steps) {
   if (h->opts.potential < 0) return set_err(COMDGB_ERR_ARG, "simulation has no potential");
   cudaGraphExec_t exec = nullptr;
   int rc = force_graph(h, after_steps, &exec);
   if (rc) return rc;
   CK(cudaGraphLaunch(exec, h->stream));
-  return finish_force(h);
+  return 0;
+}
+
+int do_force_ex(comdgb_sim *h, bool after_steps) {
+  int rc = launch_force(h, after_steps);
+  return rc ? rc : finish_force(h);
+}
+
+int enqueue_force(comdgb_sim *h) {
+  int rc = launch_force(h, false);
+  if (!rc) h->lists_built = h->pl.slot_of != nullptr;
+  return rc;
 }
 
 int do_force(comdgb_sim *h) { return do_force_ex(h, false); }
@@ -1368,7 +1391,8 @@ int relist(comdgb_sim *h) {
 
 // a velocity-Verlet step (timestep.c:129-132) as separate launches: the first
 // position half step and its rebox, then (after the caller's force call) the
-// velocity step, the second position half step and its rebox
+// velocity step, the second position half step and its rebox; the caller
+// checks the status
 int step_first_half(comdgb_sim *h, double dt_atu) {
   cudaStream_t st = h->stream;
   CK(cudaMemsetAsync(h->status + ST_REBIN_SERIAL, 0, sizeof(int), st));
@@ -1377,7 +1401,7 @@ int step_first_half(comdgb_sim *h, double dt_atu) {
   enqueue_classify_finish(h);
   enqueue_compact(h);
   CK(cudaGetLastError());
-  return check_status(h);
+  return 0;
 }
 int step_second_half(comdgb_sim *h, double dt_atu) {
   cudaStream_t st = h->stream;
@@ -1388,7 +1412,7 @@ int step_second_half(comdgb_sim *h, double dt_atu) {
   enqueue_classify_finish(h);
   enqueue_compact(h);
   CK(cudaGetLastError());
-  return check_status(h);
+  return 0;
 }
 
 // a device copy of the slot state (natoms, id, itype, mass, r, p)

@@ -153,7 +153,9 @@ enum {
   ST_OVF_BUILD = 7,   // persistent lists: overflows counted by the build in progress
   ST_FUSE = 8,        // force order: the force pass also makes the next step's velocity
                       // step and both position half steps (see fo_eam_pass2_kernel)
-  ST_COUNT = 9
+  ST_NONFINITE = 9,   // a force call's total energy was not finite, no error before it:
+                      // 1 not a number, 2 inf, 3 -inf (kept until cleared)
+  ST_COUNT = 10
 };
 
 // Persistent (skin) neighbour lists, keyed by atom id: built with cutoff

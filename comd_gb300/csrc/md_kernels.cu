@@ -943,6 +943,8 @@ __global__ void __launch_bounds__(RD_THREADS) reduce_force_kernel(ForceArgs A, d
     out[0] = e;
     out[1] = sx;
     iout[0] = np;
+    if (!isfinite(e) && A.status[ST_NONFINITE] == 0 && A.status[ST_ERROR] == 0)
+      A.status[ST_NONFINITE] = isnan(e) ? 1 : e > 0.0 ? 2 : 3;
   }
 }
 

@@ -120,6 +120,7 @@ struct comdgb_sim {
     d4 *lam = nullptr;
     double *w = nullptr, *x = nullptr, *loss = nullptr, *partial = nullptr, *out = nullptr;
     double *target = nullptr, *rb = nullptr, *pb = nullptr, *u = nullptr, *hv = nullptr;
+    double *log = nullptr;  // the gradient's sums of some backward steps
     int nblk = 0;
     std::vector<void *> snaps;  // Snapshot* (checkpoints, mid-step states, final)
   } adj;
@@ -198,6 +199,8 @@ T *track(comdgb_sim *h, T *p) {
 cg::ForceArgs force_args(comdgb_sim *h);
 comdgb_sim *find_attached(const void *s);  // the handle of an attached simflat_t
 int do_force(comdgb_sim *h);       // force call (graph), energy and stress to the host
+int enqueue_force(comdgb_sim *h);  // the same without a wait: device results only
+int check_forces(comdgb_sim *h);   // waits; the errors of the calls enqueued
 int check_status(comdgb_sim *h);
 // genDer (cheby.c:219-270): the derivative series of an n-term series on [a, b]
 void cheb_derive(double a, double b, const double *c, double *cd, int n);

@@ -250,3 +250,36 @@ def test_gpu_trajectory_adjoint_matches_finite_differences(oracle, n, every, tol
             d.close()
     finally:
         case.close()
+
+
+@pytest.mark.gpu
+def test_traj_gradient_over_segments(oracle):
+    """More steps than the device keeps gradient sums of, in one segment and in
+    nine: the same states, so the same sums (up to rounding); and an energy
+    that overflows on the way is reported as it is by a force call."""
+    case = Case(oracle, cg.POT_EAM_CHEBY, n=(5, 5, 5), amp=0.05, temp=600.0)
+    try:
+        c, x0, xn = cheb_base(case)
+        d = cg.DeviceSim(case.s, cg.opts(cg.POT_EAM_CHEBY, cg.PREC_FP64, True,
+                                         cheby_from_host=True))
+        try:
+            snap = [d.traj_energy_grad(70, 1e-15, 70)]
+            d.upload(case.s)
+            snap.append(d.traj_energy_grad(70, 1e-15, 8))
+            assert abs(snap[0][0] - snap[1][0]) <= 1e-12 * abs(snap[0][0])
+            np.testing.assert_allclose(snap[0][1], snap[1][1], rtol=0,
+                                       atol=1e-12 * np.abs(snap[0][1]).max())
+            big = np.array(c)
+            big[0] = 1.7e308  # phi's constant: infinite energy, the same forces
+            d.upload(case.s)
+            d.set_cheby(big, x0, xn)
+            with pytest.raises(cg.ComdgbError, match="total energy is inf"):
+                d.traj_energy_grad(3, 1e-15, 2)
+            d.set_cheby(c, x0, xn)
+            d.upload(case.s)
+            j, _ = d.traj_energy_grad(3, 1e-15, 2)
+            assert np.isfinite(j)
+        finally:
+            d.close()
+    finally:
+        case.close()
