@@ -471,15 +471,22 @@ __global__ void __launch_bounds__(F64_THREADS)
   hv[3 * (size_t)id + 2] = hz;
 }
 
-// per-id vectors: y = a*x + y (n triples)
-__global__ void adj_axpy_kernel(double a, const double *x, double *y, long n) {
+// per-id vectors, either side of a backward step's Hessian-vector product:
+// pb += c rb, u = -dt pb; rb += hv, pb += c rb
+__global__ void adj_before_kernel(double c, double dt, const double *rb, double *pb, double *u,
+                                  long n) {
   const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < n) y[q] = a * x[q] + y[q];
+  if (q >= n) return;
+  const double p = c * rb[q] + pb[q];
+  pb[q] = p;
+  u[q] = -dt * p;
 }
-// y = a*x
-__global__ void adj_scale_kernel(double a, const double *x, double *y, long n) {
+__global__ void adj_after_kernel(double c, const double *hv, double *rb, double *pb, long n) {
   const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < n) y[q] = a * x[q];
+  if (q >= n) return;
+  const double r = hv[q] + rb[q];
+  rb[q] = r;
+  pb[q] = c * r + pb[q];
 }
 // v[3 id] = f[slot] (the EAM force is grad U)
 __global__ void adj_force_by_id_kernel(Slots s, const int *atom_slot, int ntot, double *v) {
@@ -875,8 +882,7 @@ int comdgb_sim_traj_energy_grad(comdgb_sim *h, int n, double dt, int every, doub
     if ((rc = flush())) return rc;
     for (int t = m - 1; t >= 0; t--) {
       if ((rc = snapshot_copy(h, *mid[t], false)) || (rc = force_fresh(h, false))) return rc;
-      adj_axpy_kernel<<<blocks(nv), 256, 0, h->stream>>>(c, rb, pb, nv);
-      adj_scale_kernel<<<blocks(nv), 256, 0, h->stream>>>(-dt_atu, pb, u, nv);
+      adj_before_kernel<<<blocks(nv), 256, 0, h->stream>>>(c, dt_atu, rb, pb, u, nv);
       if ((rc = set_lambda(h, W, S, nullptr, u))) return rc;
       by_lanes(h, [&](auto lanes) {
         constexpr int L = decltype(lanes)::value;
@@ -884,8 +890,7 @@ int comdgb_sim_traj_energy_grad(comdgb_sim *h, int n, double dt, int every, doub
             force_args(h), S, h->eam64c.poly, h->eam64c.rc2, W.lam, W.x, hv);
       });
       enqueue_eam_sums(h, W, S, true, W.log + (size_t)logged * NQ * NC);
-      adj_axpy_kernel<<<blocks(nv), 256, 0, h->stream>>>(1.0, hv, rb, nv);
-      adj_axpy_kernel<<<blocks(nv), 256, 0, h->stream>>>(c, rb, pb, nv);
+      adj_after_kernel<<<blocks(nv), 256, 0, h->stream>>>(c, hv, rb, pb, nv);
       if (++logged == LOG_STEPS && (rc = flush())) return rc;
     }
   }

@@ -1428,18 +1428,25 @@ int snapshot_alloc(comdgb_sim *h, Snapshot *q) {
   return err ? set_err(COMDGB_ERR_NOMEM, "cudaMalloc failed for a state snapshot") : 0;
 }
 int snapshot_copy(comdgb_sim *h, const Snapshot &q, bool save) {
-  size_t ns = (size_t)h->nslots, nb = (size_t)h->g.nboxes;
+  const size_t ns = (size_t)h->nslots;  // a multiple of 64
   cudaStream_t st = h->stream;
-  auto cp = [&](void *dev, void *snap, size_t bytes) {
-    return save ? cudaMemcpyAsync(snap, dev, bytes, cudaMemcpyDeviceToDevice, st)
-                : cudaMemcpyAsync(dev, snap, bytes, cudaMemcpyDeviceToDevice, st);
+  CopyArrays c{};
+  int k = 0;
+  auto add = [&](void *dev, void *snap, size_t bytes) {
+    c.dst[k] = (uint4 *)(save ? snap : dev);
+    c.src[k] = (const uint4 *)(save ? dev : snap);
+    c.n[k++] = (long)(bytes / sizeof(uint4));
   };
-  CK(cp(h->s.natoms, q.natoms, nb * sizeof(int)));
-  CK(cp(h->s.id, q.id, ns * sizeof(int)));
-  CK(cp(h->s.itype, q.itype, ns * sizeof(int)));
-  CK(cp(h->s.mass, q.mass, ns * sizeof(double)));
-  CK(cp(h->s.r, q.r, ns * sizeof(d4)));
-  CK(cp(h->s.p, q.p, ns * sizeof(d4)));
+  add(h->s.id, q.id, ns * sizeof(int));
+  add(h->s.itype, q.itype, ns * sizeof(int));
+  add(h->s.mass, q.mass, ns * sizeof(double));
+  add(h->s.r, q.r, ns * sizeof(d4));
+  add(h->s.p, q.p, ns * sizeof(d4));
+  c.idst = save ? q.natoms : h->s.natoms;
+  c.isrc = save ? h->s.natoms : q.natoms;
+  c.nints = h->g.nboxes;
+  launch_copy_arrays(c, st);
+  CK(cudaGetLastError());
   if (save) return 0;
   if (h->mixed) launch_pos32(h->g, h->s, st);
   return relist(h);

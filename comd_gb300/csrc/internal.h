@@ -72,6 +72,16 @@ void launch_compact(const Geom &g, const int *natoms, int *box_start, int *atom_
                     int *partials, int npart, cudaStream_t st, const int *only_if = nullptr);
 int compact_partials(int nboxes);
 cudaError_t prepare_md_kernels();
+struct CopyArrays {
+  static constexpr int N = 5;
+  uint4 *dst[N];
+  const uint4 *src[N];
+  long n[N];
+  int *idst;
+  const int *isrc;
+  int nints;
+};
+void launch_copy_arrays(const CopyArrays &c, cudaStream_t st);
 void launch_reduce(const ForceArgs &A, double *partials, long long *ipartials, int npart,
                    unsigned *done, double *out, long long *iout, cudaStream_t st);
 int reduce_partials(int ntot);
