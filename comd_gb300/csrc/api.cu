@@ -2127,11 +2127,9 @@ int comdgb_sim_kinetic(comdgb_sim *h, double *ek) {
 
 int comdgb_sim_set_launch(comdgb_sim *h, int build_threads, int build_atoms, int pass2_threads) {
   if (!h) return set_err(COMDGB_ERR_ARG, "null handle");
-  if (build_threads == 0) build_threads = 128;
-  if (build_atoms == 0) build_atoms = 4;
   if (pass2_threads == 0) pass2_threads = 512;
-  if ((build_threads != 64 && build_threads != 128 && build_threads != 256) ||
-      (build_atoms != 2 && build_atoms != 4 && build_atoms != 8) ||
+  if ((build_threads != 0 && build_threads != 64 && build_threads != 128 && build_threads != 256) ||
+      (build_atoms != 0 && build_atoms != 2 && build_atoms != 4 && build_atoms != 8) ||
       (pass2_threads != 128 && pass2_threads != 256 && pass2_threads != 512))
     return set_err(COMDGB_ERR_ARG, "launch shape %d/%d/%d: build threads 64, 128 or 256, "
                    "atoms per load 2, 4 or 8, pass 2 threads 128, 256 or 512",

@@ -281,7 +281,7 @@ __device__ __forceinline__ int fo_code(int e) {
 // Bound by the instructions issued.  Parking the ballots in shared memory and
 // finding the h-th set bit (__fns) for full-warp stores took more of them
 // than the tests: 270 us for those lists, 129 now (65% of the issue slots).
-#define NB_ATOMS 4                 // atoms tested per candidate load
+#define NB_ATOMS 2                 // atoms tested per candidate load
 // Modes: LIST_STEP writes the per-step list (uint16 codes); LIST_ID (runs
 // only when a rebuild is due) writes neighbour ids into the atom's id-keyed
 // row and records its position; LIST_FO (also only when due) writes the

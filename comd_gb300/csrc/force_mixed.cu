@@ -121,7 +121,7 @@ cudaError_t prepare_force_kernels() {
     if (e == cudaSuccess) e = build_occupancy_nt<256>(g_build_per_sm[2]);
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &g_build_step_per_sm, nbr_build32_kernel<LIST_STEP, NB_THREADS, 2>, NB_THREADS, 0);
+          &g_build_step_per_sm, nbr_build32_kernel<LIST_STEP>, NB_THREADS, 0);
     if (e == cudaSuccess)
       e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
           &g_build_id_per_sm, nbr_build32_kernel<LIST_ID>, NB_THREADS, 0);
@@ -151,7 +151,14 @@ static void launch_fo_build_nt(const ForceArgs &A, float rc2, int na, cudaStream
     nbr_build32_kernel<LIST_FO, NT, 4><<<build_grid(A.g.nboxes, per_sm[1]), NT, 0, st>>>(A, rc2);
 }
 static void launch_fo_build(const ForceArgs &A, float rc2, cudaStream_t st, const Tune *t) {
-  const int nt = t ? t->build_threads : NB_THREADS, na = t ? t->build_atoms : NB_ATOMS;
+  // The default shape: 64 threads and 2 atoms against 128 and 4 take 200 / 243
+  // us at 282,000 atoms (13,000 boxes) and 3.83 / 4.58 ms at 4 M, other shapes
+  // between.  With few boxes (the SMs hold eight CTAs of 128 each) a box's own
+  // time counts, and 128 threads are the faster ones: 100 steps of 4,000 atoms
+  // (216 boxes) 2.39 / 2.36 ms.
+  const bool few = A.g.nboxes < 8 * g_num_sms;
+  const int nt = t && t->build_threads ? t->build_threads : few ? 128 : 64;
+  const int na = t && t->build_atoms ? t->build_atoms : few ? 4 : 2;
   if (nt == 64) launch_fo_build_nt<64>(A, rc2, na, st);
   else if (nt == 256) launch_fo_build_nt<256>(A, rc2, na, st);
   else launch_fo_build_nt<128>(A, rc2, na, st);
@@ -164,9 +171,9 @@ void launch_nbr_build(const ForceArgs &A, float rc2b, cudaStream_t st, const Tun
     nbr_build32_kernel<LIST_ID><<<build_grid(A.g.nboxes, g_build_id_per_sm), NB_THREADS, 0, st>>>(
         A, rc2b);
   else
-    // two atoms per load: boxes of a per-step list hold 10 to 20 atoms.  32 to
-    // 128 threads and 2 to 8 atoms: 129 (this) to 158 us at 256,000 atoms
-    nbr_build32_kernel<LIST_STEP, NB_THREADS, 2>
+    // (boxes of a per-step list hold 10 to 20 atoms.  32 to 128 threads and 2 to
+    // 8 atoms a load: 129 us, this, to 158 us at 256,000 atoms)
+    nbr_build32_kernel<LIST_STEP>
         <<<build_grid(A.g.nboxes, g_build_step_per_sm), NB_THREADS, 0, st>>>(A, rc2b);
 }
 

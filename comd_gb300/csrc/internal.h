@@ -135,7 +135,7 @@ void launch_fo_reslot(const Geom &g, Slots s, const ForceOrder &fo, int ntot, cu
 // candidate load, pass 2's threads per CTA and its grid cap (0: the resident
 // CTAs of the default shape)
 struct Tune {
-  int build_threads = 128, build_atoms = 4;
+  int build_threads = 0, build_atoms = 0;  // 0: by the number of boxes
   int pass2_threads = 512, pass2_blocks = 0;  // force pass: 2 CTAs of 512 per SM
   int pass2_blocks_fast = 0;  // the same for the force pass without energies (OBS = false)
 };
