@@ -19,11 +19,12 @@
 // Measured at 256,000 atoms (no energies), density + forces: table potential
 // 3,156 us before (phi, phi' and rho, then rho', a thread per atom, FP64
 // division and square root, the skin list walked in FP64), 541 + 682 with the
-// list above in FP64 geometry, 354 + 469 in fixed point; Chebyshev 1,327, 350
-// + 560, 159 + 321, where the pipe's two lanes a clock would take 135 + 310.
-// Relative rms error of the forces against extended precision (504 atoms, Cu
-// at 300 K): Chebyshev 4.6e-14 before, 2.4e-15 now, table 2.2e-15 and 1.8e-15,
-// LJ 1.4e-15 and 0.9e-15; energies and densities are closer as well.
+// list above in FP64 geometry, 354 + 469 in fixed point, 132 + 271 with its
+// intervals as polynomials; Chebyshev 1,327, 350 + 560, 159 + 321.  The pipe's
+// two lanes a clock would take 135 + 310 for the latter.  Relative rms error of
+// the forces against extended precision (504 atoms, Cu at 300 K): Chebyshev
+// 4.6e-14 before, 2.4e-15 now, table 2.2e-15 and 4.5e-16, LJ 1.4e-15 and
+// 0.9e-15; energies and densities are closer as well.
 #pragma once
 
 #include "fixed64.cuh"

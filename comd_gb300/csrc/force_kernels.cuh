@@ -209,7 +209,8 @@ __device__ __forceinline__ void for_each_neighbor(const ForceArgs &A, int a, int
 }
 
 // ---------------------------------------------------------------------------
-// neighbour-list build: one CTA per box, one warp per atom of the box
+// neighbour-list build: a CTA per box at a time, a warp per two or more of its
+// atoms
 // ---------------------------------------------------------------------------
 #define NB_THREADS 128
 #define NB_TILE 768  // candidates staged at a time (27 boxes of 64 are 1,728)
@@ -567,19 +568,11 @@ __device__ __forceinline__ void cheb_pair32(const EamPot<float, EVAL> &P, float 
     rho = cheb_low32(P.chlo, 1, r);
   }
 }
-template <int EVAL>
-__device__ __forceinline__ void cheb_pair32(const EamPot<double, EVAL> &, double, double &,
-                                            double &, double &) {}
-
 template <class T, int EVAL>
 __device__ __forceinline__ void eam_pair_terms(const EamPot<T, EVAL> &P, T r, T &phi, T &dphi,
                                                T &rho) {
-  if (EVAL == EVAL_CHEBY && sizeof(T) == 4) {
+  if (EVAL == EVAL_CHEBY) {
     cheb_pair32(P, r, phi, dphi, rho);
-  } else if (EVAL == EVAL_CHEBY) {
-    phi = cheb_series(P, 0, r);
-    dphi = cheb_series(P, 3, r);
-    rho = cheb_series(P, 1, r);
   } else {
     T drho;
     table_eval(P.phi, r, phi, dphi);
@@ -639,18 +632,6 @@ static __device__ __forceinline__ bool eam_pair_w(const EamPot<float, EVAL_CHEBY
   rho = seg_cubic(cr, t);
   return true;
 }
-// FP64 Chebyshev: the polynomials of poly64.cuh
-static __device__ __forceinline__ bool eam_pair_w(const EamPot<double, EVAL_CHEBY> &P,
-                                                  const float4 *, double r2, double &phi,
-                                                  double &w, double &rho) {
-  int k;
-  double t;
-  if (!poly_at(P.poly.pair, r2, k, t)) return false;
-  phi = poly_col(P.poly.pair, PF_PHI, k, t);
-  w = poly_col(P.poly.pair, PF_GPHI, k, t);
-  rho = poly_col(P.poly.pair, PF_RHO, k, t);
-  return true;
-}
 // the series for a pair below the table (Chebyshev only)
 template <class T, int EVAL>
 __device__ __forceinline__ void pair_w_series(const EamPot<T, EVAL> &, T, T &, T &, T &) {}
@@ -661,21 +642,9 @@ static __device__ __noinline__ void pair_w_series(const EamPot<float, EVAL_CHEBY
   cheb_pair32(P, r, phi, dphi, rho);
   w = dphi * inv_r;
 }
-static __device__ __noinline__ void pair_w_series(const EamPot<double, EVAL_CHEBY> &P, double r2,
-                                                  double &phi, double &w, double &rho) {
-  double r, inv_r, dphi;
-  r_and_inv(r2, r, inv_r);
-  eam_pair_terms<double, EVAL_CHEBY>(P, r, phi, dphi, rho);
-  w = dphi * inv_r;
-}
 template <class T, int EVAL>
 __device__ __forceinline__ bool below_seg(const EamPot<T, EVAL> &, T) {
   return false;
-}
-static __device__ __forceinline__ bool below_seg(const EamPot<double, EVAL_CHEBY> &P, double r2) {
-  int k;
-  double t;
-  return !poly_at(P.poly.pair, r2, k, t);
 }
 static __device__ __forceinline__ bool below_seg(const EamPot<float, EVAL_CHEBY> &P, float r2) {
   return !((r2 - P.seg.s_lo) * P.seg.inv_h >= 0.f);
@@ -701,15 +670,6 @@ static __device__ __forceinline__ bool eam_embed_w(const EamPot<float, EVAL_CHEB
   wr = fsum * (P.seg.dscale * seg_dcubic(sm[k], u - (float)k));
   return true;
 }
-static __device__ __forceinline__ bool eam_embed_w(const EamPot<double, EVAL_CHEBY> &P,
-                                                   const float4 *, double r2, double fsum,
-                                                   double &wr) {
-  int k;
-  double t;
-  if (!poly_at(P.poly.pair, r2, k, t)) return false;
-  wr = fsum * poly_col(P.poly.pair, PF_GRHO, k, t);
-  return true;
-}
 template <class T, int EVAL>
 __device__ __forceinline__ T embed_w_series(const EamPot<T, EVAL> &, T, T) {
   return T(0);
@@ -717,13 +677,6 @@ __device__ __forceinline__ T embed_w_series(const EamPot<T, EVAL> &, T, T) {
 static __device__ __noinline__ float embed_w_series(const EamPot<float, EVAL_CHEBY> &P, float r2,
                                                     float fsum) {
   float r, inv_r;
-  r_and_inv(r2, r, inv_r);
-  return fsum * (cheb_series(P, 4, r) * inv_r);
-}
-
-static __device__ __noinline__ double embed_w_series(const EamPot<double, EVAL_CHEBY> &P,
-                                                     double r2, double fsum) {
-  double r, inv_r;
   r_and_inv(r2, r, inv_r);
   return fsum * (cheb_series(P, 4, r) * inv_r);
 }
