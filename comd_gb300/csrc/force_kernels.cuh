@@ -944,7 +944,7 @@ __device__ __forceinline__ void fo_walk(const ForceArgs &A, const uint32_t *list
   const FoFrame fr = fo_frame<MULTI>(A, slot);
   const uint32_t *lst = list + fo_row(a, A.fo.vcap);
   const float4 *pj = NEED_FI ? A.fo.pf : A.fo.pos;
-  if constexpr (NEED_FI) {
+  if constexpr (NEED_FI && UNROLL > 1) {
     // the force pass: a batch's entries and gathers before its first pair (at
     // 4M atoms, 4 a batch: 575 us against 604 unrolled by two with the
     // Chebyshev tables, 650 against 895 with the table potential; 2 a batch
@@ -1368,23 +1368,26 @@ __global__ void __maxnreg__(OBS ? COMDGB_FO2_MAXNREG : COMDGB_FO2F_MAXNREG)
     const int n = COMDGB_FO_CUT ? A.fo.ncut[a] : A.fo.n[a];
     ForceSums<OBS> acc;
     acc.zero();
-    bool low = false;
-    auto walk = [&](auto &&fn) {
-      fo_walk<true, MULTI, FO2_UNROLL>(A, COMDGB_FO_CUT ? A.fo.cut : A.fo.list, n, a, slot, pi,
-                                       rc2, fn);
-    };
-    walk([&](float fj, float dx, float dy, float dz, float r2) {
-      if (r2 > rc2) return;
-      float phi, wphi, wrho;
-      if (!fo_pair<OBS, FORCE_COPIES>(P, dcub_sm, phi_sm, r2, phi, wphi, wrho)) {
-        low = true;
-        return;
-      }
-      const float we = r2 < rc2 ? (fii + fj) * wrho : 0.f;
-      acc.add(phi, wphi, we, dx, dy, dz);
-    });
-    if (low)  // pairs below the table: the series, in a second sweep
-      walk([&](float fj, float dx, float dy, float dz, float r2) {
+    bool low = EVAL == EVAL_CHEBY && P.seg.n == 0;  // no table: the series for all
+    const uint32_t *list = COMDGB_FO_CUT ? A.fo.cut : A.fo.list;
+    if (!low)
+      fo_walk<true, MULTI, FO2_UNROLL>(A, list, n, a, slot, pi, rc2,
+                                       [&](float fj, float dx, float dy, float dz, float r2) {
+        if (r2 > rc2) return;
+        float phi, wphi, wrho;
+        if (!fo_pair<OBS, FORCE_COPIES>(P, dcub_sm, phi_sm, r2, phi, wphi, wrho)) {
+          low = true;
+          return;
+        }
+        const float we = r2 < rc2 ? (fii + fj) * wrho : 0.f;
+        acc.add(phi, wphi, we, dx, dy, dz);
+      });
+    // pairs below the table: the series, in a second sweep, an entry at a time
+    // (its calls gain nothing from a batch: 5.85 ms a step of 4 M atoms with
+    // the series for every pair, 6.13 in batches and after an empty first sweep)
+    if (low)
+      fo_walk<true, MULTI, 1>(A, list, n, a, slot, pi, rc2,
+                              [&](float fj, float dx, float dy, float dz, float r2) {
         if (r2 > rc2 || !below_seg(P, r2)) return;
         float phi, wphi, wrho;
         fo_pair_series(P, r2, phi, wphi, wrho);
