@@ -423,8 +423,8 @@ def gpu_arm(args):
         vs_oracle = oracle_check(s, pot, mix, e_mix, st_mix, w_mix)
 
     # mixed precision with the reference's series evaluated in FP32 for every
-    # pair (no segment table): the same algorithm as the FP64 kernel, so
-    # against it the speed-up of precision alone
+    # pair (no segment table).  (The FP64 kernels take polynomials fitted to
+    # the series instead of summing it.)
     series_ms = None
     if args.series_steps > 0:
         mixed.set_pair_table(False)
@@ -544,8 +544,8 @@ def gpu_arm(args):
             "precision_only": (fp64_ms / series_ms) if fp64_ms and series_ms else None,
             "algorithm_only": (series_ms / (elapsed_s * 1e3 / args.steps))
                               if series_ms else None,
-            "what": "precision_only = FP64 kernel / mixed with the series (both sum the "
-                    "series per pair); algorithm_only = mixed with the series / mixed with "
+            "what": "precision_only = FP64 kernel (polynomials of the series) / mixed with "
+                    "the series per pair; algorithm_only = mixed with the series / mixed with "
                     "the segment table; their product is mixed_vs_fp64"},
         "force_rel_rms_mixed_vs_fp64": ferr,
         "force_rel_rms_mixed_vs_oracle": vs_oracle["f_rel_rms"] if vs_oracle else None,
