@@ -42,13 +42,12 @@ __device__ __forceinline__ void fol_atom(int ntot, F &&fn) {
 }
 
 // this lane's entries of a force-order list (skin or cut) of n entries:
-// fn(entry, q, dx, dy, dz, r2), q the neighbour's record (pos or pf)
-template <bool NEED_FI, bool MULTI, int LANES, class F>
+// fn(q, dx, dy, dz, r2), q the neighbour's record of pj (pos or pf)
+template <bool MULTI, int LANES, class F>
 __device__ __forceinline__ void fol_walk(const ForceArgs &A, const uint32_t *list, int n, int a,
-                                         int slot, int sub, float4 pi, F &&fn) {
+                                         int slot, int sub, float4 pi, const float4 *pj, F &&fn) {
   const FoFrame fr = fo_frame<MULTI>(A, slot);
   const uint32_t *lst = list + fo_row(a, A.fo.vcap);
-  const float4 *pj = NEED_FI ? A.fo.pf : A.fo.pos;
   for (int t0 = sub; t0 < n; t0 += LANES * FOL_BATCH) {
     uint32_t p[FOL_BATCH];
     float4 q[FOL_BATCH];
@@ -136,11 +135,10 @@ __device__ __forceinline__ void fol_density(const ForceArgs &A, const EamPot<flo
     }
   }
   if (low)  // pairs below the table: the series, in a second sweep
-    fol_walk<false, MULTI, LANES>(A, A.fo.list, m, a, slot, sub, pi,
-                                  [&](float4, float, float, float, float r2) {
-                                    if (!(r2 > rc2) && below_seg(P, r2))
-                                      rh.add(fo_rho_series(P, r2));
-                                  });
+    fol_walk<MULTI, LANES>(A, A.fo.list, m, a, slot, sub, pi, A.fo.pos,
+                           [&](float4, float, float, float, float r2) {
+                             if (!(r2 > rc2) && below_seg(P, r2)) rh.add(fo_rho_series(P, r2));
+                           });
   if (n <= A.fo.vcap) ncut = cnt;
   __syncwarp();
   rh = ksum_lanes<LANES>(rh);
@@ -246,8 +244,8 @@ __device__ __forceinline__ void fol_force(const ForceArgs &A, const EamPot<float
     fol_scan<true>(A, slot, sub, rc2, add);
     if (low) fol_scan<true>(A, slot, sub, rc2, add_low);
   } else {
-    fol_walk<true, MULTI, LANES>(A, A.fo.cut, n, a, slot, sub, pi, entry(add));
-    if (low) fol_walk<true, MULTI, LANES>(A, A.fo.cut, n, a, slot, sub, pi, entry(add_low));
+    fol_walk<MULTI, LANES>(A, A.fo.cut, n, a, slot, sub, pi, A.fo.pf, entry(add));
+    if (low) fol_walk<MULTI, LANES>(A, A.fo.cut, n, a, slot, sub, pi, A.fo.pf, entry(add_low));
   }
   __syncwarp();
   acc.fx = ksum_lanes<LANES>(acc.fx);
@@ -303,13 +301,14 @@ __device__ __forceinline__ void fol_lj(const ForceArgs &A, const LjPot<float> &P
     fz.add(dz * fr);
     if (OBS) sx.add(fr * dx * dx);
   };
+  const float4 *pj = fo_lj_pos<OBS>(A);
   if (n > A.fo.vcap)
     fol_scan<false>(A, slot, sub, rc2, add);
   else
-    fol_walk<false, MULTI, LANES>(A, A.fo.list, n, a, slot, sub, A.fo.pos[a],
-                                  [&](float4, float dx, float dy, float dz, float r2) {
-                                    add(0.f, dx, dy, dz, r2);
-                                  });
+    fol_walk<MULTI, LANES>(A, A.fo.list, n, a, slot, sub, pj[a], pj,
+                           [&](float4, float dx, float dy, float dz, float r2) {
+                             add(0.f, dx, dy, dz, r2);
+                           });
   __syncwarp();
   fx = ksum_lanes<LANES>(fx);
   fy = ksum_lanes<LANES>(fy);

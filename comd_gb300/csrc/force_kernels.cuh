@@ -927,12 +927,13 @@ __device__ __forceinline__ size_t fo_row(int a, int vcap) {
 
 // Visit n entries of the list `lst` (a force-order list: skin or cut) of
 // force-order atom a at FP32 position pi: fn(fj, dx, dy, dz, r2) for every
-// entry; with NEED_FI positions come from fo.pf and fj is F'(rho_j) (its w),
-// else fj is unspecified.  n > vcap (the skin list overflowed): the stencil
-// of the atom's current slot is scanned instead.
+// entry, the neighbours' positions being pj's: with NEED_FI fo.pf and fj is
+// F'(rho_j) (its w), else fj is unspecified.  n > vcap (the skin list
+// overflowed): the stencil of the atom's current slot is scanned instead.
 template <bool NEED_FI, bool MULTI, int UNROLL, class F>
 __device__ __forceinline__ void fo_walk(const ForceArgs &A, const uint32_t *list, int n, int a,
-                                        int slot, float4 pi, float rc2, F &&fn) {
+                                        int slot, float4 pi, const float4 *pj, float rc2,
+                                        F &&fn) {
   if (n > A.fo.vcap) {
     const float4 p = __ldg(A.s.pos32 + slot);
     scan_stencil<float>(A, slot >> 6, slot & 63, p.x, p.y, p.z, rc2,
@@ -943,7 +944,6 @@ __device__ __forceinline__ void fo_walk(const ForceArgs &A, const uint32_t *list
   }
   const FoFrame fr = fo_frame<MULTI>(A, slot);
   const uint32_t *lst = list + fo_row(a, A.fo.vcap);
-  const float4 *pj = NEED_FI ? A.fo.pf : A.fo.pos;
   if constexpr (NEED_FI && UNROLL > 1) {
     // the force pass: a batch's entries and gathers before its first pair (at
     // 4M atoms, 4 a batch: 575 us against 604 unrolled by two with the
@@ -984,8 +984,8 @@ __device__ __forceinline__ void fo_walk(const ForceArgs &A, const uint32_t *list
 // the skin list of force-order atom a
 template <bool NEED_FI, bool MULTI, int UNROLL = FO2_UNROLL, class F>
 __device__ __forceinline__ void fo_for_each(const ForceArgs &A, int a, int slot, float4 pi,
-                                            float rc2, F &&fn) {
-  fo_walk<NEED_FI, MULTI, UNROLL>(A, A.fo.list, A.fo.n[a], a, slot, pi, rc2, fn);
+                                            const float4 *pj, float rc2, F &&fn) {
+  fo_walk<NEED_FI, MULTI, UNROLL>(A, A.fo.list, A.fo.n[a], a, slot, pi, pj, rc2, fn);
 }
 
 // ---------------------------------------------------------------------------
@@ -1205,7 +1205,7 @@ __global__ void FO1_BOUNDS
     rh.zero();
     int cnt = 0;
     if (n > A.fo.vcap) {  // overflowed skin list: the stencil, no cut list
-      fo_walk<false, MULTI, 1>(A, A.fo.list, n, a, slot, pi, rc2,
+      fo_walk<false, MULTI, 1>(A, A.fo.list, n, a, slot, pi, A.fo.pos, rc2,
                                [&](float, float, float, float, float r2) {
                                  if (r2 > rc2) return;
                                  cnt++;
@@ -1265,7 +1265,7 @@ __global__ void FO1_BOUNDS
       }
     }
     if (low)  // pairs below the table: the series, in a second sweep
-      fo_walk<false, MULTI, 1>(A, A.fo.list, n, a, slot, pi, rc2,
+      fo_walk<false, MULTI, 1>(A, A.fo.list, n, a, slot, pi, A.fo.pos, rc2,
                                [&](float, float, float, float, float r2) {
                                  if (r2 <= rc2 && below_seg(P, r2)) rh.add(fo_rho_series(P, r2));
                                });
@@ -1317,7 +1317,8 @@ __device__ __forceinline__ void fo_host_f(const ForceArgs &A, int slot, const d4
 // (the arithmetic of the mixed-precision middle-part update), and its
 // tracking record; else its FP32 force record for the velocity step that
 // follows.  Safe inside the pass: the other atoms of the pass read the
-// positions the density pass stored (pf), never r, p, fo.pos or pos32.
+// positions that a kernel before it stored in pf (EAM: the density pass, LJ:
+// fo_lj_settle_kernel), never r, p, fo.pos or pos32.
 __device__ __forceinline__ void fo_force_end(const ForceArgs &A, int a, int slot, bool fuse,
                                              float fx, float fy, float fz) {
   if (!fuse) {
@@ -1371,7 +1372,7 @@ __global__ void __maxnreg__(OBS ? COMDGB_FO2_MAXNREG : COMDGB_FO2F_MAXNREG)
     bool low = EVAL == EVAL_CHEBY && P.seg.n == 0;  // no table: the series for all
     const uint32_t *list = COMDGB_FO_CUT ? A.fo.cut : A.fo.list;
     if (!low)
-      fo_walk<true, MULTI, FO2_UNROLL>(A, list, n, a, slot, pi, rc2,
+      fo_walk<true, MULTI, FO2_UNROLL>(A, list, n, a, slot, pi, A.fo.pf, rc2,
                                        [&](float fj, float dx, float dy, float dz, float r2) {
         if (r2 > rc2) return;
         float phi, wphi, wrho;
@@ -1386,7 +1387,7 @@ __global__ void __maxnreg__(OBS ? COMDGB_FO2_MAXNREG : COMDGB_FO2F_MAXNREG)
     // (its calls gain nothing from a batch: 5.85 ms a step of 4 M atoms with
     // the series for every pair, 6.13 in batches and after an empty first sweep)
     if (low)
-      fo_walk<true, MULTI, 1>(A, list, n, a, slot, pi, rc2,
+      fo_walk<true, MULTI, 1>(A, list, n, a, slot, pi, A.fo.pf, rc2,
                               [&](float fj, float dx, float dy, float dz, float r2) {
         if (r2 > rc2 || !below_seg(P, r2)) return;
         float phi, wphi, wrho;
@@ -1461,6 +1462,19 @@ __global__ void __launch_bounds__(128) lj_pass_kernel(ForceArgs A, LjPot<T> P) {
 
 // LJ in force order (mixed precision, persistent lists)
 // (OBS as in the EAM force pass: energy and stress only where readable)
+
+// The positions that the pass reads.  Inside a step sequence (not OBS) it ends
+// with the update, which writes fo.pos while other atoms still gather their
+// neighbours, so it reads pf, a copy that fo_lj_settle_kernel makes before it.
+// (EAM's force pass reads the copy that its density pass stores.)
+template <bool OBS>
+__device__ __forceinline__ const float4 *fo_lj_pos(const ForceArgs &A) {
+  return OBS ? A.fo.pos : A.fo.pf;
+}
+static __global__ void __launch_bounds__(PASS_THREADS) fo_lj_settle_kernel(ForceArgs A) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a < A.ntot) A.fo.pf[a] = A.fo.pos[a];
+}
 template <bool MULTI, bool OBS>
 __global__ void __launch_bounds__(PASS_THREADS) fo_lj_kernel(ForceArgs A, LjPot<float> P) {
   const float s6 = P.s6, s12 = P.s6x12, c4 = P.eps4s6, rc2 = P.rc2;
@@ -1483,7 +1497,8 @@ __global__ void __launch_bounds__(PASS_THREADS) fo_lj_kernel(ForceArgs A, LjPot<
       fz.add(dz * fr);
       if (OBS) sx.add(fr * dx * dx);
     };
-    fo_for_each<false, MULTI, FO1_UNROLL>(A, a, slot, A.fo.pos[a], rc2, fn);
+    const float4 *pj = fo_lj_pos<OBS>(A);
+    fo_for_each<false, MULTI, FO1_UNROLL>(A, a, slot, pj[a], pj, rc2, fn);
     fo_force_end(A, a, slot, fuse, fx.valuef(), fy.valuef(), fz.valuef());
     if (OBS) {
       d4 fo;

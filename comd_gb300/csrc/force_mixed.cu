@@ -296,6 +296,8 @@ int fo_pass2_blocks(int eval, bool multi, int threads, bool obs) {
 
 void launch_fo_lj(const ForceArgs &A, const LjPot<float> &P, cudaStream_t st, bool obs) {
   if (A.ntot <= 0) return;
+  if (!obs)
+    fo_lj_settle_kernel<<<(A.ntot + PASS_THREADS - 1) / PASS_THREADS, PASS_THREADS, 0, st>>>(A);
   const int lanes = fo_lj_lanes(A.ntot);
   if (lanes > 1) {
     if (lanes == 8) obs ? launch_fol_lj<true, 8>(A, P, st) : launch_fol_lj<false, 8>(A, P, st);

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(VIR_THREADS)
       slot = A.fo.slot[a];
       const float4 pi = A.fo.pf[a];
       eam_virial_sum(P, seg_sm, pi.w, acc,
-                     [&](auto &&fn) { fo_for_each<true, true>(A, a, slot, pi, P.rc2, fn); });
+                     [&](auto &&fn) { fo_for_each<true, true>(A, a, slot, pi, A.fo.pf, P.rc2, fn); });
     } else {
       slot = A.atom_slot[a];
       const int b = slot >> 6, i = slot & 63;
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(VIR_THREADS) lj_virial_kernel(ForceArgs A, LjP
     int slot;
     if constexpr (FO) {
       slot = A.fo.slot[a];
-      fo_for_each<false, true>(A, a, slot, A.fo.pos[a], (float)rc2, fn);
+      fo_for_each<false, true>(A, a, slot, A.fo.pos[a], A.fo.pos, (float)rc2, fn);
     } else {
       slot = A.atom_slot[a];
       const int b = slot >> 6, i = slot & 63;
