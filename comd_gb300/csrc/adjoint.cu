@@ -117,6 +117,30 @@ __device__ __forceinline__ double embed_d2(const ChebSet &S, const PolyTables &P
   return poly_at(P.embed, rho, k, t) ? poly_col(P.embed, EF_D2F, k, t) : cheb_der(S, 8, 2, rho);
 }
 
+// A pair's distance: from the integers in their range (plain), else in FP64 (for
+// the basis sums, which hold every register, out of line).  false: beyond the
+// cutoff; strict: within it (the embedding force).  The comparisons in FP64
+// stay in the rare branch: for every pair they took 25 us of adj_w_kernel's 304
+// at 256,000 atoms and as many of the basis sums'.
+__device__ __noinline__ Exact64 exact_distance(EntryTab et, const d4 *r, int slot,
+                                               uint32_t code) {
+  return exact64(et, r, slot, code);
+}
+template <bool OUT_OF_LINE = false>
+__device__ __forceinline__ bool distance(const ForceArgs &A, int slot, const Pair64 &q, double rc2,
+                                         Exact64 &d, bool &plain, bool &strict) {
+  plain = strict = fx_plain(A, q.s);
+  if (plain) {
+    d = Exact64{fx_length(q.x, A.fxu), fx_length(q.y, A.fxu), fx_length(q.z, A.fxu),
+                fx_area(q.s, A.fxu)};
+    return true;
+  }
+  if (q.s > A.fx_far) return false;
+  d = OUT_OF_LINE ? exact_distance(A.et, A.s.r, slot, q.code) : exact64(A, slot, q.code);
+  strict = !(d.r2 >= rc2);
+  return !(d.r2 > rc2);
+}
+
 struct Lam {
   const d4 *lam;    // [nslots] lambda by slot
   const double *x;  // [nslots] X = F'' W by slot (EAM)
@@ -167,12 +191,12 @@ __global__ void __launch_bounds__(F64_THREADS)
   const d4 li = lam[slot];
   double W = 0.0;
   walk64<LANES>(A, a, sub, slot, A.fx[slot], rc2, [&](const Pair64 &q) {
-    if (q.s >= A.fx_rc2) return;
+    Exact64 d;
+    bool plain, strict;
+    if (!distance(A, slot, q, rc2, d, plain, strict) || !strict) return;
     const d4 lj = lam[q.j];
-    const double vr = (li.x - lj.x) * fx_length(q.x, A.fxu) +
-                      (li.y - lj.y) * fx_length(q.y, A.fxu) +
-                      (li.z - lj.z) * fx_length(q.z, A.fxu);
-    W += vr * pair_grho(S, poly, q.s, A.fxu);
+    const double vr = (li.x - lj.x) * d.x + (li.y - lj.y) * d.y + (li.z - lj.z) * d.z;
+    W += vr * (plain ? pair_grho(S, poly, q.s, A.fxu) : grho_series(S, d.r2));
   });
   W = lane_sum<LANES>(W);
   if (sub != 0 || !live) return;
@@ -282,16 +306,17 @@ __global__ void __launch_bounds__(BASIS_THREADS)
     return fma(2.0, fma(fma(-t, S.b[q] - S.a[q], d), scale[q], t), -1.0);
   };
   auto pair = [&](int slot, const d4 &fi, const Pair64 &q) {
-    if (q.s > A.fx_rc2) return;
+    Exact64 d;
+    bool plain, strict;
+    if (!distance<true>(A, slot, q, rc2, d, plain, strict)) return;
     double r, inv;
-    r_and_inv(fx_area(q.s, A.fxu), r, inv);
+    r_and_inv(d.r2, r, inv);
     const double fsum = fi.w + q.fj;
     double w[3];
     if (NW == 3) {
       const d4 li = L.lam[slot], lj = L.lam[q.j];
-      w[0] = ((li.x - lj.x) * fx_length(q.x, A.fxu) + (li.y - lj.y) * fx_length(q.y, A.fxu) +
-              (li.z - lj.z) * fx_length(q.z, A.fxu)) * inv;
-      w[1] = q.s < A.fx_rc2 ? fsum * w[0] : 0.0;
+      w[0] = ((li.x - lj.x) * d.x + (li.y - lj.y) * d.y + (li.z - lj.z) * d.z) * inv;
+      w[1] = strict ? fsum * w[0] : 0.0;
       w[2] = L.x[slot] + L.x[q.j];
     } else {
       w[0] = 1.0;
@@ -447,18 +472,19 @@ __global__ void __launch_bounds__(F64_THREADS)
   const double Xk = X[slot];
   double hx = 0.0, hy = 0.0, hz = 0.0;
   walk64<LANES>(A, a, sub, slot, fi, rc2, [&](const Pair64 &q) {
-    if (q.s > A.fx_rc2) return;
-    const HessTerms h = hess_terms(S, poly, q.s, A.fxu);
+    Exact64 d;
+    bool plain, strict;
+    if (!distance(A, slot, q, rc2, d, plain, strict)) return;
+    const HessTerms h = plain ? hess_terms(S, poly, q.s, A.fxu) : hess_series(S, d.r2);
     const d4 uj = u[q.j];
-    const double dx = fx_length(q.x, A.fxu), dy = fx_length(q.y, A.fxu), dz = fx_length(q.z, A.fxu);
     const double ux = uk.x - uj.x, uy = uk.y - uj.y, uz = uk.z - uj.z;
-    const double ud = ux * dx + uy * dy + uz * dz;
-    const double fs = q.s < A.fx_rc2 ? fi.w + q.fj : 0.0;
+    const double ud = ux * d.x + uy * d.y + uz * d.z;
+    const double fs = strict ? fi.w + q.fj : 0.0;
     const double g = h.gphi + fs * h.grho;
     const double c = ud * (h.hphi + fs * h.hrho) + (Xk + X[q.j]) * h.dr;
-    hx += g * ux + c * dx;
-    hy += g * uy + c * dy;
-    hz += g * uz + c * dz;
+    hx += g * ux + c * d.x;
+    hy += g * uy + c * d.y;
+    hz += g * uz + c * d.z;
   });
   hx = lane_sum<LANES>(hx);
   hy = lane_sum<LANES>(hy);

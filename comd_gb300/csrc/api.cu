@@ -79,7 +79,10 @@ ForceArgs force_args(comdgb_sim *h) {
   A.cap = h->cap;
   A.fx = h->fx;
   A.fxu = h->fxu;
-  A.fx_rc2 = h->fx ? (u64)ldexp(h->cutoff * h->cutoff, 64 - 2 * h->fxu.m) : 0;
+  const double rc2 = ldexp(h->cutoff * h->cutoff, 64 - 2 * h->fxu.m);
+  const bool range = h->fx && rc2 > 2.0 * (FX_NEAR + FX_TIE) && rc2 < 0x1p62;
+  A.fx_span = range ? (u64)rc2 - FX_TIE - FX_NEAR : 0;  // (0: FP64 decides everywhere)
+  A.fx_far = range ? (u64)rc2 + FX_TIE : ~0ull;
   A.atom_stress = h->atom_stress;
   A.status = h->status;
   A.pl = h->pl;

@@ -10,9 +10,15 @@
 // r_i + offset - r_j is exact whatever the box size.  r^2 is the sum of the
 // high halves of three squares, in units of 2^(2m-64) A^2.  For EAM Cu (m = 4)
 // a unit is 9e-19 A and 1.4e-17 A^2: a position (a double of up to 7 A) is
-// held exactly or to 4e-19 A, and r^2 is off by less than 1.3e-16 A^2, where the FP64
-// operations they replace round to 4e-16 A and, at 6 to 25 A^2, 4e-16 to
+// held exactly or to 4e-19 A, and r^2 is off by less than 15 units, 2e-16 A^2, where the
+// FP64 operations they replace round to 4e-16 A and, at 6 to 25 A^2, 4e-16 to
 // 2e-15 A^2.
+//
+// An error of 15 units is more than those operations' where r^2 is small, and
+// r^2 = 0 is no distance at all.  So the integers serve r^2 from FX_NEAR units
+// (2^(m-5) A, 0.5 A for EAM Cu: the error is below 1e-15 of r^2) to a hair below
+// the cutoff; pairs closer, and those so near to the cutoff that rounding decides on
+// which side they lie, take the FP64 operations (exact64 in force64.cuh).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -26,6 +32,11 @@ struct FxUnit {
   int m;
   double down;
 };
+
+// r^2 from which the integers serve, and how near to the squared cutoff: past
+// what the rounding of three FP64 differences and squares comes to (2^-50 of
+// 2^(2m-2), the largest r^2)
+constexpr u64 FX_NEAR = 1ull << 54, FX_TIE = 1ull << 12;
 
 // x in units of 2^(m-64), modulo 2^m
 __device__ __forceinline__ long long fx_from(double x, const FxUnit &u) {
@@ -42,13 +53,12 @@ __device__ __forceinline__ u64 fx_square(u64 a) {
 }
 
 // a * 2^e to nearest (ties up) as a double, e + 1086 given: the leading one
-// shifted out, the exponent put in front, all in integers.  a = 0 gives a
-// number below any distance.
+// shifted out, the exponent put in front, all in integers
 __device__ __forceinline__ double fx_double(u64 a, int e1086) {
   const int lz = __clzll((long long)a);
   const u64 n = a << (lz & 63);
-  return __longlong_as_double(
-      (long long)(((u64)(unsigned)(e1086 - 1 - lz) << 52) + (n >> 11) + ((n >> 10) & 1)));
+  const unsigned top = lz < 64 ? e1086 - 1 - lz : 0;  // (0 stays 0)
+  return __longlong_as_double((long long)(((u64)top << 52) + (n >> 11) + ((n >> 10) & 1)));
 }
 // a signed difference in A
 __device__ __forceinline__ double fx_length(long long d, const FxUnit &u) {

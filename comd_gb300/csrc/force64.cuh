@@ -62,47 +62,84 @@ __device__ __forceinline__ double lane_sum(double v) {
   return v;
 }
 
-// A pair: the differences and r^2 in fixed point, F'(rho_j), j's slot
+// A pair: the differences and r^2 in fixed point, F'(rho_j), j's slot, and
+// the entry of i's stencil that it is
 struct Pair64 {
   long long x, y, z;
   u64 s;
   double fj;
   int j;
+  uint32_t code;
 };
-__device__ __forceinline__ Pair64 pair64(long long x, long long y, long long z, double fj, int j) {
-  return Pair64{x, y, z, fx_square(fx_abs(x)) + fx_square(fx_abs(y)) + fx_square(fx_abs(z)), fj, j};
-}
 // the pair of atom i (its record) and entry code of its box's stencil (off)
 __device__ __forceinline__ Pair64 pair64(const ForceArgs &A, const d4 &fi, const d4 *off,
                                          uint32_t code) {
   const d4 o = off[code >> 6];  // the offset, and the neighbour box
   const int j = __double2loint(o.w) * CG_MAXATOMS + (code & 63);
   const d4 q = A.fx[j];
-  return pair64(
-      __double_as_longlong(fi.x) + __double_as_longlong(o.x) - __double_as_longlong(q.x),
-      __double_as_longlong(fi.y) + __double_as_longlong(o.y) - __double_as_longlong(q.y),
-      __double_as_longlong(fi.z) + __double_as_longlong(o.z) - __double_as_longlong(q.z), q.w, j);
+  const long long x =
+      __double_as_longlong(fi.x) + __double_as_longlong(o.x) - __double_as_longlong(q.x);
+  const long long y =
+      __double_as_longlong(fi.y) + __double_as_longlong(o.y) - __double_as_longlong(q.y);
+  const long long z =
+      __double_as_longlong(fi.z) + __double_as_longlong(o.z) - __double_as_longlong(q.z);
+  return Pair64{x, y, z, fx_square(fx_abs(x)) + fx_square(fx_abs(y)) + fx_square(fx_abs(z)),
+                q.w, j, code};
+}
+// s in the range that the integers serve: within the cutoff
+__device__ __forceinline__ bool fx_plain(const ForceArgs &A, u64 s) {
+  return s - FX_NEAR < A.fx_span;
+}
+
+// The same pair in FP64, dr = drbox + r_i - r_j and r^2 operation by operation
+// as the reference has them (eam.c:484-521): pairs outside the range of the
+// integers.  A coincident pair has r^2 = 0 and so an infinite LJ energy, and
+// forces that are not numbers, as with the reference's divisions.
+struct Exact64 {
+  double x, y, z, r2;
+};
+__device__ __forceinline__ Exact64 exact64(const EntryTab &et, const d4 *r, int slot,
+                                           uint32_t code) {
+  const int e = (slot >> 6) * CG_NNBR + (int)(code >> 6);
+  const d4 o = et.dr64[e], ri = r[slot];
+  const d4 rj = r[et.box[e] * CG_MAXATOMS + (int)(code & 63)];
+  Exact64 q;
+  q.x = __dsub_rn(__dadd_rn(o.x, ri.x), rj.x);
+  q.y = __dsub_rn(__dadd_rn(o.y, ri.y), rj.y);
+  q.z = __dsub_rn(__dadd_rn(o.z, ri.z), rj.z);
+  q.r2 = __dadd_rn(__dadd_rn(__dmul_rn(q.x, q.x), __dmul_rn(q.y, q.y)), __dmul_rn(q.z, q.z));
+  return q;
+}
+__device__ __forceinline__ Exact64 exact64(const ForceArgs &A, int slot, uint32_t code) {
+  return exact64(A.et, A.s.r, slot, code);
 }
 
 // This lane's entries of atom a's list: fn(pair), entries past the cutoff
-// included; an overflowed list's stencil is scanned by lane 0.  fi: the
-// atom's record.
+// included; an overflowed list's stencil is scanned by lane 0 (there FP64
+// refuses the pairs first: the integers are modulo 2^m).  fi: the atom's
+// record.
 template <int LANES, class F>
 __device__ __forceinline__ void walk64(const ForceArgs &A, int a, int sub, int slot, const d4 &fi,
                                        double rc2, F &&fn) {
   const int n = A.nbr_n[a], b = slot >> 6;
+  const d4 *off = A.et.fx + b * CG_NNBR;
   if (n > A.cap) {
-    if (sub == 0) {
-      const d4 ri = A.s.r[slot];
-      scan_stencil<double>(A, b, slot & 63, ri.x, ri.y, ri.z, rc2,
-                           [&](int js, double dx, double dy, double dz, double) {
-                             fn(pair64(fx_from(dx, A.fxu), fx_from(dy, A.fxu),
-                                       fx_from(dz, A.fxu), A.fx[js].w, js));
-                           });
+    if (sub != 0) return;
+    const int ne = A.et.n[b];
+    for (int e = 0; e < ne; e++) {
+      const int jb = A.et.box[b * CG_NNBR + e], nj = A.s.natoms[jb];
+      for (int k = 0; k < nj; k++) {
+        if (jb == b && k == (slot & 63)) continue;
+        const uint32_t code = (uint32_t)(e << 6 | k);
+        const double r2 = exact64(A, slot, code).r2;
+        if (r2 > rc2) continue;
+        Pair64 q = pair64(A, fi, off, code);
+        if (r2 != r2) q.s = 0;  // (not a number: FP64, which keeps it)
+        fn(q);
+      }
     }
     return;
   }
-  const d4 *off = A.et.fx + b * CG_NNBR;
   const uint16_t *lst = A.nbr + (size_t)a * A.cap;
 #pragma unroll 1
   for (int t = sub; t < n; t += LANES) fn(pair64(A, fi, off, __ldg(lst + t)));
@@ -237,6 +274,14 @@ static __device__ __noinline__ void force64_series(const EamPot<double, EVAL_TAB
   wrho = drho * inv;
 }
 
+// the pairs of a second sweep: not far beyond the cutoff, and outside the
+// range of the integers or of the polynomials
+template <int EVAL>
+__device__ __forceinline__ bool in_rest64(const ForceArgs &A, const EamPot<double, EVAL> &P,
+                                          u64 s) {
+  return s <= A.fx_far && (!fx_plain(A, s) || outside64(P, s, A.fxu));
+}
+
 // rho_i = sum of rho(r_ij), F'(rho_i) for the force pass; OBS: also rho, F'
 // and F(rho_i) (left in f's fourth component) and the pairs counted
 template <int EVAL, int LANES, bool OBS>
@@ -247,21 +292,25 @@ __global__ void __launch_bounds__(F64_THREADS)
   if (!lane_atom<LANES>(A.ntot, a, sub, live)) return;
   const int slot = A.atom_slot[a];
   const d4 fi = A.fx[slot];
-  const u64 rc2 = A.fx_rc2;
   double rho = 0.0;
   int cnt = 0;
-  bool low = false;
+  bool rest = false;
   walk64<LANES>(A, a, sub, slot, fi, P.rc2, [&](const Pair64 &q) {
-    if (q.s > rc2) return;
-    cnt++;
     double v;
-    if (rho64(P, q.s, A.fxu, v)) rho = __dadd_rn(rho, v);
-    else low = true;
+    if (fx_plain(A, q.s) && rho64(P, q.s, A.fxu, v)) {
+      cnt++;
+      rho = __dadd_rn(rho, v);
+    } else if (q.s <= A.fx_far) {
+      rest = true;
+    }
   });
-  if (low)  // pairs below the polynomials: the series or the interpolation, in a second sweep
+  if (rest)  // pairs outside the polynomials or the integers: in FP64, in a second sweep
     walk64<LANES>(A, a, sub, slot, fi, P.rc2, [&](const Pair64 &q) {
-      if (q.s <= rc2 && outside64(P, q.s, A.fxu))
-        rho = __dadd_rn(rho, rho64_series(P, fx_area(q.s, A.fxu)));
+      if (!in_rest64(A, P, q.s)) return;
+      const double r2 = exact64(A, slot, q.code).r2;
+      if (r2 > P.rc2) return;
+      cnt++;
+      rho = __dadd_rn(rho, rho64_series(P, r2));
     });
   rho = lane_sum<LANES>(rho);
   if (OBS)
@@ -289,13 +338,11 @@ __global__ void __launch_bounds__(F64_THREADS)
   if (!lane_atom<LANES>(A.ntot, a, sub, live)) return;
   const int slot = A.atom_slot[a];
   const d4 fi = A.fx[slot];
-  const u64 rc2 = A.fx_rc2;
   const double fii = fi.w;
   double fx = 0.0, fy = 0.0, fz = 0.0, ep = 0.0, sx = 0.0;
-  bool low = false;
-  auto add = [&](const Pair64 &q, double phi, double wphi, double wrho) {
-    const double fs = q.s < rc2 ? __dadd_rn(fii, q.fj) : 0.0;
-    const double dx = fx_length(q.x, A.fxu);
+  bool rest = false;
+  auto add = [&](double dx, double dy, double dz, double fs, double phi, double wphi,
+                 double wrho) {
     double w;
     if (OBS) {
       const double we = __dmul_rn(fs, wrho);
@@ -306,21 +353,25 @@ __global__ void __launch_bounds__(F64_THREADS)
       w = fma(fs, wrho, wphi);
     }
     fx = fma(w, dx, fx);
-    fy = fma(w, fx_length(q.y, A.fxu), fy);
-    fz = fma(w, fx_length(q.z, A.fxu), fz);
+    fy = fma(w, dy, fy);
+    fz = fma(w, dz, fz);
   };
   walk64<LANES>(A, a, sub, slot, fi, P.rc2, [&](const Pair64 &q) {
-    if (q.s > rc2) return;
     double phi = 0.0, wphi, wrho;
-    if (force64<OBS>(P, q.s, A.fxu, phi, wphi, wrho)) add(q, phi, wphi, wrho);
-    else low = true;
+    if (fx_plain(A, q.s) && force64<OBS>(P, q.s, A.fxu, phi, wphi, wrho))
+      add(fx_length(q.x, A.fxu), fx_length(q.y, A.fxu), fx_length(q.z, A.fxu),
+          __dadd_rn(fii, q.fj), phi, wphi, wrho);
+    else if (q.s <= A.fx_far)
+      rest = true;
   });
-  if (low)
+  if (rest)
     walk64<LANES>(A, a, sub, slot, fi, P.rc2, [&](const Pair64 &q) {
-      if (q.s > rc2 || !outside64(P, q.s, A.fxu)) return;
+      if (!in_rest64(A, P, q.s)) return;
+      const Exact64 d = exact64(A, slot, q.code);
+      if (d.r2 > P.rc2) return;
       double phi, wphi, wrho;
-      force64_series(P, fx_area(q.s, A.fxu), phi, wphi, wrho);
-      add(q, phi, wphi, wrho);
+      force64_series(P, d.r2, phi, wphi, wrho);
+      add(d.x, d.y, d.z, d.r2 < P.rc2 ? __dadd_rn(fii, q.fj) : 0.0, phi, wphi, wrho);
     });
   fx = lane_sum<LANES>(fx);
   fy = lane_sum<LANES>(fy);
@@ -342,6 +393,19 @@ __global__ void __launch_bounds__(F64_THREADS)
   A.s.f[slot] = f;
 }
 
+// the distance of an LJ pair; false: beyond the cutoff
+__device__ __forceinline__ bool lj_pair64(const ForceArgs &A, const LjPot<double> &P, int slot,
+                                          const Pair64 &q, Exact64 &d) {
+  if (fx_plain(A, q.s)) {
+    d = Exact64{fx_length(q.x, A.fxu), fx_length(q.y, A.fxu), fx_length(q.z, A.fxu),
+                fx_area(q.s, A.fxu)};
+    return true;
+  }
+  if (q.s > A.fx_far) return false;
+  d = exact64(A, slot, q.code);
+  return !(d.r2 > P.rc2);
+}
+
 // LJ: ljForce.c:151-215 as full pairs; the kinetic stress term is added once
 // per (atom, non-empty neighbour box) as at ljForce.c:175
 template <int LANES, bool OBS>
@@ -355,18 +419,18 @@ __global__ void __launch_bounds__(F64_THREADS) lj64_kernel(ForceArgs A, LjPot<do
   double fx = 0.0, fy = 0.0, fz = 0.0, ep = 0.0, sx = 0.0;
   int cnt = 0;
   walk64<LANES>(A, a, sub, slot, fi, P.rc2, [&](const Pair64 &q) {
-    if (q.s > A.fx_rc2) return;
-    const double ir2 = reciprocal(fx_area(q.s, A.fxu));
+    Exact64 d;
+    if (!lj_pair64(A, P, slot, q, d)) return;
+    const double ir2 = reciprocal(d.r2);
     const double r6 = __dmul_rn(__dmul_rn(ir2, ir2), ir2);
     const double fr = __dmul_rn(__dmul_rn(__dmul_rn(c4, r6), ir2), fma(s12, r6, -6.0));
-    const double dx = fx_length(q.x, A.fxu);
-    fx = fma(fr, dx, fx);
-    fy = fma(fr, fx_length(q.y, A.fxu), fy);
-    fz = fma(fr, fx_length(q.z, A.fxu), fz);
+    fx = fma(fr, d.x, fx);
+    fy = fma(fr, d.y, fy);
+    fz = fma(fr, d.z, fz);
     if (OBS) {
       cnt++;
       ep = fma(r6, fma(s6, r6, -1.0), ep);
-      sx = fma(__dmul_rn(fr, dx), dx, sx);
+      sx = fma(__dmul_rn(fr, d.x), d.x, sx);
     }
   });
   fx = lane_sum<LANES>(fx);

@@ -40,10 +40,12 @@ struct ForceArgs {
   int *npair;            // [ntot] neighbours within the cutoff (written by the passes)
   int cap;
   // FP64: positions in fixed point and F'(rho) by slot (the bits of three
-  // 64-bit integers; w), their unit, and rc^2 in that of their squares
+  // 64-bit integers; w), their unit, and in that of their squares the width of the
+  // range from FX_NEAR in which a pair is surely within the cutoff, and the
+  // least r^2 that is surely beyond it
   d4 *fx;
   FxUnit fxu;
-  u64 fx_rc2;
+  u64 fx_span, fx_far;
   double *atom_stress;   // [ntot] per-atom share of the scalar stress
   int *status;
   Persist pl;            // persistent lists keyed by id (FP64)

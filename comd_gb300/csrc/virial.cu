@@ -123,8 +123,7 @@ __global__ void __launch_bounds__(VIR_THREADS)
 // FP64: the pair weight g of the terms above, times dr (x) dr
 struct Vir64 {
   double c[6];
-  __device__ __forceinline__ void add(double g, const Pair64 &q, const FxUnit &u) {
-    const double dx = fx_length(q.x, u), dy = fx_length(q.y, u), dz = fx_length(q.z, u);
+  __device__ __forceinline__ void add(double g, double dx, double dy, double dz) {
     const double gx = g * dx, gy = g * dy, gz = g * dz;
     c[0] = fma(gx, dx, c[0]);
     c[1] = fma(gy, dy, c[1]);
@@ -151,23 +150,24 @@ __global__ void __launch_bounds__(F64_THREADS)
   if (!lane_atom<LANES>(A.ntot, a, sub, live)) return;
   const int slot = A.atom_slot[a];
   const d4 fi = A.fx[slot];
-  const u64 rc2 = A.fx_rc2;
   Vir64 acc{};
-  bool low = false;
+  bool rest = false;
   walk64<LANES>(A, a, sub, slot, fi, P.rc2, [&](const Pair64 &q) {
-    if (q.s > rc2) return;
     double phi, w, wr;
-    if (force64<false>(P, q.s, A.fxu, phi, w, wr))
-      acc.add(-fma(q.s < rc2 ? fi.w + q.fj : 0.0, wr, w), q, A.fxu);
-    else
-      low = true;
+    if (fx_plain(A, q.s) && force64<false>(P, q.s, A.fxu, phi, w, wr))
+      acc.add(-fma(fi.w + q.fj, wr, w), fx_length(q.x, A.fxu), fx_length(q.y, A.fxu),
+              fx_length(q.z, A.fxu));
+    else if (q.s <= A.fx_far)
+      rest = true;
   });
-  if (low)
+  if (rest)
     walk64<LANES>(A, a, sub, slot, fi, P.rc2, [&](const Pair64 &q) {
-      if (q.s > rc2 || !outside64(P, q.s, A.fxu)) return;
+      if (!in_rest64(A, P, q.s)) return;
+      const Exact64 d = exact64(A, slot, q.code);
+      if (d.r2 > P.rc2) return;
       double phi, w, wr;
-      force64_series(P, fx_area(q.s, A.fxu), phi, w, wr);
-      acc.add(-fma(q.s < rc2 ? fi.w + q.fj : 0.0, wr, w), q, A.fxu);
+      force64_series(P, d.r2, phi, w, wr);
+      acc.add(-fma(d.r2 < P.rc2 ? fi.w + q.fj : 0.0, wr, w), d.x, d.y, d.z);
     });
   acc.template store<LANES>(sub == 0 && live, out + 6 * (size_t)slot);
 }
@@ -180,9 +180,10 @@ __global__ void __launch_bounds__(F64_THREADS)
   const int slot = A.atom_slot[a];
   Vir64 acc{};
   walk64<LANES>(A, a, sub, slot, A.fx[slot], P.rc2, [&](const Pair64 &q) {
-    if (q.s > A.fx_rc2) return;
-    const double ir2 = reciprocal(fx_area(q.s, A.fxu)), r6 = ir2 * ir2 * ir2;
-    acc.add(P.eps4s6 * r6 * ir2 * fma(P.s6x12, r6, -6.0), q, A.fxu);
+    Exact64 d;
+    if (!lj_pair64(A, P, slot, q, d)) return;
+    const double ir2 = reciprocal(d.r2), r6 = ir2 * ir2 * ir2;
+    acc.add(P.eps4s6 * r6 * ir2 * fma(P.s6x12, r6, -6.0), d.x, d.y, d.z);
   });
   acc.template store<LANES>(sub == 0 && live, out + 6 * (size_t)slot);
 }
