@@ -59,6 +59,13 @@ enum { KGF_PASS1, KGF_PASS2, KGF_REBUILD, KGF_COUNT };
 const char *kGroupNameFo[KGF_COUNT] = {"force_pass1", "force_pass2+advance_velocity_positions",
                                        "rebuild_if_due"};
 
+double widest_box(const comdgb_sim *h) {
+  double w = 0.0;
+  for (const RepGeo &R : h->reps)
+    for (int j = 0; j < 3; j++) w = std::max(w, R.boxsize[j]);
+  return w;
+}
+
 }  // namespace
 
 namespace cgapi {
@@ -762,18 +769,21 @@ void enqueue_classify_finish(comdgb_sim *h, bool lazy = false) {
 
 // The squared cutoff of an FP32 list build for pairs within rc: wider by more
 // than the FP32 distances err.  Mixed precision tests the same FP32 positions
-// in its passes: a few ulps.  FP64 tests its own: a pair's FP32 difference is
-// off by the roundings of two box-centred positions (half a box each), of two
-// box offsets (up to 1.5 boxes) and of the difference, 6 * 2^-24 box widths
-// per axis at most, atoms up to an Angstrom outside their boxes included.
+// in its passes: a few ulps.  FP64 tests its own.  With u = 2^-24, w the widest
+// box and atom i at most 1 A outside its box (atoms further out, which open
+// boundaries leave in the edge boxes, get no list: list_reach), a neighbour within rc
+// is at most 1.5 w + 1 + rc from its own box's centre, so their FP32 difference is off per
+// axis by u (w/2 + 1) and u (1.5 w + 1 + rc) of the positions, u w of the box
+// offset, u (w/2 + 1 + rc) and u rc of the two differences: u (3.5 w + 3 + 3 rc).
+// The margin is u (6 w + 6) an axis and 8 u rc in all (1.5 of it for r^2's sums).
 float list_cutoff(const comdgb_sim *h, double rc) {
   if (h->mixed) return (float)(rc * rc) * (1.0f + 4e-6f);
-  double width = 0.0;
-  for (const RepGeo &R : h->reps)
-    for (int j = 0; j < 3; j++) width = std::max(width, R.boxsize[j]);
-  const double err = 6.0 / 16777216.0 * (width + 1.0);
+  const double err = 6.0 / 16777216.0 * (widest_box(h) + 1.0);
   return (float)(rc * rc * (1.0 + 1e-6) + 4.0 * rc * err);
 }
+
+// how far from its box's centre an atom may be for that margin, per axis
+float list_reach(const comdgb_sim *h) { return (float)(0.5 * widest_box(h) + 1.0); }
 
 // compact: first the atom list of the layout a rebin has just made (every
 // other call that changes the layout leaves the list current).
@@ -822,7 +832,8 @@ void enqueue_force_parts(comdgb_sim *h, cudaEvent_t *ev, int &evi, bool obs = tr
     return;
   }
   // the build and the cut work on FP32 copies (mixed precision keeps them)
-  if (!h->mixed) launch_pos32_atoms(h->g, h->s, h->atom_slot, h->ntot, st, h->fx, h->fxu);
+  if (!h->mixed)
+    launch_pos32_atoms(h->g, h->s, h->atom_slot, h->ntot, st, h->fx, h->fxu, list_reach(h));
   launch_nbr_build(A, list_cutoff(h, h->pl.vlist ? rcl : h->cutoff), st);
   if (h->pl.vlist) {
     launch_rebuild_done(h->status, st);

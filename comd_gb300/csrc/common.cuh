@@ -6,7 +6,8 @@
 //             32-byte access per atom for gathers and the Verlet kernel
 //   rho, fi, mass  double per slot;  id, itype  int per slot
 //   pos32     float4 per slot: FP32 copy of the box-relative position
-//             (mixed precision); fi32 float per slot: F'(rho) in FP32
+//             (mixed precision; FP64: remade for every list build, w 1 where the
+//             atom is too far out for it); fi32 float per slot: F'(rho) in FP32
 //   natoms    int per box
 // Per-box link-cell stencil ("entry table"), built once: for each box the
 // up to 27 neighbour box ids in getNeighborBoxes order (domains.c:391-430)

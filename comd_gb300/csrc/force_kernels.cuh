@@ -390,6 +390,7 @@ __device__ __forceinline__ void build_box32(const ForceArgs &A, float rc2b, int 
       // all candidates
       float2 px[NA / 2], py[NA / 2], pz[NA / 2];
       int cnt[NA], id[NA];
+      bool far = false;  // an atom too far out for the margin (its stencil is scanned)
 #pragma unroll
       for (int u = 0; u < NA; u++) {
         float4 p = make_float4(-1e18f, -1e18f, -1e18f, 0.f);
@@ -399,6 +400,7 @@ __device__ __forceinline__ void build_box32(const ForceArgs &A, float rc2b, int 
           p = __ldg(A.s.pos32 + slot);
           if (MODE == LIST_ID) id[u] = A.s.id[slot];
           if (base > 0) cnt[u] = s_cnt[i0 + u];
+          far = far || p.w != 0.f;
         }
         (u & 1 ? px[u / 2].y : px[u / 2].x) = p.x;
         (u & 1 ? py[u / 2].y : py[u / 2].x) = p.y;
@@ -444,7 +446,12 @@ __device__ __forceinline__ void build_box32(const ForceArgs &A, float rc2b, int 
 #pragma unroll
         for (int u = 1; u < NA; u++) mine = lane == u ? cnt[u] : mine;
         s_cnt[i0 + lane] = mine;
-        if (base + NB_TILE >= ncand) build_count<MODE>(A, build_row<MODE>(A, b, i0 + lane), mine);
+        if (base + NB_TILE >= ncand) {
+          const int row = build_row<MODE>(A, b, i0 + lane);
+          build_count<MODE>(A, row, mine);
+          if (MODE != LIST_FO && far && __ldg(A.s.pos32 + b * CG_MAXATOMS + i0 + lane).w != 0.f)
+            (MODE == LIST_ID ? A.pl.vcount : A.nbr_n)[row] = cap + 1;
+        }
       }
       __syncwarp();
     }
@@ -479,11 +486,11 @@ static __global__ void __launch_bounds__(NB_THREADS) nbr_cut_kernel(ForceArgs A,
   if (a >= A.ntot) return;
   const int slot = A.atom_slot[a], b = slot >> 6, idi = A.s.id[slot];
   const int n = A.pl.vcount[idi];
-  if (n > A.pl.vcap) {  // overflowed skin list: the passes scan the stencil
+  const float4 pi = __ldg(A.s.pos32 + slot);
+  if (n > A.pl.vcap || pi.w != 0.f) {  // no skin list to go by: the passes scan
     if (lane == 0) A.nbr_n[a] = A.cap + 1;
     return;
   }
-  const float4 pi = __ldg(A.s.pos32 + slot);
   const int *lst = A.pl.vlist + (size_t)idi * A.pl.vcap;
   uint16_t *out = A.nbr + (size_t)a * A.cap;
   int cnt = 0;

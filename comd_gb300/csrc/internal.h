@@ -109,9 +109,10 @@ void launch_zc_upload(const HostSlots &hs, Slots s, int nboxes, bool forces, cud
 void launch_zc_download(const HostSlots &hs, Slots s, int nboxes, bool state, bool forces,
                         cudaStream_t st, int max_blocks = 0);
 void launch_pos32(const Geom &g, Slots s, cudaStream_t st, const int *only_if_overflow = nullptr);
-// the same over the atom list alone; fx: also the FP64 passes' records
+// the same over the atom list alone; fx: also the FP64 passes' records, and the
+// fourth component 1 where a coordinate is past reach (its atom gets no list)
 void launch_pos32_atoms(const Geom &g, Slots s, const int *atom_slot, int ntot, cudaStream_t st,
-                        d4 *fx = nullptr, const FxUnit &fxu = FxUnit{});
+                        d4 *fx = nullptr, const FxUnit &fxu = FxUnit{}, float reach = 0.f);
 void launch_bin_atoms(const Geom &g, const double *dcenter, Slots s, int n, const double *xyz,
                       const double *pxyz, const int *ids, const int *types, const double *masses,
                       int *tmp_index, int *status, cudaStream_t st);

@@ -1148,14 +1148,18 @@ void launch_pos32(const Geom &g, Slots s, cudaStream_t st, const int *only_if_ov
   pos32_kernel<<<slot_blocks(g), 256, 0, st>>>(g, s, only_if_overflow);
 }
 
-// fx (optional): also the fixed-point records of an FP64 force call
+// fx (optional): also the fixed-point records of an FP64 force call, and the
+// mark of an atom past reach
 __global__ void __launch_bounds__(256) pos32_atoms_kernel(Geom g, Slots s, const int *atom_slot,
-                                                          int ntot, d4 *fx, FxUnit fxu) {
+                                                          int ntot, d4 *fx, FxUnit fxu,
+                                                          float reach) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= ntot) return;
   const int slot = atom_slot[a];
   const d4 r = s.r[slot];
-  s.pos32[slot] = centred32(rep_of(g, slot >> 6), r.x, r.y, r.z);
+  float4 p = centred32(rep_of(g, slot >> 6), r.x, r.y, r.z);
+  if (fx && fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fabsf(p.z)) > reach) p.w = 1.f;
+  s.pos32[slot] = p;
   if (!fx) return;
   d4 v;
   v.x = __longlong_as_double(fx_from(r.x, fxu));
@@ -1166,9 +1170,9 @@ __global__ void __launch_bounds__(256) pos32_atoms_kernel(Geom g, Slots s, const
 }
 
 void launch_pos32_atoms(const Geom &g, Slots s, const int *atom_slot, int ntot, cudaStream_t st,
-                        d4 *fx, const FxUnit &fxu) {
+                        d4 *fx, const FxUnit &fxu, float reach) {
   if (ntot > 0)
-    pos32_atoms_kernel<<<atom_blocks(ntot), 256, 0, st>>>(g, s, atom_slot, ntot, fx, fxu);
+    pos32_atoms_kernel<<<atom_blocks(ntot), 256, 0, st>>>(g, s, atom_slot, ntot, fx, fxu, reach);
 }
 
 // ---------------------------------------------------------------------------
