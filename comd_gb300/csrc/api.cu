@@ -132,6 +132,7 @@ void free_all(comdgb_sim *h) {
   for (void *p : h->allocs)
     if (p) cudaFree(p);
   h->allocs.clear();
+  h->poly_bufs.release(cudaFree);
   for (void *q : h->adj.snaps) delete (Snapshot *)q;  // their device arrays were in allocs
   h->adj.snaps.clear();
   if (h->cond_stream) cudaStreamDestroy(h->cond_stream);
@@ -466,7 +467,8 @@ int build_pair_seg(comdgb_sim *h, const double coef[6][CG_NCHEB], const double a
 }
 
 // The polynomial tables of an FP64 simulation (poly64.cuh) from the installed
-// series.  Returns 0, or -1 when a CUDA call failed.
+// series.  Returns 0, or -1 when device memory ran out (nothing has changed
+// then) or a CUDA call failed (there are no tables and no graphs then).
 int build_poly64(comdgb_sim *h, const double coef[6][CG_NCHEB], const double a[6],
                  const double b[6], double pair_lo, double rc, PolyTables *out) {
   *out = PolyTables{};
@@ -480,35 +482,40 @@ int build_poly64(comdgb_sim *h, const double coef[6][CG_NCHEB], const double a[6
   }
   double lo = pair_lo;
   for (int s : {0, 1, 3, 4}) lo = std::max(lo, a[s]);
-  int base[PT_COUNT], n[PT_COUNT], bad[PT_COUNT], err = 0;
+  int base[PT_COUNT], n[PT_COUNT], bad[PT_COUNT];
   poly_range(PT_PAIR, lo, rc, &base[PT_PAIR], &n[PT_PAIR]);
   poly_range(PT_HESS, lo, rc, &base[PT_HESS], &n[PT_HESS]);
   poly_range(PT_EMBED, std::max(a[2], a[5]), std::min(b[2], b[5]), &base[PT_EMBED], &n[PT_EMBED]);
-  if (!h->poly_series) {
-    h->poly_series = track(h, dalloc<PolySeries>(1, &err));
-    h->poly_bad = track(h, dalloc<int>(PT_COUNT, &err));
-    if (err) return -1;
-  }
+  size_t bytes[PT_COUNT + 2] = {};
+  for (int e = 0; e < PT_COUNT; e++) bytes[e] = sizeof(double2) * poly_size(e, n[e]);
+  bytes[PT_COUNT] = sizeof(PolySeries);
+  bytes[PT_COUNT + 1] = sizeof bad;
+  auto alloc = [](size_t size) -> void * {
+    void *p = nullptr;
+    if (cudaMalloc(&p, size) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
+  };
+  if (!h->poly_bufs.reserve(bytes, alloc, cudaFree)) return -1;
+  // the graphs and the installed tables hold the former buffers
+  h->eam64c.poly = PolyTables{};
+  drop_graphs(h);
+  double2 *buf[PT_COUNT];
+  for (int e = 0; e < PT_COUNT; e++) buf[e] = (double2 *)h->poly_bufs.buf[e];
+  PolySeries *series = (PolySeries *)h->poly_bufs.buf[PT_COUNT];
+  int *first_bad = (int *)h->poly_bufs.buf[PT_COUNT + 1];
   cudaStream_t st = h->stream;
-  bool ok =
-      cudaMemcpyAsync(h->poly_series, &S, sizeof S, cudaMemcpyHostToDevice, st) == cudaSuccess &&
-      cudaMemcpyAsync(h->poly_bad, n, sizeof n, cudaMemcpyHostToDevice, st) == cudaSuccess;
-  for (int e = 0; e < PT_COUNT; e++) {
-    const size_t need = poly_size(e, n[e]);
-    if (need > h->poly_cap[e]) {
-      h->poly_buf[e] = track(h, dalloc<double2>(need, &err));
-      if (err) return -1;
-      h->poly_cap[e] = need;
-    }
-    launch_poly_fit(e, h->poly_series, base[e], n[e], h->poly_buf[e], h->poly_bad + e, st);
-  }
+  bool ok = cudaMemcpyAsync(series, &S, sizeof S, cudaMemcpyHostToDevice, st) == cudaSuccess &&
+            cudaMemcpyAsync(first_bad, n, sizeof n, cudaMemcpyHostToDevice, st) == cudaSuccess;
+  for (int e = 0; e < PT_COUNT && ok; e++)
+    launch_poly_fit(e, series, base[e], n[e], buf[e], first_bad + e, st);
   ok = ok &&
-       cudaMemcpyAsync(bad, h->poly_bad, sizeof bad, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
+       cudaMemcpyAsync(bad, first_bad, sizeof bad, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
        cudaStreamSynchronize(st) == cudaSuccess;
   if (!ok) return -1;
-  out->pair = Poly64<PT_PAIR>{h->poly_buf[PT_PAIR], base[PT_PAIR], bad[PT_PAIR]};
-  out->hess = Poly64<PT_HESS>{h->poly_buf[PT_HESS], base[PT_HESS], bad[PT_HESS]};
-  out->embed = Poly64<PT_EMBED>{h->poly_buf[PT_EMBED], base[PT_EMBED], bad[PT_EMBED]};
+  out->pair = Poly64<PT_PAIR>{buf[PT_PAIR], base[PT_PAIR], bad[PT_PAIR]};
+  out->hess = Poly64<PT_HESS>{buf[PT_HESS], base[PT_HESS], bad[PT_HESS]};
+  out->embed = Poly64<PT_EMBED>{buf[PT_EMBED], base[PT_EMBED], bad[PT_EMBED]};
   return 0;
 }
 
@@ -701,12 +708,16 @@ void cgapi::install_lj(comdgb_sim *h, double eps, double sigma, double cutoff) {
 // (h->pair_lo) take the reference coefficients in FP32 (never in practice).
 int cgapi::install_cheby(comdgb_sim *h, const double coef[6][CG_NCHEB], const double a[6],
                          const double b[6]) {
-  fill_cheb(h->eam64c.ch, h->eam32c.ch, h->eam32c.chlo, coef, a, b, h->pair_lo);
-  // each precision has its own tables of the pair functions
-  h->seg_built = no_pair_seg();
-  if (h->mixed ? build_pair_seg(h, coef, a, b, h->pair_lo, h->cutoff, &h->seg_built)
-               : build_poly64(h, coef, a, b, h->pair_lo, h->cutoff, &h->eam64c.poly))
+  // each precision has its own tables of the pair functions; nothing is installed
+  // unless they could be made
+  PairSeg seg = no_pair_seg();
+  PolyTables poly{};
+  if (h->mixed ? build_pair_seg(h, coef, a, b, h->pair_lo, h->cutoff, &seg)
+               : build_poly64(h, coef, a, b, h->pair_lo, h->cutoff, &poly))
     return set_err(COMDGB_ERR_NOMEM, "cudaMalloc failed for the pair function tables");
+  fill_cheb(h->eam64c.ch, h->eam32c.ch, h->eam32c.chlo, coef, a, b, h->pair_lo);
+  h->seg_built = seg;
+  h->eam64c.poly = poly;
   h->eam32c.seg = h->pair_table_off ? no_pair_seg() : h->seg_built;
   for (int q = 0; q < 6; q++) {
     for (int j = 0; j < CG_NCHEB; j++) h->cheb_coef[q][j] = coef[q][j];

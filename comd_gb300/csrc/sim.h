@@ -8,6 +8,7 @@
 #include <string>
 #include <vector>
 
+#include "buffer_set.h"
 #include "comdgb.h"
 #include "internal.h"
 
@@ -105,12 +106,9 @@ struct comdgb_sim {
   double cheb_a[6] = {}, cheb_b[6] = {};
   double pair_lo = 0.0;
   float4 *seg_buf = nullptr;
-  // FP64 polynomial tables (poly64.cuh): the fit's input, the tables' storage
-  // with its capacity in double2, and the first segment each misses
-  cg::PolySeries *poly_series = nullptr;
-  double2 *poly_buf[cg::PT_COUNT] = {};
-  size_t poly_cap[cg::PT_COUNT] = {};
-  int *poly_bad = nullptr;
+  // FP64 polynomial tables (poly64.cuh): their storage, then the fit's input and
+  // the first segment that each misses
+  cg::BufferSet<cg::PT_COUNT + 2> poly_bufs;
   // the FP32 pair segment table as built (seg_built) and whether the mixed
   // Chebyshev evaluator uses it (comdgb_sim_set_pair_table)
   cg::PairSeg seg_built{};
