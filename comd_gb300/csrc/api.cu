@@ -736,7 +736,10 @@ int read_status(comdgb_sim *h, int *st) {
   return 0;
 }
 
-static int status_error(const int *st) {
+// After an error the layout may lack an atom (a full box), and so may the lists
+// built from it since: the next upload has them built anew.
+static int status_error(comdgb_sim *h, const int *st) {
+  if (st[ST_ERROR]) h->lists_built = false;
   if (st[ST_ERROR] == COMDGB_ERR_MAXATOMS)
     return set_err(COMDGB_ERR_MAXATOMS, "Increase maxatoms: a box reached %d atoms",
                    CG_MAXATOMS);
@@ -750,17 +753,18 @@ static int status_error(const int *st) {
 int check_status(comdgb_sim *h) {
   int st[ST_COUNT];
   int rc = read_status(h, st);
-  return rc ? rc : status_error(st);
+  return rc ? rc : status_error(h, st);
 }
 // the force calls since ST_NONFINITE was cleared, as finish_force checks one
 int check_forces(comdgb_sim *h) {
   int st[ST_COUNT];
   int rc = read_status(h, st);
   if (rc) return rc;
+  const int error = status_error(h, st);
   if (st[ST_NONFINITE])
     return set_err(COMDGB_ERR_NONFINITE, "total energy is %s",
                    st[ST_NONFINITE] == 1 ? "nan" : st[ST_NONFINITE] == 2 ? "inf" : "-inf");
-  return status_error(st);
+  return error;
 }
 
 // ---- kernel groups of one step --------------------------------------------
