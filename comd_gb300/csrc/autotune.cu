@@ -229,7 +229,13 @@ extern "C" int comdgb_batch_autotune(const simflat_t *const *sims, int n, const 
         best.build_atoms = ba;
       }
     }
+  long ntot = 0;
+  for (const simflat_t *q : reps) ntot += q->ntot;
+  // (no kernel of a smaller batch takes pass 2's threads: noise would decide)
+  const bool pass2 =
+      o->precision == COMDGB_PREC_MIXED && cg::fo_takes_pass2_threads(o->potential, ntot);
   for (int pt : {128, 256}) {
+    if (!pass2) break;
     const double ms = time_batch(reps, ob, best.build_threads, best.build_atoms, pt, steps, dt);
     if (ms < 0) {
       free_owned();

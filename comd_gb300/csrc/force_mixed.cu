@@ -1,6 +1,10 @@
 // force_mixed.cu -- the mixed-precision force kernels (FP32 pair terms on
 // box-relative coordinates, Kahan-compensated FP32 per-atom sums) and the list
 // builds, which both precisions use.
+#include <algorithm>
+#include <climits>
+
+#include "comdgb.h"
 #include "fo_lanes.cuh"
 #include "internal.h"
 
@@ -204,6 +208,11 @@ static int fo_lanes(int eval, int ntot) {
 }
 // and the LJ pass's, whose lists are twice as long
 static int fo_lj_lanes(int ntot) { return ntot < 24000 ? 8 : ntot < 100000 ? 4 : 1; }
+bool fo_takes_pass2_threads(int potential, long ntot) {
+  return potential != COMDGB_POT_LJ &&
+         fo_lanes(potential == COMDGB_POT_EAM_TABLE ? EVAL_TABLE : EVAL_CHEBY,
+                  (int)std::min(ntot, (long)INT_MAX)) == 1;
+}
 static unsigned fol_blocks(int ntot, int lanes) {
   return (unsigned)(((long)ntot * lanes + FOL_THREADS - 1) / FOL_THREADS);
 }

@@ -159,6 +159,9 @@ template <int EVAL>
 void launch_eam64(const ForceArgs &A, const EamPot<double, EVAL> &P, int pass, cudaStream_t st,
                   bool obs);
 void launch_lj64(const ForceArgs &A, const LjPot<double> &P, cudaStream_t st, bool obs);
+// whether the force-order pass 2 of this size takes Tune::pass2_threads (the
+// thread-per-atom kernel does, those with several threads an atom and LJ do not)
+bool fo_takes_pass2_threads(int potential, long ntot);
 // force order (mixed precision only, force_mixed.cu); pass 0 or 1.  obs:
 // the caller can read this force call's energies, stress, rho and F' (else
 // forces only: the force calls inside a step sequence)
