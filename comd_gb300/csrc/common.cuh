@@ -568,11 +568,11 @@ __device__ __forceinline__ void table_eval(const Table<float> &a, float r, float
                                            float &deriv) {
   if (r < a.x0) r = a.x0;
   else if (r > a.xn) r = a.xn;
-  float t = (r - a.x0) * a.invDx;
-  float fl = floorf(t);
-  int i1 = (int)fl;
-  i1 = i1 < 0 ? 0 : (i1 > a.n - 1 ? a.n - 1 : i1);
-  float u = t - fl;
+  // (at the table's end the last interval's own end: u = 1)
+  const float t = (r - a.x0) * a.invDx;
+  const float fl = fmaxf(fminf(floorf(t), (float)(a.n - 1)), 0.f);
+  const int i1 = (int)fl;
+  const float u = t - fl;
   float4 s0 = __ldg(a.seg + 2 * i1);
   float d1 = __ldg(reinterpret_cast<const float *>(a.seg + 2 * i1 + 1));
   value = fmaf(u, fmaf(u, s0.z, s0.y), s0.x);

@@ -1060,11 +1060,10 @@ __device__ __forceinline__ const float4 *fo_copy(const float4 *sm) {
 __device__ __forceinline__ int fo_interval(const FoTab &t, float r, float &u) {
   if (r < t.x0) r = t.x0;
   else if (r > t.xn) r = t.xn;
-  const float v = (r - t.x0) * t.invDx, fl = floorf(v);
-  int i = (int)fl;
-  i = i < 0 ? 0 : (i > t.n - 1 ? t.n - 1 : i);
+  const float v = (r - t.x0) * t.invDx;
+  const float fl = fmaxf(fminf(floorf(v), (float)(t.n - 1)), 0.f);
   u = v - fl;
-  return i;
+  return (int)fl;
 }
 
 // rho(r) of one pair distance.  false: below the pair table (the series, in
