@@ -882,13 +882,16 @@ int count_kernel_nodes(cudaGraph_t graph);
 // being captured, 0 at every launch until a kernel sets it; 0 when h->stream
 // is not capturing or there is none.
 cudaGraphConditionalHandle cond_handle(comdgb_sim *h) {
-  // COMDGB_GRAPH_CONDITIONALS=0: no conditional nodes (the sections stand
-  // down by themselves instead).  ncu profiles no kernel of a graph that
-  // holds a conditional node, so the launch lists are taken with this set.
+  // COMDGB_GRAPH_CONDITIONALS=0, or a build without them (set_condition): no
+  // conditional nodes (the sections stand down by themselves instead)
+#ifdef COMDGB_NO_CONDITIONALS
+  const bool off = true;
+#else
   static const bool off = [] {
     const char *e = getenv("COMDGB_GRAPH_CONDITIONALS");
     return e && e[0] == '0';
   }();
+#endif
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   cudaGraph_t graph = nullptr;
   if (off || !h->cond_stream ||
@@ -1844,7 +1847,7 @@ int create(const simflat_t *const *sims, int nrep, const comdgb_opts *o, comdgb_
   h->cap_alloc = h->cap;
   h->pl_vcap_alloc = h->pl.vcap;
   h->fo_vcap_alloc = h->fo.vcap;
-  // per-step list: built each step, or (persistent lists) left by pass 1
+  // per-step list: built each step, or (persistent lists) cut from the skin list
   // (the force-order passes keep their own lists and never read this one)
   h->nbr = track(h, dalloc<uint16_t>((h->fo.list ? 0 : (size_t)h->ntot * h->cap) + 8, &err));
   h->nbr_n = track(h, dalloc<int>((size_t)h->ntot + 1, &err));

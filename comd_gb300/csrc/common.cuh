@@ -205,6 +205,16 @@ struct ForceOrder {
   float4 *force;     // [ntot] xyz
 };
 
+// A conditional graph node's handle set to run the node's body.  ncu profiles no
+// kernel that holds this call, nor any of a graph with such a node: in a build
+// with -DCOMDGB_NO_CONDITIONALS there are neither, and the bodies' kernels stand
+// down by themselves.
+__device__ __forceinline__ void set_condition(cudaGraphConditionalHandle cond) {
+#ifndef COMDGB_NO_CONDITIONALS
+  cudaGraphSetConditional(cond, 1);
+#endif
+}
+
 // Force order: the FP32 position of force-order atom af (now in box b at
 // box-relative FP64 position r, FP32 centred position p32) relative to its
 // build box centre -- p32 itself while the atom is in its build box, else
@@ -240,7 +250,7 @@ __device__ __forceinline__ void fo_track_at(const Geom &g, const ForceOrder &fo,
     d2 = fmaf(d, d, d2);
   }
   if ((far || !(d2 <= fo.half_skin2)) && atomicExch(status + ST_REBUILD, 1) == 0 && cond)
-    cudaGraphSetConditional(cond, 1);
+    set_condition(cond);
   fo.pos[af] = make_float4(pv[0], pv[1], pv[2], 0.f);
 }
 // What the atoms' own tests do not announce: a rebuild that was due already,
@@ -249,7 +259,7 @@ __device__ __forceinline__ void fo_track_at(const Geom &g, const ForceOrder &fo,
 __device__ __forceinline__ void cond_pending(cudaGraphConditionalHandle cond, const int *status) {
   if (cond && (*(volatile const int *)(status + ST_REBUILD) ||
                *(volatile const int *)(status + ST_NBR_OVERFLOW)))
-    cudaGraphSetConditional(cond, 1);
+    set_condition(cond);
 }
 // the slot of an atom moved by the rebin, in the maps the list mode keeps
 struct SlotMap {

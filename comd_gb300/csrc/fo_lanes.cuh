@@ -204,7 +204,7 @@ __device__ __forceinline__ void fol_force_end(const ForceArgs &A, int a, int slo
   if (a == 0) cond_pending(A.cond, A.status);
   if ((((away >> group) & 7u) != 0 || !(s <= A.fo.half_skin2)) &&
       atomicExch(A.status + ST_REBUILD, 1) == 0 && A.cond)
-    cudaGraphSetConditional(A.cond, 1);
+    set_condition(A.cond);
 }
 
 // fo_eam_pass2_kernel with LANES threads per atom
