@@ -179,7 +179,7 @@ __global__ void adj_lambda_kernel(Slots s, const int *atom_slot, int ntot, const
 // W_i = sum_j v_ij rho'(r_ij) over the embedding-force pairs (r2 < rc2,
 // eam.c:612) and X_i = F''(rho_i) W_i, per slot.  The walk of the FP64 passes
 // (fixed-point distances, LANES threads an atom): a thread per atom in FP64
-// geometry took 63 us at 3,960 atoms and 500 us at 256,000, this 12 and 279.
+// geometry took 63 us at 3,960 atoms and 500 us at 256,000, this 12 and 281.
 template <int LANES>
 __global__ void __launch_bounds__(F64_THREADS)
     adj_w_kernel(ForceArgs A, const __grid_constant__ ChebSet S, PolyTables poly, double rc2,
@@ -225,7 +225,7 @@ __device__ __forceinline__ double cheb_y(const ChebSet &S, int q, double x) {
 // a queue in shared memory and works on 32 at a time; the distances are formed
 // in fixed point, r without division.  At 256,000 and 3,960 atoms: 10,450 and
 // 750 us with sums in shared memory, 2,158 and 94 us with several threads an
-// atom each at its own pairs, 1,403 and 45 us now.
+// atom each at its own pairs, 1,406 and 45 us now.
 template <int NW>
 struct BasisAcc {
   double s[NW][NC];

@@ -19,9 +19,9 @@
 // Measured at 256,000 atoms (no energies), density + forces: table potential
 // 3,156 us before (phi, phi' and rho, then rho', a thread per atom, FP64
 // division and square root, the skin list walked in FP64), 541 + 682 with the
-// list above in FP64 geometry, 354 + 469 in fixed point, 132 + 271 with its
-// intervals as polynomials; Chebyshev 1,327, 350 + 560, 159 + 321.  The pipe's
-// two lanes a clock would take 135 + 310 for the latter.  Relative rms error of
+// list above in FP64 geometry, 354 + 469 in fixed point, 134 + 268 with its
+// intervals as polynomials; Chebyshev 1,327, 350 + 560, 160 + 321.  The pipe's
+// two lanes a clock would take 135 + 310 for the latter.  LJ: 455.  Relative rms error of
 // the forces against extended precision (504 atoms, Cu at 300 K): Chebyshev
 // 4.6e-14 before, 2.4e-15 now, table 2.2e-15 and 4.5e-16, LJ 1.4e-15 and
 // 0.9e-15; energies and densities are closer as well.
@@ -34,11 +34,18 @@ namespace cg {
 
 constexpr int F64_THREADS = 128;
 
-// Threads per atom.  Density + force pass without energies in us, Chebyshev
-// (16, 4, 1 threads): 4,000 atoms 22, 36, 99; 27,436 atoms 85, 66, 108; 256,000
-// atoms 658, 480, 523; 1,048,576 atoms 2,648, 1,903, 1,838 (lists of 42 entries
-// leave lanes of 16 short).  Eight threads lie between at every size, two at
-// 27,436 atoms 71.
+// Threads per atom.  One rule for all FP64 walks; us with 16, 4 and 1 threads,
+// density + force pass or the LJ pass without energies, then the other walks:
+//             7,488       10,976     12,600     27,436       520,200      1,016,064
+//   Chebyshev 33 39 -     42 43 -    45 43 -    83 68 126    - 957 973    - 1,845 1,848
+//   table     30 44 -     38 45 -    42 44 -    73 59 131    - 782 850    - 1,500 1,618
+//   LJ        23 29 -     30 33 -    36 34 -    64 58 90     - 912 895    - 1,773 1,732
+//   virial    28 26 -     38 32 -    41 33 -    81 60 84     - 930 865    - 1,809 1,681
+//   adj_w     17 24 -     23 25 -    26 25 -    47 38 81     - 561 543    - 1,083 1,042
+//   adj_hvp   39 42 -     53 55 -    59 55 -    115 107 144  - 1,717 1,706  - 3,344 3,322
+// (virial: Chebyshev's.)  The lines lie where most of them cross; past the second the
+// table potential would be 8% faster with four, the virial before the first
+// with four.  Lists of 42 entries leave lanes of 16 short.
 inline int lanes64(int ntot) { return ntot < 12000 ? 16 : ntot < (1 << 19) ? 4 : 1; }
 
 // The atom and sub-lane of this thread; false when its whole warp has none.
@@ -319,6 +326,8 @@ __global__ void __launch_bounds__(F64_THREADS)
   double F, dF;
   eam_embed<double, EVAL>(P, rho, F, dF);
   if (sub != 0 || !live) return;
+  // (atoms still walking gather this record for its position alone, which the
+  // store of its last 8 bytes leaves as it is)
   A.fx[slot].w = dF;
   if (OBS) {
     A.s.rho[slot] = rho;

@@ -206,7 +206,17 @@ static int fo_lanes(int eval, int ntot) {
     return ntot < 24000 ? 8 : ntot < 140000 ? 4 : ntot < 230000 ? 2 : 1;
   return ntot < 12000 ? 8 : ntot < 60000 ? 4 : 1;
 }
-// and the LJ pass's, whose lists are twice as long
+// and of the LJ pass, whose lists are twice as long (us without / with energies;
+// 8, 4, 1 threads):
+//      4,000 atoms   9.1 / 11.3  12.5 / 13.9  50.3 / 49.7
+//     16,384        11.1 / 14.4  13.1 / 15.4  49.9 / 50.3
+//     23,328        15.9 / 20.5  13.5 / 15.6  55.2 / 54.6
+//     27,436        16.6 / 22.8  14.1 / 16.6  58.7 / 57.3
+//     55,296        25.0 / 34.4  23.3 / 28.9  56.4 / 56.7
+//     97,556        40.1 / 54.4  34.2 / 42.9  59.0 / 60.7
+//    108,000        43.5 / 59.6  35.7 / 44.1  57.7 / 59.1
+//    143,748        55.4 / 76.0  45.4 / 56.8  60.5 / 62.0
+// The second line is below where four threads and one cross (past 143,748).
 static int fo_lj_lanes(int ntot) { return ntot < 24000 ? 8 : ntot < 100000 ? 4 : 1; }
 bool fo_takes_pass2_threads(int potential, long ntot) {
   return potential != COMDGB_POT_LJ &&

@@ -8,8 +8,9 @@
 // segment index is the top bits of s and the offset x in it, from -1 to 1, the
 // bits below, so an evaluation takes six FP64 operations: one for x, five
 // fused multiply-adds.  The embedding function has the same form in rho.  At
-// 256,000 atoms the first FP64 pass took 8,342 us with the series and takes
-// 750 us, the second 3,267 and 577 us.
+// 256,000 atoms the two FP64 passes took 8,342 and 3,267 us with the series and 750
+// and 577 us with the polynomials alone changed; force64.cuh has what the passes
+// take now.
 //
 // Accuracy: the coefficients interpolate the series at six Chebyshev nodes
 // of each segment, with the series summed in double-double arithmetic, and
@@ -136,7 +137,7 @@ void launch_poly_fit(int table, const PolySeries *series, int base, int n, doubl
 // of the value or of r changes.  Pairs below s_lo, inside the first interval
 // after the last that misses it (the Cu tables' first, next to their guard
 // value, at 1 A), take the formula.
-// 256,000 atoms, density + forces: 354 + 469 -> 132 + 271 us.
+// 256,000 atoms, density + forces: 354 + 469 -> 134 + 268 us.
 struct TabPoly {
   const double4_32a *rho;    // [2 n] (S0, S1, c0, c1) (c2, c3, c4, -), S the bits of the ends
   const double4_32a *force;  // [3 n] (S0, S1, a0, a1) (a2, a3, a4, b0) (b1, b2, b3, b4):
